@@ -388,7 +388,7 @@ extern "C" int mgp_destroy(mgp_ctx *c) {
     free(c->box_cosmo);
   }
   free(c->box_p);
-  void *bufs[] = {c->ic_scratch, c->s, c->v, c->D1, c->D2, c->dstate, c->partials, c->stage, c->rho, c->dk, c->frc, c->mg1,
+  void *bufs[] = {c->ic_scratch, c->ic_amp, c->s, c->v, c->D1, c->D2, c->dstate, c->partials, c->stage, c->rho, c->dk, c->frc, c->mg1,
                   c->fft_work, c->rk_bin, c->pk_thr, c->win1d, c->pk_block, c->pk_sum, c->rsd_block, c->rsd_sum,
                   c->pk_sum_tot, c->nu_tab_d, c->nu_row_d, c->nu_x_d, c->nu_den_d, c->scr_tab};
   for (size_t i = 0; i < sizeof(bufs) / sizeof(bufs[0]); i++)
@@ -554,6 +554,52 @@ extern "C" int mgp_batch_create(const mgp_params *p, int nbox, const mgp_box_par
 }
 
 // ---------------------------------------------------------------- IC
+// Amplitudes per integer |k|^2 < namp of the Gaussian draw (k in h/Mpc = 2 pi/Box
+// sqrt(RK)) into c->ic_amp, with the P(k) rescaling for MG runs whose input
+// spectrum is LCDM (2LPT.c:323-327, 395-407): mg_pofk_ratio(k, 1), per k when
+// the growth is scale dependent.  The analytic spectrum is evaluated on the
+// device; tabulated spectra and CAMB files on the host.
+static int ic_amplitudes(mgp_ctx *c, const mgp_params *pb, const mgp_cosmo *cb, int namp) {
+  const double box = pb->Box, kf = 2.0 * M_PI / box;
+  const bool rescale = pb->modified_gravity_active && pb->input_pofk_is_for_lcdm;
+  const int ny = cb->sd ? cb->sd_tab[0].ny : 0;
+  if (!c->ic_amp) MGP_CUDA(cudaMalloc(&c->ic_amp, sizeof(double) * ((size_t)namp + 2 * ny)));
+  double s8fac = 1.0;
+  if (rescale && !pb->input_sigma8_is_for_lcdm) {
+    const double e = mgp_cosmo_sigma8_enh(cb, 1.0);
+    s8fac = 1.0 / (e * e);
+  }
+  mgp_eh_spectrum eh;
+  if (mgp_cosmo_power_eh(cb, &eh)) {
+    double fac = s8fac;
+    if (rescale && cb->sd) {
+      // per k: the growth table at a = 1 over the LCDM growth factor
+      std::vector<double> col(2 * (size_t)ny);
+      RET_IF(mgp_cosmo_sd_column(cb, 0, 1.0, col.data(), col.data() + ny));
+      const double *y = cb->sd_tab[0].y, dy = (y[ny - 1] - y[0]) / (double)(ny - 1);
+      double *dcol = c->ic_amp + namp;
+      MGP_CUDA(cudaMemcpyAsync(dcol, col.data(), sizeof(double) * 2 * ny, cudaMemcpyHostToDevice, c->stream));
+      RET_IF(mgp_launch_ic_amp(c->ic_amp, namp, kf, pow(box, -1.5), &eh, fac, dcol, ny, y[0], dy,
+                               mgp_cosmo_growth_lcdm0(cb), c->stream));
+      return MGP_OK;
+    }
+    if (rescale) {
+      double k1 = kf, r1 = 1.0;
+      mgp_cosmo_pofk_ratio_many(cb, 1.0, 1, &k1, &r1);
+      fac *= r1;
+    }
+    return mgp_launch_ic_amp(c->ic_amp, namp, kf, pow(box, -1.5), &eh, fac, NULL, 0, 0.0, 1.0, 1.0, c->stream);
+  }
+  std::vector<double> amp(namp, 0.0), kk(namp), ratio(namp, 1.0);
+  for (int rk = 0; rk < namp; rk++) kk[rk] = kf * sqrt((double)rk);
+  if (rescale) mgp_cosmo_pofk_ratio_many(cb, 1.0, namp - 1, kk.data() + 1, ratio.data() + 1);
+  for (int rk = 1; rk < namp; rk++)
+    amp[rk] = pow(box, -1.5) * sqrt(mgp_cosmo_power(cb, kk[rk]) * ratio[rk] * s8fac);
+  // pageable source: the copy has been staged when the call returns
+  MGP_CUDA(cudaMemcpyAsync(c->ic_amp, amp.data(), sizeof(double) * namp, cudaMemcpyHostToDevice, c->stream));
+  return MGP_OK;
+}
+
 // displacement_fields + the particle assignment of main.c:231-309 for box b
 // (single-grid transforms; box b's particle arrays and state).
 // 2LPT initial conditions of box bx (displacement_fields, src/2LPT.c:185-495,
@@ -568,50 +614,14 @@ static int ic_box(mgp_ctx *c, int bx, const double *pos01 = NULL, size_t npos = 
   const size_t po = (size_t)bx * 3 * c->np;
   const int N = c->g.N, Ns = c->Ns, h = N / 2;
   const double box = pb->Box;
-  // seed table, src/2LPT.c:262-271
-  std::vector<uint32_t> seeds((size_t)N * N);
+  // cube cut of 2LPT.c:383-386 with the reference's double expression: the
+  // largest |d| it keeps
+  int kc = Ns / 2 < h ? Ns / 2 : h;
   {
-    uint64_t n = 0;
-    uint32_t sd = (uint32_t)pb->Seed;
-    auto draw = [&]() { return (uint32_t)(0x7fffffff * mgp_uniform(sd, n++)); };
-    for (int i = 0; i < N / 2; i++) {
-      for (int j = 0; j < i; j++) seeds[(size_t)i * N + j] = draw();
-      for (int j = 0; j < i + 1; j++) seeds[(size_t)j * N + i] = draw();
-      for (int j = 0; j < i; j++) seeds[(size_t)(N - 1 - i) * N + j] = draw();
-      for (int j = 0; j < i + 1; j++) seeds[(size_t)(N - 1 - j) * N + i] = draw();
-      for (int j = 0; j < i; j++) seeds[(size_t)i * N + (N - 1 - j)] = draw();
-      for (int j = 0; j < i + 1; j++) seeds[(size_t)j * N + (N - 1 - i)] = draw();
-      for (int j = 0; j < i; j++) seeds[(size_t)(N - 1 - i) * N + (N - 1 - j)] = draw();
-      for (int j = 0; j < i + 1; j++) seeds[(size_t)(N - 1 - j) * N + (N - 1 - i)] = draw();
-    }
+    const double kv = kc * 2 * 3.14159265358979323846 / box;
+    if (fabs(kv) * box / (2 * 3.14159265358979323846) > Ns / 2) kc--;
   }
-  // amplitude per integer |k|^2 (k in h/Mpc = 2 pi/Box sqrt(RK)), with the
-  // P(k) rescaling for MG runs whose input spectrum is LCDM (2LPT.c:323-327,
-  // 395-407): mg_pofk_ratio(k, 1), per k when the growth is scale dependent
-  const int rkmax = 3 * h * h;
-  std::vector<double> amp(rkmax + 1), kk(rkmax + 1), ratio(rkmax + 1, 1.0);
-  for (int rk = 0; rk <= rkmax; rk++) kk[rk] = 2.0 * M_PI / box * sqrt((double)rk);
-  double s8fac = 1.0;
-  if (pb->modified_gravity_active && pb->input_pofk_is_for_lcdm) {
-    mgp_cosmo_pofk_ratio_many(cb, 1.0, rkmax, kk.data() + 1, ratio.data() + 1);
-    if (!pb->input_sigma8_is_for_lcdm) {
-      double e = mgp_cosmo_sigma8_enh(cb, 1.0);
-      s8fac = 1.0 / (e * e);
-    }
-  }
-  for (int rk = 0; rk <= rkmax; rk++) {
-    double pk = rk == 0 ? 0.0 : mgp_cosmo_power(cb, kk[rk]) * ratio[rk] * s8fac;
-    amp[rk] = pow(box, -1.5) * sqrt(pk);
-  }
-  // cube cut of 2LPT.c:383-386 with the reference's double expression
-  std::vector<unsigned char> cut(h + 1);
-  for (int d = 0; d <= h; d++) {
-    double kv = d * 2 * 3.14159265358979323846 / box;
-    cut[d] = (fabs(kv) * box / (2 * 3.14159265358979323846) > Ns / 2) ? 1 : 0;
-  }
-  uint32_t *d_seeds = NULL;
-  double *d_amp = NULL;
-  unsigned char *d_cut = NULL;
+  const int namp = 3 * (Ns / 2 < h ? (Ns / 2) * (Ns / 2) : h * h) + 1;  // |k|^2 up to the cut
   float *g6 = NULL;
   int rc = MGP_OK;
   const long long gf = c->g.nreal;
@@ -642,22 +652,18 @@ static int ic_box(mgp_ctx *c, int bx, const double *pos01 = NULL, size_t npos = 
       goto cleanup;                                                                                    \
     }                                                                                                  \
   } while (0)
-  CKC(cudaMalloc(&d_seeds, sizeof(uint32_t) * seeds.size()));
-  CKC(cudaMalloc(&d_amp, sizeof(double) * amp.size()));
-  CKC(cudaMalloc(&d_cut, cut.size()));
   // six scratch grids for the displacement gradients and the six
   // displacement fields (2LPT.c:1214-1219, 1300-1306), kept by the context
   // for its next IC (runs of many ICs -- the boxes of a batch, repeated
   // runs -- allocate them once)
   if (!c->ic_scratch) CKC(cudaMalloc(&c->ic_scratch, sizeof(float) * 6 * (size_t)gf));
   g6 = c->ic_scratch;
-  CKC(cudaMemcpyAsync(d_seeds, seeds.data(), sizeof(uint32_t) * seeds.size(), cudaMemcpyHostToDevice, c->stream));
-  CKC(cudaMemcpyAsync(d_amp, amp.data(), sizeof(double) * amp.size(), cudaMemcpyHostToDevice, c->stream));
-  CKC(cudaMemcpyAsync(d_cut, cut.data(), cut.size(), cudaMemcpyHostToDevice, c->stream));
   if (pos01) {
     // the particles' CIC density at a_i as the LCDM linear field, brought to
     // a = 1 (readICfromfile.c:640-676), deconvolved and rescaled (701-777)
-    std::vector<double> gcw(h + 1), resc(rkmax + 1);
+    const int rkmax = 3 * h * h;
+    std::vector<double> gcw(h + 1), resc(rkmax + 1), kk(rkmax + 1);
+    for (int rk = 0; rk <= rkmax; rk++) kk[rk] = 2.0 * M_PI / box * sqrt((double)rk);
     for (int d = 0; d <= h; d++) {
       const double x = M_PI * d / (double)N, sc = d == 0 ? 1.0 : sin(x) / x;
       gcw[d] = 1.0 / (sc * sc);
@@ -691,8 +697,8 @@ static int ic_box(mgp_ctx *c, int bx, const double *pos01 = NULL, size_t npos = 
     cudaStreamSynchronize(c->stream);
     if (rc != MGP_OK) goto cleanup;
   } else {
-    CKC(cudaMemsetAsync(dkb, 0, sizeof(float) * (size_t)gf, c->stream));
-    CK(mgp_launch_ic_delta(d_seeds, d_amp, d_cut, N, Ns, box, pb->amplitude_fixed_initial_condition,
+    CK(ic_amplitudes(c, pb, cb, namp));
+    CK(mgp_launch_ic_delta((uint32_t)pb->Seed, c->ic_amp, N, Ns, kc, box, pb->amplitude_fixed_initial_condition,
                            pb->inverted_initial_condition, pb->SphereMode == 1, dkb, c->stream));
   }
   CK(mgp_launch_ic_grad6(dkb, g6, gf, N, c->stream));
@@ -724,9 +730,6 @@ static int ic_box(mgp_ctx *c, int bx, const double *pos01 = NULL, size_t npos = 
   CKC(cudaStreamSynchronize(c->stream));
   c->have_density = c->have_forces = 0;
 cleanup:
-  if (d_seeds) cudaFree(d_seeds);
-  if (d_amp) cudaFree(d_amp);
-  if (d_cut) cudaFree(d_cut);
   (void)g6;  // the context's IC scratch, freed by mgp_destroy
 #undef CK
 #undef CKC

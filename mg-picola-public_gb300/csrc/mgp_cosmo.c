@@ -907,19 +907,35 @@ double mgp_cosmo_drift_dyyy(const mgp_cosmo *c, double a, double aff, double af)
 
 /* -------------------------------------------------------- power spectrum */
 /* Eisenstein & Hu no-wiggle transfer function (src/power.c:447-476). */
-static double transfer_eh(const mgp_cosmo *c, double k) {
+static void eh_constants(const mgp_cosmo *c, mgp_eh_spectrum *e) {
   const double h = c->p.HubbleParam, om = c->p.Omega;
   double ombh2 = c->p.OmegaBaryon * h * h;
   if (c->p.OmegaBaryon == 0) ombh2 = 0.04 * h * h;
-  k *= 3.085678e24 / c->p.UnitLength_in_cm;
-  double theta = 2.728 / 2.7, ommh2 = om * h * h;
-  double s = 44.5 * log(9.83 / ommh2) / sqrt(1. + 10. * exp(0.75 * log(ombh2))) * h;
-  double fb = ombh2 / ommh2;
-  double alpha = 1. - 0.328 * log(431. * ommh2) * fb + 0.380 * log(22.3 * ommh2) * fb * fb;
-  double gamma = (alpha + (1. - alpha) / (1. + exp(4 * log(0.43 * k * s)))) * om * h;
-  double q = k * theta * theta / gamma;
+  double ommh2 = om * h * h, fb = ombh2 / ommh2;
+  e->norm = c->norm;
+  e->ns = c->p.PrimordialIndex;
+  e->kunit = 3.085678e24 / c->p.UnitLength_in_cm;
+  e->theta = 2.728 / 2.7;
+  e->s = 44.5 * log(9.83 / ommh2) / sqrt(1. + 10. * exp(0.75 * log(ombh2))) * h;
+  e->alpha = 1. - 0.328 * log(431. * ommh2) * fb + 0.380 * log(22.3 * ommh2) * fb * fb;
+  e->gamma0 = om * h;
+}
+
+static double transfer_eh(const mgp_cosmo *c, double k) {
+  mgp_eh_spectrum e;
+  eh_constants(c, &e);
+  k *= e.kunit;
+  double gamma = (e.alpha + (1. - e.alpha) / (1. + exp(4 * log(0.43 * k * e.s)))) * e.gamma0;
+  double q = k * e.theta * e.theta / gamma;
   double L0 = log(2. * exp(1.) + 1.8 * q), C0 = 14.2 + 731. / (1. + 62.5 * q);
   return L0 / (L0 + C0 * q * q);
+}
+
+int mgp_cosmo_power_eh(const mgp_cosmo *c, mgp_eh_spectrum *e) {
+  if (c->p.massive_neutrinos || c->p.WhichSpectrum == 1 || (c->p.WhichSpectrum == 0 && c->p.WhichTransfer == 1))
+    return 0;
+  eh_constants(c, e);
+  return 1;
 }
 
 static double table_interp(const mgp_cosmo *c, double k) {
@@ -1054,6 +1070,8 @@ void mgp_cosmo_pofk_ratio_many(const mgp_cosmo *c, double a, int n, const double
   }
   free(col);
 }
+
+double mgp_cosmo_growth_lcdm0(const mgp_cosmo *c) { return spline_eval(&c->DL, 0.0); }
 
 /* mg_sigma8_enhancement(a) (src/cosmo.c:713-756): the ratio of growth
  * factors, or in the scale-dependent build the ratio of the sigma_8

@@ -101,6 +101,15 @@ double mgp_cosmo_drift_dyyy(const mgp_cosmo *c, double a, double aff, double af)
 
 /* PowerSpec (src/power.c:373-394) in (Mpc/h)^3, k in h/Mpc */
 double mgp_cosmo_power(const mgp_cosmo *c, double k);
+/* The constants of the analytic spectrum norm k^ns T(k)^2 with the Eisenstein
+ * & Hu no-wiggle T (src/power.c:447-476); returns 0 when the spectrum is
+ * tabulated or comes from CAMB files. */
+typedef struct {
+  double norm, ns, kunit, s, alpha, gamma0, theta;
+} mgp_eh_spectrum;
+int mgp_cosmo_power_eh(const mgp_cosmo *c, mgp_eh_spectrum *e);
+/* the LCDM growth factor at a = 1 in the units of the D(k, a) table */
+double mgp_cosmo_growth_lcdm0(const mgp_cosmo *c);
 /* mg_pofk_ratio(k, a) and mg_sigma8_enhancement(a) (src/cosmo.c:688-756) */
 double mgp_cosmo_pofk_ratio(const mgp_cosmo *c, double k, double a);
 void mgp_cosmo_pofk_ratio_many(const mgp_cosmo *c, double a, int n, const double *k, double *out);

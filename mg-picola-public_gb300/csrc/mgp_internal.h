@@ -79,6 +79,7 @@ struct mgp_ctx {
   /* grids */
   float *rho, *dk, *frc, *mg1;
   float *ic_scratch;        /* six grids for the 2LPT IC (lazy, kept for the next IC) */
+  double *ic_amp;           /* device: amplitude per integer |k|^2 up to the IC's mode cut (lazy), then a growth column */
   void *fft_work;
   size_t fft_work_bytes;
   cufftHandle plan_r2c_oop, plan_r2c_ip, plan_c2r_1;
@@ -369,9 +370,10 @@ int mgp_launch_screen_table(float *rho, const float *arg, long long n, float mul
                             double t0, double dt, cudaStream_t st);
 
 /* IC */
-int mgp_launch_ic_delta(const uint32_t *seedtable, const double *amp_rk, const unsigned char *cut1d,
-                        int N, int Ns, double box, int fixed, int inverted, int sphere, float *dk,
-                        cudaStream_t st);
+int mgp_launch_ic_amp(double *amp, int n, double kf, double vol, const mgp_eh_spectrum *e, double fac,
+                      const double *col, int ny, double y0, double dy, double DL, cudaStream_t st);
+int mgp_launch_ic_delta(uint32_t seed, const double *amp_rk, int N, int Ns, int kc, double box, int fixed, int inverted,
+                        int sphere, float *dk, cudaStream_t st);
 int mgp_launch_ic_grad6(const float *dk, float *out6, long long grid_floats, int N, cudaStream_t st);
 int mgp_launch_ic_source(float *g6, long long grid_floats, int N, long long P, cudaStream_t st);
 int mgp_launch_ic_disp(const float *dk, const float *src, float *out6, long long grid_floats, int N, double box,

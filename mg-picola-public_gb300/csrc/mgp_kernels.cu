@@ -864,73 +864,159 @@ int mgp_launch_scale_complex(float *c, long long ncomplex, float factor, cudaStr
 }
 
 // ------------------------------------------------------------------ IC
-// displacement_fields, Gaussian branch (src/2LPT.c:276-495): one thread per
-// (i, j) column of the k grid replays that column's white-noise stream
-// (seeded by seedtable[i N + j], 2LPT.c:344) in the reference's draw order --
-// phase, then amplitude unless amplitude-fixed -- and writes delta(k) for
-// kz < N/2, including the Hermitian partners on the kz = 0 plane.
-// amp_rk[RK] = Box^-1.5 sqrt(P(k) * rescale) is tabulated on the host in FP64;
-// cut1d[|d|] is the cube cut of 2LPT.c:383-386 evaluated on the host with the
-// reference's exact double expression.
-__global__ void __launch_bounds__(MGP_THREADS) k_ic_delta(const uint32_t *__restrict__ seedtable,
-                                                          const double *__restrict__ amp_rk,
-                                                          const unsigned char *__restrict__ cut1d, int N, int Ns,
-                                                          double box, int fixed, int inverted, int sphere,
-                                                          float2 *__restrict__ dk) {
-  long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= (long long)N * N) return;
-  const int NH = N / 2 + 1;
-  int i = (int)(col / N), j = (int)(col % N);
-  uint32_t seed = seedtable[col];
-  uint64_t n = 0;
-  const double twopi = 2 * 3.14159265358979323846;
-  for (int k = 0; k < N / 2; k++) {
-    double phase = mgp_uniform(seed, n++);
-    double ampl = 1.0;
-    if (!fixed) {
-      do { ampl = mgp_uniform(seed, n++); } while (ampl == 0.0);
-    }
-    if (2 * i == N || 2 * j == N) continue;
-    if (i == 0 && j == 0 && k == 0) continue;
-    int di = i < N / 2 ? i : i - N, dj = j < N / 2 ? j : j - N, dkz = k;
-    int ai = di < 0 ? -di : di, aj = dj < 0 ? -dj : dj;
-    if (sphere) {
-      double kx = (di < 0 ? -(N - i) * 2 * 3.14159265358979323846 / box : i * 2 * 3.14159265358979323846 / box);
-      double ky = (dj < 0 ? -(N - j) * 2 * 3.14159265358979323846 / box : j * 2 * 3.14159265358979323846 / box);
-      double kzv = k * 2 * 3.14159265358979323846 / box;
-      double km = sqrt(kx * kx + ky * ky + kzv * kzv);
-      if (km * box / twopi > Ns / 2) continue;
-    } else {
-      if (cut1d[ai] || cut1d[aj] || cut1d[dkz]) continue;
-    }
-    int rk = ai * ai + aj * aj + dkz * dkz;
-    double delta = amp_rk[rk];
-    if (!fixed) delta *= sqrt(-log(ampl));
-    if (inverted) delta = -delta;
-    float sn, cs;
-    sincospif((float)(2.0 * phase), &sn, &cs);
-    float re = (float)delta * cs, im = (float)delta * sn;
-    if (k > 0) {
-      dk[((long long)i * N + j) * NH + k] = make_float2(re, im);
-    } else if (i == 0) {
-      if (j >= N / 2) continue;
-      dk[((long long)j) * NH] = make_float2(re, im);
-      dk[((long long)(N - j)) * NH] = make_float2(re, -im);
-    } else {
-      if (i >= N / 2) continue;
-      int ii = N - i, jj = (N - j) % N;
-      dk[((long long)i * N + j) * NH] = make_float2(re, im);
-      dk[((long long)ii * N + jj) * NH] = make_float2(re, -im);
-    }
-  }
-  (void)twopi;
+// displacement_fields, Gaussian branch (src/2LPT.c:262-495).
+//
+// Entry (i, j) of the seed table (2LPT.c:262-271): the reference fills the
+// table in shells m = 0 .. N/2-1, eight runs per shell (the four quadrants,
+// each a row run and a column run of lengths m and m + 1); shell m starts at
+// draw 4 m^2, so the position of an entry in the stream has a closed form and
+// every entry is one counter-based draw.
+__device__ __forceinline__ uint32_t ic_column_seed(uint32_t seed, int i, int j, int N) {
+  const bool hi = i >= N / 2, hj = j >= N / 2;
+  const int x = hi ? N - 1 - i : i, y = hj ? N - 1 - j : j;
+  const int m = x > y ? x : y, run = x > y ? y : m + x;  // row run (m, y < m), column run (x <= m, m)
+  const uint64_t n = 4ull * m * m + (uint64_t)((hj ? 2 : 0) + (hi ? 1 : 0)) * (2 * m + 1) + run;
+  return (uint32_t)(0x7fffffff * mgp_uniform(seed, n));
 }
 
-int mgp_launch_ic_delta(const uint32_t *seedtable, const double *amp_rk, const unsigned char *cut1d, int N, int Ns,
-                        double box, int fixed, int inverted, int sphere, float *dk, cudaStream_t st) {
-  long long cols = (long long)N * N;
-  int nb = (int)((cols + MGP_THREADS - 1) / MGP_THREADS);
-  k_ic_delta<<<nb, MGP_THREADS, 0, st>>>(seedtable, amp_rk, cut1d, N, Ns, box, fixed, inverted, sphere, (float2 *)dk);
+// Amplitude Box^-1.5 sqrt(P(k) rescaling) per integer |k|^2 = rk for the
+// analytic spectrum (Eisenstein & Hu no-wiggle transfer function,
+// src/power.c:447-476; the constants from mgp_cosmo_power_eh), FP64: `fac`
+// is the k-independent part of the rescaling (2LPT.c:395-407); with a
+// growth-table column (ny > 0, cubic Hermite in ln k) the rescaling also
+// carries (D(k) / DL)^2.  A host loop over the 3 (Ns/2)^2 values took 20 ms
+// at Nsample 512 (100 ns each).
+__global__ void k_ic_amp(double *__restrict__ amp, int n, double kf, double vol, mgp_eh_spectrum e, double fac,
+                         const double *__restrict__ col, int ny, double y0, double dy, double DL) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int rk = blockIdx.x * blockDim.x + threadIdx.x; rk < n; rk += stride) {
+    if (rk == 0) {
+      amp[0] = 0.0;
+      continue;
+    }
+    const double k = kf * sqrt((double)rk), ku = k * e.kunit;
+    const double gamma = (e.alpha + (1. - e.alpha) / (1. + exp(4 * log(0.43 * ku * e.s)))) * e.gamma0;
+    const double q = ku * e.theta * e.theta / gamma;
+    const double L0 = log(2. * exp(1.) + 1.8 * q), C0 = 14.2 + 731. / (1. + 62.5 * q), T = L0 / (L0 + C0 * q * q);
+    double pk = e.norm * pow(k, e.ns) * T * T * fac;
+    if (ny > 0) {
+      double t = (log(k) - y0) / dy;
+      t = fmin(fmax(t, 0.0), (double)(ny - 1));
+      int j = (int)t;
+      if (j > ny - 2) j = ny - 2;
+      const double u = t - (double)j;
+      const double D = (1 + 2 * u) * (1 - u) * (1 - u) * col[j] + u * u * (3 - 2 * u) * col[j + 1] +
+                       u * (1 - u) * (1 - u) * dy * col[ny + j] + u * u * (u - 1) * dy * col[ny + j + 1];
+      pk *= (D / DL) * (D / DL);
+    }
+    amp[rk] = vol * sqrt(pk);
+  }
+}
+
+int mgp_launch_ic_amp(double *amp, int n, double kf, double vol, const mgp_eh_spectrum *e, double fac,
+                      const double *col, int ny, double y0, double dy, double DL, cudaStream_t st) {
+  k_ic_amp<<<blocks_for(n, 8), MGP_THREADS, 0, st>>>(amp, n, kf, vol, *e, fac, col, ny, y0, dy, DL);
+  MGP_CHECK_LAUNCH();
+  g_kernel_launches++;
+  return MGP_OK;
+}
+
+// delta(k) of the Gaussian draw: one warp per (i, j) row, lanes along kz, so
+// the row is written once, coalesced, zeros included (one thread per column
+// wrote 8-byte entries 4 KB apart after a separate memset).  Mode kz takes
+// draws 2 kz (phase) and 2 kz + 1 (amplitude) of the column's stream, or draw
+// kz when amplitudes are fixed; the reference draws again when an amplitude
+// is zero (probability 2^-53 each), which shifts every later draw of the
+// column: a chunk of 32 modes that meets one replays its draws in order.
+// Modes outside the cube |d| <= kc (2LPT.c:383-386; kc = Ns/2, or one less
+// where the reference's double expression rounds above it) need no draws at
+// all.  The kz = 0 entries of the half the reference fills by symmetry take
+// the conjugate of the partner column's first mode.  With the seed table and
+// the amplitudes also made on the device, the whole IC of 256^3 particles on
+// a 512^3 mesh went from 36 to 17 ms (the rest is its transforms).
+__global__ void __launch_bounds__(MGP_THREADS) k_ic_delta(uint32_t seed0, const double *__restrict__ amp_rk, int N,
+                                                          int Ns, int kc, double box, int fixed, int inverted,
+                                                          int sphere, float2 *__restrict__ dk) {
+  const double twopi = 2 * 3.14159265358979323846;
+  const int NH = N / 2 + 1, lane = threadIdx.x & 31;
+  const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int reach = sphere ? Ns / 2 + 1 : kc;  // no mode beyond it survives the cut
+  for (long long row = wid; row < (long long)N * N; row += nw) {
+    const int i = (int)(row / N), j = (int)(row - (long long)i * N);
+    const int ai = i < N / 2 ? i : N - i, aj = j < N / 2 ? j : N - j;
+    float2 *__restrict__ out = dk + row * NH;
+    const bool dead = 2 * i == N || 2 * j == N || ai > reach || aj > reach;
+    const int kend = dead ? 0 : min(N / 2, reach + 1);  // modes kz < kend are drawn
+    const uint32_t seed = dead ? 0u : ic_column_seed(seed0, i, j, N);
+    // kz = 0: rows i > N/2, or i = 0 and j > N/2, mirror their partner's draw
+    const bool mirror = i > N / 2 || (i == 0 && j > N / 2);
+    uint64_t base = 0;  // draws used by the modes before this chunk
+    for (int k0 = 0; k0 < NH; k0 += 32) {
+      const int k = k0 + lane;
+      if (k0 >= kend) {
+        if (k < NH) out[k] = make_float2(0.f, 0.f);
+        continue;
+      }
+      double phase = 0.0, ampl = 1.0;
+      if (k < kend) {
+        uint32_t sd = seed;
+        if (k == 0 && mirror) sd = ic_column_seed(seed0, i ? N - i : 0, j ? N - j : 0, N);
+        if (fixed) {
+          phase = mgp_uniform(sd, (uint64_t)k);
+        } else {
+          const uint64_t n = base + 2ull * lane;
+          phase = mgp_uniform(sd, n);
+          ampl = mgp_uniform(sd, n + 1);
+          if (k == 0 && mirror)
+            for (uint64_t m = n + 2; ampl == 0.0; m++) ampl = mgp_uniform(sd, m);
+        }
+      }
+      if (!fixed) {
+        // the column's own stream at kz = 0 decides what the later modes draw
+        const bool zero = k < kend && (k == 0 && mirror ? mgp_uniform(seed, base + 1) == 0.0 : ampl == 0.0);
+        uint64_t used = 64;
+        if (__any_sync(0xffffffffu, zero)) {
+          uint64_t n = base;
+          for (int l = 0; l < 32; l++) {
+            const double ph = mgp_uniform(seed, n++);
+            double am;
+            do { am = mgp_uniform(seed, n++); } while (am == 0.0);
+            if (l == lane && !(k == 0 && mirror)) {
+              phase = ph;
+              ampl = am;
+            }
+          }
+          used = n - base;
+        }
+        base += used;
+      }
+      float2 z = make_float2(0.f, 0.f);
+      bool live = k < kend && !(row == 0 && k == 0);
+      if (live && sphere) {
+        const double kx = ai * twopi / box, ky = aj * twopi / box, kzv = k * twopi / box;
+        const double km = sqrt(kx * kx + ky * ky + kzv * kzv);
+        live = !(km * box / twopi > Ns / 2);
+      }
+      if (live) {
+        const int rk = ai * ai + aj * aj + k * k;
+        double delta = amp_rk[rk];
+        if (!fixed) delta *= sqrt(-log(ampl));
+        if (inverted) delta = -delta;
+        float sn, cs;
+        sincospif((float)(2.0 * phase), &sn, &cs);
+        z = make_float2((float)delta * cs, (float)delta * sn);
+        if (k == 0 && mirror) z.y = -z.y;
+      }
+      if (k < NH) out[k] = z;
+    }
+  }
+}
+
+int mgp_launch_ic_delta(uint32_t seed, const double *amp_rk, int N, int Ns, int kc, double box, int fixed, int inverted,
+                        int sphere, float *dk, cudaStream_t st) {
+  k_ic_delta<<<blocks_for((long long)N * N * 32, 8), MGP_THREADS, 0, st>>>(seed, amp_rk, N, Ns, kc, box, fixed, inverted,
+                                                                          sphere, (float2 *)dk);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
