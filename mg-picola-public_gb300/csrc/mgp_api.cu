@@ -144,14 +144,22 @@ extern "C" int mgp_set_particle_order(mgp_ctx *c, int tiles) {
   return MGP_OK;
 }
 
+static void drop_graph(mgp_ctx *c) {
+  if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
+  if (c->graph) cudaGraphDestroy(c->graph);
+  c->graph_exec = NULL;
+  c->graph = NULL;
+}
+
 extern "C" int mgp_set_fft_mode(mgp_ctx *c, int mode) {
   if (!c) return mgp_set_error(MGP_EINVAL, "null context");
   if (mode < 0 || mode > 1) return mgp_set_error(MGP_EINVAL, "FFT mode %d (0 or 1)", mode);
+  if (mode != c->fft_mode) drop_graph(c);  // a batch captures its next run anew
   c->fft_mode = mode;
   return MGP_OK;
 }
 
-// Whether this context's transforms take the strided passes of mgp_fft.cu.
+// Whether this context's transforms are those of mgp_fft.cu.
 static bool own_fft(const mgp_ctx *c) { return c->fft_mode && mgp_fft_supported(c); }
 
 extern "C" int mgp_mark(mgp_ctx *c, int slot) {
@@ -525,6 +533,7 @@ static int create_impl(const mgp_params *p, int nbox, const mgp_box_params *boxe
   TRYCUDA(cudaMalloc(&c->frc, 3 * gbytes));
   if (needs_mg1(p)) TRYCUDA(cudaMalloc(&c->mg1, gbytes));
   TRY(make_plans(c));
+  TRY(mgp_fft_setup(c));
   TRY(setup_pofk(c));
   c->tune[0] = c->tune[1] = c->tune[2] = MGP_BUDGET_DEFAULT;  // deposit, grid passes, kick
   c->tune[3] = 4;                                             // P(k) binning
@@ -611,6 +620,7 @@ static int ic_box(mgp_ctx *c, int bx, const double *pos01 = NULL, size_t npos = 
   const mgp_params *pb = &c->box_p[bx];
   const mgp_cosmo *cb = cosmo_of(c, bx);
   float *dkb = c->dk + (size_t)bx * c->g.nreal;
+  c->dk_planar = c->rho_planar = 0;
   const size_t po = (size_t)bx * 3 * c->np;
   const int N = c->g.N, Ns = c->Ns, h = N / 2;
   const double box = pb->Box;
@@ -819,25 +829,14 @@ static int fifth_force(mgp_ctx *c, double A, int filtered, int *mg_kind, float *
     // ComputeFifthForce_PotentialScreening, src/mg.h:147-189
     if (p->include_screening) {
       double norm = 1.0 / pow((double)N, 3) * 1.5 * p->Omega / A * pow(p->Box / 2997.92458 / (2.0 * M_PI), 2);
-      if (own_fft(c) && !filtered) {
-        // the inverse Laplacian applied in the first inverse pass (mgp_fft.cu)
-        RET_IF(mgp_fft_c2r_filtered(c, c->dk, c->mg1, 2, 0, 0.f, (float)norm));
-      } else {
-        if (!filtered) RET_IF(mgp_launch_div_laplacian(c->dk, c->mg1, N, (float)norm, c->stream));
-        if (own_fft(c))
-          RET_IF(mgp_fft_c2r(c, c->mg1));
-        else
-          MGP_CUFFT(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)c->mg1, (cufftReal *)c->mg1));
-      }
+      if (!filtered) RET_IF(mgp_launch_div_laplacian(c->dk, c->mg1, N, (float)norm, c->stream));
+      MGP_CUFFT(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)c->mg1, (cufftReal *)c->mg1));
       if (mgp_cosmo_user_screening(&c->cosmo, 0))
         RET_IF(user_screening(c, A, 0, 1.0, nr));
       else
         RET_IF(mgp_launch_screen_potential(c->rho, c->mg1, nr, (float)mgp_phicrit(&c->cosmo, A), c->stream));
     }
-    if (own_fft(c))
-      RET_IF(mgp_fft_r2c(c, c->rho, c->rho));
-    else
-      MGP_CUFFT(cufftExecR2C(c->plan_r2c_ip, (cufftReal *)c->rho, (cufftComplex *)c->rho));
+    MGP_CUFFT(cufftExecR2C(c->plan_r2c_ip, (cufftReal *)c->rho, (cufftComplex *)c->rho));
     *mg_kind = 1;
     *coupling = (float)mgp_coupling(&c->cosmo, A);
     *mass2 = (float)(A * A * mgp_mass2_of_a(&c->cosmo, A) / pow(2.0 * M_PI * 2997.92458 / p->Box, 2));
@@ -850,19 +849,10 @@ static int fifth_force(mgp_ctx *c, double A, int filtered, int *mg_kind, float *
       return MGP_OK;
     }
     double kR1 = 2.0 * M_PI / p->Box * p->Rsmooth;
-    if (own_fft(c) && !filtered) {
-      // the smoothing filter applied in the first inverse pass (mgp_fft.cu)
-      RET_IF(mgp_fft_c2r_filtered(c, c->dk, c->mg1, 1, p->smoothing_filter, (float)kR1,
-                                  (float)(1.0 / pow((double)N, 3))));
-    } else {
-      if (!filtered)
-        RET_IF(mgp_launch_smooth(c->dk, c->mg1, N, p->smoothing_filter, (float)kR1,
-                                 (float)(1.0 / pow((double)N, 3)), c->stream));
-      if (own_fft(c))
-        RET_IF(mgp_fft_c2r(c, c->mg1));
-      else
-        MGP_CUFFT(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)c->mg1, (cufftReal *)c->mg1));
-    }
+    if (!filtered)
+      RET_IF(mgp_launch_smooth(c->dk, c->mg1, N, p->smoothing_filter, (float)kR1, (float)(1.0 / pow((double)N, 3)),
+                               c->stream));
+    MGP_CUFFT(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)c->mg1, (cufftReal *)c->mg1));
     // Without massive neutrinos delta(k) is the transform of rho itself, so
     // the screening pass writes delta + source, rho (1 + coupling S), and the
     // force pass reads that one spectrum (mg_kind 4) instead of delta(k) and
@@ -875,10 +865,7 @@ static int fifth_force(mgp_ctx *c, double A, int filtered, int *mg_kind, float *
       RET_IF(mgp_launch_screen_density(c->rho, c->mg1, nr, (float)coupling_d,
                                        (float)mgp_dgp_screen_prefactor(&c->cosmo, A), c->stream, 1, NULL,
                                        fold ? 1.0f : 0.0f));
-    if (own_fft(c))
-      RET_IF(mgp_fft_r2c(c, c->rho, c->rho));
-    else
-      MGP_CUFFT(cufftExecR2C(c->plan_r2c_ip, (cufftReal *)c->rho, (cufftComplex *)c->rho));
+    MGP_CUFFT(cufftExecR2C(c->plan_r2c_ip, (cufftReal *)c->rho, (cufftComplex *)c->rho));
     *mg_kind = fold ? 4 : 2;
   } else if (p->model == MGP_MODEL_BRANSDICKE) {
     // ComputeFifthForce_TimeDepGeffModels (src/mg.h:127-137): the source
@@ -912,7 +899,7 @@ static int pofk_now(mgp_ctx *c, int fuse_kind, double A, double *sums = NULL) {
   }
   RET_IF(mgp_launch_pofk_thr(c->dk, N, c->pk_thr, c->win1d, c->pk_nbins, c->pk_bintype, c->pk_kmin, c->pk_kmax,
                              c->pk_block, c->pk_blocks, sums ? sums : c->pk_sum, fuse_kind, p->smoothing_filter,
-                             fuse_kind ? c->mg1 : NULL, fa, fb, c->stream));
+                             fuse_kind ? c->mg1 : NULL, fa, fb, c->stream, 1, 0, 0, c->dk_planar));
   return MGP_OK;
 }
 
@@ -958,7 +945,7 @@ static int nu_prepare(mgp_ctx *c, double A) {
 // which the MG solver reads from the total field.
 static int add_neutrinos(mgp_ctx *c, double A, int fuse_kind) {
   if (!c->sd_dk[0]) return mgp_set_error(MGP_ESTATE, "massive neutrinos need the scale-dependent IC field");
-  RET_IF(mgp_launch_nu_add(c->dk, c->sd_dk[0], c->g.N, c->nu_cdmfac, c->nu_tab_d, c->stream));
+  RET_IF(mgp_launch_nu_add(c->dk, c->sd_dk[0], c->g.N, c->nu_cdmfac, c->nu_tab_d, c->dk_planar, c->stream));
   if (c->p.pofk_compute_every_step) {
     if (!c->pk_sum_tot) MGP_CUDA(cudaMalloc(&c->pk_sum_tot, sizeof(double) * c->pk_nbins));
     RET_IF(pofk_now(c, fuse_kind, A, c->pk_sum_tot));
@@ -996,25 +983,122 @@ extern "C" int mgp_get_displacements(mgp_ctx *c, double A) {
   return fields_from_density(c, A);
 }
 
+// The field passes of a step at scale factor A for the transforms of
+// mgp_fft.cu: the solver's filter and screening (ComputeFifthForce,
+// src/user_defined_functions.h:687-719) and how its source enters the forces.
+// bs: per-box scalars of a batch (device), which replace the growth- and
+// model-dependent ones.
+static mgp_fft_plan field_plan(const mgp_ctx *c, double A, const mgp_box_scalars *bs) {
+  const mgp_params *p = &c->p;
+  const double n3 = pow((double)c->g.N, 3);
+  mgp_fft_plan f;
+  memset(&f, 0, sizeof(f));
+  f.A = A;
+  f.bs = bs;
+  f.cfac = (float)(-1.0 / (n3 * (2.0 * M_PI / p->Box)));
+  f.split = c->cosmo.nu;
+  f.filter = p->smoothing_filter;
+  f.filter_kind = mg_filter_kind(p);
+  if (f.filter_kind == 1) {
+    f.kR1 = (float)(2.0 * M_PI / p->Box * p->Rsmooth);
+    f.norm = (float)(1.0 / n3);
+  } else if (f.filter_kind == 2) {
+    f.norm = (float)(1.0 / n3 * 1.5 * p->Omega / A * pow(p->Box / 2997.92458 / (2.0 * M_PI), 2));
+  }
+  if (!p->modified_gravity_active) return f;
+  if (p->model == MGP_MODEL_FOFR || p->model == MGP_MODEL_MBETA) {
+    // ComputeFifthForce_PotentialScreening, src/mg.h:147-189
+    f.from_rho = 1;
+    f.mg_kind = 1;
+    if (!bs) {
+      f.coupling = (float)mgp_coupling(&c->cosmo, A);
+      f.mass2 = (float)(A * A * mgp_mass2_of_a(&c->cosmo, A) / pow(2.0 * M_PI * 2997.92458 / p->Box, 2));
+      if (f.filter_kind) f.phicrit = (float)mgp_phicrit(&c->cosmo, A);
+    }
+  } else if (p->model == MGP_MODEL_DGP && p->include_screening) {
+    // ComputeFifthForce_DensityScreening, src/mg.h:197-260.  Without massive
+    // neutrinos delta(k) is the transform of rho itself, so the screening
+    // writes delta + source, rho (1 + coupling S), and the force pass reads
+    // that one spectrum (the sum P3D + P3D_mg of auxPM.c:450-455, formed in
+    // real space; the transform is linear)
+    const int fold = !c->cosmo.nu && !mgp_cosmo_user_screening(&c->cosmo, 1);
+    f.from_rho = 1;
+    f.mg_kind = fold ? 0 : 2;
+    f.screen_base = fold ? 1.0f : 0.0f;
+    if (!bs) {
+      f.screen_coupling = (float)mgp_coupling(&c->cosmo, A);
+      f.screen_pref = (float)mgp_dgp_screen_prefactor(&c->cosmo, A);
+    }
+  } else if (p->model == MGP_MODEL_DGP || p->model == MGP_MODEL_BRANSDICKE) {
+    // a multiple of delta(k) (src/mg.h:127-137, 209-215)
+    f.mg_kind = 3;
+    if (!bs)
+      f.coupling = (float)(p->model == MGP_MODEL_DGP ? mgp_coupling(&c->cosmo, A) : mgp_geff(&c->cosmo, A, 0.0) - 1.0);
+  }
+  return f;
+}
+
+// A user's screening function applied between the solver's inverse and the
+// density's forward z rows.
+static int user_screen_pass(mgp_ctx *c, const mgp_fft_plan *f) {
+  const int density = f->filter_kind == 1;
+  return user_screening(c, f->A, density, density ? (double)f->screen_coupling : 1.0, c->g.nreal);
+}
+
+static int fields_own(mgp_ctx *c, double A) {
+  mgp_fft_plan f = field_plan(c, A, NULL);
+  tstart(c, T_R2C);
+  RET_IF(mgp_fft_density(c, &f));
+  tstop(c, T_R2C);
+  c->have_density = 1;
+  c->last_density_a = A;
+  if (c->p.pofk_compute_every_step) {
+    tstart(c, T_POFK);
+    RET_IF(pofk_now(c, 0, A));
+    tstop(c, T_POFK);
+  }
+  if (c->cosmo.nu) RET_IF(add_neutrinos(c, A, 0));
+  tstart(c, T_MG);
+  if (f.from_rho) {
+    const bool user = f.filter_kind && mgp_cosmo_user_screening(&c->cosmo, f.filter_kind == 1);
+    RET_IF(mgp_fft_screen(c, &f, user ? user_screen_pass : NULL));
+  }
+  tstop(c, T_MG);
+  tstart(c, T_FORCES);
+  if (f.from_rho || f.split) RET_IF(mgp_fft_force_x(c, &f));
+  RET_IF(mgp_fft_force_y(c));
+  tstop(c, T_FORCES);
+  tstart(c, T_C2R);
+  RET_IF(mgp_fft_force_z(c));
+  tstop(c, T_C2R);
+  if (c->closure) {  // learned residual force, added to the force grids
+    tstart(c, T_NN);
+    RET_IF(mgp_closure_apply(c->closure, c, A, 1));
+    tstop(c, T_NN);
+  }
+  c->have_forces = 1;
+  return MGP_OK;
+}
+
 // The rest of GetDisplacements once the density is on the mesh: R2C, P(k),
 // neutrinos, fifth force, forces and the three C2R.
 static int fields_from_density(mgp_ctx *c, double A) {
+  c->rho_planar = 0;
+  // a closure whose high-pass keeps more than the mean out adds its residual
+  // to force spectra in cuFFT's layout
+  if (own_fft(c) && !(c->closure && !mgp_closure_real(c->closure))) return fields_own(c, A);
   const int N = c->g.N;
+  c->dk_planar = 0;
   tstart(c, T_R2C);
-  if (own_fft(c))
-    RET_IF(mgp_fft_r2c(c, c->rho, c->dk));
-  else
-    MGP_CUFFT(cufftExecR2C(c->plan_r2c_oop, (cufftReal *)c->rho, (cufftComplex *)c->dk));
+  MGP_CUFFT(cufftExecR2C(c->plan_r2c_oop, (cufftReal *)c->rho, (cufftComplex *)c->dk));
   tstop(c, T_R2C);
   c->have_density = 1;
   c->last_density_a = A;
   int fused = 0;
   if (c->p.pofk_compute_every_step) {
     // with massive neutrinos the fifth-force filter reads the total field:
-    // it is fused into the total P(k) pass instead of the CDM one.  With the
-    // y pass of mgp_fft.cu the filter rides on the first inverse pass of
-    // the solver's transform instead (P(k) then only reads delta(k)).
-    fused = own_fft(c) ? 0 : mg_filter_kind(&c->p);
+    // it is fused into the total P(k) pass instead of the CDM one
+    fused = mg_filter_kind(&c->p);
     tstart(c, T_POFK);
     RET_IF(pofk_now(c, c->cosmo.nu ? 0 : fused, A));
     tstop(c, T_POFK);
@@ -1026,14 +1110,6 @@ static int fields_from_density(mgp_ctx *c, double A) {
   RET_IF(fifth_force(c, A, fused, &mg_kind, &coupling, &mass2));
   tstop(c, T_MG);
   // Forces, src/auxPM.c:437-555
-  if (own_fft(c) && !c->closure && (mg_kind == 0 || mg_kind == 3 || mg_kind == 4)) {
-    // one spectrum: the force pass fused into the inverse x and y passes
-    // (mgp_fft.cu); nDGP without screening scales delta by 1 + coupling
-    const float *spec = mg_kind == 4 ? c->rho : c->dk;
-    RET_IF(mgp_fft_forces(c, spec, mg_kind == 3 ? 1.0f + coupling : 1.0f, T_FORCES, T_C2R));
-    c->have_forces = 1;
-    return MGP_OK;
-  }
   tstart(c, T_FORCES);
   if (mg_kind == 4)  // rho holds delta + the fifth-force source
     RET_IF(mgp_launch_forces(c->rho, NULL, 0.f, 0.f, 0, N, c->p.Box, c->frc, c->g.nreal, c->stream));
@@ -1042,17 +1118,13 @@ static int fields_from_density(mgp_ctx *c, double A) {
   tstop(c, T_FORCES);
   if (c->closure) {  // learned residual force, added to the force transforms
     tstart(c, T_NN);
-    RET_IF(mgp_closure_apply(c->closure, c, A));
+    RET_IF(mgp_closure_apply(c->closure, c, A, 0));
     tstop(c, T_NN);
   }
   tstart(c, T_C2R);
-  for (int g = 0; g < 3; g++) {
-    if (own_fft(c))
-      RET_IF(mgp_fft_c2r(c, c->frc + g * c->g.nreal));
-    else
-      MGP_CUFFT(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)(c->frc + g * c->g.nreal),
-                             (cufftReal *)(c->frc + g * c->g.nreal)));
-  }
+  for (int g = 0; g < 3; g++)
+    MGP_CUFFT(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)(c->frc + g * c->g.nreal),
+                           (cufftReal *)(c->frc + g * c->g.nreal)));
   tstop(c, T_C2R);
   c->have_forces = 1;
   return MGP_OK;
@@ -1473,6 +1545,28 @@ extern "C" int mgp_copy_grid(mgp_ctx *c, int which, float *host, size_t count) {
   }
   if (!src) return mgp_set_error(MGP_ESTATE, "grid %d is not allocated", which);
   if ((long long)count > c->g.nreal) return mgp_set_error(MGP_EINVAL, "count %zu exceeds grid size", count);
+  if ((which == 1 && c->dk_planar) || ((which == 0 || which == 5) && c->rho_planar)) {
+    // a planar spectrum, rearranged by up to 64 MB of x planes at a time
+    const int N = c->g.N;
+    const size_t plane = (size_t)c->g.N * c->g.P;
+    const int step = (int)(((size_t)16 << 20) / plane) + 1;
+    float *rows = NULL;
+    MGP_CUDA(cudaMalloc(&rows, sizeof(float) * plane * step));
+    int rc = MGP_OK;
+    for (int x = 0; x < N && (size_t)x * plane < count && rc == MGP_OK; x += step) {
+      const int x1 = x + step < N ? x + step : N;
+      size_t n = (size_t)(x1 - x) * plane;
+      if (n > count - (size_t)x * plane) n = count - (size_t)x * plane;
+      rc = mgp_fft_planar_rows(N, src, rows, x, x1, c->stream);
+      if (rc == MGP_OK &&
+          (cudaMemcpyAsync(host + (size_t)x * plane, rows, sizeof(float) * n, cudaMemcpyDeviceToHost, c->stream) !=
+               cudaSuccess ||
+           cudaStreamSynchronize(c->stream) != cudaSuccess))
+        rc = mgp_set_error(MGP_ECUDA, "copy of grid %d", which);
+    }
+    cudaFree(rows);
+    return rc;
+  }
   MGP_CUDA(cudaStreamSynchronize(c->stream));
   MGP_CUDA(cudaMemcpy(host, src, sizeof(float) * count, cudaMemcpyDeviceToHost));
   return MGP_OK;
@@ -1573,8 +1667,15 @@ static int batch_step_launch(mgp_ctx *c, const batch_step &q, const mgp_box_scal
     RET_IF(mgp_cic_tiles(c, (float)wpar, c->tune[0]));
   else
     RET_IF(mgp_launch_cic(c->s, c->dstate, c->np, c->Ns, N, p->Box, (float)wpar, c->rho, c->g.P, c->stream, B, gf));
-  MGP_CUFFT(cufftExecR2C(r2c_oop, (cufftReal *)c->rho, (cufftComplex *)c->dk));
-  const int fused = p->pofk_compute_every_step ? mg_filter_kind(p) : 0;
+  const bool own = own_fft(c);
+  mgp_fft_plan f;
+  if (own) {
+    f = field_plan(c, q.A, bs);
+    RET_IF(mgp_fft_density(c, &f));
+  } else {
+    MGP_CUFFT(cufftExecR2C(r2c_oop, (cufftReal *)c->rho, (cufftComplex *)c->dk));
+  }
+  const int fused = p->pofk_compute_every_step && !own ? mg_filter_kind(p) : 0;
   const double n3 = pow((double)N, 3);
   if (p->pofk_compute_every_step) {
     float fa = 0.f, fb = 0.f;
@@ -1586,10 +1687,17 @@ static int batch_step_launch(mgp_ctx *c, const batch_step &q, const mgp_box_scal
     }
     RET_IF(mgp_launch_pofk_thr(c->dk, N, c->pk_thr, c->win1d, c->pk_nbins, c->pk_bintype, c->pk_kmin, c->pk_kmax,
                                c->pk_block, c->pk_blocks, pk_sums, fused, p->smoothing_filter, fused ? c->mg1 : NULL,
-                               fa, fb, c->stream, B, gf, c->pk_nbins));
+                               fa, fb, c->stream, B, gf, c->pk_nbins, own));
   }
   int mg_kind = 0;
-  if (p->modified_gravity_active) {
+  if (own) {
+    if (f.from_rho) {
+      RET_IF(mgp_fft_screen(c, &f, NULL));
+      RET_IF(mgp_fft_force_x(c, &f));
+    }
+    RET_IF(mgp_fft_force_y(c));
+    RET_IF(mgp_fft_force_z(c));
+  } else if (p->modified_gravity_active) {
     if (p->model == MGP_MODEL_FOFR || p->model == MGP_MODEL_MBETA) {
       if (p->include_screening) {
         double norm = 1.0 / n3 * 1.5 * p->Omega / q.A * pow(p->Box / 2997.92458 / (2.0 * M_PI), 2);
@@ -1615,9 +1723,11 @@ static int batch_step_launch(mgp_ctx *c, const batch_step &q, const mgp_box_scal
       mg_kind = 3;
     }
   }
-  RET_IF(mgp_launch_forces(c->dk, c->rho, 0.f, 0.f, mg_kind, N, p->Box, c->frc, gf, c->stream, B, bs));
-  for (int g = 0; g < 3; g++)
-    MGP_CUFFT(cufftExecC2R(c2r_frc, (cufftComplex *)(c->frc + g * gf), (cufftReal *)(c->frc + g * gf)));
+  if (!own) {
+    RET_IF(mgp_launch_forces(c->dk, c->rho, 0.f, 0.f, mg_kind, N, p->Box, c->frc, gf, c->stream, B, bs));
+    for (int g = 0; g < 3; g++)
+      MGP_CUFFT(cufftExecC2R(c2r_frc, (cufftComplex *)(c->frc + g * gf), (cufftReal *)(c->frc + g * gf)));
+  }
   int nblk = mgp_blocks_per_box(c->np, c->tune[2], B);
   if (nblk > c->max_blocks) nblk = c->max_blocks;  // the per-block partials buffer
   RET_IF(mgp_launch_ikd(c->frc, gf, N, c->g.P, c->Ns, c->np, c->s, c->v, c->D1, c->D2, c->dstate, c->partials, nblk,
@@ -1650,6 +1760,7 @@ static int batch_build_graph(mgp_ctx *c, int nsteps, double zf) {
   if (c->pk_blocks > c->pk_blocks_cap) c->pk_blocks = c->pk_blocks_cap;
   mgp_set_launch_budget(c->tune[0], c->tune[1]);
   if (c->batch_tile) RET_IF(mgp_tiles_alloc(c, c->batch_tile));  // no allocation inside the capture
+  if (own_fft(c)) RET_IF(mgp_fft_scratch(c));
   MGP_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   const long long k0 = g_kernel_launches;
   int rc = MGP_OK;
@@ -1710,10 +1821,7 @@ extern "C" int mgp_batch_set_tuning(mgp_ctx *c, const int *tune) {
   for (int q = 0; q < 4; q++)
     if (tune[q] < 1 || tune[q] > 64) return mgp_set_error(MGP_EINVAL, "launch budget %d out of [1, 64]", tune[q]);
   for (int q = 0; q < 4; q++) c->tune[q] = tune[q];
-  if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
-  if (c->graph) cudaGraphDestroy(c->graph);
-  c->graph_exec = NULL;
-  c->graph = NULL;
+  drop_graph(c);
   return MGP_OK;
 }
 
@@ -1733,10 +1841,7 @@ extern "C" int mgp_batch_set_deposit_tiles(mgp_ctx *c, int side) {
   if (!c) return mgp_set_error(MGP_EINVAL, "null context");
   if (side) RET_IF(mgp_tiles_check(c, side));
   c->batch_tile = side;
-  if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
-  if (c->graph) cudaGraphDestroy(c->graph);
-  c->graph_exec = NULL;
-  c->graph = NULL;
+  drop_graph(c);
   return MGP_OK;
 }
 

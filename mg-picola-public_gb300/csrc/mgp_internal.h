@@ -83,15 +83,14 @@ struct mgp_ctx {
   void *fft_work;
   size_t fft_work_bytes;
   cufftHandle plan_r2c_oop, plan_r2c_ip, plan_c2r_1;
-  /* 1024^3 grids (mgp_fft.cu): the y pass by this library's kernel (the
-   * force pass fused into the inverse one), z rows and x lines by cuFFT's
-   * 1D plans.  fft_mode 1 (default where supported) uses them, 0 the 3D
-   * cuFFT plans. */
-  int fft_mode, fft_ready;
-  cufftHandle zplan_r2c_oop, zplan_r2c_ip, zplan_c2r, xplan;
-  float *fft_tw;            /* device: W_1024^m, m = 0..1023 (float2) */
-  float *fft_gauss;         /* device: Gaussian smoothing factor per stored index (lazy) */
-  float fft_gauss_kR1;      /* the kR1 it was made for */
+  /* power-of-two meshes (mgp_fft.cu): fft_mode 1 (the default) transforms
+   * them with this library's kernels, 0 with cuFFT's 3D plans.  Tables of the
+   * mesh and of the lattice size (W_N^m, then the row passes'), and the
+   * Gaussian smoothing factor per stored index */
+  int fft_mode;
+  float *fft_tw, *fft_tw_s, *fft_gauss;
+  float *fft_scr;           /* scratch spectra (lazy): the IC's grids, or a batch's own */
+  int dk_planar, rho_planar; /* dk / rho hold a spectrum in the planar layout of mgp_fft.cuh */
 
   /* P(k) */
   int pk_nbins, pk_bintype, pk_sub;
@@ -289,16 +288,40 @@ typedef struct {
 extern long long g_kernel_launches;
 int mgp_blocks_for(long long n, int per_sm);
 
-/* the y pass of 1024^3 transforms and the fused force pass (mgp_fft.cu) */
+/* power-of-two transforms and the field passes fused into them (mgp_fft.cu).
+ * The plan of one step's field passes:
+ *   split        delta(k) is changed between the density and the forces
+ *                (neutrinos), or the forces are made elsewhere (closure)
+ *   filter_kind  the solver's filter, 1 smoothing, 2 inverse Laplacian (mg_kfilter)
+ *   from_rho     the source spectrum is the transform of rho after the screening
+ *   mg_kind      how it enters the forces: 0 alone, 1, 2, 3 as k_forces */
+typedef struct {
+  int split, filter_kind, filter;
+  float kR1, norm;
+  float phicrit, screen_coupling, screen_pref, screen_base;
+  int from_rho, mg_kind;
+  float cfac, coupling, mass2;
+  const mgp_box_scalars *bs; /* per box, in place of phicrit, couplings, pref and mass2 */
+  double A;
+} mgp_fft_plan;
+int mgp_fft_has(int N);
 int mgp_fft_supported(const mgp_ctx *c);
 int mgp_fft_setup(mgp_ctx *c);
 void mgp_fft_free(mgp_ctx *c);
-int mgp_fft_r2c(mgp_ctx *c, float *in, float *out);
-int mgp_fft_c2r(mgp_ctx *c, float *grid);
-int mgp_fft_forces(mgp_ctx *c, const float *spec, float mult, int t_x, int t_rest);
-int mgp_fft_c2r_filtered(mgp_ctx *c, const float *in, float *out, int kind, int filter, float kR1, float norm);
-/* learned force closure (mgp_nn.cu): adds its residual to the force grids */
-int mgp_closure_apply(struct mgp_closure *cl, mgp_ctx *c, double A);
+int mgp_fft_scratch(mgp_ctx *c);
+int mgp_fft_r2c(mgp_ctx *c, const float *in, float *out, int n, long long gs);
+int mgp_fft_c2r(mgp_ctx *c, int N, float *in, float *out, int n, long long gs);
+int mgp_fft_planar_rows(int N, const float *in, float *out, int x0, int x1, cudaStream_t st);
+int mgp_fft_density(mgp_ctx *c, const mgp_fft_plan *f);
+int mgp_fft_screen(mgp_ctx *c, const mgp_fft_plan *f, int (*user)(mgp_ctx *, const mgp_fft_plan *));
+int mgp_fft_force_x(mgp_ctx *c, const mgp_fft_plan *f);
+int mgp_fft_force_y(mgp_ctx *c);
+int mgp_fft_force_z(mgp_ctx *c);
+/* learned force closure (mgp_nn.cu): adds its residual to the force spectra
+ * in frc, or (real != 0, possible when mgp_closure_real says so) to the force
+ * grids themselves */
+int mgp_closure_apply(struct mgp_closure *cl, mgp_ctx *c, double A, int real);
+int mgp_closure_real(const struct mgp_closure *cl);
 /* waits for a pending snapshot write and frees the output buffers (mgp_destroy) */
 int mgp_run_release(mgp_ctx *c);
 
@@ -323,7 +346,7 @@ int mgp_launch_pofk(const float *dk, int N, const int *rk_bin, const float *win,
 int mgp_launch_pofk_thr(const float *dk, int N, const int *thr, const float *win, int nbins, int bintype, double kmin,
                         double kmax, double *block_part, int nblocks, double *sums, int fuse_kind, int filter,
                         float *fuse_out, float fuse_a, float fuse_b, cudaStream_t st, int nbox = 1,
-                        long long g_bs = 0, long long sum_bs = 0);
+                        long long g_bs = 0, long long sum_bs = 0, int planar = 0);
 int mgp_launch_forces(const float *dk, const float *mgk, float mg_coupling, float mg_mass2, int mg_kind,
                       int N, double box, float *frc, long long grid_floats, cudaStream_t st, int nbox = 1,
                       const mgp_box_scalars *bs = NULL);
@@ -348,7 +371,8 @@ int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a, int *nblocks_out);
 int mgp_particles_canonical(mgp_ctx *c);
 int mgp_launch_nu_table(float *tab, int nrk, double kfac, double fac, const double *x, const double *val,
                         const double *dval, int nx, const double *den, cudaStream_t st);
-int mgp_launch_nu_add(float *dk, const float *dk0, int N, double cdmfac, const float *nufac, cudaStream_t st);
+int mgp_launch_nu_add(float *dk, const float *dk0, int N, double cdmfac, const float *nufac, int planar,
+                      cudaStream_t st);
 int mgp_launch_cic_unit(const double *pos, long long n, int N, long long P, float wpar, float *rho, cudaStream_t st);
 int mgp_launch_ic_from_density(float *dk, int N, int Ns, double normfac, const double *gc, const double *rescale,
                                cudaStream_t st);

@@ -205,6 +205,7 @@ struct mgp_pofk_kargs {
   int priv;
   long long dk_bs;     // box stride of dk / fuse_out (complex values)
   long long part_bs;   // box stride of block_part (doubles)
+  int planar;          // layout of dk: planar (mgp_fft.cuh) or rows of N/2 + 1
 };
 
 // Bin sums: native FP32 shared-memory atomics made exact to second order by
@@ -248,11 +249,19 @@ __global__ void __launch_bounds__(MGP_THREADS) k_pofk(mgp_pofk_kargs a) {
     const long long rows[4] = {(long long)d0 * N + d1, (long long)d0 * N + (N - d1), (long long)(N - d0) * N + d1,
                                (long long)(N - d0) * N + (N - d1)};
     const bool use[4] = {true, mj, mi, mi && mj};
+    // offsets of kz = 0 and of kz = N/2 of every row
+    long long r0[4], rl[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const long long i = t < 2 ? d0 : N - d0, j = rows[t] - i * N, plane = i * ((long long)N * NH);
+      r0[t] = a.planar ? plane + j * h : rows[t] * NH;
+      rl[t] = a.planar ? plane + (long long)N * h + j : r0[t] + h;
+    }
     // the rows' next 32 modes are loaded while the current ones are binned
     float2 zn[4];
 #pragma unroll
     for (int t = 0; t < 4; t++)
-      if (use[t] && lane < NH) zn[t] = dkb[rows[t] * NH + lane];
+      if (use[t] && lane < NH) zn[t] = dkb[lane == h ? rl[t] : r0[t] + lane];
     for (int k0 = 0; k0 < NH; k0 += 32) {
       const int kz = k0 + lane;
       float2 z[4];
@@ -261,7 +270,7 @@ __global__ void __launch_bounds__(MGP_THREADS) k_pofk(mgp_pofk_kargs a) {
       if (kz + 32 < NH) {
 #pragma unroll
         for (int t = 0; t < 4; t++)
-          if (use[t]) zn[t] = dkb[rows[t] * NH + kz + 32];
+          if (use[t]) zn[t] = dkb[kz + 32 == h ? rl[t] : r0[t] + kz + 32];
       }
       int bin = -1;
       float pk = 0.0f;
@@ -375,7 +384,7 @@ int mgp_launch_pofk(const float *dk, int N, const int *rk_bin, const float *win,
 int mgp_launch_pofk_thr(const float *dk, int N, const int *thr, const float *win, int nbins, int bintype, double kmin,
                         double kmax, double *block_part, int nblocks, double *sums, int fuse_kind, int filter,
                         float *fuse_out, float fuse_a, float fuse_b, cudaStream_t st, int nbox, long long g_bs,
-                        long long sum_bs) {
+                        long long sum_bs, int planar) {
   mgp_pofk_kargs ka;
   memset(&ka, 0, sizeof(ka));
   ka.dk = (const float2 *)dk;
@@ -393,6 +402,7 @@ int mgp_launch_pofk_thr(const float *dk, int N, const int *thr, const float *win
   ka.fuse_a = fuse_a;
   ka.fuse_b = fuse_b;
   ka.dk_bs = g_bs / 2;
+  ka.planar = planar;
   return launch_pofk(ka, nblocks, sums, st, nbox, sum_bs);
 }
 
@@ -1028,8 +1038,9 @@ int mgp_launch_ic_delta(uint32_t seed, const double *amp_rk, int N, int Ns, int 
 // One warp per (i, j) row of the half-complex grid, lanes along kz; FP32
 // arithmetic (the grids are FP32, and FP64 runs at a small fraction of the
 // FP32 rate on this part).
+// planar: the layout of dk (mgp_fft.cuh).
 __global__ void k_nu_add(float2 *__restrict__ dk, const float2 *__restrict__ dk0, int N, float cdmfac,
-                         const float *__restrict__ nufac) {
+                         const float *__restrict__ nufac, int planar) {
   const int NH = N / 2 + 1;
   const int lane = threadIdx.x & 31;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1040,9 +1051,10 @@ __global__ void k_nu_add(float2 *__restrict__ dk, const float2 *__restrict__ dk0
     const int r2 = di * di + dj * dj;
     for (int kz = lane; kz < NH; kz += 32) {
       if (r == 0 && kz == 0) continue;
-      const long long c = r * NH + kz;
+      const long long c0 = r * NH + kz, plane = (long long)i * N * NH;
+      const long long c = !planar ? c0 : (2 * kz == N ? plane + (long long)N * kz + j : plane + (long long)j * (N / 2) + kz);
       const float f = nufac[r2 + kz * kz];
-      const float2 a = dk[c], b = dk0[c];
+      const float2 a = dk[c], b = dk0[c0];
       dk[c] = make_float2(fmaf(f, b.x, cdmfac * a.x), fmaf(f, b.y, cdmfac * a.y));
     }
   }
@@ -1083,10 +1095,11 @@ int mgp_launch_nu_table(float *tab, int nrk, double kfac, double fac, const doub
   return MGP_OK;
 }
 
-int mgp_launch_nu_add(float *dk, const float *dk0, int N, double cdmfac, const float *nufac, cudaStream_t st) {
+int mgp_launch_nu_add(float *dk, const float *dk0, int N, double cdmfac, const float *nufac, int planar,
+                      cudaStream_t st) {
   const long long rows = (long long)N * N;
   k_nu_add<<<blocks_for(rows * 32, 8), MGP_THREADS, 0, st>>>((float2 *)dk, (const float2 *)dk0, N, (float)cdmfac,
-                                                             nufac);
+                                                             nufac, planar);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;

@@ -733,6 +733,62 @@ __global__ void k_highpass(float2 *__restrict__ src, long long cstride, int N, f
   }
 }
 
+// Per-block sums of three padded real grids (FP64; fixed order).
+__global__ void __launch_bounds__(256) k_grid_sums(const float *__restrict__ u, long long gs, int N, long long P,
+                                                   double *__restrict__ part) {
+  __shared__ double sh[3][8];
+  const long long rows = (long long)N * N;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n2 = N / 2;
+  float acc[3] = {0.f, 0.f, 0.f};
+  for (long long r = (long long)blockIdx.x * 8 + w; r < rows; r += (long long)gridDim.x * 8)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const float2 *p = reinterpret_cast<const float2 *>(u + c * gs + r * P);
+      for (int k = lane; k < n2; k += 32) acc[c] += p[k].x + p[k].y;
+    }
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    double x = (double)acc[c];
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) sh[c][w] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double t = 0.0;
+    for (int k = 0; k < 8; k++) t += sh[threadIdx.x][k];
+    part[blockIdx.x * 3 + threadIdx.x] = t;
+  }
+}
+
+// frc += scale (u - <u>) on three padded real grids, <u> from the block sums.
+__global__ void __launch_bounds__(256) k_add_residual(float *__restrict__ frc, const float *__restrict__ u, long long gs,
+                                                      int N, long long P, const double *__restrict__ part, int nparts,
+                                                      float scale) {
+  __shared__ float mean[3];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n2 = N / 2;
+  if (w < 3) {
+    double t = 0.0;
+    for (int b = lane; b < nparts; b += 32) t += part[b * 3 + w];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) mean[w] = (float)(t / ((double)N * N * N));
+  }
+  __syncthreads();
+  const long long rows = (long long)N * N;
+  for (long long r = (long long)blockIdx.x * 8 + w; r < rows; r += (long long)gridDim.x * 8)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const float2 *p = reinterpret_cast<const float2 *>(u + c * gs + r * P);
+      float2 *f = reinterpret_cast<float2 *>(frc + c * gs + r * P);
+      for (int k = lane; k < n2; k += 32) {
+        const float2 a = p[k];
+        float2 o = f[k];
+        o.x = fmaf(scale, a.x - mean[c], o.x);
+        o.y = fmaf(scale, a.y - mean[c], o.y);
+        f[k] = o;
+      }
+    }
+}
+
 // Keep the modes of a fine-mesh transform [Nf][Nf][Nf/2+1] that the coarse
 // mesh represents (|k_x|, |k_y|, k_z < kc in fine integer units), scaled by
 // norm (the 1/Nf^3 of the round trip); zero the rest.
@@ -1139,10 +1195,13 @@ static int closure_features(mgp_closure *cl, mgp_ctx *c, double A) {
     MGP_CUDA(cudaMalloc(&cl->grid_b, sizeof(float) * gf));
   }
   MGP_CUFFT(cufftSetStream(c->plan_c2r_1, cl->stream));
-  MGP_CUDA(cudaMemcpyAsync(cl->grid_a, c->dk, sizeof(float) * gf, cudaMemcpyDeviceToDevice, cl->stream));
+  if (c->dk_planar)
+    NN_RET(mgp_fft_planar_rows(N, c->dk, cl->grid_a, 0, N, cl->stream));
+  else
+    MGP_CUDA(cudaMemcpyAsync(cl->grid_a, c->dk, sizeof(float) * gf, cudaMemcpyDeviceToDevice, cl->stream));
   const mgp_params *p = &c->p;
   const double norm = 1.0 / pow((double)N, 3) * 1.5 * p->Omega / A * pow(p->Box / 2997.92458 / (2.0 * M_PI), 2);
-  NN_RET(mgp_launch_div_laplacian(c->dk, cl->grid_b, N, (float)norm, cl->stream));
+  NN_RET(mgp_launch_div_laplacian(cl->grid_a, cl->grid_b, N, (float)norm, cl->stream));
   cufftResult r1 = cufftExecC2R(c->plan_c2r_1, (cufftComplex *)cl->grid_a, (cufftReal *)cl->grid_a);
   cufftResult r2 = cufftExecC2R(c->plan_c2r_1, (cufftComplex *)cl->grid_b, (cufftReal *)cl->grid_b);
   cufftSetStream(c->plan_c2r_1, c->stream);
@@ -1446,7 +1505,12 @@ static double closure_scale(const mgp_closure *cl, double A) {
 // three output grids), their R2C, and out_scale * H(k) / N^3 times them
 // added to the three force transforms, so the context's C2R yields the PM
 // force plus the high-passed closure force; all on the context's stream.
-int mgp_closure_apply(mgp_closure *cl, mgp_ctx *c, double A) {
+// real: called after the C2R instead.  With the default high-pass, which
+// removes the mean and nothing else, out_scale (u - <u>) is added to the force
+// grids without a transform (three R2C and a pass over six spectra less).
+int mgp_closure_real(const mgp_closure *cl) { return cl->hp_lambda == 0.f; }
+
+int mgp_closure_apply(mgp_closure *cl, mgp_ctx *c, double A, int real) {
   cudaStream_t keep = cl->stream;
   cl->stream = c->stream;
   int rc = ensure_hp(cl);
@@ -1459,6 +1523,18 @@ int mgp_closure_apply(mgp_closure *cl, mgp_ctx *c, double A) {
     rc = conv_fwd(cl, cl->act[NN_LAYERS - 1], cl->w16[NN_LAYERS - 1], cl->b32[NN_LAYERS - 1], NULL, 3, NULL, NULL,
                   cl->ugrid, gf, cl->P, 0.f);
   mgp_tstop(c, T_NNCONV);
+  if (real) {
+    cl->stream = keep;
+    if (rc != MGP_OK) return rc;
+    const int nb = mgp_blocks_for(cl->V, 4);  // at most max_blocks: the context's partials hold 6 a block
+    k_grid_sums<<<nb, 256, 0, c->stream>>>(cl->ugrid, gf, cl->N, cl->P, c->partials);
+    MGP_CHECK_LAUNCH();
+    k_add_residual<<<nb, 256, 0, c->stream>>>(c->frc, cl->ugrid, gf, cl->N, cl->P, c->partials, nb,
+                                              (float)closure_scale(cl, A));
+    MGP_CHECK_LAUNCH();
+    g_kernel_launches += 2;
+    return MGP_OK;
+  }
   if (rc == MGP_OK && cufftSetStream(cl->plan_r2c, c->stream) != CUFFT_SUCCESS)
     rc = mgp_set_error(MGP_ECUFFT, "closure transform stream");
   for (int q = 0; q < 3 && rc == MGP_OK; q++)

@@ -498,9 +498,9 @@ class Context:
         _check(lib().mgp_set_particle_order(self.h, int(tiles)))
 
     def set_fft_mode(self, mode):
-        """Transforms of a 1024^3 single box (mgp_set_fft_mode): 1 the
-        default, own strided y/x passes with the force pass fused in; 0
-        cuFFT's 3D plans and the separate force pass."""
+        """Transforms of power-of-two meshes of 64 to 1024 (mgp_set_fft_mode):
+        1 the default, the library's own passes with the force, filter and
+        screening passes fused in; 0 cuFFT's 3D plans and separate passes."""
         _check(lib().mgp_set_fft_mode(self.h, int(mode)))
 
     def mark(self, slot):
