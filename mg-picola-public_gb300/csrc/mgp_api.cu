@@ -396,7 +396,7 @@ extern "C" int mgp_destroy(mgp_ctx *c) {
     free(c->box_cosmo);
   }
   free(c->box_p);
-  void *bufs[] = {c->ic_scratch, c->ic_amp, c->s, c->v, c->D1, c->D2, c->dstate, c->partials, c->stage, c->rho, c->dk, c->frc, c->mg1,
+  void *bufs[] = {c->ic_scratch, c->ic_amp, c->ic_box, c->s, c->v, c->D1, c->D2, c->dstate, c->partials, c->stage, c->rho, c->dk, c->frc, c->mg1,
                   c->fft_work, c->rk_bin, c->pk_thr, c->win1d, c->pk_block, c->pk_sum, c->rsd_block, c->rsd_sum,
                   c->pk_sum_tot, c->nu_tab_d, c->nu_row_d, c->nu_x_d, c->nu_den_d, c->scr_tab};
   for (size_t i = 0; i < sizeof(bufs) / sizeof(bufs[0]); i++)
@@ -563,207 +563,245 @@ extern "C" int mgp_batch_create(const mgp_params *p, int nbox, const mgp_box_par
 }
 
 // ---------------------------------------------------------------- IC
-// Amplitudes per integer |k|^2 < namp of the Gaussian draw (k in h/Mpc = 2 pi/Box
-// sqrt(RK)) into c->ic_amp, with the P(k) rescaling for MG runs whose input
-// spectrum is LCDM (2LPT.c:323-327, 395-407): mg_pofk_ratio(k, 1), per k when
+// What the IC kernels need of every box (device, c->ic_box), and with `draw` the
+// amplitudes per integer |k|^2 < namp of the Gaussian draw (k in h/Mpc = 2 pi/Box
+// sqrt(RK)) into c->ic_amp, namp a box, with the P(k) rescaling for MG runs whose
+// input spectrum is LCDM (2LPT.c:323-327, 395-407): mg_pofk_ratio(k, 1), per k when
 // the growth is scale dependent.  The analytic spectrum is evaluated on the
 // device; tabulated spectra and CAMB files on the host.
-static int ic_amplitudes(mgp_ctx *c, const mgp_params *pb, const mgp_cosmo *cb, int namp) {
-  const double box = pb->Box, kf = 2.0 * M_PI / box;
-  const bool rescale = pb->modified_gravity_active && pb->input_pofk_is_for_lcdm;
-  const int ny = cb->sd ? cb->sd_tab[0].ny : 0;
-  if (!c->ic_amp) MGP_CUDA(cudaMalloc(&c->ic_amp, sizeof(double) * ((size_t)namp + 2 * ny)));
-  double s8fac = 1.0;
-  if (rescale && !pb->input_sigma8_is_for_lcdm) {
-    const double e = mgp_cosmo_sigma8_enh(cb, 1.0);
-    s8fac = 1.0 / (e * e);
-  }
+static int ic_prepare(mgp_ctx *c, int namp, int draw) {
+  const int n = c->nbox;
+  const double box = c->p.Box, kf = 2.0 * M_PI / box, ai = 1.0 / (1.0 + c->p.Init_Redshift);
+  const mgp_cosmo *c0 = &c->cosmo;
+  const int ny = c0->sd ? c0->sd_tab[0].ny : 0;
+  if (!c->ic_box) MGP_CUDA(cudaMalloc(&c->ic_box, sizeof(mgp_ic_box) * n));
+  if (!c->ic_amp) MGP_CUDA(cudaMalloc(&c->ic_amp, sizeof(double) * ((size_t)namp * n + 2 * ny)));
+  std::vector<mgp_ic_box> hb(n);
   mgp_eh_spectrum eh;
-  if (mgp_cosmo_power_eh(cb, &eh)) {
-    double fac = s8fac;
-    if (rescale && cb->sd) {
-      // per k: the growth table at a = 1 over the LCDM growth factor
-      std::vector<double> col(2 * (size_t)ny);
-      RET_IF(mgp_cosmo_sd_column(cb, 0, 1.0, col.data(), col.data() + ny));
-      const double *y = cb->sd_tab[0].y, dy = (y[ny - 1] - y[0]) / (double)(ny - 1);
-      double *dcol = c->ic_amp + namp;
-      MGP_CUDA(cudaMemcpyAsync(dcol, col.data(), sizeof(double) * 2 * ny, cudaMemcpyHostToDevice, c->stream));
-      RET_IF(mgp_launch_ic_amp(c->ic_amp, namp, kf, pow(box, -1.5), &eh, fac, dcol, ny, y[0], dy,
-                               mgp_cosmo_growth_lcdm0(cb), c->stream));
-      return MGP_OK;
+  const int analytic = mgp_cosmo_power_eh(c0, &eh);
+  bool per_k = false;
+  for (int b = 0; b < n; b++) {
+    const mgp_params *pb = &c->box_p[b];
+    const mgp_cosmo *cb = cosmo_of(c, b);
+    mgp_ic_box &o = hb[b];
+    memset(&o, 0, sizeof(o));
+    o.seed = (uint32_t)pb->Seed;
+    o.fixed = pb->amplitude_fixed_initial_condition;
+    o.inverted = pb->inverted_initial_condition;
+    o.sphere = pb->SphereMode == 1;
+    o.Di = (float)mgp_cosmo_growth(cb, 0, ai);
+    o.Di2 = (float)mgp_cosmo_growth(cb, 3, ai);
+    // without COLA the particles start with the 2LPT velocity (main.c:276-283)
+    o.vD = pb->UseCOLA ? 0.0f : (float)mgp_cosmo_growth(cb, 1, ai);
+    o.vD2 = pb->UseCOLA ? 0.0f : (float)mgp_cosmo_growth(cb, 4, ai);
+    o.fac = 1.0;
+    if (!draw) continue;
+    const bool rescale = pb->modified_gravity_active && pb->input_pofk_is_for_lcdm;
+    if (rescale && !pb->input_sigma8_is_for_lcdm) {
+      const double e = mgp_cosmo_sigma8_enh(cb, 1.0);
+      o.fac = 1.0 / (e * e);
     }
-    if (rescale) {
-      double k1 = kf, r1 = 1.0;
-      mgp_cosmo_pofk_ratio_many(cb, 1.0, 1, &k1, &r1);
-      fac *= r1;
+    if (analytic) {
+      mgp_eh_spectrum eb;
+      mgp_cosmo_power_eh(cb, &eb);
+      o.norm = eb.norm;
+      if (rescale && cb->sd) {
+        per_k = true;  // one box: batches run scale-independent growth
+      } else if (rescale) {
+        double k1 = kf, r1 = 1.0;
+        mgp_cosmo_pofk_ratio_many(cb, 1.0, 1, &k1, &r1);
+        o.fac *= r1;
+      }
+      continue;
     }
-    return mgp_launch_ic_amp(c->ic_amp, namp, kf, pow(box, -1.5), &eh, fac, NULL, 0, 0.0, 1.0, 1.0, c->stream);
+    std::vector<double> amp(namp, 0.0), kk(namp), ratio(namp, 1.0);
+    for (int rk = 0; rk < namp; rk++) kk[rk] = kf * sqrt((double)rk);
+    if (rescale) mgp_cosmo_pofk_ratio_many(cb, 1.0, namp - 1, kk.data() + 1, ratio.data() + 1);
+    for (int rk = 1; rk < namp; rk++)
+      amp[rk] = pow(box, -1.5) * sqrt(mgp_cosmo_power(cb, kk[rk]) * ratio[rk] * o.fac);
+    // pageable sources: the copies have been staged when the calls return
+    MGP_CUDA(cudaMemcpyAsync(c->ic_amp + (size_t)b * namp, amp.data(), sizeof(double) * namp, cudaMemcpyHostToDevice,
+                             c->stream));
   }
-  std::vector<double> amp(namp, 0.0), kk(namp), ratio(namp, 1.0);
-  for (int rk = 0; rk < namp; rk++) kk[rk] = kf * sqrt((double)rk);
-  if (rescale) mgp_cosmo_pofk_ratio_many(cb, 1.0, namp - 1, kk.data() + 1, ratio.data() + 1);
-  for (int rk = 1; rk < namp; rk++)
-    amp[rk] = pow(box, -1.5) * sqrt(mgp_cosmo_power(cb, kk[rk]) * ratio[rk] * s8fac);
-  // pageable source: the copy has been staged when the call returns
-  MGP_CUDA(cudaMemcpyAsync(c->ic_amp, amp.data(), sizeof(double) * namp, cudaMemcpyHostToDevice, c->stream));
+  MGP_CUDA(cudaMemcpyAsync(c->ic_box, hb.data(), sizeof(mgp_ic_box) * n, cudaMemcpyHostToDevice, c->stream));
+  if (!draw || !analytic) return MGP_OK;
+  if (!per_k)
+    return mgp_launch_ic_amp(c->ic_amp, namp, kf, pow(box, -1.5), &eh, c->ic_box, n, NULL, 0, 0.0, 1.0, 1.0, c->stream);
+  // the growth table at a = 1 over the LCDM growth factor
+  std::vector<double> col(2 * (size_t)ny);
+  RET_IF(mgp_cosmo_sd_column(c0, 0, 1.0, col.data(), col.data() + ny));
+  const double *y = c0->sd_tab[0].y, dy = (y[ny - 1] - y[0]) / (double)(ny - 1);
+  double *dcol = c->ic_amp + namp;
+  MGP_CUDA(cudaMemcpyAsync(dcol, col.data(), sizeof(double) * 2 * ny, cudaMemcpyHostToDevice, c->stream));
+  return mgp_launch_ic_amp(c->ic_amp, namp, kf, pow(box, -1.5), &eh, c->ic_box, 1, dcol, ny, y[0], dy,
+                           mgp_cosmo_growth_lcdm0(c0), c->stream);
+}
+
+// Mode cut of the draw (the cube cut of 2LPT.c:383-386 with the reference's
+// double expression: the largest |d| it keeps) and the number of amplitudes.
+static int ic_cut(const mgp_ctx *c, int *namp) {
+  const int h = c->g.N / 2, k = c->Ns / 2 < h ? c->Ns / 2 : h;
+  *namp = 3 * k * k + 1;
+  const double box = c->p.Box, kv = k * 2 * 3.14159265358979323846 / box;
+  return fabs(kv) * box / (2 * 3.14159265358979323846) > c->Ns / 2 ? k - 1 : k;
+}
+
+// delta(k) of box 0 in dk from particles in [0,1) of the box, as the linear field at
+// a = 1: their CIC density at a_i (readICfromfile.c:640-676), deconvolved and
+// rescaled (701-777).
+static int ic_density(mgp_ctx *c, const double *pos01, size_t npos, bool own) {
+  const mgp_params *pb = &c->box_p[0];
+  const mgp_cosmo *cb = &c->cosmo;
+  const int N = c->g.N, Ns = c->Ns, h = N / 2, rkmax = 3 * h * h;
+  const double box = pb->Box;
+  std::vector<double> gcw(h + 1), resc(rkmax + 1), kk(rkmax + 1), r2(rkmax + 1, 1.0);
+  for (int rk = 0; rk <= rkmax; rk++) kk[rk] = 2.0 * M_PI / box * sqrt((double)rk);
+  for (int d = 0; d <= h; d++) {
+    const double x = M_PI * d / (double)N, sc = d == 0 ? 1.0 : sin(x) / x;
+    gcw[d] = 1.0 / (sc * sc);
+  }
+  mgp_cosmo_pofk_ratio_many(cb, 1.0, rkmax, kk.data() + 1, r2.data() + 1);
+  const double s8 = pb->input_sigma8_is_for_lcdm ? 1.0 : mgp_cosmo_sigma8_enh(cb, 1.0);
+  for (int rk = 0; rk <= rkmax; rk++) resc[rk] = sqrt(r2[rk]) / s8;
+  const double normfac = 1.0 / ((double)N * N * N) / mgp_cosmo_growth(cb, 6, 1.0 / (1.0 + pb->Init_Redshift));
+  struct dbuf {  // freed on every exit
+    double *p = NULL;
+    ~dbuf() {
+      if (p) cudaFree(p);
+    }
+  } b_pos, b_gc, b_resc;
+  MGP_CUDA(cudaMalloc(&b_pos.p, sizeof(double) * 3 * npos));
+  MGP_CUDA(cudaMalloc(&b_gc.p, sizeof(double) * gcw.size()));
+  MGP_CUDA(cudaMalloc(&b_resc.p, sizeof(double) * resc.size()));
+  MGP_CUDA(cudaMemcpyAsync(b_pos.p, pos01, sizeof(double) * 3 * npos, cudaMemcpyHostToDevice, c->stream));
+  MGP_CUDA(cudaMemcpyAsync(b_gc.p, gcw.data(), sizeof(double) * gcw.size(), cudaMemcpyHostToDevice, c->stream));
+  MGP_CUDA(cudaMemcpyAsync(b_resc.p, resc.data(), sizeof(double) * resc.size(), cudaMemcpyHostToDevice, c->stream));
+  int rc = mgp_launch_fill(c->rho, c->g.nreal, -1.0f, c->stream);
+  if (rc == MGP_OK)
+    rc = mgp_launch_cic_unit(b_pos.p, (long long)npos, N, c->g.P, (float)pow((double)N / Ns, 3), c->rho, c->stream);
+  if (rc == MGP_OK && own)
+    rc = mgp_fft_r2c(c, c->rho, c->dk, 1, c->g.nreal);
+  else if (rc == MGP_OK && cufftExecR2C(c->plan_r2c_oop, (cufftReal *)c->rho, (cufftComplex *)c->dk) != CUFFT_SUCCESS)
+    rc = mgp_set_error(MGP_ECUFFT, "IC density transform");
+  if (rc == MGP_OK) rc = mgp_launch_ic_from_density(c->dk, N, Ns, normfac, b_gc.p, b_resc.p, own, c->stream);
+  cudaStreamSynchronize(c->stream);
+  return rc;
+}
+
+// After the fields: the scale-dependent build keeps delta(k) and the source
+// (2LPT.c:1336-1344), then x = q + D + D2 and v = dDdy + dD2dy (or 0) at a_i
+// (main.c:244-307).
+static int ic_sd(mgp_ctx *c, const float *src, int planar) {
+  const double Ai = 1.0 / (1.0 + c->p.Init_Redshift);
+  const int types[2] = {MGP_FIELD_D, MGP_FIELD_dDdy};
+  RET_IF(mgp_sd_store(c, c->dk, src, planar));
+  RET_IF(mgp_sd_fields(c, Ai, Ai, 2, types));
+  return mgp_sd_init_particles(c);
+}
+
+// The IC of every box with the transforms of mgp_fft.cu.
+static int ic_own(mgp_ctx *c, const double *pos01, size_t npos) {
+  const int N = c->g.N, Ns = c->Ns;
+  int namp, kc = ic_cut(c, &namp);
+  c->dk_planar = 1;
+  RET_IF(ic_prepare(c, namp, pos01 == NULL));
+  if (pos01) {
+    RET_IF(ic_density(c, pos01, npos, true));
+    kc = N > Ns ? Ns / 2 : N / 2;
+  } else {
+    RET_IF(mgp_launch_ic_delta(c->ic_box, c->nbox, c->ic_amp, namp, N, Ns, kc, c->p.Box, c->dk, c->g.nreal, 1, c->stream));
+    // spherical cut: modes up to Ns/2 + 1 may survive its rounding
+    if (c->p.SphereMode == 1) kc = Ns / 2 + 1 < N / 2 ? Ns / 2 + 1 : N / 2;
+  }
+  RET_IF(mgp_fft_ic_source(c, kc));
+  RET_IF(c->sd ? ic_sd(c, c->rho, 1) : mgp_fft_ic_fields(c));
   return MGP_OK;
 }
 
-// displacement_fields + the particle assignment of main.c:231-309 for box b
-// (single-grid transforms; box b's particle arrays and state).
-// 2LPT initial conditions of box bx (displacement_fields, src/2LPT.c:185-495,
-// 1209-1519): delta(k) from the Gaussian draw, or, given pos01 (particles in
-// [0,1) of the box, the ReadParticlesFromFile path of
-// src/readICfromfile.c:533-777), from the particles' density; then the 2LPT
-// fields, the lattice read-out and the particle state.
-static int ic_box(mgp_ctx *c, int bx, const double *pos01 = NULL, size_t npos = 0) {
+// 2LPT initial conditions of box bx with cuFFT's 3D plans (displacement_fields,
+// src/2LPT.c:185-495, 1209-1519): delta(k), the 2LPT fields, the lattice
+// read-out and the particle state.
+static int ic_box(mgp_ctx *c, int bx, const double *pos01, size_t npos) {
   const mgp_params *pb = &c->box_p[bx];
   const mgp_cosmo *cb = cosmo_of(c, bx);
   float *dkb = c->dk + (size_t)bx * c->g.nreal;
-  c->dk_planar = c->rho_planar = 0;
   const size_t po = (size_t)bx * 3 * c->np;
-  const int N = c->g.N, Ns = c->Ns, h = N / 2;
+  const int N = c->g.N, Ns = c->Ns;
   const double box = pb->Box;
-  // cube cut of 2LPT.c:383-386 with the reference's double expression: the
-  // largest |d| it keeps
-  int kc = Ns / 2 < h ? Ns / 2 : h;
-  {
-    const double kv = kc * 2 * 3.14159265358979323846 / box;
-    if (fabs(kv) * box / (2 * 3.14159265358979323846) > Ns / 2) kc--;
-  }
-  const int namp = 3 * (Ns / 2 < h ? (Ns / 2) * (Ns / 2) : h * h) + 1;  // |k|^2 up to the cut
-  float *g6 = NULL;
-  int rc = MGP_OK;
+  int namp;
+  const int kc = ic_cut(c, &namp);
   const long long gf = c->g.nreal;
-  const double Di = mgp_cosmo_growth(cb, 0, 1.0 / (1.0 + pb->Init_Redshift));
-  const double Di2 = mgp_cosmo_growth(cb, 3, 1.0 / (1.0 + pb->Init_Redshift));
+  const double ai = 1.0 / (1.0 + pb->Init_Redshift);
+  const double Di = mgp_cosmo_growth(cb, 0, ai), Di2 = mgp_cosmo_growth(cb, 3, ai);
   // without COLA the particles start with the 2LPT velocity (main.c:276-283)
-  const double vD = pb->UseCOLA ? 0.0 : mgp_cosmo_growth(cb, 1, 1.0 / (1.0 + pb->Init_Redshift));
-  const double vD2 = pb->UseCOLA ? 0.0 : mgp_cosmo_growth(cb, 4, 1.0 / (1.0 + pb->Init_Redshift));
+  const double vD = pb->UseCOLA ? 0.0 : mgp_cosmo_growth(cb, 1, ai);
+  const double vD2 = pb->UseCOLA ? 0.0 : mgp_cosmo_growth(cb, 4, ai);
   const int nblk = mgp_ikd_blocks(c->np);
-#define CK(x)                      \
-  do {                             \
-    rc = (x);                      \
-    if (rc != MGP_OK) goto cleanup; \
-  } while (0)
-#define CKC(x)                                                                                           \
-  do {                                                                                                   \
-    cudaError_t e_ = (x);                                                                                \
-    if (e_ != cudaSuccess) {                                                                             \
-      rc = mgp_set_error(MGP_ECUDA, "%s:%d %s: %s", __FILE__, __LINE__, #x, cudaGetErrorString(e_));   \
-      goto cleanup;                                                                                      \
-    }                                                                                                    \
-  } while (0)
-#define CKF(x)                                                                                         \
-  do {                                                                                                 \
-    cufftResult r_ = (x);                                                                              \
-    if (r_ != CUFFT_SUCCESS) {                                                                         \
-      rc = mgp_set_error(MGP_ECUFFT, "%s:%d %s: cufft error %d", __FILE__, __LINE__, #x, (int)r_);   \
-      goto cleanup;                                                                                    \
-    }                                                                                                  \
-  } while (0)
   // six scratch grids for the displacement gradients and the six
   // displacement fields (2LPT.c:1214-1219, 1300-1306), kept by the context
   // for its next IC (runs of many ICs -- the boxes of a batch, repeated
   // runs -- allocate them once)
-  if (!c->ic_scratch) CKC(cudaMalloc(&c->ic_scratch, sizeof(float) * 6 * (size_t)gf));
-  g6 = c->ic_scratch;
-  if (pos01) {
-    // the particles' CIC density at a_i as the LCDM linear field, brought to
-    // a = 1 (readICfromfile.c:640-676), deconvolved and rescaled (701-777)
-    const int rkmax = 3 * h * h;
-    std::vector<double> gcw(h + 1), resc(rkmax + 1), kk(rkmax + 1);
-    for (int rk = 0; rk <= rkmax; rk++) kk[rk] = 2.0 * M_PI / box * sqrt((double)rk);
-    for (int d = 0; d <= h; d++) {
-      const double x = M_PI * d / (double)N, sc = d == 0 ? 1.0 : sin(x) / x;
-      gcw[d] = 1.0 / (sc * sc);
-    }
-    {
-      std::vector<double> r2(rkmax + 1, 1.0);
-      mgp_cosmo_pofk_ratio_many(cb, 1.0, rkmax, kk.data() + 1, r2.data() + 1);
-      const double s8 = pb->input_sigma8_is_for_lcdm ? 1.0 : mgp_cosmo_sigma8_enh(cb, 1.0);
-      for (int rk = 0; rk <= rkmax; rk++) resc[rk] = sqrt(r2[rk]) / s8;
-    }
-    const double normfac = 1.0 / ((double)N * N * N) / mgp_cosmo_growth(cb, 6, 1.0 / (1.0 + pb->Init_Redshift));
-    struct dbuf {  // freed on every exit from this block
-      double *p = NULL;
-      ~dbuf() {
-        if (p) cudaFree(p);
-      }
-    } b_pos, b_gc, b_resc;
-    CKC(cudaMalloc(&b_pos.p, sizeof(double) * 3 * npos));
-    CKC(cudaMalloc(&b_gc.p, sizeof(double) * gcw.size()));
-    CKC(cudaMalloc(&b_resc.p, sizeof(double) * resc.size()));
-    double *d_pos = b_pos.p, *d_gc = b_gc.p, *d_resc = b_resc.p;
-    CKC(cudaMemcpyAsync(d_pos, pos01, sizeof(double) * 3 * npos, cudaMemcpyHostToDevice, c->stream));
-    CKC(cudaMemcpyAsync(d_gc, gcw.data(), sizeof(double) * gcw.size(), cudaMemcpyHostToDevice, c->stream));
-    CKC(cudaMemcpyAsync(d_resc, resc.data(), sizeof(double) * resc.size(), cudaMemcpyHostToDevice, c->stream));
-    rc = mgp_launch_fill(c->rho, gf, -1.0f, c->stream);
-    if (rc == MGP_OK)
-      rc = mgp_launch_cic_unit(d_pos, (long long)npos, N, c->g.P, (float)pow((double)N / Ns, 3), c->rho, c->stream);
-    if (rc == MGP_OK && cufftExecR2C(c->plan_r2c_oop, (cufftReal *)c->rho, (cufftComplex *)dkb) != CUFFT_SUCCESS)
-      rc = mgp_set_error(MGP_ECUFFT, "IC density transform");
-    if (rc == MGP_OK) rc = mgp_launch_ic_from_density(dkb, N, Ns, normfac, d_gc, d_resc, c->stream);
-    cudaStreamSynchronize(c->stream);
-    if (rc != MGP_OK) goto cleanup;
-  } else {
-    CK(ic_amplitudes(c, pb, cb, namp));
-    CK(mgp_launch_ic_delta((uint32_t)pb->Seed, c->ic_amp, N, Ns, kc, box, pb->amplitude_fixed_initial_condition,
-                           pb->inverted_initial_condition, pb->SphereMode == 1, dkb, c->stream));
-  }
-  CK(mgp_launch_ic_grad6(dkb, g6, gf, N, c->stream));
-  for (int g = 0; g < 3; g++) CKF(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)(g6 + g * gf), (cufftReal *)(g6 + g * gf)));
-  for (int g = 3; g < 6; g++) CKF(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)(g6 + g * gf), (cufftReal *)(g6 + g * gf)));
-  CK(mgp_launch_ic_source(g6, gf, N, c->g.P, c->stream));
-  CKF(cufftExecR2C(c->plan_r2c_ip, (cufftReal *)(g6 + 3 * gf), (cufftComplex *)(g6 + 3 * gf)));
-  if (c->sd) {
-    // SCALEDEPENDENT: keep delta(k) and the source (2LPT.c:1336-1344), then
-    // x = q + D + D2 and v = dDdy + dD2dy (or 0) at a_i (main.c:244-307)
-    const double Ai = 1.0 / (1.0 + c->p.Init_Redshift);
-    const int types[2] = {MGP_FIELD_D, MGP_FIELD_dDdy};
-    CK(mgp_sd_store(c, c->dk, g6 + 3 * gf));
-    CK(mgp_sd_fields(c, Ai, Ai, 2, types));
-    CK(mgp_sd_init_particles(c));
-    CKC(cudaMemsetAsync(c->dstate, 0, sizeof(mgp_dstate), c->stream));
-    CKC(cudaStreamSynchronize(c->stream));
-    c->have_density = c->have_forces = 0;
-    goto cleanup;
-  }
-  CK(mgp_launch_ic_disp(dkb, g6 + 3 * gf, g6, gf, N, box, c->stream));
-  for (int g = 0; g < 3; g++) CKF(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)(g6 + g * gf), (cufftReal *)(g6 + g * gf)));
-  for (int g = 3; g < 6; g++) CKF(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)(g6 + g * gf), (cufftReal *)(g6 + g * gf)));
-  CK(mgp_launch_ic_readout(g6, gf, N, c->g.P, Ns, c->D1 + po, c->D2 + po, c->partials, nblk, c->stream));
-  CK(mgp_launch_ic_finish(c->D1 + po, c->D2 + po, c->s + po, c->v + po, c->np, c->partials, nblk, (float)Di,
-                          (float)Di2, (float)vD, (float)vD2, c->stream));
-  c->lpt_ver++;  // new D1/D2
-  CKC(cudaMemsetAsync(c->dstate + bx, 0, sizeof(mgp_dstate), c->stream));
-  CKC(cudaStreamSynchronize(c->stream));
+  if (!c->ic_scratch) MGP_CUDA(cudaMalloc(&c->ic_scratch, sizeof(float) * 6 * (size_t)gf));
+  float *g6 = c->ic_scratch;
+  if (pos01)
+    RET_IF(ic_density(c, pos01, npos, false));
+  else
+    RET_IF(mgp_launch_ic_delta(c->ic_box + bx, 1, c->ic_amp + (size_t)bx * namp, namp, N, Ns, kc, box, dkb, gf, 0,
+                               c->stream));
+  RET_IF(mgp_launch_ic_grad6(dkb, g6, gf, N, c->stream));
+  for (int g = 0; g < 6; g++)
+    MGP_CUFFT(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)(g6 + g * gf), (cufftReal *)(g6 + g * gf)));
+  RET_IF(mgp_launch_ic_source(g6, gf, N, c->g.P, c->stream));
+  MGP_CUFFT(cufftExecR2C(c->plan_r2c_ip, (cufftReal *)(g6 + 3 * gf), (cufftComplex *)(g6 + 3 * gf)));
+  if (c->sd) return ic_sd(c, g6 + 3 * gf, 0);
+  RET_IF(mgp_launch_ic_disp(dkb, g6 + 3 * gf, g6, gf, N, box, c->stream));
+  for (int g = 0; g < 6; g++)
+    MGP_CUFFT(cufftExecC2R(c->plan_c2r_1, (cufftComplex *)(g6 + g * gf), (cufftReal *)(g6 + g * gf)));
+  RET_IF(mgp_launch_ic_readout(g6, gf, N, c->g.P, Ns, c->D1 + po, c->D2 + po, c->partials, nblk, c->stream));
+  return mgp_launch_ic_finish(c->D1 + po, c->D2 + po, c->s + po, c->v + po, c->np, c->partials, nblk, (float)Di,
+                              (float)Di2, (float)vD, (float)vD2, c->stream);
+}
+
+// displacement_fields + the particle assignment of main.c:231-309 for every box of
+// the context: delta(k) from the Gaussian draw, or, given pos01 (one box), from
+// those particles' density (the ReadParticlesFromFile path,
+// src/readICfromfile.c:533-777).  With the transforms of mgp_fft.cu where the
+// lattice points are mesh points and the lattice size has them too.
+static int ic_boxes(mgp_ctx *c, const double *pos01, size_t npos) {
+  const int N = c->g.N, Ns = c->Ns;
+  // the IC writes every particle array in lattice order
+  c->permuted = 0;
+  c->tile_ready = 0;
+  c->dk_planar = c->rho_planar = 0;
   c->have_density = c->have_forces = 0;
-cleanup:
-  (void)g6;  // the context's IC scratch, freed by mgp_destroy
-#undef CK
-#undef CKC
-#undef CKF
-  return rc;
+  if (own_fft(c) && (N == Ns || (N % Ns == 0 && mgp_fft_has(Ns)))) {
+    RET_IF(ic_own(c, pos01, npos));
+  } else {
+    int namp;
+    ic_cut(c, &namp);
+    RET_IF(ic_prepare(c, namp, pos01 == NULL));
+    for (int b = 0; b < c->nbox; b++) RET_IF(ic_box(c, b, pos01, npos));
+  }
+  c->lpt_ver++;  // new D1/D2
+  MGP_CUDA(cudaMemsetAsync(c->dstate, 0, sizeof(mgp_dstate) * c->nbox, c->stream));
+  MGP_CUDA(cudaStreamSynchronize(c->stream));
+  return MGP_OK;
 }
 
 extern "C" int mgp_displacement_fields(mgp_ctx *c) {
   if (!c) return mgp_set_error(MGP_EINVAL, "null context");
   if (c->nbox != 1) return mgp_set_error(MGP_ESTATE, "single-box call on a batch of %d boxes", c->nbox);
   MGP_CUDA(cudaSetDevice(c->device));
-  // the IC writes every particle array in lattice order
-  c->permuted = 0;
-  c->tile_ready = 0;
   if (c->p.ReadParticlesFromFile) {
     // ReadFilesMakeDisplacementField (src/readICfromfile.c:533-699)
     double *pos = NULL;
     size_t n = 0;
     RET_IF(mgp_read_particle_files(&c->p, &pos, &n));
-    const int rc = ic_box(c, 0, pos, n);
+    const int rc = ic_boxes(c, pos, n);
     free(pos);
     return rc;
   }
-  return ic_box(c, 0);
+  return ic_boxes(c, NULL, 0);
 }
 
 // The same from particles held by the caller: positions in Mpc/h, [n][3],
@@ -772,9 +810,6 @@ extern "C" int mgp_displacement_fields_from_positions(mgp_ctx *c, const double *
   if (!c || (!pos && n)) return mgp_set_error(MGP_EINVAL, "null argument");
   if (c->nbox != 1) return mgp_set_error(MGP_ESTATE, "single-box call on a batch of %d boxes", c->nbox);
   MGP_CUDA(cudaSetDevice(c->device));
-  // the IC writes every particle array in lattice order
-  c->permuted = 0;
-  c->tile_ready = 0;
   std::vector<double> u(3 * n);
   const double inv = 1.0 / c->p.Box;
   for (size_t q = 0; q < 3 * n; q++) {
@@ -783,7 +818,7 @@ extern "C" int mgp_displacement_fields_from_positions(mgp_ctx *c, const double *
     if (x >= 1.0) x = 0.0;
     u[q] = x;
   }
-  return ic_box(c, 0, u.data(), n);
+  return ic_boxes(c, u.data(), n);
 }
 
 // ------------------------------------------------------------ PM step
@@ -945,7 +980,8 @@ static int nu_prepare(mgp_ctx *c, double A) {
 // which the MG solver reads from the total field.
 static int add_neutrinos(mgp_ctx *c, double A, int fuse_kind) {
   if (!c->sd_dk[0]) return mgp_set_error(MGP_ESTATE, "massive neutrinos need the scale-dependent IC field");
-  RET_IF(mgp_launch_nu_add(c->dk, c->sd_dk[0], c->g.N, c->nu_cdmfac, c->nu_tab_d, c->dk_planar, c->stream));
+  RET_IF(mgp_launch_nu_add(c->dk, c->sd_dk[0], c->g.N, c->nu_cdmfac, c->nu_tab_d, c->dk_planar, c->sd_planar,
+                           c->stream));
   if (c->p.pofk_compute_every_step) {
     if (!c->pk_sum_tot) MGP_CUDA(cudaMalloc(&c->pk_sum_tot, sizeof(double) * c->pk_nbins));
     RET_IF(pofk_now(c, fuse_kind, A, c->pk_sum_tot));
@@ -1545,7 +1581,7 @@ extern "C" int mgp_copy_grid(mgp_ctx *c, int which, float *host, size_t count) {
   }
   if (!src) return mgp_set_error(MGP_ESTATE, "grid %d is not allocated", which);
   if ((long long)count > c->g.nreal) return mgp_set_error(MGP_EINVAL, "count %zu exceeds grid size", count);
-  if ((which == 1 && c->dk_planar) || ((which == 0 || which == 5) && c->rho_planar)) {
+  if ((which == 1 && c->dk_planar) || ((which == 0 || which == 5) && c->rho_planar) || (which == 7 && c->sd_planar)) {
     // a planar spectrum, rearranged by up to 64 MB of x planes at a time
     const int N = c->g.N;
     const size_t plane = (size_t)c->g.N * c->g.P;
@@ -1793,12 +1829,9 @@ extern "C" int mgp_batch_run(mgp_ctx *c, int nsteps, double z_final) {
     MGP_CUDA(cudaEventCreate(&c->bev[1]));
   }
   if (c->sd) return mgp_set_error(MGP_EINVAL, "batch runs use scale-independent growth");
-  // 2LPT ICs of every box (not captured: host-side seed tables), written
-  // in lattice order
-  c->permuted = 0;
-  c->tile_ready = 0;
+  // 2LPT ICs of every box (not captured), written in lattice order
   MGP_CUDA(cudaEventRecord(c->bev[0], c->stream));
-  for (int b = 0; b < c->nbox; b++) RET_IF(ic_box(c, b));
+  RET_IF(ic_boxes(c, NULL, 0));
   MGP_CUDA(cudaEventRecord(c->bev[1], c->stream));
   MGP_CUDA(cudaEventSynchronize(c->bev[1]));
   MGP_CUDA(cudaEventElapsedTime(&c->batch_ic_ms, c->bev[0], c->bev[1]));

@@ -100,12 +100,10 @@ int mgp_fft_setup(mgp_ctx *c) {
 }
 
 void mgp_fft_free(mgp_ctx *c) {
-  if (c->fft_scr && c->nbox > 1) cudaFree(c->fft_scr);
-  c->fft_scr = NULL;
-  float *b[] = {c->fft_tw, c->fft_tw_s, c->fft_gauss};
+  float *b[] = {c->fft_tw, c->fft_tw_s, c->fft_gauss, c->fft_scr};
   for (float *p : b)
     if (p) cudaFree(p);
-  c->fft_tw = c->fft_tw_s = c->fft_gauss = NULL;
+  c->fft_tw = c->fft_tw_s = c->fft_gauss = c->fft_scr = NULL;
 }
 
 // ---------------------------------------------------------------- passes
@@ -223,14 +221,8 @@ int mgp_fft_planar_rows(int N, const float *in, float *out, int x0, int x1, cuda
   return MGP_OK;
 }
 
-// Scratch spectra of the field passes: three per box (a single box shares the
-// IC's grids).
+// Scratch spectra of the field passes and the IC: three per box.
 int mgp_fft_scratch(mgp_ctx *c) {
-  if (c->nbox == 1 && c->g.nreal) {
-    if (!c->ic_scratch) MGP_CUDA(cudaMalloc(&c->ic_scratch, sizeof(float) * 6 * (size_t)c->g.nreal));
-    c->fft_scr = c->ic_scratch;
-    return MGP_OK;
-  }
   if (!c->fft_scr) MGP_CUDA(cudaMalloc(&c->fft_scr, sizeof(float) * 3 * (size_t)c->g.nreal * c->nbox));
   return MGP_OK;
 }
@@ -339,25 +331,124 @@ int mgp_fft_force_x(mgp_ctx *c, const mgp_fft_plan *f) {
   return MGP_OK;
 }
 
-int mgp_fft_force_y(mgp_ctx *c) {
-  const passes p(c, c->g.N);
-  float2 *f0 = (float2 *)scr(c, 0), *f1 = (float2 *)scr(c, 1), *f2 = (float2 *)scr(c, 2);
+// y pass of the force fields f[0] (kx G) and f[2] (G) after their x lines
+static mgp_fft_y force_y_args(float2 *const *f) {
   mgp_fft_y a;
   memset(&a, 0, sizeof(a));
   a.ntask = 2;
-  a.task[0].in = f0;
-  a.task[0].out[0] = f0;
+  a.task[0].in = f[0];
+  a.task[0].out[0] = f[0];
   a.task[0].nout = 1;
-  a.task[1].in = f2;  // inverse x transform of G: F_y = ky G, F_z = kz G
-  a.task[1].out[0] = f1;
+  a.task[1].in = f[2];  // inverse x transform of G: F_y = ky G, F_z = kz G
+  a.task[1].out[0] = f[1];
   a.task[1].ypow[0] = 1;
-  a.task[1].out[1] = f2;
+  a.task[1].out[1] = f[2];
   a.task[1].zpow[1] = 1;
   a.task[1].nout = 2;
-  return p.y(1, 1, a, 3 * c->g.nreal, c->nbox);
+  return a;
+}
+
+int mgp_fft_force_y(mgp_ctx *c) {
+  const passes p(c, c->g.N);
+  float2 *f[3] = {(float2 *)scr(c, 0), (float2 *)scr(c, 1), (float2 *)scr(c, 2)};
+  return p.y(1, 1, force_y_args(f), 3 * c->g.nreal, c->nbox);
 }
 
 int mgp_fft_force_z(mgp_ctx *c) {
   const passes p(c, c->g.N);
   return p.z_c2r(scr(c, 0), c->frc, c->g.nreal, 3 * c->nbox);
+}
+
+// The 2LPT source's spectrum in rho from delta(k) in dk (src/2LPT.c:1224-1290),
+// both planar, for all boxes: three inverse x transforms of -delta / k^2 times 1,
+// kx, kx^2, from them six y transforms of the gradients, then one row pass that
+// inverts the six rows, forms the source and transforms it forward.  delta is
+// zero beyond |k| <= kc: columns and tiles beyond it are skipped (at Nmesh = 2
+// Nsample a quarter of the x columns and half of the y columns are left).
+// Gradients 00, 01, 02 in the force grids, 11, 12, 22 in the scratch spectra.
+int mgp_fft_ic_source(mgp_ctx *c, int kc) {
+  const passes p(c, c->g.N);
+  const int n = c->nbox;
+  const long long gs = c->g.nreal;
+  RET_IF(mgp_fft_scratch(c));
+  float2 *g[6];
+  for (int q = 0; q < 6; q++) g[q] = (float2 *)((q < 3 ? c->frc : c->fft_scr) + (q % 3) * gs);
+  mgp_fft_x x = x_args(c->dk, gs);
+  x.o[0] = g[5];
+  x.o[1] = g[2];
+  x.o[2] = g[0];
+  x.bs_o = 3 * gs / 2;
+  x.kc = kc;
+  RET_IF(p.x(0, MGP_X_IC, x, n));
+  mgp_fft_y y;
+  memset(&y, 0, sizeof(y));
+  y.ntask = 3;
+  y.neg = 1;
+  y.task[0].in = y.task[0].out[0] = g[0];
+  y.task[0].nout = 1;
+  y.task[1].in = g[2];
+  y.task[1].out[0] = g[1];
+  y.task[1].ypow[0] = 1;
+  y.task[1].out[1] = g[2];
+  y.task[1].zpow[1] = 1;
+  y.task[1].nout = 2;
+  y.task[2].in = g[5];
+  y.task[2].out[0] = g[3];
+  y.task[2].ypow[0] = 2;
+  y.task[2].out[1] = g[4];
+  y.task[2].ypow[1] = y.task[2].zpow[1] = 1;
+  y.task[2].out[2] = g[5];
+  y.task[2].zpow[2] = 2;
+  y.task[2].nout = 3;
+  RET_IF(p.y(1, 1, y, 3 * gs, n, kc));
+  mgp_fft_z z;
+  memset(&z, 0, sizeof(z));
+  for (int q = 0; q < 6; q++) z.grad[q] = g[q];
+  z.out = (float2 *)c->rho;
+  z.rows = p.rows(n);
+  z.bs_in = 3 * gs / 2;
+  z.bs_out = gs / 2;
+  z.kc = kc;
+  RET_IF(p.z(MGP_Z_SOURCE, z));
+  RET_IF(p.y(-1, c->rho, gs, n));
+  c->rho_planar = 1;
+  return p.x(1, MGP_X_NONE, x_args(c->rho, gs), n);
+}
+
+// The particles' D1, D2, s and v from delta(k) in dk and the 2LPT source in rho.
+int mgp_fft_ic_fields(mgp_ctx *c) {
+  const int N = c->g.N, Ns = c->Ns, n = c->nbox;
+  const long long gs = c->g.nreal;
+  const float mult = (float)(-3.0 / 7.0 / ((double)N * N * N));
+  // D1: three cuFFT transforms in the force grids
+  RET_IF(mgp_launch_ic_za(c->dk, c->frc, gs, N, c->p.Box, n, c->stream));
+  for (int g = 0; g < 3; g++)
+    MGP_CUFFT(cufftExecC2R(n > 1 ? c->plan_c2r_frc_b : c->plan_c2r_1, (cufftComplex *)(c->frc + g * gs),
+                           (cufftReal *)(c->frc + g * gs)));
+  RET_IF(mgp_launch_ic_take(c->frc, 3 * gs, gs, N, N / Ns, Ns, c->np, c->ic_box, n, 0, 1.0f, c->D1, c->D2, c->s, c->v,
+                            c->stream));
+  if (N != Ns) {
+    // three lattice grids a box, from the scratch spectra to the force grids
+    const long long ls = (long long)Ns * Ns * (Ns + 2);
+    RET_IF(mgp_launch_ic_fold(c->rho, gs, N, Ns, c->p.Box, c->fft_scr, ls, n, c->stream));
+    RET_IF(mgp_fft_c2r(c, Ns, c->fft_scr, c->frc, 3 * n, ls));
+    return mgp_launch_ic_take(c->frc, 3 * ls, ls, Ns, 1, Ns, c->np, c->ic_box, n, 1, mult, c->D1, c->D2, c->s, c->v,
+                              c->stream);
+  }
+  // the force pass's x and y passes with g = -Box/2pi / k^2 on the source
+  const passes p(c, N);
+  float2 *f[3] = {(float2 *)c->frc, (float2 *)(c->frc + gs), (float2 *)(c->frc + 2 * gs)};
+  mgp_fft_x x = x_args(c->rho, gs);
+  x.o[0] = f[0];
+  x.o[1] = f[2];
+  x.bs_o = 3 * gs / 2;
+  x.cfac = (float)(-c->p.Box / (2.0 * M_PI));
+  x.neg = 1;
+  RET_IF(p.x(0, MGP_X_FORCE, x, n));
+  mgp_fft_y y = force_y_args(f);
+  y.neg = 1;
+  RET_IF(p.y(1, 1, y, 3 * gs, n));
+  RET_IF(p.z_c2r(c->frc, c->fft_scr, gs, 3 * n));
+  return mgp_launch_ic_take(c->fft_scr, 3 * gs, gs, N, 1, Ns, c->np, c->ic_box, n, 1, mult, c->D1, c->D2, c->s, c->v,
+                            c->stream);
 }

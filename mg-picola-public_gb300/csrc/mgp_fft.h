@@ -24,6 +24,7 @@ typedef struct {
   float cfac, coupling, mass2;
   const mgp_box_scalars *bs;
   int kc;
+  int neg; /* X_FORCE: wave number -N/2 at the Nyquist index (the IC's convention), else +N/2 */
 } mgp_fft_x;
 
 typedef struct {
@@ -37,12 +38,13 @@ typedef struct {
   int ntask, nbox;
   long long bs;
   const float2 *tw;
-  int kc;
+  int kc, neg;
 } mgp_fft_y;
 
 /* z rows; strides between grids in float2 */
 typedef struct {
   const float2 *in;             /* real (Z_R2C) or spectra */
+  const float2 *grad[6];        /* Z_SOURCE: the gradient spectra of a box, bs_in to the next */
   float2 *out;                  /* spectra */
   float2 *real;                 /* real rows written */
   const float2 *rho;            /* Z_SCREEN: the density */

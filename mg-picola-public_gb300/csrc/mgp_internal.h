@@ -53,6 +53,14 @@ typedef struct {
   float pref;                       /* density-screening prefactor */
 } mgp_box_scalars;
 
+/* What the IC kernels need of a box. */
+typedef struct {
+  uint32_t seed;
+  int fixed, inverted, sphere;
+  double norm, fac;         /* of the analytic spectrum: amplitude, k-independent rescaling */
+  float Di, Di2, vD, vD2;   /* initial displacement and velocity per unit of D1, D2 */
+} mgp_ic_box;
+
 struct mgp_ctx {
   mgp_params p;
   mgp_cosmo cosmo;
@@ -79,7 +87,8 @@ struct mgp_ctx {
   /* grids */
   float *rho, *dk, *frc, *mg1;
   float *ic_scratch;        /* six grids for the 2LPT IC (lazy, kept for the next IC) */
-  double *ic_amp;           /* device: amplitude per integer |k|^2 up to the IC's mode cut (lazy), then a growth column */
+  double *ic_amp;           /* device: per box the amplitude per integer |k|^2 up to the IC's mode cut, then a growth column (lazy) */
+  mgp_ic_box *ic_box;       /* device: per box (lazy) */
   void *fft_work;
   size_t fft_work_bytes;
   cufftHandle plan_r2c_oop, plan_r2c_ip, plan_c2r_1;
@@ -89,7 +98,7 @@ struct mgp_ctx {
    * Gaussian smoothing factor per stored index */
   int fft_mode;
   float *fft_tw, *fft_tw_s, *fft_gauss;
-  float *fft_scr;           /* scratch spectra (lazy): the IC's grids, or a batch's own */
+  float *fft_scr;           /* scratch spectra, three a box (lazy) */
   int dk_planar, rho_planar; /* dk / rho hold a spectrum in the planar layout of mgp_fft.cuh */
 
   /* P(k) */
@@ -133,7 +142,8 @@ struct mgp_ctx {
                                not a multiple of Nsample (full-mesh path) */
   float *sd_full;           /* full-mesh path: one padded real N^3 grid */
   double *sd_part;          /* full-mesh path: read-out partial sums */
-  float *sd_dk[2];          /* delta(k), -source(k): complex [N][N][NH] */
+  float *sd_dk[2];          /* delta(k), -source(k): complex [N][N][NH], or planar (mgp_fft.cuh) */
+  int sd_planar;
   float *sd_slot[3];        /* 3 components x sd_grid floats each */
   long long sd_grid;        /* Ns*Ns*Ps floats */
   int sd_pitch;             /* Ps */
@@ -311,6 +321,8 @@ void mgp_fft_free(mgp_ctx *c);
 int mgp_fft_scratch(mgp_ctx *c);
 int mgp_fft_r2c(mgp_ctx *c, const float *in, float *out, int n, long long gs);
 int mgp_fft_c2r(mgp_ctx *c, int N, float *in, float *out, int n, long long gs);
+int mgp_fft_ic_source(mgp_ctx *c, int kc);
+int mgp_fft_ic_fields(mgp_ctx *c);
 int mgp_fft_planar_rows(int N, const float *in, float *out, int x0, int x1, cudaStream_t st);
 int mgp_fft_density(mgp_ctx *c, const mgp_fft_plan *f);
 int mgp_fft_screen(mgp_ctx *c, const mgp_fft_plan *f, int (*user)(mgp_ctx *, const mgp_fft_plan *));
@@ -330,7 +342,7 @@ int mgp_sd_alloc(mgp_ctx *c);
 void mgp_sd_free(mgp_ctx *c);
 /* keep delta(k) and the complex 2LPT source S(k) of the IC (stored as
  * delta and -S, src/2LPT.c:301-309, 1336-1344) */
-int mgp_sd_store(mgp_ctx *c, const float *deltak, const float *source2k);
+int mgp_sd_store(mgp_ctx *c, const float *deltak, const float *source2k, int planar);
 /* fields of `types` (one per slot) at A (and AFF for deltaD) */
 int mgp_sd_fields(mgp_ctx *c, double A, double AFF, int n, const int *types);
 /* IC particle state from the D (slot 0) and dDdy (slot 2) fields */
@@ -372,10 +384,10 @@ int mgp_particles_canonical(mgp_ctx *c);
 int mgp_launch_nu_table(float *tab, int nrk, double kfac, double fac, const double *x, const double *val,
                         const double *dval, int nx, const double *den, cudaStream_t st);
 int mgp_launch_nu_add(float *dk, const float *dk0, int N, double cdmfac, const float *nufac, int planar,
-                      cudaStream_t st);
+                      int planar0, cudaStream_t st);
 int mgp_launch_cic_unit(const double *pos, long long n, int N, long long P, float wpar, float *rho, cudaStream_t st);
 int mgp_launch_ic_from_density(float *dk, int N, int Ns, double normfac, const double *gc, const double *rescale,
-                               cudaStream_t st);
+                               int planar, cudaStream_t st);
 long long mgp_kernel_launches(void);
 
 /* MG real-space and k-space passes */
@@ -394,10 +406,16 @@ int mgp_launch_screen_table(float *rho, const float *arg, long long n, float mul
                             double t0, double dt, cudaStream_t st);
 
 /* IC */
-int mgp_launch_ic_amp(double *amp, int n, double kf, double vol, const mgp_eh_spectrum *e, double fac,
-                      const double *col, int ny, double y0, double dy, double DL, cudaStream_t st);
-int mgp_launch_ic_delta(uint32_t seed, const double *amp_rk, int N, int Ns, int kc, double box, int fixed, int inverted,
-                        int sphere, float *dk, cudaStream_t st);
+int mgp_launch_ic_amp(double *amp, int n, double kf, double vol, const mgp_eh_spectrum *e, const mgp_ic_box *boxes,
+                      int nbox, const double *col, int ny, double y0, double dy, double DL, cudaStream_t st);
+int mgp_launch_ic_delta(const mgp_ic_box *boxes, int nbox, const double *amp_rk, int namp, int N, int Ns, int kc,
+                        double box, float *dk, long long g_bs, int planar, cudaStream_t st);
+int mgp_launch_ic_za(const float *dk, float *out, long long gs, int N, double box, int nbox, cudaStream_t st);
+int mgp_launch_ic_fold(const float *src, long long g_bs, int N, int Ns, double box, float *out, long long out_gs,
+                       int nbox, cudaStream_t st);
+int mgp_launch_ic_take(const float *g, long long bs, long long gs, int n, int step, int Ns, long long np,
+                       const mgp_ic_box *boxes, int nbox, int second, float mult, float *D1, float *D2, float *s,
+                       float *v, cudaStream_t st);
 int mgp_launch_ic_grad6(const float *dk, float *out6, long long grid_floats, int N, cudaStream_t st);
 int mgp_launch_ic_source(float *g6, long long grid_floats, int N, long long P, cudaStream_t st);
 int mgp_launch_ic_disp(const float *dk, const float *src, float *out6, long long grid_floats, int N, double box,

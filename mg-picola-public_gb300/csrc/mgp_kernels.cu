@@ -214,7 +214,9 @@ struct mgp_pofk_kargs {
 // array; hi + lo carries about twice FP32's precision.
 // priv != 0: every warp owns its own hi/lo bin arrays (the run tails of one
 // warp always hit distinct bins), so the sums need no atomics at all.
-__global__ void __launch_bounds__(MGP_THREADS) k_pofk(mgp_pofk_kargs a) {
+// Four blocks an SM (64 registers): the launch has four, and a fourth that waits
+// for a slot doubles the pass (0.97 -> 1.53 ms at 1024^3 with 78 registers).
+__global__ void __launch_bounds__(MGP_THREADS, 4) k_pofk(mgp_pofk_kargs a) {
   extern __shared__ float shf[];
   const int N = a.N, nbins = a.nbins, NH = N / 2 + 1, h = N / 2;
   const float2 *__restrict__ dkb = a.dk + blockIdx.y * a.dk_bs;
@@ -246,22 +248,22 @@ __global__ void __launch_bounds__(MGP_THREADS) k_pofk(mgp_pofk_kargs a) {
     const int rk01 = d0 * d0 + d1 * d1;
     const float w01 = swin[d0] * swin[d1];
     const bool mi = !(d0 == 0 || d0 == h), mj = !(d1 == 0 || d1 == h);
-    const long long rows[4] = {(long long)d0 * N + d1, (long long)d0 * N + (N - d1), (long long)(N - d0) * N + d1,
-                               (long long)(N - d0) * N + (N - d1)};
     const bool use[4] = {true, mj, mi, mi && mj};
-    // offsets of kz = 0 and of kz = N/2 of every row
-    long long r0[4], rl[4];
+    // row (i, j): its kz = 0 value, and the distance to its kz = N/2 value
+    const float2 *row[4];
+    long long last[4];
 #pragma unroll
     for (int t = 0; t < 4; t++) {
-      const long long i = t < 2 ? d0 : N - d0, j = rows[t] - i * N, plane = i * ((long long)N * NH);
-      r0[t] = a.planar ? plane + j * h : rows[t] * NH;
-      rl[t] = a.planar ? plane + (long long)N * h + j : r0[t] + h;
+      const int i = t < 2 ? d0 : N - d0, j = t & 1 ? N - d1 : d1;
+      const long long plane = (long long)i * N * NH;
+      row[t] = dkb + (a.planar ? plane + (long long)j * h : plane + (long long)j * NH);
+      last[t] = a.planar ? (long long)(N - j) * h + j : h;
     }
     // the rows' next 32 modes are loaded while the current ones are binned
     float2 zn[4];
 #pragma unroll
     for (int t = 0; t < 4; t++)
-      if (use[t] && lane < NH) zn[t] = dkb[lane == h ? rl[t] : r0[t] + lane];
+      if (use[t] && lane < NH) zn[t] = row[t][lane == h ? last[t] : lane];
     for (int k0 = 0; k0 < NH; k0 += 32) {
       const int kz = k0 + lane;
       float2 z[4];
@@ -270,7 +272,7 @@ __global__ void __launch_bounds__(MGP_THREADS) k_pofk(mgp_pofk_kargs a) {
       if (kz + 32 < NH) {
 #pragma unroll
         for (int t = 0; t < 4; t++)
-          if (use[t]) zn[t] = dkb[kz + 32 == h ? rl[t] : r0[t] + kz + 32];
+          if (use[t]) zn[t] = row[t][kz + 32 == h ? last[t] : kz + 32];
       }
       int bin = -1;
       float pk = 0.0f;
@@ -295,7 +297,7 @@ __global__ void __launch_bounds__(MGP_THREADS) k_pofk(mgp_pofk_kargs a) {
         for (int t = 0; t < 4; t++)
           if (use[t]) {
             p2 += z[t].x * z[t].x + z[t].y * z[t].y;
-            if (a.fuse_kind) fob[rows[t] * NH + kz] = make_float2(f * z[t].x, f * z[t].y);
+            if (a.fuse_kind) fob[(row[t] - dkb) + kz] = make_float2(f * z[t].x, f * z[t].y);
           }
         if (bin >= 0) {
           float w = (kz == 0 || 2 * kz == N) ? 1.0f : 2.0f;
@@ -896,8 +898,12 @@ __device__ __forceinline__ uint32_t ic_column_seed(uint32_t seed, int i, int j, 
 // growth-table column (ny > 0, cubic Hermite in ln k) the rescaling also
 // carries (D(k) / DL)^2.  A host loop over the 3 (Ns/2)^2 values took 20 ms
 // at Nsample 512 (100 ns each).
-__global__ void k_ic_amp(double *__restrict__ amp, int n, double kf, double vol, mgp_eh_spectrum e, double fac,
-                         const double *__restrict__ col, int ny, double y0, double dy, double DL) {
+// Box blockIdx.y has its own normalisation and `fac` and fills its own n values.
+__global__ void k_ic_amp(double *__restrict__ amp, int n, double kf, double vol, mgp_eh_spectrum e,
+                         const mgp_ic_box *__restrict__ boxes, const double *__restrict__ col, int ny, double y0,
+                         double dy, double DL) {
+  amp += (size_t)blockIdx.y * n;
+  const double norm = boxes[blockIdx.y].norm, fac = boxes[blockIdx.y].fac;
   const int stride = gridDim.x * blockDim.x;
   for (int rk = blockIdx.x * blockDim.x + threadIdx.x; rk < n; rk += stride) {
     if (rk == 0) {
@@ -908,7 +914,7 @@ __global__ void k_ic_amp(double *__restrict__ amp, int n, double kf, double vol,
     const double gamma = (e.alpha + (1. - e.alpha) / (1. + exp(4 * log(0.43 * ku * e.s)))) * e.gamma0;
     const double q = ku * e.theta * e.theta / gamma;
     const double L0 = log(2. * exp(1.) + 1.8 * q), C0 = 14.2 + 731. / (1. + 62.5 * q), T = L0 / (L0 + C0 * q * q);
-    double pk = e.norm * pow(k, e.ns) * T * T * fac;
+    double pk = norm * pow(k, e.ns) * T * T * fac;
     if (ny > 0) {
       double t = (log(k) - y0) / dy;
       t = fmin(fmax(t, 0.0), (double)(ny - 1));
@@ -923,9 +929,9 @@ __global__ void k_ic_amp(double *__restrict__ amp, int n, double kf, double vol,
   }
 }
 
-int mgp_launch_ic_amp(double *amp, int n, double kf, double vol, const mgp_eh_spectrum *e, double fac,
-                      const double *col, int ny, double y0, double dy, double DL, cudaStream_t st) {
-  k_ic_amp<<<blocks_for(n, 8), MGP_THREADS, 0, st>>>(amp, n, kf, vol, *e, fac, col, ny, y0, dy, DL);
+int mgp_launch_ic_amp(double *amp, int n, double kf, double vol, const mgp_eh_spectrum *e, const mgp_ic_box *boxes,
+                      int nbox, const double *col, int ny, double y0, double dy, double DL, cudaStream_t st) {
+  k_ic_amp<<<dim3(blocks_for(n, 8), nbox), MGP_THREADS, 0, st>>>(amp, n, kf, vol, *e, boxes, col, ny, y0, dy, DL);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
@@ -944,18 +950,24 @@ int mgp_launch_ic_amp(double *amp, int n, double kf, double vol, const mgp_eh_sp
 // the conjugate of the partner column's first mode.  With the seed table and
 // the amplitudes also made on the device, the whole IC of 256^3 particles on
 // a 512^3 mesh went from 36 to 17 ms (the rest is its transforms).
-__global__ void __launch_bounds__(MGP_THREADS) k_ic_delta(uint32_t seed0, const double *__restrict__ amp_rk, int N,
-                                                          int Ns, int kc, double box, int fixed, int inverted,
-                                                          int sphere, float2 *__restrict__ dk) {
+__global__ void __launch_bounds__(MGP_THREADS) k_ic_delta(const mgp_ic_box *__restrict__ boxes,
+                                                          const double *__restrict__ amp_rk, int namp, int N, int Ns,
+                                                          int kc, double box, float2 *__restrict__ dk, long long bs,
+                                                          int planar) {
   const double twopi = 2 * 3.14159265358979323846;
   const int NH = N / 2 + 1, lane = threadIdx.x & 31;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  const uint32_t seed0 = boxes[blockIdx.y].seed;
+  const int fixed = boxes[blockIdx.y].fixed, inverted = boxes[blockIdx.y].inverted, sphere = boxes[blockIdx.y].sphere;
+  amp_rk += (size_t)blockIdx.y * namp;
+  dk += blockIdx.y * bs;
   const int reach = sphere ? Ns / 2 + 1 : kc;  // no mode beyond it survives the cut
   for (long long row = wid; row < (long long)N * N; row += nw) {
     const int i = (int)(row / N), j = (int)(row - (long long)i * N);
     const int ai = i < N / 2 ? i : N - i, aj = j < N / 2 ? j : N - j;
-    float2 *__restrict__ out = dk + row * NH;
+    float2 *__restrict__ out = planar ? dk + (long long)i * N * NH + (long long)j * (N / 2) : dk + row * NH;
+    float2 *__restrict__ last = planar ? dk + (long long)i * N * NH + (long long)N * (N / 2) + j : out + N / 2;
     const bool dead = 2 * i == N || 2 * j == N || ai > reach || aj > reach;
     const int kend = dead ? 0 : min(N / 2, reach + 1);  // modes kz < kend are drawn
     const uint32_t seed = dead ? 0u : ic_column_seed(seed0, i, j, N);
@@ -965,7 +977,7 @@ __global__ void __launch_bounds__(MGP_THREADS) k_ic_delta(uint32_t seed0, const 
     for (int k0 = 0; k0 < NH; k0 += 32) {
       const int k = k0 + lane;
       if (k0 >= kend) {
-        if (k < NH) out[k] = make_float2(0.f, 0.f);
+        if (k < NH) *(k == N / 2 ? last : out + k) = make_float2(0.f, 0.f);
         continue;
       }
       double phase = 0.0, ampl = 1.0;
@@ -1018,15 +1030,15 @@ __global__ void __launch_bounds__(MGP_THREADS) k_ic_delta(uint32_t seed0, const 
         z = make_float2((float)delta * cs, (float)delta * sn);
         if (k == 0 && mirror) z.y = -z.y;
       }
-      if (k < NH) out[k] = z;
+      if (k < NH) *(k == N / 2 ? last : out + k) = z;
     }
   }
 }
 
-int mgp_launch_ic_delta(uint32_t seed, const double *amp_rk, int N, int Ns, int kc, double box, int fixed, int inverted,
-                        int sphere, float *dk, cudaStream_t st) {
-  k_ic_delta<<<blocks_for((long long)N * N * 32, 8), MGP_THREADS, 0, st>>>(seed, amp_rk, N, Ns, kc, box, fixed, inverted,
-                                                                          sphere, (float2 *)dk);
+int mgp_launch_ic_delta(const mgp_ic_box *boxes, int nbox, const double *amp_rk, int namp, int N, int Ns, int kc,
+                        double box, float *dk, long long g_bs, int planar, cudaStream_t st) {
+  k_ic_delta<<<grid_boxes((long long)N * N * 32, 8, nbox), MGP_THREADS, 0, st>>>(boxes, amp_rk, namp, N, Ns, kc, box,
+                                                                                (float2 *)dk, g_bs / 2, planar);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
@@ -1038,9 +1050,9 @@ int mgp_launch_ic_delta(uint32_t seed, const double *amp_rk, int N, int Ns, int 
 // One warp per (i, j) row of the half-complex grid, lanes along kz; FP32
 // arithmetic (the grids are FP32, and FP64 runs at a small fraction of the
 // FP32 rate on this part).
-// planar: the layout of dk (mgp_fft.cuh).
+// planar, planar0: the layouts of dk and dk0 (mgp_fft.cuh).
 __global__ void k_nu_add(float2 *__restrict__ dk, const float2 *__restrict__ dk0, int N, float cdmfac,
-                         const float *__restrict__ nufac, int planar) {
+                         const float *__restrict__ nufac, int planar, int planar0) {
   const int NH = N / 2 + 1;
   const int lane = threadIdx.x & 31;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1052,9 +1064,10 @@ __global__ void k_nu_add(float2 *__restrict__ dk, const float2 *__restrict__ dk0
     for (int kz = lane; kz < NH; kz += 32) {
       if (r == 0 && kz == 0) continue;
       const long long c0 = r * NH + kz, plane = (long long)i * N * NH;
-      const long long c = !planar ? c0 : (2 * kz == N ? plane + (long long)N * kz + j : plane + (long long)j * (N / 2) + kz);
+      const long long cp = 2 * kz == N ? plane + (long long)N * kz + j : plane + (long long)j * (N / 2) + kz;
+      const long long c = planar ? cp : c0;
       const float f = nufac[r2 + kz * kz];
-      const float2 a = dk[c], b = dk0[c0];
+      const float2 a = dk[c], b = dk0[planar0 ? cp : c0];
       dk[c] = make_float2(fmaf(f, b.x, cdmfac * a.x), fmaf(f, b.y, cdmfac * a.y));
     }
   }
@@ -1096,10 +1109,10 @@ int mgp_launch_nu_table(float *tab, int nrk, double kfac, double fac, const doub
 }
 
 int mgp_launch_nu_add(float *dk, const float *dk0, int N, double cdmfac, const float *nufac, int planar,
-                      cudaStream_t st) {
+                      int planar0, cudaStream_t st) {
   const long long rows = (long long)N * N;
   k_nu_add<<<blocks_for(rows * 32, 8), MGP_THREADS, 0, st>>>((float2 *)dk, (const float2 *)dk0, N, (float)cdmfac,
-                                                             nufac, planar);
+                                                             nufac, planar, planar0);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
@@ -1149,9 +1162,10 @@ int mgp_launch_cic_unit(const double *pos, long long n, int N, long long P, floa
 // three Nyquist planes, whose sign conventions differ between the
 // reference's displacement and gradient passes); the CIC window divided out
 // (gc[|d|] = 1/sinc^2(pi d/N) per axis) and the P(k) rescaling per integer
-// |k|^2; the k = 0 mode zeroed.  In place on [N][N][N/2+1].
+// |k|^2; the k = 0 mode zeroed.  In place on [N][N][N/2+1]
+// (planar: the layout of the transforms of mgp_fft.cuh).
 __global__ void k_ic_from_density(float2 *__restrict__ dk, int N, int Ns, double normfac,
-                                  const double *__restrict__ gc, const double *__restrict__ rescale) {
+                                  const double *__restrict__ gc, const double *__restrict__ rescale, int planar) {
   const int NH = N / 2 + 1;
   const long long n = (long long)N * N * NH;
   const long long cut2 = (long long)(Ns / 2) * (Ns / 2);
@@ -1165,17 +1179,19 @@ __global__ void k_ic_from_density(float2 *__restrict__ dk, int N, int Ns, double
     const bool zero = d2 == 0 || (N > Ns && d2 > cut2) ||
                       (N <= Ns && (2 * i == N || 2 * j == N || 2 * kz == N));
     const double f = zero ? 0.0 : normfac * gc[di] * gc[dj] * gc[kz] * rescale[d2];
-    float2 v = dk[q];
+    const long long plane = (long long)i * N * NH;
+    float2 *z = dk + (!planar ? q : 2 * kz == N ? plane + (long long)N * kz + j : plane + (long long)j * (N / 2) + kz);
+    float2 v = *z;
     v.x = (float)(f * v.x);
     v.y = (float)(f * v.y);
-    dk[q] = v;
+    *z = v;
   }
 }
 
 int mgp_launch_ic_from_density(float *dk, int N, int Ns, double normfac, const double *gc, const double *rescale,
-                               cudaStream_t st) {
+                               int planar, cudaStream_t st) {
   const long long n = (long long)N * N * (N / 2 + 1);
-  k_ic_from_density<<<blocks_for(n, 8), MGP_THREADS, 0, st>>>((float2 *)dk, N, Ns, normfac, gc, rescale);
+  k_ic_from_density<<<blocks_for(n, 8), MGP_THREADS, 0, st>>>((float2 *)dk, N, Ns, normfac, gc, rescale, planar);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
@@ -1283,6 +1299,162 @@ int mgp_launch_ic_disp(const float *dk, const float *src, float *out6, long long
   const long long total = (long long)N * N * (N / 2 + 1);
   k_ic_disp<<<blocks_for(total, 8), MGP_THREADS, 0, st>>>((const float2 *)dk, src, out6, gf, N,
                                                           (float)(box / (2.0 * M_PI)));
+  MGP_CHECK_LAUNCH();
+  g_kernel_launches++;
+  return MGP_OK;
+}
+
+// The ZA displacement spectra Psi_a = i k_a / k^2 delta (src/2LPT.c:406-425) of
+// box blockIdx.y in rows of N/2 + 1 for cuFFT, from a planar delta(k): the
+// expressions of k_ic_disp.  These three transforms stay cuFFT's: a run carries
+// D1 through every step, and a D1 that rounds differently (this library's
+// transforms are nearer to FP64, 2.1e-7 against 2.5e-7 relative rms at
+// 256^3/512^3) moves the float positions of a host-buffer run by units in the
+// last place, which its steps amplify (1.3e-5 relative in the final velocities
+// without, 2.0e-5 with it).
+__global__ void __launch_bounds__(MGP_THREADS) k_ic_za(const float2 *__restrict__ dk, long long bs,
+                                                       float2 *__restrict__ out, long long og, int N,
+                                                       float box_over_2pi) {
+  dk += blockIdx.y * bs;
+  out += blockIdx.y * 3 * og;
+  const int NH = N / 2 + 1, lane = threadIdx.x & 31;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < (long long)N * N; r += nw) {
+    const int i = (int)(r / N), j = (int)(r - (long long)i * N);
+    const float2 *in = dk + (long long)i * N * NH;
+#pragma unroll 4
+    for (int kz = lane; kz < NH; kz += 32) {
+      const float2 z = 2 * kz == N ? in[(long long)N * kz + j] : in[(long long)j * (N / 2) + kz];
+      const int d[3] = {ic_d(i, N), ic_d(j, N), ic_d(kz, N)};
+      const int rk = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+      const float inv = rk == 0 ? 0.0f : box_over_2pi / (float)rk;
+      const bool edge = kz == 0 || 2 * kz == N;
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        float f = inv * (float)d[a];
+        if (edge && ((a == 0 && 2 * i == N) || (a == 1 && 2 * j == N) || a == 2)) f = 0.0f;
+        out[a * og + r * NH + kz] = make_float2(-f * z.y, f * z.x);
+      }
+    }
+  }
+}
+
+int mgp_launch_ic_za(const float *dk, float *out, long long gs, int N, double box, int nbox, cudaStream_t st) {
+  k_ic_za<<<grid_boxes((long long)N * N * 32, 8, nbox), MGP_THREADS, 0, st>>>((const float2 *)dk, gs / 2, (float2 *)out,
+                                                                             gs / 2, N, (float)(box / (2.0 * M_PI)));
+  MGP_CHECK_LAUNCH();
+  g_kernel_launches++;
+  return MGP_OK;
+}
+
+// The 2LPT displacement field on the lattice when Nmesh = r Nsample, r >= 2
+// (src/2LPT.c:1343-1355, 1424-1491): the lattice points are mesh points (the
+// read-out's trilinear weights are 1 and 0), and sampling every r-th point of
+// an N^3 inverse transform is an Ns^3 inverse transform of the spectrum folded
+// onto the Ns grid, G(k') = the sum over the r^3 aliases k' + Ns a of the Hermitian-
+// extended spectrum.  So three Ns^3 transforms take the place of three N^3
+// ones.  One warp per folded (kx, ky) row; out: the three folded spectra of box
+// blockIdx.y, planar, og complex values apart.  G(0) = 0 removes the lattice
+// mean (src/2LPT.c:1493-1508).  The Nyquist conventions are k_ic_disp's.
+__global__ void __launch_bounds__(MGP_THREADS) k_ic_fold(const float2 *__restrict__ src, long long bs, int N, int Ns,
+                                                         int r, float fac, float2 *__restrict__ out, long long og) {
+  src += blockIdx.y * bs;
+  out += blockIdx.y * 3 * og;
+  const int NH = N / 2 + 1, NHs = Ns / 2 + 1, lane = threadIdx.x & 31;
+  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < (long long)Ns * Ns; row += nw) {
+    const int kxp = (int)(row / Ns), kyp = (int)(row - (long long)kxp * Ns);
+    for (int kzp = lane; kzp < NHs; kzp += 32) {
+      float2 G[3];
+#pragma unroll
+      for (int q = 0; q < 3; q++) G[q] = make_float2(0.f, 0.f);
+      for (int ax = 0; ax < r; ax++)
+        for (int ay = 0; ay < r; ay++)
+          for (int az = 0; az < r; az++) {
+            const int kx = kxp + Ns * ax, ky = kyp + Ns * ay, kz = kzp + Ns * az;
+            // stored half space, or the conjugate of the mirrored mode
+            const bool cj = 2 * kz > N;
+            const int sx = cj ? (kx == 0 ? 0 : N - kx) : kx, sy = cj ? (ky == 0 ? 0 : N - ky) : ky,
+                      sz = cj ? N - kz : kz;
+            const long long plane = (long long)sx * N * NH;
+            const float2 S =
+                __ldg(src + (2 * sz == N ? plane + (long long)N * sz + sy : plane + (long long)sy * (N / 2) + sz));
+            const int dx = ic_d(sx, N), dy = ic_d(sy, N), rk = dx * dx + dy * dy + sz * sz;
+            float m[3] = {(float)dx, (float)dy, (float)sz};
+            if (sz == 0 || 2 * sz == N) {
+              if (2 * sx == N) m[0] = 0.f;
+              if (2 * sy == N) m[1] = 0.f;
+              m[2] = 0.f;
+            }
+            const float inv = rk == 0 ? 0.0f : fac / (float)rk, sg = cj ? -1.f : 1.f;
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+              const float g = inv * m[a];
+              G[a].x += g * S.y;
+              G[a].y -= sg * g * S.x;
+            }
+          }
+      if (row == 0 && kzp == 0)
+#pragma unroll
+        for (int q = 0; q < 3; q++) G[q] = make_float2(0.f, 0.f);
+      const long long plane = (long long)kxp * Ns * NHs;
+      float2 *o = out + (2 * kzp == Ns ? plane + (long long)Ns * kzp + kyp : plane + (long long)kyp * (Ns / 2) + kzp);
+#pragma unroll
+      for (int q = 0; q < 3; q++) o[q * og] = G[q];
+    }
+  }
+}
+
+int mgp_launch_ic_fold(const float *src, long long g_bs, int N, int Ns, double box, float *out, long long out_gs,
+                       int nbox, cudaStream_t st) {
+  k_ic_fold<<<grid_boxes((long long)Ns * Ns * 32, 8, nbox), MGP_THREADS, 0, st>>>(
+      (const float2 *)src, g_bs / 2, N, Ns, N / Ns, (float)(box / (2.0 * M_PI)), (float2 *)out, out_gs / 2);
+  MGP_CHECK_LAUNCH();
+  g_kernel_launches++;
+  return MGP_OK;
+}
+
+// A displacement field at the lattice points to the particle arrays: every
+// `step`-th point of three real grids of n^3 (rows of n + 2 floats, gs apart; box
+// blockIdx.y bs floats on).  second 0: D1; 1: D2, times mult, and with it the
+// initial state (main.c:257-309) s = D1 Di + D2 Di2, v = D1 vD + D2 vD2.
+__global__ void __launch_bounds__(MGP_THREADS) k_ic_take(const float *__restrict__ g, long long bs, long long gs, int n,
+                                                         int step, int Ns, long long np,
+                                                         const mgp_ic_box *__restrict__ boxes, int second, float mult,
+                                                         float *__restrict__ D1, float *__restrict__ D2,
+                                                         float *__restrict__ s, float *__restrict__ v) {
+  const mgp_ic_box b = boxes[blockIdx.y];
+  g += blockIdx.y * bs;
+  const long long po = blockIdx.y * 3 * np;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += stride) {
+    int i, j, k;
+    if (np <= 0xffffffffLL)
+      lattice_ijk((unsigned)p, Ns, i, j, k);
+    else
+      lattice_ijk(p, Ns, i, j, k);
+    const long long e = ((long long)i * step * n + j * step) * (n + 2) + k * step;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const long long o = po + a * np + p;
+      const float d = g[a * gs + e];
+      if (!second) {
+        D1[o] = d;
+        continue;
+      }
+      const float d1 = D1[o], d2 = mult * d;
+      D2[o] = d2;
+      s[o] = d1 * b.Di + d2 * b.Di2;
+      v[o] = d1 * b.vD + d2 * b.vD2;
+    }
+  }
+}
+
+int mgp_launch_ic_take(const float *g, long long bs, long long gs, int n, int step, int Ns, long long np,
+                       const mgp_ic_box *boxes, int nbox, int second, float mult, float *D1, float *D2, float *s,
+                       float *v, cudaStream_t st) {
+  k_ic_take<<<grid_boxes(np, 16, nbox), MGP_THREADS, 0, st>>>(g, bs, gs, n, step, Ns, np, boxes, second, mult, D1, D2,
+                                                              s, v);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;

@@ -34,6 +34,12 @@
 
 #include "mgp_internal.h"
 
+#define RET_IF(x)                  \
+  do {                             \
+    int rc_ = (x);                 \
+    if (rc_ != MGP_OK) return rc_; \
+  } while (0)
+
 namespace {
 
 constexpr int kThreads = 256;
@@ -89,11 +95,13 @@ __global__ void k_sd_table(const double *__restrict__ cols, SdRecipe r, long lon
 
 // One thread per output mode k' of the Ns half-complex grid; sums the r^3
 // aliases of the full spectrum F_a(k) = i d_a T(|k|^2) . (delta, -S2) for one
-// or two fields (table components xy -> field 0, zw -> field 1).
+// or two fields (table components xy -> field 0, zw -> field 1;
+// nfields -1: field 1 alone, to out0).  planar, oplanar: the layouts of the stored and the folded spectra (mgp_fft.cuh).
 __global__ void __launch_bounds__(kThreads) k_sd_fold(const float2 *__restrict__ d1, const float2 *__restrict__ d2,
                                                        const float4 *__restrict__ tab, int N, int Ns, int r,
                                                        int nfields, float2 *__restrict__ out0,
-                                                       float2 *__restrict__ out1, long long ostride) {
+                                                       float2 *__restrict__ out1, long long ostride, int planar,
+                                                       int oplanar) {
   const int NH = N / 2 + 1, NHs = Ns / 2 + 1;
   // one warp per folded (kx, ky) row, lanes along kz: no division per mode
   const int lane = threadIdx.x & 31;
@@ -117,9 +125,12 @@ __global__ void __launch_bounds__(kThreads) k_sd_fold(const float2 *__restrict__
             // stored half space, or the conjugate of the mirrored mode
             const bool cj = 2 * kz > N;
             const int sx = cj ? (kx == 0 ? 0 : N - kx) : kx, sy = cj ? (ky == 0 ? 0 : N - ky) : ky, sz = cj ? N - kz : kz;
-            const long long c = ((long long)sx * N + sy) * NH + sz;
+            const long long plane = (long long)sx * N * NH;
+            const long long c = !planar ? plane + (long long)sy * NH + sz
+                                : 2 * sz == N ? plane + (long long)N * sz + sy : plane + (long long)sy * (N / 2) + sz;
             const int dx = sd_d(sx, N), dy = sd_d(sy, N), dz = sd_d(sz, N);
-            const float4 t = __ldg(tab + ((long long)dx * dx + (long long)dy * dy + (long long)dz * dz));
+            float4 t = __ldg(tab + ((long long)dx * dx + (long long)dy * dy + (long long)dz * dz));
+            if (nfields < 0) t = make_float4(t.z, t.w, 0.f, 0.f);
             const float2 u = __ldg(d1 + c), w = __ldg(d2 + c);
             float m[3] = {(float)dx, (float)dy, (float)dz};
             if (sz == 0 || 2 * sz == N) {
@@ -146,11 +157,13 @@ __global__ void __launch_bounds__(kThreads) k_sd_fold(const float2 *__restrict__
         }
       }
     }
+    const long long op = (long long)kxp * Ns * NHs;
+    const long long w = !oplanar ? o : 2 * kzp == Ns ? op + (long long)Ns * kzp + kyp : op + (long long)kyp * (Ns / 2) + kzp;
 #pragma unroll
-    for (int a = 0; a < 3; a++) out0[a * ostride + o] = G[0][a];
+    for (int a = 0; a < 3; a++) out0[a * ostride + w] = G[0][a];
     if (nfields > 1) {
 #pragma unroll
-      for (int a = 0; a < 3; a++) out1[a * ostride + o] = G[1][a];
+      for (int a = 0; a < 3; a++) out1[a * ostride + w] = G[1][a];
     }
   }
 }
@@ -335,7 +348,8 @@ void mgp_sd_free(mgp_ctx *c) {
   c->sd = 0;
 }
 
-int mgp_sd_store(mgp_ctx *c, const float *deltak, const float *source2k) {
+int mgp_sd_store(mgp_ctx *c, const float *deltak, const float *source2k, int planar) {
+  c->sd_planar = planar;
   const long long n = c->g.ncomplex;
   k_sd_store<<<mgp_blocks_for(n, 8), kThreads, 0, c->stream>>>((const float2 *)deltak, (const float2 *)source2k, n,
                                                               (float2 *)c->sd_dk[0], (float2 *)c->sd_dk[1]);
@@ -429,18 +443,37 @@ static int fields_pass(mgp_ctx *c, double A, double AFF, int n, const int *types
     }
     return MGP_OK;
   }
-  float *o0 = c->sd_slot[slot_of(types[0])], *o1 = n > 1 ? c->sd_slot[slot_of(types[1])] : NULL;
-  k_sd_fold<<<mgp_blocks_for((long long)Ns * Ns * 32, 8), kThreads, 0, c->stream>>>(
-      (const float2 *)c->sd_dk[0], (const float2 *)c->sd_dk[1], (const float4 *)c->sd_tab, c->g.N, Ns, c->sd_fold, n,
-      (float2 *)o0, (float2 *)o1, c->sd_grid / 2);
-  MGP_CHECK_LAUNCH();
-  g_kernel_launches++;
-  for (int f = 0; f < n; f++) {
-    float *base = c->sd_slot[slot_of(types[f])];
-    for (int a = 0; a < 3; a++) {
-      float *g = base + a * c->sd_grid;
-      MGP_CUFFT(cufftExecC2R(c->plan_c2r_s, (cufftComplex *)g, (cufftReal *)g));
+  // the Ns^3 inverse transforms: this library's (from planar spectra in
+  // scratch, six at most 3/4 of three mesh grids for Nmesh >= 2 Nsample, or
+  // two calls of three) where the lattice size has them, else cuFFT's in place
+  const bool own = c->fft_mode && mgp_fft_has(Ns) && mgp_fft_supported(c);
+  if (own) RET_IF(mgp_fft_scratch(c));
+  const int per = own && c->g.N == Ns ? 1 : n;  // fields per fold
+  for (int f0 = 0; f0 < n; f0 += per) {
+    float *o[2] = {c->sd_slot[slot_of(types[f0])], per > 1 ? c->sd_slot[slot_of(types[f0 + 1])] : NULL};
+    if (own) {
+      o[0] = c->fft_scr;
+      o[1] = c->fft_scr + 3 * c->sd_grid;
     }
+    const float4 *tab = (const float4 *)c->sd_tab;
+    k_sd_fold<<<mgp_blocks_for((long long)Ns * Ns * 32, 8), kThreads, 0, c->stream>>>(
+        (const float2 *)c->sd_dk[0], (const float2 *)c->sd_dk[1], tab, c->g.N, Ns, c->sd_fold, f0 ? -per : per,
+        (float2 *)o[0], (float2 *)o[1], c->sd_grid / 2, c->sd_planar, own);
+    MGP_CHECK_LAUNCH();
+    g_kernel_launches++;
+    for (int f = 0; f < per; f++) {
+      float *base = c->sd_slot[slot_of(types[f0 + f])];
+      if (own) {
+        RET_IF(mgp_fft_c2r(c, Ns, o[f], base, 3, c->sd_grid));
+        continue;
+      }
+      for (int a = 0; a < 3; a++) {
+        float *g = base + a * c->sd_grid;
+        MGP_CUFFT(cufftExecC2R(c->plan_c2r_s, (cufftComplex *)g, (cufftReal *)g));
+      }
+    }
+  }
+  for (int f = 0; f < n; f++) {
     const int s = slot_of(types[f]);
     c->sd_kind[s] = types[f];
     c->sd_a[s] = A;
