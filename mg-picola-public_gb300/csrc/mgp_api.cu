@@ -1001,7 +1001,7 @@ extern "C" int mgp_get_displacements(mgp_ctx *c, double A) {
     // bucket the particles by cell tile (mgp_tiles.cu) for the deposit and
     // the kick of this step
     tstart(c, T_SORT);
-    RET_IF(mgp_tiles_sort(c, mgp_tile_side(N, c->np)));
+    RET_IF(mgp_tiles_sort(c, mgp_tile_side(N, c->np), c->s));
     tstop(c, T_SORT);
   }
   // the tile deposit stores every cell of the mesh itself (owner writes),
@@ -1012,7 +1012,7 @@ extern "C" int mgp_get_displacements(mgp_ctx *c, double A) {
   tstart(c, T_CIC);
   double wpar = pow((double)N / (double)c->Ns, 3);
   if (tiles)
-    RET_IF(mgp_cic_tiles_own(c, (float)wpar));
+    RET_IF(mgp_cic_tiles_own(c, (float)wpar, c->s, c->rho));
   else
     RET_IF(mgp_launch_cic(c->s, c->dstate, c->np, c->Ns, N, c->p.Box, (float)wpar, c->rho, c->g.P, c->stream));
   tstop(c, T_CIC);
@@ -1299,18 +1299,32 @@ extern "C" int mgp_pofk_total(mgp_ctx *c, int cap, int *nbins, double *k, double
   return pofk_out(c, 1, cap, nbins, k, pk, kmean, n);
 }
 
+static int ensure_stage(mgp_ctx *c, int arrays = 2) {
+  // `arrays` [np][3] float staging arrays
+  if (c->stage_arrays < arrays) {
+    if (c->stage) {
+      MGP_CUDA(cudaStreamSynchronize(c->stream));
+      cudaFree(c->stage);
+      c->stage = NULL;
+      c->stage_arrays = 0;
+    }
+    MGP_CUDA(cudaMalloc(&c->stage, sizeof(float) * 3 * arrays * (size_t)c->np));
+    c->stage_arrays = arrays;
+  }
+  return MGP_OK;
+}
+
 // compute_RSD_powerspectrum (src/compute_pofk.c:403-512): redshift-space
 // deposits with the y and z axes as line of sight, P0/P2/P4 per axis, their
 // mean and |difference|/sqrt(2).  Uses the force grids as scratch.
 extern "C" int mgp_pofk_rsd(mgp_ctx *c, double A, int cap, int *nbins, double *k, double *P0, double *P2, double *P4,
                             double *s0, double *s2, double *s4, double *n) {
   RET_IF(require_particles(c));
-  RET_IF(mgp_particles_canonical(c));  // lattice order for the caller's arrays
   const int nb = c->pk_nbins, N = c->g.N;
   if (nbins) *nbins = nb;
   if (cap < nb) return mgp_set_error(MGP_EINVAL, "RSD capacity %d < %d bins", cap, nb);
   if (!c->rsd_block) {
-    MGP_CUDA(cudaMalloc(&c->rsd_block, sizeof(double) * 3 * (size_t)nb * c->pk_blocks));
+    MGP_CUDA(cudaMalloc(&c->rsd_block, sizeof(double) * 3 * (size_t)nb * (c->pk_blocks + 1)));
     MGP_CUDA(cudaMalloc(&c->rsd_sum, sizeof(double) * 3 * (size_t)nb));
   }
   const mgp_params *p = &c->p;
@@ -1336,15 +1350,38 @@ extern "C" int mgp_pofk_rsd(mgp_ctx *c, double A, int cap, int *nbins, double *k
     lpitch = c->sd_pitch;
   }
   const double wpar = pow((double)N / (double)c->Ns, 3);
+  // the particles bucketed by cell tile at their redshift-space positions, as the
+  // step's deposit, with the grid axes as they are; where the mesh has no tiles,
+  // the lattice-order deposit with the line of sight on the third axis
+  const int side = c->tile_mode ? mgp_tile_side(N, c->np) : 0;
+  const bool own = own_fft(c);
+  if (side) {
+    RET_IF(ensure_stage(c));
+    c->tile_ready = 0;  // the sort's arrays describe the shifted positions
+  } else {
+    RET_IF(mgp_particles_canonical(c));
+  }
   float *dens = c->frc, *dkr = c->frc + c->g.nreal;
   std::vector<double> sums(3 * (size_t)nb), res[2][3];
   const double norm = pow(p->Box, 3) / pow((double)N, 6), shot = c->pk_sub ? pow(p->Box / (double)c->Ns, 3) : 0.0;
   for (int ax = 0; ax < 2; ax++) {
-    RET_IF(mgp_launch_fill(dens, c->g.nreal, -1.0f, c->stream));
-    RET_IF(mgp_launch_cic_rsd(c->s, c->v, L1, L2, lstride, lpitch, c->dstate, c->np, c->Ns, N, p->Box, (float)wpar,
-                              ax + 1, (float)vnorm, g1, g2, dens, c->g.P, c->stream));
-    MGP_CUFFT(cufftExecR2C(c->plan_r2c_oop, (cufftReal *)dens, (cufftComplex *)dkr));
-    RET_IF(mgp_launch_pofk_mu(dkr, N, c->rk_bin, c->win1d, nb, c->rsd_block, c->pk_blocks, c->rsd_sum, c->stream));
+    if (side) {
+      RET_IF(mgp_launch_rsd_shift(c->s, c->v, L1, L2, lstride, lpitch, c->dstate, c->np, c->Ns, ax + 1,
+                                  (float)(vnorm * p->Box / N), g1, g2, c->permuted ? c->q : NULL, c->stage, c->stream));
+      RET_IF(mgp_tiles_sort(c, side, c->stage));
+      RET_IF(mgp_cic_tiles_own(c, (float)wpar, c->stage, dens));
+      c->tile_ready = 0;
+    } else {
+      RET_IF(mgp_launch_fill(dens, c->g.nreal, -1.0f, c->stream));
+      RET_IF(mgp_launch_cic_rsd(c->s, c->v, L1, L2, lstride, lpitch, c->dstate, c->np, c->Ns, N, p->Box, (float)wpar,
+                                ax + 1, (float)vnorm, g1, g2, dens, c->g.P, c->stream));
+    }
+    if (own)
+      RET_IF(mgp_fft_r2c(c, dens, dkr, 1, c->g.nreal));
+    else
+      MGP_CUFFT(cufftExecR2C(c->plan_r2c_oop, (cufftReal *)dens, (cufftComplex *)dkr));
+    RET_IF(mgp_launch_pofk_mu(dkr, N, c->pk_thr, c->win1d, nb, c->pk_bintype, c->pk_kmin, c->pk_kmax, side ? ax + 1 : 2,
+                              own, c->rsd_block, c->pk_blocks, c->rsd_sum, c->stream));
     MGP_CUDA(cudaMemcpyAsync(sums.data(), c->rsd_sum, sizeof(double) * 3 * nb, cudaMemcpyDeviceToHost, c->stream));
     MGP_CUDA(cudaStreamSynchronize(c->stream));
     for (int q = 0; q < 3; q++) res[ax][q].assign(nb, 0.0);
@@ -1375,54 +1412,30 @@ extern "C" int mgp_pofk_rsd(mgp_ctx *c, double A, int cap, int *nbins, double *k
 }
 
 // ---------------------------------------------------------- particles
-static int ensure_stage(mgp_ctx *c, int arrays = 2) {
-  // `arrays` [np][3] float staging arrays
-  if (c->stage_arrays < arrays) {
-    if (c->stage) {
-      MGP_CUDA(cudaStreamSynchronize(c->stream));
-      cudaFree(c->stage);
-      c->stage = NULL;
-      c->stage_arrays = 0;
-    }
-    MGP_CUDA(cudaMalloc(&c->stage, sizeof(float) * 3 * arrays * (size_t)c->np));
-    c->stage_arrays = arrays;
-  }
-  return MGP_OK;
-}
-
 extern "C" int mgp_get_particles(mgp_ctx *c, float *pos, float *vel, float *D1, float *D2, size_t np) {
   RET_IF(require_particles(c));
-  RET_IF(mgp_particles_canonical(c));  // lattice order for the caller's arrays
   if ((long long)np != c->np) return mgp_set_error(MGP_EINVAL, "np = %zu, context holds %lld", np, c->np);
   RET_IF(ensure_stage(c));
   const size_t bytes = sizeof(float) * 3 * np;
-  float *dpos = c->stage, *dvel = c->stage + 3 * np;
+  float *st[2] = {c->stage, c->stage + 3 * np};
+  // particles in tile order go straight to their lattice places; D1 and D2 (with
+  // scale-dependent growth the slots the kick and the drift read) take the
+  // staging arrays after the copies before them
   if (pos || vel) {
-    RET_IF(mgp_launch_positions(c->s, c->dstate, c->np, c->Ns, c->p.Box, pos ? dpos : NULL, vel ? dvel : NULL, c->v,
-                                c->stream));
-    if (pos) MGP_CUDA(cudaMemcpyAsync(pos, dpos, bytes, cudaMemcpyDeviceToHost, c->stream));
-    if (vel) MGP_CUDA(cudaMemcpyAsync(vel, dvel, bytes, cudaMemcpyDeviceToHost, c->stream));
+    RET_IF(mgp_launch_positions(c->s, c->dstate, c->np, c->Ns, c->p.Box, pos ? st[0] : NULL, vel ? st[1] : NULL, c->v,
+                                c->stream, c->permuted ? c->q : NULL));
+    if (pos) MGP_CUDA(cudaMemcpyAsync(pos, st[0], bytes, cudaMemcpyDeviceToHost, c->stream));
+    if (vel) MGP_CUDA(cudaMemcpyAsync(vel, st[1], bytes, cudaMemcpyDeviceToHost, c->stream));
   }
-  MGP_CUDA(cudaStreamSynchronize(c->stream));
-  // D1/D2 SoA -> AoS on the host; with scale-dependent growth the two slots
-  // the kick and the drift read (lattice rows of pitch Ps)
   const float *srcs[2] = {c->sd ? c->sd_slot[0] : c->D1, c->sd ? c->sd_slot[1] : c->D2};
   float *dsts[2] = {D1, D2};
-  std::vector<float> h;
   for (int q = 0; q < 2; q++) {
     if (!dsts[q]) continue;
-    h.resize(3 * np);
-    if (c->sd) {
-      for (int a = 0; a < 3; a++)
-        MGP_CUDA(cudaMemcpy2D(h.data() + a * np, sizeof(float) * c->Ns, srcs[q] + a * c->sd_grid,
-                              sizeof(float) * c->sd_pitch, sizeof(float) * c->Ns, (size_t)c->Ns * c->Ns,
-                              cudaMemcpyDeviceToHost));
-    } else {
-      MGP_CUDA(cudaMemcpy(h.data(), srcs[q], bytes, cudaMemcpyDeviceToHost));
-    }
-    for (size_t i = 0; i < np; i++)
-      for (int a = 0; a < 3; a++) dsts[q][3 * i + a] = h[a * np + i];
+    RET_IF(mgp_launch_soa_to_aos(srcs[q], c->sd ? c->sd_grid : c->np, c->Ns, c->sd ? c->sd_pitch : c->Ns, st[q], c->np,
+                                 c->stream));
+    MGP_CUDA(cudaMemcpyAsync(dsts[q], st[q], bytes, cudaMemcpyDeviceToHost, c->stream));
   }
+  MGP_CUDA(cudaStreamSynchronize(c->stream));
   return MGP_OK;
 }
 
@@ -1697,7 +1710,7 @@ static int batch_step_launch(mgp_ctx *c, const batch_step &q, const mgp_box_scal
   const cufftHandle c2r = B > 1 ? c->plan_c2r_b : c->plan_c2r_1;
   const cufftHandle c2r_frc = B > 1 ? c->plan_c2r_frc_b : c->plan_c2r_1;
   const double wpar = pow((double)N / (double)c->Ns, 3);
-  if (c->batch_tile) RET_IF(mgp_tiles_sort(c, c->batch_tile));  // all boxes' particles by tile
+  if (c->batch_tile) RET_IF(mgp_tiles_sort(c, c->batch_tile, c->s));  // all boxes' particles by tile
   RET_IF(mgp_launch_fill(c->rho, gf * B, -1.0f, c->stream));
   if (c->batch_tile)
     RET_IF(mgp_cic_tiles(c, (float)wpar, c->tune[0]));

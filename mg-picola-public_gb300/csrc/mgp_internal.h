@@ -372,10 +372,10 @@ int mgp_tile_side(int N, long long np);
 int mgp_tiles_check(const mgp_ctx *c, int T);
 int mgp_tiles_alloc(mgp_ctx *c, int T);
 void mgp_tiles_free(mgp_ctx *c);
-int mgp_tiles_sort(mgp_ctx *c, int T);
+int mgp_tiles_sort(mgp_ctx *c, int T, const float *s);
 int mgp_cic_tiles(mgp_ctx *c, float wpar, int per_sm = 0);
 /* single-box tile deposit writing every cell itself (no pre-set mesh) */
-int mgp_cic_tiles_own(mgp_ctx *c, float wpar);
+int mgp_cic_tiles_own(mgp_ctx *c, float wpar, const float *s, float *rho);
 /* kick + drift in the order of the last mgp_tiles_sort, the particle
  * arrays rewritten in that order */
 int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a, int *nblocks_out);
@@ -423,8 +423,16 @@ int mgp_launch_ic_disp(const float *dk, const float *src, float *out6, long long
 int mgp_launch_cic_rsd(const float *s, const float *v, const float *D1, const float *D2, long long lpt_stride,
                        int lpt_pitch, const mgp_dstate *st, long long np, int Ns, int N, double box, float wpar,
                        int axis, float vnorm, float g1, float g2, float *rho, long long P, cudaStream_t stream);
-int mgp_launch_pofk_mu(const float *dk, int N, const int *rk_bin, const float *win, int nbins, double *block_part,
-                       int nblocks, double *sums, cudaStream_t st);
+int mgp_launch_rsd_shift(const float *s, const float *v, const float *D1, const float *D2, long long lpt_stride,
+                         int lpt_pitch, const mgp_dstate *st, long long np, int Ns, int axis, float shift, float g1,
+                         float g2, const unsigned *qlat, float *out, cudaStream_t stream);
+/* sums of P, P mu^2, P mu^4 per bin, mu along grid axis `los` (1 y, 2 z);
+ * block_part: 3 nbins (nblocks + 1) values */
+int mgp_launch_pofk_mu(const float *dk, int N, const int *thr, const float *win, int nbins, int bintype, double kmin,
+                       double kmax, int los, int planar, double *block_part, int nblocks, double *sums,
+                       cudaStream_t st);
+int mgp_launch_soa_to_aos(const float *in, long long stride, int Ns, int pitch, float *out, long long np,
+                          cudaStream_t st);
 int mgp_launch_aos_to_soa(const float *in, float *out, long long np, cudaStream_t st);
 int mgp_launch_output(const float *s, const float *v, const float *D1, const float *D2, long long lpt_stride,
                       int lpt_pitch, const mgp_dstate *dst, long long np, int Ns, double box, double lengthfac,
@@ -436,7 +444,8 @@ int mgp_launch_ic_finish(float *D1, float *D2, float *s, float *v, long long np,
 int mgp_launch_finalize_kd(mgp_dstate *dst, const double *partials, int nblocks, long long np,
                            double dda_omega, double dyyy, int do_drift, cudaStream_t st);
 int mgp_launch_positions(const float *s, const mgp_dstate *dst, long long np, int Ns, double box,
-                         float *out_pos, float *out_vel, const float *v, cudaStream_t st);
+                         float *out_pos, float *out_vel, const float *v, cudaStream_t st,
+                         const unsigned *qlat = NULL);
 int mgp_launch_set_state(float *s, float *v, const float *pos, const float *vel, long long np, int Ns,
                          double box, cudaStream_t st);
 int mgp_launch_set_state_range(float *s, float *v, const float *pos, const float *vel, long long np, int Ns,

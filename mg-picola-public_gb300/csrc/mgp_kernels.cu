@@ -949,7 +949,7 @@ int mgp_launch_ic_amp(double *amp, int n, double kf, double vol, const mgp_eh_sp
 // all.  The kz = 0 entries of the half the reference fills by symmetry take
 // the conjugate of the partner column's first mode.  With the seed table and
 // the amplitudes also made on the device, the whole IC of 256^3 particles on
-// a 512^3 mesh went from 36 to 17 ms (the rest is its transforms).
+// a 512^3 mesh went from 36 to 16 ms (the rest is its transforms).
 __global__ void __launch_bounds__(MGP_THREADS) k_ic_delta(const mgp_ic_box *__restrict__ boxes,
                                                           const double *__restrict__ amp_rk, int namp, int N, int Ns,
                                                           int kc, double box, float2 *__restrict__ dk, long long bs,
@@ -1553,8 +1553,11 @@ int mgp_launch_ic_finish(float *D1, float *D2, float *s, float *v, long long np,
 }
 
 // ---------------------------------------------------- particle export
-// Absolute positions wrap(q + s + cx) and velocities v + cv, AoS [np][3].
-// FP32 arithmetic: the outputs are FP32 and the wrap needs no division.
+// Absolute positions wrap(q + s + cx) and velocities v + cv, AoS [np][3] in lattice
+// order; qlat: the lattice point of every slot when the arrays are in tile order
+// (12-byte stores to the particle's place instead of restoring the order of six
+// arrays first).  FP32 arithmetic: the outputs are FP32 and the wrap needs no
+// division.
 __device__ __forceinline__ float wrap_box(float x, float box) {
   x -= box * floorf(x / box);  // no loop: bounded work for any input
   if (x >= box) x -= box;
@@ -1563,27 +1566,29 @@ __device__ __forceinline__ float wrap_box(float x, float box) {
 }
 
 __global__ void k_positions(const float *__restrict__ s, const float *__restrict__ v, const mgp_dstate *__restrict__ st,
-                            long long np, int Ns, double box, float *__restrict__ pos, float *__restrict__ vel) {
+                            long long np, int Ns, double box, float *__restrict__ pos, float *__restrict__ vel,
+                            const unsigned *__restrict__ qlat) {
   long long stride = (long long)gridDim.x * blockDim.x;
   const float dq = (float)(box / (double)Ns), fbox = (float)box;
   const float cx[3] = {(float)st->cx[0], (float)st->cx[1], (float)st->cx[2]};
   const float cv[3] = {(float)st->cv[0], (float)st->cv[1], (float)st->cv[2]};
   for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += stride) {
+    const long long l = qlat ? (long long)qlat[p] : p;
     int li[3];
     if (np <= 0xffffffffLL)
-      lattice_ijk((unsigned)p, Ns, li[0], li[1], li[2]);
+      lattice_ijk((unsigned)l, Ns, li[0], li[1], li[2]);
     else
-      lattice_ijk(p, Ns, li[0], li[1], li[2]);
+      lattice_ijk(l, Ns, li[0], li[1], li[2]);
     for (int a = 0; a < 3; a++) {
-      if (pos) pos[3 * p + a] = wrap_box((float)li[a] * dq + (s[a * np + p] + cx[a]), fbox);
-      if (vel) vel[3 * p + a] = v[a * np + p] + cv[a];
+      if (pos) pos[3 * l + a] = wrap_box((float)li[a] * dq + (s[a * np + p] + cx[a]), fbox);
+      if (vel) vel[3 * l + a] = v[a * np + p] + cv[a];
     }
   }
 }
 
 int mgp_launch_positions(const float *s, const mgp_dstate *dst, long long np, int Ns, double box, float *out_pos,
-                         float *out_vel, const float *v, cudaStream_t st) {
-  k_positions<<<blocks_for(np, 8), MGP_THREADS, 0, st>>>(s, v, dst, np, Ns, box, out_pos, out_vel);
+                         float *out_vel, const float *v, cudaStream_t st, const unsigned *qlat) {
+  k_positions<<<blocks_for(np, 8), MGP_THREADS, 0, st>>>(s, v, dst, np, Ns, box, out_pos, out_vel, qlat);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
@@ -1636,6 +1641,25 @@ __global__ void k_aos_to_soa(const float *__restrict__ in, float *__restrict__ o
 }
 int mgp_launch_aos_to_soa(const float *in, float *out, long long np, cudaStream_t st) {
   k_aos_to_soa<<<blocks_for(np, 4), MGP_THREADS, 0, st>>>(in, out, np);
+  MGP_CHECK_LAUNCH();
+  g_kernel_launches++;
+  return MGP_OK;
+}
+
+// Three lattice fields (component a of point (i, j, k) at a stride + (i Ns + j) pitch
+// + k) to AoS [np][3].
+__global__ void k_soa_to_aos(const float *__restrict__ in, long long stride, int Ns, int pitch, float *__restrict__ out,
+                             long long np) {
+  const long long step = (long long)gridDim.x * blockDim.x;
+  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += step) {
+    const long long row = pitch == Ns ? 0 : p / Ns, e = pitch == Ns ? p : row * pitch + (p - row * Ns);
+#pragma unroll
+    for (int a = 0; a < 3; a++) out[3 * p + a] = in[a * stride + e];
+  }
+}
+int mgp_launch_soa_to_aos(const float *in, long long stride, int Ns, int pitch, float *out, long long np,
+                          cudaStream_t st) {
+  k_soa_to_aos<<<blocks_for(np, 8), MGP_THREADS, 0, st>>>(in, stride, Ns, pitch, out, np);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
@@ -1731,50 +1755,207 @@ int mgp_launch_cic_rsd(const float *s, const float *v, const float *D1, const fl
   return MGP_OK;
 }
 
-// bin_up_RSD_power_spectrum (src/compute_pofk.c:518-753): sums of P, P mu^2
-// and P mu^4 per bin with mu = kz/|k| (kz is the LOS index), mu = 0 for the
-// k = 0 mode; FP64 shared-memory bins (used at output time only).
-__global__ void __launch_bounds__(MGP_THREADS) k_pofk_mu(const float2 *__restrict__ dk, int N,
-                                                         const int *__restrict__ rk_bin, const float *__restrict__ win,
-                                                         int nbins, double *__restrict__ block_part) {
-  extern __shared__ double smu[];
-  const int NH = N / 2 + 1, h = N / 2;
-  for (int b = threadIdx.x; b < 3 * nbins; b += blockDim.x) smu[b] = 0.0;
+// The displacements in redshift space for the tile deposit (PtoMesh_RSD,
+// src/compute_pofk.c:280-393): component `axis` moved by V shift, V as in k_cic_rsd,
+// shift in Mpc/h per unit of V; the axes stay the grid's, and the binning takes
+// mu along the line of sight's own axis.  qlat: the lattice point of every slot
+// when the arrays are in tile order.
+__global__ void __launch_bounds__(MGP_THREADS) k_rsd_shift(const float *__restrict__ s, const float *__restrict__ v,
+                                                           const float *__restrict__ D1, const float *__restrict__ D2,
+                                                           long long lstride, int lpitch,
+                                                           const mgp_dstate *__restrict__ st, long long np, int Ns,
+                                                           int axis, float shift, float g1, float g2,
+                                                           const unsigned *__restrict__ qlat, float *__restrict__ out) {
+  const float cvl = (float)st->cv[axis];
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += stride) {
+    const long long l = qlat ? (long long)qlat[p] : p;
+    long long od = axis * lstride + l;
+    if (lpitch != Ns) {
+      const long long row = l / Ns;
+      od = axis * lstride + row * lpitch + (l - row * Ns);
+    }
+    const float V = (v[axis * np + p] + cvl) + D1[od] * g1 + D2[od] * g2;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const float x = s[a * np + p];
+      out[a * np + p] = a == axis ? fmaf(V, shift, x) : x;
+    }
+  }
+}
+
+int mgp_launch_rsd_shift(const float *s, const float *v, const float *D1, const float *D2, long long lpt_stride,
+                         int lpt_pitch, const mgp_dstate *st, long long np, int Ns, int axis, float shift, float g1,
+                         float g2, const unsigned *qlat, float *out, cudaStream_t stream) {
+  k_rsd_shift<<<blocks_for(np, 8), MGP_THREADS, 0, stream>>>(s, v, D1, D2, lpt_stride, lpt_pitch, st, np, Ns, axis,
+                                                             shift, g1, g2, qlat, out);
+  MGP_CHECK_LAUNCH();
+  g_kernel_launches++;
+  return MGP_OK;
+}
+
+// bin_up_RSD_power_spectrum (src/compute_pofk.c:518-753): sums of P, P mu^2 and
+// P mu^4 per bin with mu = k_los/|k|, mu = 0 for the k = 0 mode.  As k_pofk: a warp
+// takes the four rows that share (|kx|, |ky|), 32 modes at a time, sums the runs
+// of equal bin with a segmented scan (three values), and adds each run's total to
+// its own bins in FP32 with the rounding error kept apart; blocks write FP64
+// partials.  One FP64 shared-memory addition per mode and moment -- a
+// compare-and-swap loop, with all modes of a row falling into few bins -- took 2.9
+// of the 5.5 ms of a line of sight at 512^3.  The modes with all |k_i| < 32, whose
+// bins hold few modes and carry the multipoles' weight (35 P4 - 30 P2 + 3 P0
+// amplifies their rounding), are FP64 throughout, added to the partial row after
+// the blocks' (zeroed by the launcher).
+#define MGP_MU_THREADS 128
+__global__ void __launch_bounds__(MGP_MU_THREADS) k_pofk_mu(mgp_pofk_kargs a, int los) {
+  extern __shared__ float shf[];
+  const int N = a.N, nbins = a.nbins, NH = N / 2 + 1, h = N / 2, nwb = blockDim.x >> 5;
+  float *acc0 = shf;  // [warp][moment][hi, lo][nbins]
+  const int *sthr = a.thr;  // priv: with room for them, the tables in shared memory too
+  const float *swin = a.win;
+  for (int b = threadIdx.x; b < 6 * nwb * nbins; b += blockDim.x) acc0[b] = 0.0f;
+  if (a.priv) {
+    int *t = (int *)(acc0 + 6 * (size_t)nwb * nbins);
+    float *w = (float *)(t + nbins + 1);
+    for (int b = threadIdx.x; b <= nbins; b += blockDim.x) t[b] = a.thr[b];
+    for (int d = threadIdx.x; d <= h; d += blockDim.x) w[d] = a.win[d];
+    sthr = t;
+    swin = w;
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31;
+  float *acc = acc0 + 6 * (size_t)(threadIdx.x >> 5) * nbins;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long r = wid; r < (long long)N * N; r += nw) {
-    const int i = (int)(r / N), j = (int)(r - (long long)i * N);
-    const int d0 = i > h ? N - i : i, d1 = j > h ? N - j : j;
-    for (int kz = lane; kz < NH; kz += 32) {
-      const int rk = d0 * d0 + d1 * d1 + kz * kz;
-      const int bin = rk_bin[rk];
-      if (bin < 0) continue;
-      float2 z = dk[r * NH + kz];
-      double w = (kz == 0 || 2 * kz == N) ? 1.0 : 2.0;
-      double pk = (double)(z.x * z.x + z.y * z.y) * (double)(win[d0] * win[d1] * win[kz]) * w;
-      double mu2 = rk == 0 ? 0.0 : (double)(kz * kz) / (double)rk;
-      atomicAdd(&smu[bin], pk);
-      atomicAdd(&smu[nbins + bin], pk * mu2);
-      atomicAdd(&smu[2 * nbins + bin], pk * mu2 * mu2);
+  const float inv_span = (float)nbins / (a.kmax - a.kmin);
+  const float inv_logspan = a.bintype ? (float)nbins / logf(a.kmax / a.kmin) : 0.0f;
+  const int lo = sthr[0], hi = sthr[nbins];
+  const long long npair = (long long)(h + 1) * (h + 1);
+  for (long long q = wid; q < npair; q += nw) {
+    const int d0 = (int)(q / (h + 1)), d1 = (int)(q - (long long)d0 * (h + 1));
+    const int rk01 = d0 * d0 + d1 * d1;
+    const float w01 = swin[d0] * swin[d1];
+    const bool mi = !(d0 == 0 || d0 == h), mj = !(d1 == 0 || d1 == h);
+    const bool use[4] = {true, mj, mi, mi && mj};
+    const float2 *row[4];
+    long long last[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const int i = t < 2 ? d0 : N - d0, j = t & 1 ? N - d1 : d1;
+      const long long plane = (long long)i * N * NH;
+      row[t] = a.dk + (a.planar ? plane + (long long)j * h : plane + (long long)j * NH);
+      last[t] = a.planar ? (long long)(N - j) * h + j : h;
+    }
+    for (int k0 = 0; k0 < NH; k0 += 32) {
+      const int kz = k0 + lane;
+      int bin = -1;
+      float m0 = 0.0f, m2 = 0.0f, m4 = 0.0f;
+      if (kz < NH) {
+        const int rk = rk01 + kz * kz;
+        if (rk >= lo && rk < hi) {
+          float p2 = 0.0f;
+          double e2 = 0.0;
+          const bool exact = k0 == 0 && d0 < 32 && d1 < 32;
+#pragma unroll
+          for (int t = 0; t < 4; t++)
+            if (use[t]) {
+              const float2 z = row[t][kz == h ? last[t] : kz];
+              const float p1 = z.x * z.x + z.y * z.y;
+              p2 += p1;
+              if (exact) e2 += (double)p1;
+            }
+          const float km = sqrtf((float)rk);
+          const float x = a.bintype ? logf(km / a.kmin) * inv_logspan : (km - a.kmin) * inv_span;
+          int b = (int)floorf(x + 0.5f);
+          b = b < 0 ? 0 : (b >= nbins ? nbins - 1 : b);
+          while (b > 0 && sthr[b] > rk) b--;
+          while (b + 1 < nbins && sthr[b + 1] <= rk) b++;
+          bin = b;
+          const int kl = los == 2 ? kz : d1;
+          if (exact) {
+            const double w = (double)(w01 * swin[kz]) * ((kz == 0 || 2 * kz == N) ? 1.0 : 2.0);
+            const double mu = rk == 0 ? 0.0 : (double)(kl * kl) / (double)rk, pk = e2 * w;
+            double *o = a.block_part + (long long)gridDim.x * 3 * nbins + b;
+            atomicAdd(o, pk);
+            atomicAdd(o + nbins, pk * mu);
+            atomicAdd(o + 2 * nbins, pk * mu * mu);
+            p2 = 0.0f;
+          }
+          const float mu2 = rk == 0 ? 0.0f : (float)(kl * kl) / (float)rk;
+          m0 = p2 * (w01 * swin[kz] * ((kz == 0 || 2 * kz == N) ? 1.0f : 2.0f));
+          m2 = m0 * mu2;
+          m4 = m2 * mu2;
+        }
+      }
+      const int prev = __shfl_up_sync(0xffffffffu, bin, 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != bin);
+      const int seg0 = 31 - __clz(heads & ((2u << lane) - 1u));
+      for (int o = 1; o < 32; o <<= 1) {
+        const float t0 = __shfl_up_sync(0xffffffffu, m0, o), t2 = __shfl_up_sync(0xffffffffu, m2, o),
+                    t4 = __shfl_up_sync(0xffffffffu, m4, o);
+        if (lane - o >= seg0) {
+          m0 += t0;
+          m2 += t2;
+          m4 += t4;
+        }
+      }
+      const int nbin = __shfl_down_sync(0xffffffffu, bin, 1);
+      if ((lane == 31 || nbin != bin) && bin >= 0) {
+        const float m[3] = {m0, m2, m4};
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          float *p = acc + 2 * c * nbins + bin;
+          const float old = p[0], sum = old + m[c], bp = sum - old;
+          p[0] = sum;
+          p[nbins] += (old - (sum - bp)) + (m[c] - bp);
+        }
+      }
+      __syncwarp();  // a bin may go on in the next 32 modes
     }
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < 3 * nbins; b += blockDim.x) block_part[(long long)blockIdx.x * 3 * nbins + b] = smu[b];
+  for (int b = threadIdx.x; b < 3 * nbins; b += blockDim.x) {
+    const int c = b / nbins, k = b - c * nbins;
+    double t = 0.0;
+    for (int w = 0; w < nwb; w++) {
+      const float *p = acc0 + 6 * (size_t)w * nbins + 2 * c * nbins + k;
+      t += (double)p[0] + (double)p[nbins];
+    }
+    a.block_part[(long long)blockIdx.x * 3 * nbins + b] = t;
+  }
 }
 
-int mgp_launch_pofk_mu(const float *dk, int N, const int *rk_bin, const float *win, int nbins, double *block_part,
-                       int nblocks, double *sums, cudaStream_t st) {
-  size_t shmem = sizeof(double) * 3 * (size_t)nbins;
+int mgp_launch_pofk_mu(const float *dk, int N, const int *thr, const float *win, int nbins, int bintype, double kmin,
+                       double kmax, int los, int planar, double *block_part, int nblocks, double *sums,
+                       cudaStream_t st) {
+  mgp_pofk_kargs ka;
+  memset(&ka, 0, sizeof(ka));
+  ka.dk = (const float2 *)dk;
+  ka.N = N;
+  ka.nbins = nbins;
+  ka.bintype = bintype;
+  ka.thr = thr;
+  ka.win = win;
+  ka.kmin = (float)kmin;
+  ka.kmax = (float)kmax;
+  ka.block_part = block_part;
+  ka.planar = planar;
+  // as many warps a block as the bins leave room for
+  int threads = MGP_MU_THREADS;
+  const size_t tables = sizeof(int) * (size_t)(nbins + 1) + sizeof(float) * (size_t)(N / 2 + 1);
+  while (threads > 32 && tables + 24 * (size_t)nbins * (threads / 32) > 100 * 1024) threads /= 2;
+  ka.priv = tables + 24 * (size_t)nbins <= 200 * 1024;
+  const size_t shmem = (ka.priv ? tables : 0) + 24 * (size_t)nbins * (threads / 32);
   if (shmem > 48 * 1024) {
-    if (cudaFuncSetAttribute(k_pofk_mu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_pofk_mu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem) != cudaSuccess) {
+      cudaGetLastError();
       return mgp_set_error(MGP_EINVAL, "RSD P(k) needs %zu bytes of shared memory", shmem);
+    }
   }
-  k_pofk_mu<<<nblocks, MGP_THREADS, shmem, st>>>((const float2 *)dk, N, rk_bin, win, nbins, block_part);
+  MGP_CUDA(cudaMemsetAsync(block_part + (size_t)nblocks * 3 * nbins, 0, sizeof(double) * 3 * nbins, st));
+  k_pofk_mu<<<nblocks, threads, shmem, st>>>(ka, los);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
-  k_pofk_reduce<<<(3 * nbins + 127) / 128, 128, 0, st>>>(block_part, nblocks, 3 * nbins, sums, 0, 0);
+  k_pofk_reduce<<<(3 * nbins + 127) / 128, 128, 0, st>>>(block_part, nblocks + 1, 3 * nbins, sums, 0, 0);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;

@@ -788,9 +788,10 @@ int mgp_particles_canonical(mgp_ctx *c) {
   return MGP_OK;
 }
 
-// Bucket the particles of every box by tile of side T (their current
-// positions).
-int mgp_tiles_sort(mgp_ctx *c, int T) {
+// Bucket the particles of every box by tile of side T at the displacements s (c->s:
+// their current positions; with another array the sort describes that one, and
+// tile_ready is cleared by the caller).
+int mgp_tiles_sort(mgp_ctx *c, int T, const float *s) {
   int rc = mgp_tiles_alloc(c, T);
   if (rc != MGP_OK) return rc;
   const int N = c->g.N, Ns = c->Ns, nt1 = c->tile_n1, ntz = c->tile_nz, B = c->nbox;
@@ -804,10 +805,10 @@ int mgp_tiles_sort(mgp_ctx *c, int T) {
   MGP_CUDA(cudaMemsetAsync(c->tile_count, 0, sizeof(unsigned) * (size_t)ntiles, c->stream));
   const dim3 gk(mgp_blocks_per_box(c->np, 8, B), B);
   if (ls >= 0)
-    k_tile_key<true><<<gk, kThreads, 0, c->stream>>>(c->s, c->dstate, c->np, Ns, ls, N, scale, sx, sz, nt1, ntz, qp,
+    k_tile_key<true><<<gk, kThreads, 0, c->stream>>>(s, c->dstate, c->np, Ns, ls, N, scale, sx, sz, nt1, ntz, qp,
                                                      c->tile_of, c->tile_count);
   else
-    k_tile_key<false><<<gk, kThreads, 0, c->stream>>>(c->s, c->dstate, c->np, Ns, ls, N, scale, sx, sz, nt1, ntz, qp,
+    k_tile_key<false><<<gk, kThreads, 0, c->stream>>>(s, c->dstate, c->np, Ns, ls, N, scale, sx, sz, nt1, ntz, qp,
                                                       c->tile_of, c->tile_count);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
@@ -861,10 +862,11 @@ int mgp_cic_tiles(mgp_ctx *c, float wpar, int per_sm) {
   return MGP_OK;
 }
 
-// Single-box tile deposit with owner writes (after mgp_tiles_sort; the
-// mesh needs no pre-set): k_cic_tiles_own stores every tile's interior and
-// its halo pairs, k_cic_halo adds the halos and the listed particles.
-int mgp_cic_tiles_own(mgp_ctx *c, float wpar) {
+// Single-box tile deposit with owner writes of the displacements s onto rho (after
+// mgp_tiles_sort of the same s; the mesh needs no pre-set): k_cic_tiles_own stores
+// every tile's interior and its halo pairs, k_cic_halo adds the halos and the
+// listed particles.
+int mgp_cic_tiles_own(mgp_ctx *c, float wpar, const float *s, float *rho) {
   if (c->nbox != 1 || !c->tile_ready) return mgp_set_error(MGP_ESTATE, "owner-writes deposit without a current tile sort");
   const int N = c->g.N, Ns = c->Ns, T = c->tile_side, nt1 = c->tile_n1, ntz = c->tile_nz;
   if (c->g.P != N + 2) return mgp_set_error(MGP_EINVAL, "mesh rows of %lld floats, expected %d", c->g.P, N + 2);
@@ -890,12 +892,12 @@ int mgp_cic_tiles_own(mgp_ctx *c, float wpar) {
   const int nh = mgp_blocks_for(ntiles * pairs, 8);
 #define MGP_CIC_OWN(TT, PP)                                                                                          \
   do {                                                                                                               \
-    k_cic_tiles_own<TT, PP><<<nb, kThreads, 0, c->stream>>>(c->s, c->dstate, c->np, Ns, ls, N, scale, wpar, c->rho, \
+    k_cic_tiles_own<TT, PP><<<nb, kThreads, 0, c->stream>>>(s, c->dstate, c->np, Ns, ls, N, scale, wpar, rho,       \
                                                             c->g.P, c->tile_off, c->tile_order, c->q_alt, nt1, ntz, \
                                                             halo, c->tile_spill, nspill);                            \
     MGP_CHECK_LAUNCH();                                                                                              \
     g_kernel_launches++;                                                                                             \
-    k_cic_halo<TT, PP><<<nh, kThreads, 0, c->stream>>>(halo, nt1, ntz, c->rho, c->g.P, c->s, c->dstate, c->np, Ns,  \
+    k_cic_halo<TT, PP><<<nh, kThreads, 0, c->stream>>>(halo, nt1, ntz, rho, c->g.P, s, c->dstate, c->np, Ns,        \
                                                        ls, N, scale, wpar, c->tile_order, c->q_alt, c->tile_spill,   \
                                                        nspill);                                                      \
     MGP_CHECK_LAUNCH();                                                                                              \
