@@ -337,17 +337,23 @@ __global__ void __launch_bounds__(MGP_THREADS, 4) k_pofk(mgp_pofk_kargs a) {
   }
 }
 
-// Deterministic cross-block sum in FP64 (the MPI_Allreduce of compute_pofk.c:225).
+// Cross-block sum in FP64 (the MPI_Allreduce of compute_pofk.c:225), one warp per
+// bin: each lane its blocks in order, then a fixed shuffle tree, so the sums do not
+// depend on scheduling.  (One thread per bin walked 608 dependent loads: 80 us a
+// call at 256 bins, as long as the binning of a 256^3 mesh.)
 __global__ void k_pofk_reduce(const double *__restrict__ block_part, int nblocks, int nbins, double *__restrict__ sums,
                               long long part_bs, long long sum_bs) {
   block_part += blockIdx.y * part_bs;
   sums += blockIdx.y * sum_bs;
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (b >= nbins) return;
   double s = 0.0;
-  for (int k = 0; k < nblocks; k++) s += block_part[(long long)k * nbins + b];
-  sums[b] = s;
+#pragma unroll 4
+  for (int k = lane; k < nblocks; k += 32) s += block_part[(long long)k * nbins + b];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) sums[b] = s;
 }
+static int reduce_blocks(int nbins) { return (int)((32LL * nbins + 127) / 128); }
 
 static int launch_pofk(mgp_pofk_kargs ka, int nblocks, double *sums, cudaStream_t st, int nbox = 1,
                        long long sum_bs = 0) {
@@ -363,7 +369,7 @@ static int launch_pofk(mgp_pofk_kargs ka, int nblocks, double *sums, cudaStream_
   k_pofk<<<dim3(nblocks, nbox), MGP_THREADS, shmem, st>>>(ka);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
-  k_pofk_reduce<<<dim3((ka.nbins + 127) / 128, nbox), 128, 0, st>>>(ka.block_part, nblocks, ka.nbins, sums, ka.part_bs,
+  k_pofk_reduce<<<dim3(reduce_blocks(ka.nbins), nbox), 128, 0, st>>>(ka.block_part, nblocks, ka.nbins, sums, ka.part_bs,
                                                                    sum_bs);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
@@ -1955,7 +1961,7 @@ int mgp_launch_pofk_mu(const float *dk, int N, const int *thr, const float *win,
   k_pofk_mu<<<nblocks, threads, shmem, st>>>(ka, los);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
-  k_pofk_reduce<<<(3 * nbins + 127) / 128, 128, 0, st>>>(block_part, nblocks + 1, 3 * nbins, sums, 0, 0);
+  k_pofk_reduce<<<reduce_blocks(3 * nbins), 128, 0, st>>>(block_part, nblocks + 1, 3 * nbins, sums, 0, 0);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;

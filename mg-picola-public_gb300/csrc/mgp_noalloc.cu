@@ -102,11 +102,14 @@ __global__ void k_na_geometry(int N, const int *rkbin, unsigned *rkcnt, int *bin
   const int h = N / 2, rkmax = 3 * h * h;
   const long long nthr = (long long)gridDim.x * blockDim.x;
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  for (long long t = t0; t < (long long)(h + 1) * (h + 1); t += nthr) {
-    int d0 = (int)(t / (h + 1)), d1 = (int)(t % (h + 1));
-    unsigned m = ((d0 == 0 || d0 == h) ? 1u : 2u) * ((d1 == 0 || d1 == h) ? 1u : 2u);
-    int base = d0 * d0 + d1 * d1;
-    for (int d2 = 0; d2 <= h; d2++) atomicAdd(&rkcnt[base + d2 * d2], m * ((d2 == 0 || d2 == h) ? 1u : 2u));
+  // a warp per (d0, d1 >= d0), lanes along d2
+  const int lane = threadIdx.x & 31;
+  for (long long t = t0 >> 5; t < (long long)(h + 1) * (h + 1); t += nthr >> 5) {
+    const int d0 = (int)(t / (h + 1)), d1 = (int)(t % (h + 1));
+    if (d1 < d0) continue;
+    const unsigned m = ((d0 == 0 || d0 == h) ? 1u : 2u) * ((d1 == 0 || d1 == h) ? 1u : 2u) * (d0 == d1 ? 1u : 2u);
+    const int base = d0 * d0 + d1 * d1;
+    for (int d2 = lane; d2 <= h; d2 += 32) atomicAdd(&rkcnt[base + d2 * d2], m * ((d2 == 0 || d2 == h) ? 1u : 2u));
   }
   for (long long rk = t0; rk <= rkmax; rk += nthr) {
     int b = rkbin[rk];
@@ -140,7 +143,8 @@ __global__ void k_na_binsum(int nbins, const unsigned *rkcnt, const int *binrk, 
   }
 }
 
-// Normalisation and shot noise (compute_pofk.c:229-236): out = [P, kmean, n].
+// Normalisation and shot noise (compute_pofk.c:229-236): out = [P, kmean, n],
+// nbins each.
 __global__ void k_na_finalize(int nbins, const double *sums, const double *geo_n, const double *geo_k, double norm,
                               double shot, double kunit, double *out) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -151,8 +155,8 @@ __global__ void k_na_finalize(int nbins, const double *sums, const double *geo_n
     K = geo_k[b] / n * kunit;
   }
   out[b] = P;
-  out[MGP_NA_MAX_BINS + b] = K;
-  out[2 * MGP_NA_MAX_BINS + b] = n;
+  out[nbins + b] = K;
+  out[2 * nbins + b] = n;
 }
 
 extern "C" int mgp_pofk_noalloc(const float *d_deltak, int Nmesh, int Nsample, double Box, int nbins, int bintype,
@@ -196,7 +200,7 @@ extern "C" int mgp_pofk_noalloc(const float *d_deltak, int Nmesh, int Nsample, d
   k_na_tables<<<(3 * h * h + 256) / 256, 256, 0, st>>>(Nmesh, kmin, kmax, nbins, bintype, rkbin, rkcnt, binrk, win);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
-  k_na_geometry<<<mgp_blocks_for((long long)(h + 1) * (h + 1), 8), 256, 0, st>>>(Nmesh, rkbin, rkcnt, binrk);
+  k_na_geometry<<<mgp_blocks_for(32LL * (h + 1) * (h + 1), 8), 256, 0, st>>>(Nmesh, rkbin, rkcnt, binrk);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   k_na_binsum<<<(nbins * 32 + 255) / 256, 256, 0, st>>>(nbins, rkcnt, binrk, geo_n, geo_k);
@@ -212,10 +216,14 @@ extern "C" int mgp_pofk_noalloc(const float *d_deltak, int Nmesh, int Nsample, d
   k_na_finalize<<<(nbins + 127) / 128, 128, 0, st>>>(nbins, sums, geo_n, geo_k, norm, shot, 2.0 * M_PI / Box, out);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
-  MGP_CUDA(cudaMemcpyAsync(pk, out, sizeof(double) * nbins, cudaMemcpyDeviceToHost, st));
-  if (kmean) MGP_CUDA(cudaMemcpyAsync(kmean, out + MGP_NA_MAX_BINS, sizeof(double) * nbins, cudaMemcpyDeviceToHost, st));
-  if (n) MGP_CUDA(cudaMemcpyAsync(n, out + 2 * MGP_NA_MAX_BINS, sizeof(double) * nbins, cudaMemcpyDeviceToHost, st));
+  // one copy for the three arrays (each copy to pageable memory waits for the
+  // stream)
+  double res[3 * MGP_NA_MAX_BINS];
+  MGP_CUDA(cudaMemcpyAsync(res, out, sizeof(double) * 3 * nbins, cudaMemcpyDeviceToHost, st));
   MGP_CUDA(cudaStreamSynchronize(st));
+  memcpy(pk, res, sizeof(double) * nbins);
+  if (kmean) memcpy(kmean, res + nbins, sizeof(double) * nbins);
+  if (n) memcpy(n, res + 2 * nbins, sizeof(double) * nbins);
   if (k)
     for (int b = 0; b < nbins; b++)
       k[b] = (bintype == 0 ? (kmin + (kmax - kmin) / (double)nbins * b)
