@@ -128,9 +128,16 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 // Forward convolution, persistent: a CTA keeps all weights in shared memory
 // and walks tiles of CT_I x CT_J output rows (i, j) by CT_SEG voxels (k).
 // For a tile it stages the (CT_I+2) x (CT_J+2) input rows around it, each
-// with one halo voxel on either side (cp.async), so a staged row serves up
-// to 9 output rows; warp w computes output row (i0 + w / CT_J, j0 + w % CT_J)
-// as 4 groups of 16 voxels, reusing each tap's B fragment for the 4 groups.
+// with one halo voxel on either side (cp.async).  A warp computes four output
+// rows in j by 32 voxels: an input fragment (row, k shift, 16 voxels) it loads
+// serves up to three of its rows, so it issues 135 ldmatrix for 432 MMAs.  (One
+// output row by 64 voxels a warp took 135 for 216, and shared memory, 71% busy,
+// held the tensor pipe at 47%: 352 us a layer at 192^3; now 260, the pipe 65%
+// busy, and 178 for the last layer's one n-tile.)  What is left is the wait on
+// dependent MMAs and fragments with 16 warps an SM.  Rows are copied by a warp
+// each, so an index is worked out once a row.  Per output the taps are added in
+// ascending order, as with one row a warp.  NT: n-tiles of 8
+// output channels (1 for the last layer, whose channels 3..15 are zero).
 // Shared-memory layout of a [voxel][16] bf16 row: the two 16-byte halves of
 // voxel q are swapped when bit 2 of q is set, so the 8 row addresses of any
 // ldmatrix (8 consecutive voxels or 8 consecutive output channels) fall in 8
@@ -139,10 +146,10 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 // (data gradient through the previous layer's ReLU, gate = its output); 2: f32
 // out [V][4] (channels 0-3), bias; 3: out + bias into three padded real
 // grids (channels 0-2; grid c at frc + c gstride, rows of P floats).
-constexpr int CT_I = 2, CT_J = 4, CT_SEG = 64;
+constexpr int CT_I = 4, CT_J = 4, CT_SEG = 64;
 constexpr int CT_ROWS = (CT_I + 2) * (CT_J + 2);  // staged rows
 constexpr int CT_Q = CT_SEG + 2;                  // staged voxels per row
-constexpr int kThreadsConv = 32 * CT_I * CT_J;    // one warp per output row
+constexpr int kThreadsConv = 32 * CT_I * 2;       // a warp per i and half segment
 constexpr size_t kConvSmem = sizeof(bf16) * (NN_WSIZE + (size_t)CT_ROWS * CT_Q * NN_CH);
 
 __device__ __forceinline__ int swz_half(int q, int h) { return h ^ ((q >> 2) & 1); }
@@ -153,7 +160,26 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
-__global__ void __launch_bounds__(kThreadsConv, 3) k_conv_fwd(const bf16 *__restrict__ X, const bf16 *__restrict__ W,
+__device__ __forceinline__ int wrap(int i, int N) { return i < 0 ? i + N : (i >= N ? i - N : i); }
+
+// One warp copies the staged voxels q = 0 .. count - 1 (k = k0 + q, periodic) of the
+// row at `row` ([N][16] bf16); those past qmax are zero.
+template <int COUNT>
+__device__ __forceinline__ void stage_row(bf16 *dst, const bf16 *__restrict__ row, int k0, int N, int qmax, int lane) {
+#pragma unroll
+  for (int c0 = 0; c0 < 2 * COUNT; c0 += 32) {
+    const int c = c0 + lane, q = c >> 1, h = c & 1;
+    if (2 * COUNT % 32 && c >= 2 * COUNT) break;
+    bf16 *d = dst + q * NN_CH + 8 * swz_half(q, h);
+    if (q > qmax)
+      *reinterpret_cast<uint4 *>(d) = make_uint4(0, 0, 0, 0);
+    else
+      cp_async16(d, row + wrap(k0 + q, N) * NN_CH + 8 * h);
+  }
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kThreadsConv, 2) k_conv_fwd(const bf16 *__restrict__ X, const bf16 *__restrict__ W,
                                                               const float *__restrict__ bias,
                                                               const bf16 *__restrict__ gate, int N, int mode,
                                                               bf16 *__restrict__ Y16, float *__restrict__ Y32,
@@ -169,7 +195,7 @@ __global__ void __launch_bounds__(kThreadsConv, 3) k_conv_fwd(const bf16 *__rest
   }
   const int nseg = (N + CT_SEG - 1) / CT_SEG, tiles_j = N / CT_J;
   const long long ntiles = (long long)(N / CT_I) * tiles_j * nseg;
-  const int wi = warp / CT_J, wj = warp % CT_J;
+  const int wi = warp >> 1, kh = 32 * (warp & 1);  // the warp's i and first voxel in the segment
   // ldmatrix lane roles: A (16 voxels x 16 ch), B (16 out x 16 in)
   const int a_vox = (lane & 7) + 8 * ((lane >> 3) & 1), a_half = lane >> 4;
   const int b_out = (lane & 7) + 8 * (lane >> 4), b_half = (lane >> 3) & 1;
@@ -180,89 +206,100 @@ __global__ void __launch_bounds__(kThreadsConv, 3) k_conv_fwd(const bf16 *__rest
     const int i0 = (int)(rest / tiles_j) * CT_I, j0 = (int)(rest % tiles_j) * CT_J, k0 = seg * CT_SEG;
     const int qmax = min(CT_SEG + 1, N - k0 + 1);  // staged voxels past qmax are zero
     __syncthreads();  // the previous tile's reads of xs are done
-    for (int c = tid; c < CT_ROWS * CT_Q * 2; c += kThreadsConv) {
-      const int r = c / (CT_Q * 2), rem = c - r * (CT_Q * 2), q = rem >> 1, h = rem & 1;
-      bf16 *dst = &xs[r][q][8 * swz_half(q, h)];
-      if (q > qmax) {
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-        continue;
-      }
-      int ii = i0 + r / (CT_J + 2) - 1, jj = j0 + r % (CT_J + 2) - 1, kk = k0 - 1 + q;
-      ii += ii < 0 ? N : 0;
-      ii -= ii >= N ? N : 0;
-      jj += jj < 0 ? N : 0;
-      jj -= jj >= N ? N : 0;
-      kk += kk < 0 ? N : 0;
-      kk -= kk >= N ? N : 0;
-      cp_async16(dst, X + (((long long)ii * N + jj) * N + kk) * NN_CH + 8 * h);
+    for (int r = warp; r < CT_ROWS; r += kThreadsConv / 32) {
+      const int ii = wrap(i0 + r / (CT_J + 2) - 1, N), jj = wrap(j0 + r % (CT_J + 2) - 1, N);
+      stage_row<CT_Q>(&xs[r][0][0], X + (size_t)(ii * N + jj) * N * NN_CH, k0 - 1, N, qmax, lane);
     }
     cp_async_wait_all();
     __syncthreads();
-    const int ng = min(4, (N - k0) / 16);  // valid 16-voxel groups (N is a multiple of 16)
-    float acc[4][2][4];
+    const int ng = min(2, (N - k0 - kh) / 16);  // valid 16-voxel groups (N is a multiple of 16)
+    if (ng <= 0) continue;
+    float acc[CT_J][2][NT][4];
 #pragma unroll
-    for (int g = 0; g < 4; g++)
+    for (int w = 0; w < CT_J; w++)
 #pragma unroll
-      for (int n = 0; n < 2; n++)
+      for (int g = 0; g < 2; g++)
 #pragma unroll
-        for (int q = 0; q < 4; q++) acc[g][n][q] = 0.f;
-#pragma unroll 3
-    for (int tap = 0; tap < NN_TAPS; tap++) {
-      const int di = tap / 9, dj = (tap / 3) % 3, dk = tap % 3;
-      const int r = (wi + di) * (CT_J + 2) + (wj + dj);
-      uint32_t b0, b1, b2, b3;
-      ldsm_x4(smem_u32(&ws[tap * NN_CH + b_out][8 * swz_half(b_out, b_half)]), b0, b1, b2, b3);
+        for (int n = 0; n < NT; n++)
 #pragma unroll
-      for (int g = 0; g < 4; g++) {
-        if (g < ng) {
-          const int q = 16 * g + a_vox + dk;
-          uint32_t a0, a1, a2, a3;
-          ldsm_x4(smem_u32(&xs[r][q][8 * swz_half(q, a_half)]), a0, a1, a2, a3);
-          mma16816(acc[g][0], a0, a1, a2, a3, b0, b1);
-          mma16816(acc[g][1], a0, a1, a2, a3, b2, b3);
+          for (int q = 0; q < 4; q++) acc[w][g][n][q] = 0.f;
+#pragma unroll 1
+    for (int di = 0; di < 3; di++) {
+      uint32_t b[9][4];
+#pragma unroll
+      for (int q = 0; q < 9; q++)
+        ldsm_x4(smem_u32(&ws[(9 * di + q) * NN_CH + b_out][8 * swz_half(b_out, b_half)]), b[q][0], b[q][1], b[q][2],
+                b[q][3]);
+#pragma unroll
+      for (int jr = 0; jr < CT_J + 2; jr++) {
+#pragma unroll
+        for (int dk = 0; dk < 3; dk++) {
+#pragma unroll
+          for (int g = 0; g < 2; g++) {
+            if (g < ng) {
+              const int q = kh + 16 * g + a_vox + dk;
+              uint32_t a0, a1, a2, a3;
+              ldsm_x4(smem_u32(&xs[(wi + di) * (CT_J + 2) + jr][q][8 * swz_half(q, a_half)]), a0, a1, a2, a3);
+#pragma unroll
+              for (int w = 0; w < CT_J; w++) {
+                const int dj = jr - w;
+                if (dj < 0 || dj > 2) continue;
+                const uint32_t *bt = b[3 * dj + dk];
+                mma16816(acc[w][g][0], a0, a1, a2, a3, bt[0], bt[1]);
+                if (NT > 1) mma16816(acc[w][g][NT - 1], a0, a1, a2, a3, bt[2], bt[3]);
+              }
+            }
+          }
         }
       }
     }
     // fragment: rows (voxels) lane/4 and lane/4 + 8, columns 2 (lane%4) + {0,1}
-    const int i = i0 + wi, j = j0 + wj;
+    const int i = i0 + wi;
 #pragma unroll
-    for (int g = 0; g < 4; g++) {
-      if (g >= ng) continue;
-      const int kw = k0 + 16 * g;
-      const long long vb = ((long long)i * N + j) * N + kw;
+    for (int w = 0; w < CT_J; w++) {
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const long long v = vb + vr + 8 * h;
-        float o[4] = {acc[g][0][2 * h], acc[g][0][2 * h + 1], acc[g][1][2 * h], acc[g][1][2 * h + 1]};  // cc, cc+1, cc+8, cc+9
-        if (mode != 1 && bias) {
-          o[0] += bias[cc];
-          o[1] += bias[cc + 1];
-          o[2] += bias[cc + 8];
-          o[3] += bias[cc + 9];
-        }
-        if (mode <= 1) {
-          if (mode == 0) {
+      for (int g = 0; g < 2; g++) {
+        if (g >= ng) continue;
+        const int j = j0 + w, kw = k0 + kh + 16 * g;
+        const size_t vb = (size_t)(i * N + j) * N + kw + vr;
 #pragma unroll
-            for (int q = 0; q < 4; q++) o[q] = fmaxf(o[q], 0.f);
-          } else if (gate) {
-            const __nv_bfloat162 g0 = reinterpret_cast<const __nv_bfloat162 *>(gate + v * NN_CH + cc)[0];
-            const __nv_bfloat162 g1 = reinterpret_cast<const __nv_bfloat162 *>(gate + v * NN_CH + cc + 8)[0];
-            if (!(__bfloat162float(g0.x) > 0.f)) o[0] = 0.f;
-            if (!(__bfloat162float(g0.y) > 0.f)) o[1] = 0.f;
-            if (!(__bfloat162float(g1.x) > 0.f)) o[2] = 0.f;
-            if (!(__bfloat162float(g1.y) > 0.f)) o[3] = 0.f;
+        for (int h = 0; h < 2; h++) {
+          const size_t v = vb + 8 * h;
+          // channels cc, cc + 1, cc + 8, cc + 9
+          float o[4] = {acc[w][g][0][2 * h], acc[w][g][0][2 * h + 1], acc[w][g][NT - 1][2 * h],
+                        acc[w][g][NT - 1][2 * h + 1]};
+          if (mode != 1 && bias) {
+            o[0] += bias[cc];
+            o[1] += bias[cc + 1];
+            if (NT > 1) {
+              o[2] += bias[cc + 8];
+              o[3] += bias[cc + 9];
+            }
           }
-          reinterpret_cast<__nv_bfloat162 *>(Y16 + v * NN_CH + cc)[0] = __floats2bfloat162_rn(o[0], o[1]);
-          reinterpret_cast<__nv_bfloat162 *>(Y16 + v * NN_CH + cc + 8)[0] = __floats2bfloat162_rn(o[2], o[3]);
-        } else if (cc < 4) {
-          if (mode == 2) {
-            Y32[v * 4 + cc] = o[0];
-            Y32[v * 4 + cc + 1] = o[1];
-          } else {
-            const int kk = kw + vr + 8 * h;
-            const long long gi = ((long long)i * N + j) * P + kk;
-            frc[cc * gstride + gi] = o[0];
-            if (cc + 1 < 3) frc[(cc + 1) * gstride + gi] = o[1];
+          if (NT > 1) {  // modes 0 and 1
+            if (mode == 0) {
+#pragma unroll
+              for (int q = 0; q < 4; q++) o[q] = fmaxf(o[q], 0.f);
+            } else if (gate) {
+              const __nv_bfloat162 g0 = reinterpret_cast<const __nv_bfloat162 *>(gate + v * NN_CH + cc)[0];
+              const __nv_bfloat162 g1 = reinterpret_cast<const __nv_bfloat162 *>(gate + v * NN_CH + cc + 8)[0];
+              if (!(__bfloat162float(g0.x) > 0.f)) o[0] = 0.f;
+              if (!(__bfloat162float(g0.y) > 0.f)) o[1] = 0.f;
+              if (!(__bfloat162float(g1.x) > 0.f)) o[2] = 0.f;
+              if (!(__bfloat162float(g1.y) > 0.f)) o[3] = 0.f;
+            }
+            reinterpret_cast<__nv_bfloat162 *>(Y16 + v * NN_CH + cc)[0] = __floats2bfloat162_rn(o[0], o[1]);
+            reinterpret_cast<__nv_bfloat162 *>(Y16 + v * NN_CH + cc + 8)[0] = __floats2bfloat162_rn(o[2], o[3]);
+          } else if (cc < 4) {
+            if (mode == 2) {
+              Y32[v * 4 + cc] = o[0];
+              Y32[v * 4 + cc + 1] = o[1];
+            } else {
+              const int kk = kw + vr + 8 * h;
+              const long long gi = ((long long)i * N + j) * P + kk;
+              frc[cc * gstride + gi] = o[0];
+              if (cc + 1 < 3) frc[(cc + 1) * gstride + gi] = o[1];
+            }
           }
         }
       }
@@ -270,115 +307,122 @@ __global__ void __launch_bounds__(kThreadsConv, 3) k_conv_fwd(const bf16 *__rest
   }
 }
 
-// Weight and bias gradients, dW[tap][o][c] = sum_v dY[v][o] X[v + d(tap)][c]
-// and db[o] = sum_v dY[v][o], over the same tiles as the forward kernel: a
-// persistent block stages the 4 x 6 input rows and the 8 dY rows of a tile
-// (cp.async, swizzled rows), and warp w owns the three taps dk = 0..2 of
-// staged-row offset (di, dj) = (w / 3, w % 3): for each output row it loads
-// the dY^T fragments once (ldmatrix.trans) and runs them against the three
-// dk-shifted X fragments; warp o < 8 also multiplies output row o's dY^T by a
-// ones fragment for the bias.  Sums stay in registers across tiles and are
-// written once per block to `partial` [block][NN_WSIZE + 8 x 16]; a second
-// kernel adds the blocks in a fixed order (deterministic gradients).
-constexpr int kThreadsWg = 32 * 9;
-constexpr int kWgPartial = NN_WSIZE + 8 * NN_CH;
-constexpr size_t kWgSmem = sizeof(bf16) * ((size_t)CT_ROWS * CT_Q * NN_CH + (size_t)CT_I * CT_J * CT_SEG * NN_CH);
+// Weight and bias gradients, dW[tap][o][c] = sum_v dY[v][o] X[v + d(tap)][c] and
+// db[o] = sum_v dY[v][o]: a persistent block walks tiles of 2 x 4 output rows by 64
+// voxels, the next tile's 4 x 6 X rows and 8 dY rows copied (cp.async) while this
+// one is computed.  Warp (dk, ks) owns the nine taps of its k shift and 16 of the
+// 64 voxels: it holds the dY^T fragments of the 8 rows (ldmatrix.trans) and runs
+// every X fragment against all of them whose tap it is, 32 ldmatrix for 144 MMAs;
+// the dk = 1 warps also multiply dY^T by a ones fragment for the bias.  (A warp
+// per staged-row offset, three taps, took 4 for 6: 384 us a layer at 192^3; now
+// 315, the tensor pipe 55% busy with the 12 warps that the sums leave room for.)
+// Sums stay in registers across tiles; at the end the four voxel quarters are
+// added in order in shared memory and written once per block to `partial`
+// [block][NN_WSIZE + NN_CH]; a second kernel adds the blocks in a fixed order
+// (deterministic gradients).  NT: n-tiles of 8 input channels (1 for the first
+// layer, whose channels 3..15 are zero).
+constexpr int WG_I = 2, WG_J = 4, WG_ROWS = (WG_I + 2) * (WG_J + 2), WG_OUT = WG_I * WG_J;
+constexpr int kThreadsWg = 32 * 12;
+constexpr int kWgPartial = NN_WSIZE + NN_CH;
+constexpr int kWgX = WG_ROWS * CT_Q * NN_CH, kWgY = WG_OUT * CT_SEG * NN_CH;  // bf16 values of a buffer
+constexpr size_t kWgSmem = 2 * sizeof(bf16) * (size_t)(kWgX + kWgY);
 
-__global__ void __launch_bounds__(kThreadsWg, 3) k_conv_wgrad(const bf16 *__restrict__ X, const bf16 *__restrict__ dY,
+template <int NT>
+__global__ void __launch_bounds__(kThreadsWg, 1) k_conv_wgrad(const bf16 *__restrict__ X, const bf16 *__restrict__ dY,
                                                               int N, float *__restrict__ partial) {
   extern __shared__ __align__(16) unsigned char wg_smem[];
-  bf16(*xs)[CT_Q][NN_CH] = reinterpret_cast<bf16(*)[CT_Q][NN_CH]>(wg_smem);
-  bf16(*ys)[CT_SEG][NN_CH] =
-      reinterpret_cast<bf16(*)[CT_SEG][NN_CH]>(wg_smem + sizeof(bf16) * (size_t)CT_ROWS * CT_Q * NN_CH);
+  bf16 *buf = reinterpret_cast<bf16 *>(wg_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rdi = warp / 3, rdj = warp % 3;
-  float acc[3][2][4], bacc[4] = {0.f, 0.f, 0.f, 0.f};
+  const int dk = warp % 3, ks = warp / 3;
+  float acc[9][NT][4], bacc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int t = 0; t < 3; t++)
+  for (int t = 0; t < 9; t++)
 #pragma unroll
-    for (int n = 0; n < 2; n++)
+    for (int n = 0; n < NT; n++)
 #pragma unroll
       for (int q = 0; q < 4; q++) acc[t][n][q] = 0.f;
   const uint32_t ones = 0x3F803F80u;  // two bf16 1.0
   // ldmatrix.trans lane roles: A = dY^T (16 out x 16 voxels), B = X (16 voxels x 16 in)
   const int a_vox = (lane & 7) + 8 * (lane >> 4), a_half = (lane >> 3) & 1;
   const int b_vox = (lane & 7) + 8 * ((lane >> 3) & 1), b_half = lane >> 4;
-  const int nseg = (N + CT_SEG - 1) / CT_SEG, tiles_j = N / CT_J;
-  const long long ntiles = (long long)(N / CT_I) * tiles_j * nseg;
-  for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int seg = (int)(t % nseg);
-    const long long rest = t / nseg;
-    const int i0 = (int)(rest / tiles_j) * CT_I, j0 = (int)(rest % tiles_j) * CT_J, k0 = seg * CT_SEG;
-    const int qmax = min(CT_SEG + 1, N - k0 + 1);  // staged voxels past qmax are zero
-    __syncthreads();                              // the previous tile's reads are done
-    for (int c = tid; c < CT_ROWS * CT_Q * 2; c += kThreadsWg) {
-      const int r = c / (CT_Q * 2), rem = c - r * (CT_Q * 2), q = rem >> 1, h = rem & 1;
-      bf16 *dst = &xs[r][q][8 * swz_half(q, h)];
-      if (q > qmax) {
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-        continue;
-      }
-      int ii = i0 + r / (CT_J + 2) - 1, jj = j0 + r % (CT_J + 2) - 1, kk = k0 - 1 + q;
-      ii += ii < 0 ? N : 0;
-      ii -= ii >= N ? N : 0;
-      jj += jj < 0 ? N : 0;
-      jj -= jj >= N ? N : 0;
-      kk += kk < 0 ? N : 0;
-      kk -= kk >= N ? N : 0;
-      cp_async16(dst, X + (((long long)ii * N + jj) * N + kk) * NN_CH + 8 * h);
-    }
-    for (int c = tid; c < CT_I * CT_J * CT_SEG * 2; c += kThreadsWg) {
-      const int o = c / (CT_SEG * 2), rem = c - o * (CT_SEG * 2), q = rem >> 1, h = rem & 1;
-      bf16 *dst = &ys[o][q][8 * swz_half(q, h)];
-      const int kk = k0 + q;
-      if (kk >= N) {
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-        continue;
-      }
-      const int i = i0 + o / CT_J, j = j0 + o % CT_J;
-      cp_async16(dst, dY + (((long long)i * N + j) * N + kk) * NN_CH + 8 * h);
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    const int ng = min(CT_SEG / 16, (N - k0) / 16);  // 16-voxel steps holding data
-    for (int o = 0; o < CT_I * CT_J; o++) {
-      const int r = (o / CT_J + rdi) * (CT_J + 2) + (o % CT_J + rdj);
-#pragma unroll
-      for (int ks = 0; ks < CT_SEG / 16; ks++) {
-        if (ks >= ng) break;
-        const int qa = 16 * ks + a_vox;
-        uint32_t a0, a1, a2, a3;
-        ldsm_x4_t(smem_u32(&ys[o][qa][8 * swz_half(qa, a_half)]), a0, a1, a2, a3);
-        if (o == warp) mma16816(bacc, a0, a1, a2, a3, ones, ones);
-#pragma unroll
-        for (int dk = 0; dk < 3; dk++) {
-          const int qb = 16 * ks + dk + b_vox;
-          uint32_t b0, b1, b2, b3;
-          ldsm_x4_t(smem_u32(&xs[r][qb][8 * swz_half(qb, b_half)]), b0, b1, b2, b3);
-          mma16816(acc[dk][0], a0, a1, a2, a3, b0, b1);
-          mma16816(acc[dk][1], a0, a1, a2, a3, b2, b3);
+  const int nseg = (N + CT_SEG - 1) / CT_SEG, tiles_j = N / WG_J;
+  const int ntiles = (N / WG_I) * tiles_j * nseg;
+  auto stage = [&](int t, int slot) {
+    if (t < ntiles) {
+      bf16 *xs = buf + slot * (kWgX + kWgY), *ys = xs + kWgX;
+      const int seg = t % nseg, rest = t / nseg;
+      const int i0 = rest / tiles_j * WG_I, j0 = rest % tiles_j * WG_J, k0 = seg * CT_SEG;
+      const int qmax = min(CT_SEG + 1, N - k0 + 1);  // staged voxels past qmax are zero
+      for (int r = warp; r < WG_ROWS + WG_OUT; r += kThreadsWg / 32) {
+        if (r < WG_ROWS) {
+          const int ii = wrap(i0 + r / (WG_J + 2) - 1, N), jj = wrap(j0 + r % (WG_J + 2) - 1, N);
+          stage_row<CT_Q>(xs + r * CT_Q * NN_CH, X + (size_t)(ii * N + jj) * N * NN_CH, k0 - 1, N, qmax, lane);
+        } else {
+          const int o = r - WG_ROWS, i = i0 + o / WG_J, j = j0 + o % WG_J;
+          stage_row<CT_SEG>(ys + o * CT_SEG * NN_CH, dY + (size_t)(i * N + j) * N * NN_CH, k0, N, N - k0 - 1, lane);
         }
       }
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  int slot = 0;
+  stage((int)blockIdx.x, 0);
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x, slot ^= 1) {
+    stage(t + (int)gridDim.x, slot ^ 1);
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    __syncthreads();
+    const bf16 *xs = buf + slot * (kWgX + kWgY), *ys = xs + kWgX;
+    if (16 * ks < N - t % nseg * CT_SEG) {  // the warp's voxels hold data
+      uint32_t a[WG_OUT][4];
+#pragma unroll
+      for (int o = 0; o < WG_OUT; o++) {
+        const int q = 16 * ks + a_vox;
+        ldsm_x4_t(smem_u32(ys + (o * CT_SEG + q) * NN_CH + 8 * swz_half(q, a_half)), a[o][0], a[o][1], a[o][2], a[o][3]);
+        if (dk == 1) mma16816(bacc, a[o][0], a[o][1], a[o][2], a[o][3], ones, ones);
+      }
+#pragma unroll
+      for (int r = 0; r < WG_ROWS; r++) {
+        const int q = 16 * ks + dk + b_vox;
+        uint32_t b0, b1, b2, b3;
+        ldsm_x4_t(smem_u32(xs + (r * CT_Q + q) * NN_CH + 8 * swz_half(q, b_half)), b0, b1, b2, b3);
+#pragma unroll
+        for (int o = 0; o < WG_OUT; o++) {
+          const int di = r / (WG_J + 2) - o / WG_J, dj = r % (WG_J + 2) - o % WG_J;
+          if (di < 0 || di > 2 || dj < 0 || dj > 2) continue;
+          mma16816(acc[3 * di + dj][0], a[o][0], a[o][1], a[o][2], a[o][3], b0, b1);
+          if (NT > 1) mma16816(acc[3 * di + dj][NT - 1], a[o][0], a[o][1], a[o][2], a[o][3], b2, b3);
+        }
+      }
+    }
+    __syncthreads();  // this buffer is staged again in the next round
   }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
   // fragment: rows (out) lane/4, lane/4 + 8; columns (in) 2 (lane%4) + {0,1} (+8 for n-tile 1)
-  float *pb = partial + (size_t)blockIdx.x * kWgPartial;
+  float *sum = reinterpret_cast<float *>(wg_smem);  // [tap][out][in], then the bias
+  for (int e = tid; e < kWgPartial; e += kThreadsWg) sum[e] = 0.f;
   const int o0 = lane >> 2, c0 = 2 * (lane & 3);
+  for (int turn = 0; turn < 4; turn++) {
+    __syncthreads();
+    if (turn != ks) continue;
 #pragma unroll
-  for (int dk = 0; dk < 3; dk++) {
-    float *w = pb + (3 * warp + dk) * NN_CH * NN_CH;
+    for (int t = 0; t < 9; t++)
 #pragma unroll
-    for (int n = 0; n < 2; n++) {
-      w[o0 * NN_CH + c0 + 8 * n] = acc[dk][n][0];
-      w[o0 * NN_CH + c0 + 8 * n + 1] = acc[dk][n][1];
-      w[(o0 + 8) * NN_CH + c0 + 8 * n] = acc[dk][n][2];
-      w[(o0 + 8) * NN_CH + c0 + 8 * n + 1] = acc[dk][n][3];
+      for (int n = 0; n < NT; n++) {
+        float *w = sum + (3 * t + dk) * NN_CH * NN_CH + c0 + 8 * n;
+        w[o0 * NN_CH] += acc[t][n][0];
+        w[o0 * NN_CH + 1] += acc[t][n][1];
+        w[(o0 + 8) * NN_CH] += acc[t][n][2];
+        w[(o0 + 8) * NN_CH + 1] += acc[t][n][3];
+      }
+    if (dk == 1 && (lane & 3) == 0) {  // every column of the ones product holds the row sum
+      sum[NN_WSIZE + o0] += bacc[0];
+      sum[NN_WSIZE + o0 + 8] += bacc[2];
     }
   }
-  if (warp < CT_I * CT_J && (lane & 3) == 0) {  // every column of the ones product holds the row sum
-    pb[NN_WSIZE + warp * NN_CH + o0] = bacc[0];
-    pb[NN_WSIZE + warp * NN_CH + o0 + 8] = bacc[2];
-  }
+  __syncthreads();
+  float *pb = partial + (size_t)blockIdx.x * kWgPartial;
+  for (int e = tid; e < kWgPartial; e += kThreadsWg) pb[e] = sum[e];
 }
 
 // dW and db from the per-block partial sums in a fixed order: thread row ty
@@ -389,13 +433,8 @@ __global__ void k_wgrad_reduce(const float *__restrict__ partial, int nblk, floa
   __shared__ float sh[8][32];
   const int tx = threadIdx.x, ty = threadIdx.y, e = blockIdx.x * 32 + tx;
   float s = 0.f;
-  if (e < NN_WSIZE) {
+  if (e < kWgPartial)
     for (int b = ty; b < nblk; b += 8) s += partial[(size_t)b * kWgPartial + e];
-  } else if (e < NN_WSIZE + NN_CH) {
-    const int c = e - NN_WSIZE;
-    for (int b = ty; b < nblk; b += 8)
-      for (int w = 0; w < 8; w++) s += partial[(size_t)b * kWgPartial + NN_WSIZE + w * NN_CH + c];
-  }
   sh[ty][tx] = s;
   __syncthreads();
   if (ty == 0) {
@@ -870,39 +909,41 @@ static int highpass_grids(mgp_closure *cl, float *g, cudaStream_t st) {
   return MGP_OK;
 }
 
+// Resident blocks of a persistent kernel on the closure's device.
+template <class K>
+static int resident(const mgp_closure *cl, K kernel, int threads, size_t smem, int *grid) {
+  MGP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0, sms = 0;
+  MGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem));
+  MGP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cl->device));
+  *grid = sms * (per_sm > 0 ? per_sm : 1);
+  return MGP_OK;
+}
+
 static int conv_fwd(mgp_closure *cl, const bf16 *X, const bf16 *W, const float *bias, const bf16 *gate, int mode,
                     bf16 *Y16, float *Y32,
                     float *frc, long long gstride, long long P, float scale) {
-  static int grid = 0;  // resident CTAs of the persistent kernel (one device per process)
-  if (!grid) {
-    MGP_CUDA(cudaFuncSetAttribute(k_conv_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kConvSmem));
-    int per_sm = 0, sms = 0;
-    MGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv_fwd, kThreadsConv, kConvSmem));
-    MGP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cl->device));
-    grid = sms * (per_sm > 0 ? per_sm : 1);
-  }
+  const auto kernel = mode >= 2 ? k_conv_fwd<1> : k_conv_fwd<2>;
+  static int grids[2] = {0, 0};  // (one device per process)
+  int &grid = grids[mode >= 2];
+  if (!grid) NN_RET(resident(cl, kernel, kThreadsConv, kConvSmem, &grid));
   const int N = cl->N;
   const long long tiles = (long long)(N / CT_I) * (N / CT_J) * ((N + CT_SEG - 1) / CT_SEG);
   const unsigned blocks = (unsigned)(tiles < grid ? tiles : grid);
-  k_conv_fwd<<<blocks, kThreadsConv, kConvSmem, cl->stream>>>(X, W, bias, gate, N, mode, Y16, Y32, frc, gstride, P,
-                                                              scale);
+  kernel<<<blocks, kThreadsConv, kConvSmem, cl->stream>>>(X, W, bias, gate, N, mode, Y16, Y32, frc, gstride, P, scale);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
 }
 
-static int conv_wgrad(mgp_closure *cl, const bf16 *X, const bf16 *dY, float *dW, float *db) {
-  static int grid = 0;  // resident blocks of the persistent kernel (one device per process)
-  if (!grid) {
-    MGP_CUDA(cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem));
-    MGP_CUDA(cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    int per_sm = 0, sms = 0;
-    MGP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv_wgrad, kThreadsWg, kWgSmem));
-    MGP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cl->device));
-    grid = sms * (per_sm > 0 ? per_sm : 1);
-  }
+// first: X holds the network's inputs (channels 3..15 zero)
+static int conv_wgrad(mgp_closure *cl, const bf16 *X, const bf16 *dY, float *dW, float *db, bool first) {
+  const auto kernel = first ? k_conv_wgrad<1> : k_conv_wgrad<2>;
+  static int grids[2] = {0, 0};  // (one device per process)
+  int &grid = grids[first];
+  if (!grid) NN_RET(resident(cl, kernel, kThreadsWg, kWgSmem, &grid));
   const int N = cl->N;
-  const long long tiles = (long long)(N / CT_I) * (N / CT_J) * ((N + CT_SEG - 1) / CT_SEG);
+  const long long tiles = (long long)(N / WG_I) * (N / WG_J) * ((N + CT_SEG - 1) / CT_SEG);
   const int blocks = (int)(tiles < grid ? tiles : grid);
   if (cl->wg_blocks < blocks) {
     if (cl->wg_partial) cudaFree(cl->wg_partial);
@@ -911,9 +952,9 @@ static int conv_wgrad(mgp_closure *cl, const bf16 *X, const bf16 *dY, float *dW,
     MGP_CUDA(cudaMalloc(&cl->wg_partial, sizeof(float) * (size_t)kWgPartial * blocks));
     cl->wg_blocks = blocks;
   }
-  k_conv_wgrad<<<blocks, kThreadsWg, kWgSmem, cl->stream>>>(X, dY, N, cl->wg_partial);
+  kernel<<<blocks, kThreadsWg, kWgSmem, cl->stream>>>(X, dY, N, cl->wg_partial);
   MGP_CHECK_LAUNCH();
-  k_wgrad_reduce<<<(NN_WSIZE + NN_CH + 31) / 32, dim3(32, 8), 0, cl->stream>>>(cl->wg_partial, blocks, dW, db);
+  k_wgrad_reduce<<<(kWgPartial + 31) / 32, dim3(32, 8), 0, cl->stream>>>(cl->wg_partial, blocks, dW, db);
   MGP_CHECK_LAUNCH();
   g_kernel_launches += 2;
   return MGP_OK;
@@ -961,7 +1002,7 @@ static int closure_backward(mgp_closure *cl) {
   }
   bf16 *g = cl->g0, *gn = cl->g1;
   for (int l = NN_LAYERS - 1; l >= 0; l--) {
-    NN_RET(conv_wgrad(cl, cl->act[l], g, cl->gw[l], cl->gb[l]));
+    NN_RET(conv_wgrad(cl, cl->act[l], g, cl->gw[l], cl->gb[l], l == 0));
     if (l == 0) break;
     k_mirror_transpose<<<(NN_WSIZE + 255) / 256, 256, 0, cl->stream>>>(cl->w16[l], cl->wt16);
     MGP_CHECK_LAUNCH();
