@@ -396,7 +396,7 @@ extern "C" int mgp_destroy(mgp_ctx *c) {
     free(c->box_cosmo);
   }
   free(c->box_p);
-  void *bufs[] = {c->ic_scratch, c->ic_amp, c->ic_box, c->s, c->v, c->D1, c->D2, c->dstate, c->partials, c->stage, c->rho, c->dk, c->frc, c->mg1,
+  void *bufs[] = {c->ic_scratch, c->ic_amp, c->ic_box, c->s, c->v, c->D1, c->D2, c->dstate, c->partials, c->kd_done, c->stage, c->rho, c->dk, c->frc, c->mg1,
                   c->fft_work, c->rk_bin, c->pk_thr, c->win1d, c->pk_block, c->pk_sum, c->rsd_block, c->rsd_sum,
                   c->pk_sum_tot, c->nu_tab_d, c->nu_row_d, c->nu_x_d, c->nu_den_d, c->scr_tab};
   for (size_t i = 0; i < sizeof(bufs) / sizeof(bufs[0]); i++)
@@ -456,7 +456,7 @@ static int create_impl(const mgp_params *p, int nbox, const mgp_box_params *boxe
   for (int b = 0; b < nbox; b++) c->box_p[b] = boxes ? box_params(p, &boxes[b]) : *p;
   c->p = c->box_p[0];
   c->device = device;
-  c->tile_mode = nbox == 1;
+  c->tile_mode = nbox == 1 ? 2 : 0;
   c->tile_kick = nbox == 1;
   c->fft_mode = 1;
   char err[512] = "";
@@ -527,6 +527,8 @@ static int create_impl(const mgp_params *p, int nbox, const mgp_box_params *boxe
   TRYCUDA(cudaMemset(c->dstate, 0, sizeof(mgp_dstate) * nbox));
   c->max_blocks = mgp_ikd_blocks(c->np) > 4096 ? mgp_ikd_blocks(c->np) : 4096;
   TRYCUDA(cudaMalloc(&c->partials, sizeof(double) * 6 * (size_t)c->max_blocks * nbox));
+  TRYCUDA(cudaMalloc(&c->kd_done, sizeof(unsigned) * nbox));
+  TRYCUDA(cudaMemset(c->kd_done, 0, sizeof(unsigned) * nbox));
   const size_t gbytes = sizeof(float) * (size_t)c->g.nreal * nbox;
   TRYCUDA(cudaMalloc(&c->rho, gbytes));
   TRYCUDA(cudaMalloc(&c->dk, gbytes));
@@ -991,17 +993,24 @@ static int add_neutrinos(mgp_ctx *c, double A, int fuse_kind) {
 
 static int fields_from_density(mgp_ctx *c, double A);
 
+// Tile shape of a single box's deposit, 0: in lattice order.
+static int tile_side(const mgp_ctx *c) {
+  if (!c->tile_mode || (c->tile_mode == 2 && !mgp_tiles_pay(c->g.N))) return 0;
+  return mgp_tile_side(c->g.N, c->np);
+}
+
 extern "C" int mgp_get_displacements(mgp_ctx *c, double A) {
   RET_IF(require_particles(c));
   const int N = c->g.N;
   if (c->cosmo.nu) RET_IF(nu_prepare(c, A));
   // PtoMesh, src/auxPM.c:280-432
-  const bool tiles = c->tile_mode && mgp_tile_side(N, c->np) > 0;
+  const int side = tile_side(c);
+  const bool tiles = side > 0;
   if (tiles) {
     // bucket the particles by cell tile (mgp_tiles.cu) for the deposit and
     // the kick of this step
     tstart(c, T_SORT);
-    RET_IF(mgp_tiles_sort(c, mgp_tile_side(N, c->np), c->s));
+    RET_IF(mgp_tiles_sort(c, side, c->s));
     tstop(c, T_SORT);
   }
   // the tile deposit stores every cell of the mesh itself (owner writes),
@@ -1175,6 +1184,7 @@ static void kd_args(mgp_ctx *c, double AI, double AF, double A, double AFF, int 
   a->inv_scale = (float)(c->p.Box / c->g.N);
   a->kick_disp = (float)(-1.5 * om * dda);
   a->dda_omega = 1.5 * om * dda;
+  a->inv_np = 1.0 / (double)c->np;
   a->do_drift = do_drift;
   if (c->sd) {
     // scale-dependent Kick/Drift (main.c:703-719, 758-770): D1 is the slot of
@@ -1221,20 +1231,18 @@ extern "C" int mgp_kick_drift(mgp_ctx *c, double AI, double AF, double A, double
   }
   mgp_kd_args a;
   kd_args(c, AI, AF, A, AFF, do_drift, &a);
-  int nblk = mgp_ikd_blocks(c->np);
   const float *D1 = c->sd ? c->sd_slot[0] : c->D1, *D2 = c->sd ? c->sd_slot[1] : c->D2;
   tstart(c, T_IKD);
   if (c->tile_kick && c->tile_ready && !c->sd) {
     // per cell tile of this step's deposit sort, forces staged in shared
     // memory; the particle arrays are rewritten in the tile order
-    RET_IF(mgp_ikd_tiles(c, &a, &nblk));
-    RET_IF(mgp_launch_finalize_kd(c->dstate, c->partials, nblk, c->np, a.dda_omega, a.dyyy_d, a.do_drift,
-                                  c->stream));
+    RET_IF(mgp_ikd_tiles(c, &a));
   } else {
     // particles in array order; with the arrays in tile order, q gives the
     // lattice points
     RET_IF(mgp_launch_ikd(c->frc, c->g.nreal, c->g.N, c->g.P, c->Ns, c->np, c->s, c->v, D1, D2, c->dstate,
-                          c->partials, nblk, &a, c->stream, 1, NULL, c->permuted ? c->q : NULL));
+                          c->partials, c->kd_done, mgp_blocks_for(c->np, 4), &a, c->stream, 1, NULL,
+                          c->permuted ? c->q : NULL));
   }
   tstop(c, T_IKD);
   if (do_drift) c->have_density = 0;
@@ -1350,37 +1358,34 @@ extern "C" int mgp_pofk_rsd(mgp_ctx *c, double A, int cap, int *nbins, double *k
     lpitch = c->sd_pitch;
   }
   const double wpar = pow((double)N / (double)c->Ns, 3);
-  // the particles bucketed by cell tile at their redshift-space positions, as the
-  // step's deposit, with the grid axes as they are; where the mesh has no tiles,
-  // the lattice-order deposit with the line of sight on the third axis
-  const int side = c->tile_mode ? mgp_tile_side(N, c->np) : 0;
+  // the particles at their redshift-space positions, deposited as in a step, with
+  // the grid axes as they are
+  const int side = tile_side(c);
   const bool own = own_fft(c);
-  if (side) {
-    RET_IF(ensure_stage(c));
+  RET_IF(ensure_stage(c));
+  if (side)
     c->tile_ready = 0;  // the sort's arrays describe the shifted positions
-  } else {
+  else
     RET_IF(mgp_particles_canonical(c));
-  }
   float *dens = c->frc, *dkr = c->frc + c->g.nreal;
   std::vector<double> sums(3 * (size_t)nb), res[2][3];
   const double norm = pow(p->Box, 3) / pow((double)N, 6), shot = c->pk_sub ? pow(p->Box / (double)c->Ns, 3) : 0.0;
   for (int ax = 0; ax < 2; ax++) {
+    RET_IF(mgp_launch_rsd_shift(c->s, c->v, L1, L2, lstride, lpitch, c->dstate, c->np, c->Ns, ax + 1,
+                                (float)(vnorm * p->Box / N), g1, g2, c->permuted ? c->q : NULL, c->stage, c->stream));
     if (side) {
-      RET_IF(mgp_launch_rsd_shift(c->s, c->v, L1, L2, lstride, lpitch, c->dstate, c->np, c->Ns, ax + 1,
-                                  (float)(vnorm * p->Box / N), g1, g2, c->permuted ? c->q : NULL, c->stage, c->stream));
       RET_IF(mgp_tiles_sort(c, side, c->stage));
       RET_IF(mgp_cic_tiles_own(c, (float)wpar, c->stage, dens));
       c->tile_ready = 0;
     } else {
       RET_IF(mgp_launch_fill(dens, c->g.nreal, -1.0f, c->stream));
-      RET_IF(mgp_launch_cic_rsd(c->s, c->v, L1, L2, lstride, lpitch, c->dstate, c->np, c->Ns, N, p->Box, (float)wpar,
-                                ax + 1, (float)vnorm, g1, g2, dens, c->g.P, c->stream));
+      RET_IF(mgp_launch_cic(c->stage, c->dstate, c->np, c->Ns, N, p->Box, (float)wpar, dens, c->g.P, c->stream));
     }
     if (own)
       RET_IF(mgp_fft_r2c(c, dens, dkr, 1, c->g.nreal));
     else
       MGP_CUFFT(cufftExecR2C(c->plan_r2c_oop, (cufftReal *)dens, (cufftComplex *)dkr));
-    RET_IF(mgp_launch_pofk_mu(dkr, N, c->pk_thr, c->win1d, nb, c->pk_bintype, c->pk_kmin, c->pk_kmax, side ? ax + 1 : 2,
+    RET_IF(mgp_launch_pofk_mu(dkr, N, c->pk_thr, c->win1d, nb, c->pk_bintype, c->pk_kmin, c->pk_kmax, ax + 1,
                               own, c->rsd_block, c->pk_blocks, c->rsd_sum, c->stream));
     MGP_CUDA(cudaMemcpyAsync(sums.data(), c->rsd_sum, sizeof(double) * 3 * nb, cudaMemcpyDeviceToHost, c->stream));
     MGP_CUDA(cudaStreamSynchronize(c->stream));
@@ -1663,6 +1668,7 @@ static void batch_schedule(const mgp_ctx *c, int nsteps, double zf, std::vector<
     q.kd.inv_scale = (float)(p->Box / c->g.N);
     q.kd.kick_disp = (float)(-1.5 * om * dda);
     q.kd.dda_omega = 1.5 * om * dda;
+    q.kd.inv_np = 1.0 / (double)c->np;
     q.kd.do_drift = q.drift;
     q.kd.lpt_stride = c->np;
     q.kd.lpt_pitch = c->Ns;
@@ -1779,8 +1785,8 @@ static int batch_step_launch(mgp_ctx *c, const batch_step &q, const mgp_box_scal
   }
   int nblk = mgp_blocks_per_box(c->np, c->tune[2], B);
   if (nblk > c->max_blocks) nblk = c->max_blocks;  // the per-block partials buffer
-  RET_IF(mgp_launch_ikd(c->frc, gf, N, c->g.P, c->Ns, c->np, c->s, c->v, c->D1, c->D2, c->dstate, c->partials, nblk,
-                        &q.kd, c->stream, B, bs));
+  RET_IF(mgp_launch_ikd(c->frc, gf, N, c->g.P, c->Ns, c->np, c->s, c->v, c->D1, c->D2, c->dstate, c->partials,
+                        c->kd_done, nblk, &q.kd, c->stream, B, bs));
   return MGP_OK;
 }
 

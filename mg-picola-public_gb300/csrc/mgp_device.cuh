@@ -1,7 +1,9 @@
 // Device helpers shared by the PM kernels and the closure kernels: the
-// particle's lattice point and its cell coordinates on a mesh.
+// particle's lattice point, its cell coordinates on a mesh, the means of a kick.
 #ifndef MGP_DEVICE_CUH
 #define MGP_DEVICE_CUH
+
+#include "mgp_internal.h"
 
 // Lattice coordinates of particle p (src/main.c:257-262 ordering).
 __device__ __forceinline__ void lattice_ijk(long long p, int Ns, int &i, int &j, int &k) {
@@ -83,6 +85,60 @@ __host__ __device__ __forceinline__ int lattice_log2(int Ns) {
   return l;
 }
 
+// Means over all particles of the interpolated forces and the new velocities
+// at the end of a kick, and the FP64 offsets they move (Kick and Drift subtract
+// them, src/main.c:688-787).  Every block adds its threads' FP32 sums in FP64
+// and leaves six numbers in `partials`; the block that arrives last at `done`
+// adds the blocks' in index order and updates the state (done returns to 0 for
+// the next launch).  red: 6 NT floats of shared memory that are free.
+// FP64 runs at 1/64 of the FP32 rate here, so the adds are what counts: six
+// warps sum NT / 32 values a lane and then one tree each, instead of six trees
+// in every warp and a serial sum over warps (2^18 particles: 38 us the kick and
+// 11 us a kernel for the blocks' sums; one kernel of 21 us now).
+template <int NT>
+__device__ __forceinline__ void kd_means(const float (&accD)[3], const float (&accV)[3], float *red,
+                                         double *partials, int block, int nblocks, unsigned *done, mgp_dstate *st,
+                                         const mgp_kd_args &a) {
+  __shared__ double tot[6];
+  __shared__ int last;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+    red[q * NT + tid] = accD[q];
+    red[(3 + q) * NT + tid] = accV[q];
+  }
+  __syncthreads();
+  if (w < 6) {
+    double x = 0.0;
+#pragma unroll 4
+    for (int i = 0; i < NT / 32; i++) x += (double)red[w * NT + 32 * i + lane];
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) {
+      partials[(long long)block * 6 + w] = x;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(done, 1u) == (unsigned)nblocks - 1u;
+  __syncthreads();
+  if (!last) return;
+  if (w < 6) {
+    __threadfence();
+    double x = 0.0;
+    for (int b = lane; b < nblocks; b += 32) x += __ldcg(partials + (long long)b * 6 + w);
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) tot[w] = x;
+  }
+  __syncthreads();
+  if (tid < 3) {
+    const double mD = tot[tid] * a.inv_np, mV = tot[3 + tid] * a.inv_np;
+    st->mean_disp[tid] = mD;
+    st->cv[tid] += a.dda_omega * mD;
+    st->mean_v[tid] = mV;
+    if (a.do_drift) st->cx[tid] -= mV * a.dyyy_d;
+  }
+  if (tid == 0) *done = 0u;
+}
 
 // Fourier-space filter of the fifth-force solvers per integer |k|^2 = rk
 // (grid units): kind 1 SmoothDensityField (src/mg.h:268-309) with the

@@ -74,6 +74,7 @@ struct mgp_ctx {
   float *s, *v, *D1, *D2;  /* each 3*np */
   mgp_dstate *dstate;      /* device */
   double *partials;        /* per-block reduction scratch (double) */
+  unsigned *kd_done;       /* blocks of a kick that have left their sums, per box (0 between kicks) */
   float *stage;            /* host-interface staging, stage_arrays x 3 np floats (lazy) */
   int stage_arrays;
   cudaStream_t side;       /* host-buffer step: copies that only the kick waits for */
@@ -193,7 +194,7 @@ struct mgp_ctx {
   size_t tile_halo_bytes;
   unsigned *tile_spill;
   int batch_tile;           /* batch deposit: tile side (8, 16) or 0 for the lattice-order deposit */
-  int tile_mode;            /* 1 (default): tile deposit where it applies; 0: particle order */
+  int tile_mode;            /* tile deposit: 2 (default) where it pays, 1 where it applies, 0 never */
   /* particle arrays held in cell-tile order (single box, scale-independent
    * growth): with tile_kick the kick of every step reads the particles in
    * the deposit's tile order and writes s, v in that order (into the *_alt
@@ -288,6 +289,7 @@ typedef struct {
   int do_drift;
   double dda_omega;   /* 1.5 * Omega * dda for the velocity offset */
   double dyyy_d;
+  double inv_np;      /* 1 / particles, for the means */
   /* layout of D1/D2: component c of particle (i, j, k) is at
    * c * lpt_stride + (i*Ns + j) * lpt_pitch + k (Np and Ns for the particle
    * arrays, the slot grid size and Ps for the scale-dependent slots) */
@@ -364,11 +366,12 @@ int mgp_launch_forces(const float *dk, const float *mgk, float mg_coupling, floa
                       const mgp_box_scalars *bs = NULL);
 int mgp_launch_ikd(const float *frc, long long grid_floats, int N, long long P, int Ns, long long np,
                    float *s, float *v, const float *D1, const float *D2, mgp_dstate *dst,
-                   double *partials, int nblocks, const mgp_kd_args *a, cudaStream_t st, int nbox = 1,
+                   double *partials, unsigned *done, int nblocks, const mgp_kd_args *a, cudaStream_t st, int nbox = 1,
                    const mgp_box_scalars *bs = NULL, const unsigned *qlat = NULL);
 int mgp_ikd_blocks(long long np);
 /* cell-tile order (mgp_tiles.cu) */
 int mgp_tile_side(int N, long long np);
+bool mgp_tiles_pay(int N);
 int mgp_tiles_check(const mgp_ctx *c, int T);
 int mgp_tiles_alloc(mgp_ctx *c, int T);
 void mgp_tiles_free(mgp_ctx *c);
@@ -378,7 +381,7 @@ int mgp_cic_tiles(mgp_ctx *c, float wpar, int per_sm = 0);
 int mgp_cic_tiles_own(mgp_ctx *c, float wpar, const float *s, float *rho);
 /* kick + drift in the order of the last mgp_tiles_sort, the particle
  * arrays rewritten in that order */
-int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a, int *nblocks_out);
+int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a);
 /* lattice order of the particle arrays (no-op unless permuted) */
 int mgp_particles_canonical(mgp_ctx *c);
 int mgp_launch_nu_table(float *tab, int nrk, double kfac, double fac, const double *x, const double *val,
@@ -420,9 +423,6 @@ int mgp_launch_ic_grad6(const float *dk, float *out6, long long grid_floats, int
 int mgp_launch_ic_source(float *g6, long long grid_floats, int N, long long P, cudaStream_t st);
 int mgp_launch_ic_disp(const float *dk, const float *src, float *out6, long long grid_floats, int N, double box,
                        cudaStream_t st);
-int mgp_launch_cic_rsd(const float *s, const float *v, const float *D1, const float *D2, long long lpt_stride,
-                       int lpt_pitch, const mgp_dstate *st, long long np, int Ns, int N, double box, float wpar,
-                       int axis, float vnorm, float g1, float g2, float *rho, long long P, cudaStream_t stream);
 int mgp_launch_rsd_shift(const float *s, const float *v, const float *D1, const float *D2, long long lpt_stride,
                          int lpt_pitch, const mgp_dstate *st, long long np, int Ns, int axis, float shift, float g1,
                          float g2, const unsigned *qlat, float *out, cudaStream_t stream);
@@ -441,8 +441,6 @@ int mgp_launch_ic_readout(const float *g6, long long grid_floats, int N, long lo
                           float *D1, float *D2, double *partials, int nblocks, cudaStream_t st);
 int mgp_launch_ic_finish(float *D1, float *D2, float *s, float *v, long long np, const double *partials,
                          int nblocks, float Di, float Di2, float vD, float vD2, cudaStream_t st);
-int mgp_launch_finalize_kd(mgp_dstate *dst, const double *partials, int nblocks, long long np,
-                           double dda_omega, double dyyy, int do_drift, cudaStream_t st);
 int mgp_launch_positions(const float *s, const mgp_dstate *dst, long long np, int Ns, double box,
                          float *out_pos, float *out_vel, const float *v, cudaStream_t st,
                          const unsigned *qlat = NULL);

@@ -124,6 +124,13 @@ __global__ void __launch_bounds__(MGP_THREADS) k_cic(const float *__restrict__ s
     const IDX y0 = (IDX)iy * Pi, y1 = (iy + 1 == N ? 0 : (IDX)(iy + 1) * Pi);
     const IDX z0 = (IDX)iz, z1 = (iz + 1 == N ? 0 : (IDX)(iz + 1));
     float *r00 = rho + (x0 + y0), *r01 = rho + (x0 + y1), *r10 = rho + (x1 + y0), *r11 = rho + (x1 + y1);
+    if (!(iz & 1) && iz + 1 < N) {  // mesh rows have even length: the pair is 8-byte aligned
+      atomicAdd(reinterpret_cast<float2 *>(r00 + z0), make_float2(TX * TY * TZ, TX * TY * DZ));
+      atomicAdd(reinterpret_cast<float2 *>(r01 + z0), make_float2(TX * DY * TZ, TX * DY * DZ));
+      atomicAdd(reinterpret_cast<float2 *>(r10 + z0), make_float2(DX * TY * TZ, DX * TY * DZ));
+      atomicAdd(reinterpret_cast<float2 *>(r11 + z0), make_float2(DX * DY * TZ, DX * DY * DZ));
+      continue;
+    }
     atomicAdd(r00 + z0, TX * TY * TZ);
     atomicAdd(r00 + z1, TX * TY * DZ);
     atomicAdd(r01 + z0, TX * DY * TZ);
@@ -510,7 +517,7 @@ int mgp_launch_forces(const float *dk, const float *mgk, float mg_coupling, floa
 //   x += (v - <v>) dyyy + UseCOLA (D1 dD + D2 dD2).
 // The global means only shift all velocities (or all positions) by one
 // vector, so the kernel applies the particle-local part and carries the
-// uniform part in the FP64 offsets cv / cx (k_finalize_kd), which removes
+// uniform part in the FP64 offsets cv / cx (kd_means), which removes
 // the two extra passes over the particles the reference makes.
 __device__ __forceinline__ double block_sum_d(double v, double *sh) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -532,9 +539,9 @@ template <typename IDX, bool P2>
 __global__ void __launch_bounds__(MGP_THREADS, 4) k_interp_kick_drift(
     const float *__restrict__ frc, long long gf, int N, long long P, int Ns, long long np, float *__restrict__ s,
     float *__restrict__ v, const float *__restrict__ D1, const float *__restrict__ D2,
-    const mgp_dstate *__restrict__ st, double *__restrict__ partials, mgp_kd_args a,
+    mgp_dstate *st, double *__restrict__ partials, unsigned *__restrict__ done, mgp_kd_args a,
     const mgp_box_scalars *__restrict__ bs, int ls, const unsigned *__restrict__ qlat) {
-  __shared__ double sh[MGP_THREADS / 32];
+  __shared__ float red[6 * MGP_THREADS];
   {
     // box blockIdx.y of a batch: force grids 3 gf apart, particle arrays 3 np
     const int bx = blockIdx.y;
@@ -545,6 +552,7 @@ __global__ void __launch_bounds__(MGP_THREADS, 4) k_interp_kick_drift(
     D2 += bx * 3 * a.lpt_stride;
     st += bx;
     partials += (long long)bx * gridDim.x * 6;
+    done += bx;
     if (bs) {
       a.kick_d1 = bs[bx].kick_d1;
       a.kick_d2 = bs[bx].kick_d2;
@@ -611,80 +619,30 @@ __global__ void __launch_bounds__(MGP_THREADS, 4) k_interp_kick_drift(
       accV[ax] += vn;
     }
   }
-#pragma unroll
-  for (int q = 0; q < 3; q++) {
-    double t = block_sum_d((double)accD[q], sh);
-    if (threadIdx.x == 0) partials[(long long)blockIdx.x * 6 + q] = t;
-    t = block_sum_d((double)accV[q], sh);
-    if (threadIdx.x == 0) partials[(long long)blockIdx.x * 6 + 3 + q] = t;
-  }
-}
-
-// Means over all particles and offset update (one block, fixed order).
-__global__ void k_finalize_kd(mgp_dstate *st, const double *__restrict__ partials, int nblocks, double inv_np,
-                              double dda_omega, double dyyy, int do_drift) {
-  __shared__ double sh[6][MGP_THREADS / 32];
-  st += blockIdx.x;  // one block per box
-  partials += (long long)blockIdx.x * nblocks * 6;
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nblocks; b += blockDim.x)
-    for (int q = 0; q < 6; q++) acc[q] += partials[(long long)b * 6 + q];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int q = 0; q < 6; q++) {
-    double x = acc[q];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[q][w] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t[6];
-    for (int q = 0; q < 6; q++) {
-      t[q] = 0.0;
-      for (int k = 0; k < (int)(blockDim.x >> 5); k++) t[q] += sh[q][k];
-    }
-    for (int ax = 0; ax < 3; ax++) {
-      double mD = t[ax] * inv_np, mV = t[3 + ax] * inv_np;
-      st->mean_disp[ax] = mD;
-      st->cv[ax] += dda_omega * mD;
-      st->mean_v[ax] = mV;
-      if (do_drift) st->cx[ax] -= mV * dyyy;
-    }
-  }
+  kd_means<MGP_THREADS>(accD, accV, red, partials, blockIdx.x, gridDim.x, done, st, a);
 }
 
 int mgp_ikd_blocks(long long np) { return blocks_for(np, 8); }
 
 int mgp_launch_ikd(const float *frc, long long gf, int N, long long P, int Ns, long long np, float *s, float *v,
-                   const float *D1, const float *D2, mgp_dstate *dst, double *partials, int nblocks,
+                   const float *D1, const float *D2, mgp_dstate *dst, double *partials, unsigned *done, int nblocks,
                    const mgp_kd_args *a, cudaStream_t st, int nbox, const mgp_box_scalars *bs,
                    const unsigned *qlat) {
   const dim3 g(nblocks, nbox);
   const int ls = lattice_log2(Ns);
   const bool p2 = ls >= 0 && np <= 0xffffffffLL;
   if (gf < (1LL << 31) && p2)
-    k_interp_kick_drift<int, true><<<g, MGP_THREADS, 0, st>>>(frc, gf, N, P, Ns, np, s, v, D1, D2, dst, partials, *a,
+    k_interp_kick_drift<int, true><<<g, MGP_THREADS, 0, st>>>(frc, gf, N, P, Ns, np, s, v, D1, D2, dst, partials, done, *a,
                                                               bs, ls, qlat);
   else if (gf < (1LL << 31))
-    k_interp_kick_drift<int, false><<<g, MGP_THREADS, 0, st>>>(frc, gf, N, P, Ns, np, s, v, D1, D2, dst, partials, *a,
+    k_interp_kick_drift<int, false><<<g, MGP_THREADS, 0, st>>>(frc, gf, N, P, Ns, np, s, v, D1, D2, dst, partials, done, *a,
                                                                bs, ls, qlat);
   else if (p2)
     k_interp_kick_drift<long long, true><<<g, MGP_THREADS, 0, st>>>(frc, gf, N, P, Ns, np, s, v, D1, D2, dst, partials,
-                                                                    *a, bs, ls, qlat);
+                                                                    done, *a, bs, ls, qlat);
   else
     k_interp_kick_drift<long long, false><<<g, MGP_THREADS, 0, st>>>(frc, gf, N, P, Ns, np, s, v, D1, D2, dst,
-                                                                     partials, *a, bs, ls, qlat);
-  MGP_CHECK_LAUNCH();
-  g_kernel_launches++;
-  k_finalize_kd<<<nbox, MGP_THREADS, 0, st>>>(dst, partials, nblocks, 1.0 / (double)np, a->dda_omega, a->dyyy_d,
-                                              a->do_drift);
-  MGP_CHECK_LAUNCH();
-  g_kernel_launches++;
-  return MGP_OK;
-}
-
-int mgp_launch_finalize_kd(mgp_dstate *dst, const double *partials, int nblocks, long long np, double dda_omega,
-                           double dyyy, int do_drift, cudaStream_t st) {
-  k_finalize_kd<<<1, MGP_THREADS, 0, st>>>(dst, partials, nblocks, 1.0 / (double)np, dda_omega, dyyy, do_drift);
+                                                                     partials, done, *a, bs, ls, qlat);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
@@ -1707,65 +1665,12 @@ int mgp_launch_output(const float *s, const float *v, const float *D1, const flo
 }
 
 // ------------------------------------------------------ RSD multipoles
-// PtoMesh_RSD (src/compute_pofk.c:280-393): CIC in redshift space with the
-// line of sight mapped onto the grid's third axis (y LOS: grid axes (x, z, y);
-// z LOS: (x, y, z)); the LOS coordinate moves by V * vnorm cells with
-// V = Vel + UseCOLA (D1 dD/dy + D2 dD2/dy) (the reference does not subtract
-// the mean velocity here) and wraps periodically.
-__global__ void __launch_bounds__(MGP_THREADS) k_cic_rsd(const float *__restrict__ s, const float *__restrict__ v,
-                                                         const float *__restrict__ D1, const float *__restrict__ D2,
-                                                         long long lstride, int lpitch,
-                                                         const mgp_dstate *__restrict__ st, long long np, int Ns,
-                                                         int N, float scale, float wpar, int axis, float vnorm,
-                                                         float g1, float g2, float *__restrict__ rho, long long P) {
-  const int map[2][3] = {{0, 2, 1}, {0, 1, 2}};  // grid axis g takes particle axis map[.][g]
-  const int *m = map[axis == 1 ? 0 : 1];
-  float off[3];
-  for (int g = 0; g < 3; g++) off[g] = (float)(st->cx[m[g]] * scale);
-  const float cvl = (float)st->cv[m[2]];
-  long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += stride) {
-    int li[3];
-    lattice_ijk(p, Ns, li[0], li[1], li[2]);
-    const long long ol = m[2] * np + p;
-    const long long od = m[2] * lstride + ((long long)li[0] * Ns + li[1]) * lpitch + li[2];
-    float V = (v[ol] + cvl) + D1[od] * g1 + D2[od] * g2;
-    int ix, iy, iz;
-    float DX, DY, DZ;
-    cell_frac(li[m[0]], s[m[0] * np + p], off[0], N, Ns, scale, ix, DX);
-    cell_frac(li[m[1]], s[m[1] * np + p], off[1], N, Ns, scale, iy, DY);
-    cell_frac(li[m[2]], s[ol], off[2] + V * vnorm, N, Ns, scale, iz, DZ);
-    float TX = 1.0f - DX, TY = (1.0f - DY) * wpar, TZ = 1.0f - DZ;
-    DY *= wpar;
-    int ixn = ix + 1 == N ? 0 : ix + 1, iyn = iy + 1 == N ? 0 : iy + 1, izn = iz + 1 == N ? 0 : iz + 1;
-    long long r00 = ((long long)ix * N + iy) * P, r01 = ((long long)ix * N + iyn) * P;
-    long long r10 = ((long long)ixn * N + iy) * P, r11 = ((long long)ixn * N + iyn) * P;
-    atomicAdd(rho + r00 + iz, TX * TY * TZ);
-    atomicAdd(rho + r00 + izn, TX * TY * DZ);
-    atomicAdd(rho + r01 + iz, TX * DY * TZ);
-    atomicAdd(rho + r01 + izn, TX * DY * DZ);
-    atomicAdd(rho + r10 + iz, DX * TY * TZ);
-    atomicAdd(rho + r10 + izn, DX * TY * DZ);
-    atomicAdd(rho + r11 + iz, DX * DY * TZ);
-    atomicAdd(rho + r11 + izn, DX * DY * DZ);
-  }
-}
-
-int mgp_launch_cic_rsd(const float *s, const float *v, const float *D1, const float *D2, long long lpt_stride,
-                       int lpt_pitch, const mgp_dstate *st, long long np, int Ns, int N, double box, float wpar,
-                       int axis, float vnorm, float g1, float g2, float *rho, long long P, cudaStream_t stream) {
-  k_cic_rsd<<<blocks_for(np, 8), MGP_THREADS, 0, stream>>>(s, v, D1, D2, lpt_stride, lpt_pitch, st, np, Ns, N,
-                                                           (float)(N / box), wpar, axis, vnorm, g1, g2, rho, P);
-  MGP_CHECK_LAUNCH();
-  g_kernel_launches++;
-  return MGP_OK;
-}
-
-// The displacements in redshift space for the tile deposit (PtoMesh_RSD,
-// src/compute_pofk.c:280-393): component `axis` moved by V shift, V as in k_cic_rsd,
-// shift in Mpc/h per unit of V; the axes stay the grid's, and the binning takes
-// mu along the line of sight's own axis.  qlat: the lattice point of every slot
-// when the arrays are in tile order.
+// The displacements in redshift space (PtoMesh_RSD, src/compute_pofk.c:280-393), for
+// the deposit of a step: component `axis` moved by V shift, with
+// V = Vel + UseCOLA (D1 dD/dy + D2 dD2/dy) (the reference does not subtract the
+// mean velocity here) and shift in Mpc/h per unit of V; the axes stay the grid's,
+// and the binning takes mu along the line of sight's own axis.  qlat: the lattice
+// point of every slot when the arrays are in tile order.
 __global__ void __launch_bounds__(MGP_THREADS) k_rsd_shift(const float *__restrict__ s, const float *__restrict__ v,
                                                            const float *__restrict__ D1, const float *__restrict__ D2,
                                                            long long lstride, int lpitch,

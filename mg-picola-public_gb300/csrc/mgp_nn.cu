@@ -126,9 +126,9 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 }
 
 // Forward convolution, persistent: a CTA keeps all weights in shared memory
-// and walks tiles of CT_I x CT_J output rows (i, j) by CT_SEG voxels (k).
-// For a tile it stages the (CT_I+2) x (CT_J+2) input rows around it, each
-// with one halo voxel on either side (cp.async).  A warp computes four output
+// and walks tiles of CT_I x CJ output rows (i, j) by CT_SEG voxels (k).
+// For a tile it stages the (CT_I+2) x (CJ+2) input rows around it, each
+// with one halo voxel on either side (cp.async).  A warp computes CJ = 4 output
 // rows in j by 32 voxels: an input fragment (row, k shift, 16 voxels) it loads
 // serves up to three of its rows, so it issues 135 ldmatrix for 432 MMAs.  (One
 // output row by 64 voxels a warp took 135 for 216, and shared memory, 71% busy,
@@ -146,11 +146,14 @@ __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1
 // (data gradient through the previous layer's ReLU, gate = its output); 2: f32
 // out [V][4] (channels 0-3), bias; 3: out + bias into three padded real
 // grids (channels 0-2; grid c at frc + c gstride, rows of P floats).
-constexpr int CT_I = 4, CT_J = 4, CT_SEG = 64;
-constexpr int CT_ROWS = (CT_I + 2) * (CT_J + 2);  // staged rows
+constexpr int CT_I = 4, CT_SEG = 64;
 constexpr int CT_Q = CT_SEG + 2;                  // staged voxels per row
 constexpr int kThreadsConv = 32 * CT_I * 2;       // a warp per i and half segment
-constexpr size_t kConvSmem = sizeof(bf16) * (NN_WSIZE + (size_t)CT_ROWS * CT_Q * NN_CH);
+template <int CJ>
+struct conv_tile {
+  static constexpr int ROWS = (CT_I + 2) * (CJ + 2);  // staged rows
+  static constexpr size_t SMEM = sizeof(bf16) * (NN_WSIZE + (size_t)ROWS * CT_Q * NN_CH);
+};
 
 __device__ __forceinline__ int swz_half(int q, int h) { return h ^ ((q >> 2) & 1); }
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
@@ -178,7 +181,7 @@ __device__ __forceinline__ void stage_row(bf16 *dst, const bf16 *__restrict__ ro
   }
 }
 
-template <int NT>
+template <int NT, int CJ>
 __global__ void __launch_bounds__(kThreadsConv, 2) k_conv_fwd(const bf16 *__restrict__ X, const bf16 *__restrict__ W,
                                                               const float *__restrict__ bias,
                                                               const bf16 *__restrict__ gate, int N, int mode,
@@ -193,7 +196,7 @@ __global__ void __launch_bounds__(kThreadsConv, 2) k_conv_fwd(const bf16 *__rest
     const int row = c >> 1, h = c & 1;  // row = tap * 16 + out
     cp_async16(&ws[row][8 * swz_half(row & 15, h)], W + (size_t)c * 8);
   }
-  const int nseg = (N + CT_SEG - 1) / CT_SEG, tiles_j = N / CT_J;
+  const int nseg = (N + CT_SEG - 1) / CT_SEG, tiles_j = N / CJ;
   const long long ntiles = (long long)(N / CT_I) * tiles_j * nseg;
   const int wi = warp >> 1, kh = 32 * (warp & 1);  // the warp's i and first voxel in the segment
   // ldmatrix lane roles: A (16 voxels x 16 ch), B (16 out x 16 in)
@@ -203,20 +206,20 @@ __global__ void __launch_bounds__(kThreadsConv, 2) k_conv_fwd(const bf16 *__rest
   for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int seg = (int)(t % nseg);
     const long long rest = t / nseg;
-    const int i0 = (int)(rest / tiles_j) * CT_I, j0 = (int)(rest % tiles_j) * CT_J, k0 = seg * CT_SEG;
+    const int i0 = (int)(rest / tiles_j) * CT_I, j0 = (int)(rest % tiles_j) * CJ, k0 = seg * CT_SEG;
     const int qmax = min(CT_SEG + 1, N - k0 + 1);  // staged voxels past qmax are zero
     __syncthreads();  // the previous tile's reads of xs are done
-    for (int r = warp; r < CT_ROWS; r += kThreadsConv / 32) {
-      const int ii = wrap(i0 + r / (CT_J + 2) - 1, N), jj = wrap(j0 + r % (CT_J + 2) - 1, N);
+    for (int r = warp; r < conv_tile<CJ>::ROWS; r += kThreadsConv / 32) {
+      const int ii = wrap(i0 + r / (CJ + 2) - 1, N), jj = wrap(j0 + r % (CJ + 2) - 1, N);
       stage_row<CT_Q>(&xs[r][0][0], X + (size_t)(ii * N + jj) * N * NN_CH, k0 - 1, N, qmax, lane);
     }
     cp_async_wait_all();
     __syncthreads();
     const int ng = min(2, (N - k0 - kh) / 16);  // valid 16-voxel groups (N is a multiple of 16)
     if (ng <= 0) continue;
-    float acc[CT_J][2][NT][4];
+    float acc[CJ][2][NT][4];
 #pragma unroll
-    for (int w = 0; w < CT_J; w++)
+    for (int w = 0; w < CJ; w++)
 #pragma unroll
       for (int g = 0; g < 2; g++)
 #pragma unroll
@@ -231,7 +234,7 @@ __global__ void __launch_bounds__(kThreadsConv, 2) k_conv_fwd(const bf16 *__rest
         ldsm_x4(smem_u32(&ws[(9 * di + q) * NN_CH + b_out][8 * swz_half(b_out, b_half)]), b[q][0], b[q][1], b[q][2],
                 b[q][3]);
 #pragma unroll
-      for (int jr = 0; jr < CT_J + 2; jr++) {
+      for (int jr = 0; jr < CJ + 2; jr++) {
 #pragma unroll
         for (int dk = 0; dk < 3; dk++) {
 #pragma unroll
@@ -239,9 +242,9 @@ __global__ void __launch_bounds__(kThreadsConv, 2) k_conv_fwd(const bf16 *__rest
             if (g < ng) {
               const int q = kh + 16 * g + a_vox + dk;
               uint32_t a0, a1, a2, a3;
-              ldsm_x4(smem_u32(&xs[(wi + di) * (CT_J + 2) + jr][q][8 * swz_half(q, a_half)]), a0, a1, a2, a3);
+              ldsm_x4(smem_u32(&xs[(wi + di) * (CJ + 2) + jr][q][8 * swz_half(q, a_half)]), a0, a1, a2, a3);
 #pragma unroll
-              for (int w = 0; w < CT_J; w++) {
+              for (int w = 0; w < CJ; w++) {
                 const int dj = jr - w;
                 if (dj < 0 || dj > 2) continue;
                 const uint32_t *bt = b[3 * dj + dk];
@@ -256,7 +259,7 @@ __global__ void __launch_bounds__(kThreadsConv, 2) k_conv_fwd(const bf16 *__rest
     // fragment: rows (voxels) lane/4 and lane/4 + 8, columns 2 (lane%4) + {0,1}
     const int i = i0 + wi;
 #pragma unroll
-    for (int w = 0; w < CT_J; w++) {
+    for (int w = 0; w < CJ; w++) {
 #pragma unroll
       for (int g = 0; g < 2; g++) {
         if (g >= ng) continue;
@@ -923,14 +926,22 @@ static int resident(const mgp_closure *cl, K kernel, int threads, size_t smem, i
 static int conv_fwd(mgp_closure *cl, const bf16 *X, const bf16 *W, const float *bias, const bf16 *gate, int mode,
                     bf16 *Y16, float *Y32,
                     float *frc, long long gstride, long long P, float scale) {
-  const auto kernel = mode >= 2 ? k_conv_fwd<1> : k_conv_fwd<2>;
-  static int grids[2] = {0, 0};  // (one device per process)
-  int &grid = grids[mode >= 2];
-  if (!grid) NN_RET(resident(cl, kernel, kThreadsConv, kConvSmem, &grid));
+  // tiles of 4 x 4 rows, or 4 x 2 where those would leave SMs without a block: on a
+  // small mesh a tile's latency is what the layer takes (a whole gradient at 32^3:
+  // 248 us with 4 x 4 tiles, 228 with 4 x 2; at 48^3, 144 tiles of 4 x 4, 266 both)
   const int N = cl->N;
-  const long long tiles = (long long)(N / CT_I) * (N / CT_J) * ((N + CT_SEG - 1) / CT_SEG);
+  const long long rows = (long long)(N / CT_I) * ((N + CT_SEG - 1) / CT_SEG), quads = rows * (N / 4);
+  static int grids[2][2] = {{0, 0}, {0, 0}}, sms = 0;  // (one device per process)
+  if (!sms) MGP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cl->device));
+  const bool pairs = quads <= sms;
+  const auto kernel = pairs ? (mode >= 2 ? k_conv_fwd<1, 2> : k_conv_fwd<2, 2>)
+                            : (mode >= 2 ? k_conv_fwd<1, 4> : k_conv_fwd<2, 4>);
+  const size_t smem = pairs ? conv_tile<2>::SMEM : conv_tile<4>::SMEM;
+  int &grid = grids[pairs][mode >= 2];
+  if (!grid) NN_RET(resident(cl, kernel, kThreadsConv, smem, &grid));
+  const long long tiles = pairs ? 2 * quads : quads;
   const unsigned blocks = (unsigned)(tiles < grid ? tiles : grid);
-  kernel<<<blocks, kThreadsConv, kConvSmem, cl->stream>>>(X, W, bias, gate, N, mode, Y16, Y32, frc, gstride, P, scale);
+  kernel<<<blocks, kThreadsConv, smem, cl->stream>>>(X, W, bias, gate, N, mode, Y16, Y32, frc, gstride, P, scale);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;

@@ -528,19 +528,6 @@ __global__ void __launch_bounds__(kThreads) k_pack_lpt(long long np, const float
   }
 }
 
-// Block sum of one double per thread (the result in thread 0).
-__device__ __forceinline__ double block_sum_tiles(double x, double *sh) {
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) sh[w] = x;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int k = 0; k < (int)(blockDim.x >> 5); k++) t += sh[k];
-  return t;
-}
-
 // Force tile in shared memory: three components, each (TX+1)^2 rows of
 // R = TZ + 4 floats (tile shape TX x TX x TZ, tile_tx).  A grid row (x, y)
 // of N + 2 floats starts on a 16-byte boundary when y is even and 8 bytes
@@ -578,8 +565,7 @@ __device__ __forceinline__ int tile_row(int c, int xx, int yy) {
 // k_interp_kick_drift does (same expressions in the same order), and writes
 // slot j of the output arrays (s, v; qs is the new order's lattice map).  D1/D2
 // (scale-independent growth) stay in lattice order, packed 32 bytes per
-// particle in `lpt` and read through the lattice point.  Per-block sums of the
-// interpolated forces and new velocities go to partials for k_finalize_kd.
+// particle in `lpt` and read through the lattice point.  kd_means takes the means.
 // PI: particle-array offset type, 32-bit when 3 np < 2^32 (fewer integer
 // instructions per access); NT: threads per block (512: two blocks per SM
 // within 64 registers a thread).
@@ -588,13 +574,12 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 2 : 0) k_ikd_tiles(
     const float *__restrict__ frc, long long gf, int N, long long P, int Ns, int ls, long long np,
     const float *__restrict__ s, const float *__restrict__ v, const float4 *__restrict__ lpt,
     const unsigned *__restrict__ qs, const unsigned *__restrict__ off, const unsigned *__restrict__ order, int ntx,
-    int ntz, const mgp_dstate *__restrict__ st, float *__restrict__ s2, float *__restrict__ v2,
-    double *__restrict__ partials, mgp_kd_args a) {
+    int ntz, mgp_dstate *st, float *__restrict__ s2, float *__restrict__ v2, double *__restrict__ partials,
+    unsigned *__restrict__ done, mgp_kd_args a) {
   using FT = force_tile<T>;
   constexpr int X = FT::X, R = FT::R, COMP = FT::COMP, K = FT::PIECES, KX = FT::TX, KZ = FT::TZ;
   constexpr int ROWS = NT / K;  // rows copied per pass of the block
   extern __shared__ __align__(16) float fs[];  // FT::FLOATS
-  __shared__ double sh[NT / 32];
   __shared__ long long rowoff[X * X];  // grid offset of row (x0 + xx, y0 + yy), periodic
   const int sub = threadIdx.x / K, k = threadIdx.x - sub * K;  // this thread's row in a pass, its piece
   const float ox = (float)(st->cx[0] * a.scale), oy = (float)(st->cx[1] * a.scale), oz = (float)(st->cx[2] * a.scale);
@@ -679,16 +664,22 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 2 : 0) k_ikd_tiles(
       }
     }
   }
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    double t = block_sum_tiles((double)accD[c], sh);
-    if (threadIdx.x == 0) partials[(long long)blockIdx.x * 6 + c] = t;
-    t = block_sum_tiles((double)accV[c], sh);
-    if (threadIdx.x == 0) partials[(long long)blockIdx.x * 6 + 3 + c] = t;
-  }
+  static_assert(6 * NT <= FT::FLOATS, "the sums reuse the force tile");
+  __syncthreads();  // the last tile's reads of fs are done
+  kd_means<NT>(accD, accV, fs, partials, blockIdx.x, gridDim.x, done, st, a);
 }
 
 }  // namespace
+
+// Whether a context left to choose buckets its particles.  Below 512^3 the mesh
+// and much of the three force grids stay in L2, the lattice-order deposit and
+// kick find their cells there, and the sort and the tiles cost more than they
+// save.  Microseconds a step (tiles; lattice order), Ns = N/2, cells of 0.5 and
+// of 2 Mpc/h: N = 64 96; 56 and 90; 55, 128 156; 97 and 142; 93, 256 578; 432 and
+// 528; 416, 384 3024; 2631 and 2923; 2553.  At 512 the two are even (3691; 3648 and
+// 3580; 3247) and at 1024 the tiles lead where the particles have moved far (29975;
+// 39071 and 29147; 29442).
+bool mgp_tiles_pay(int N) { return N >= 512; }
 
 // Tile shape of the single-box tile path, or 0 when it does not apply (the
 // mesh must split into whole tiles and the indices fit 32 bits): 8 x 8 x 64
@@ -922,9 +913,8 @@ int mgp_cic_tiles_own(mgp_ctx *c, float wpar, const float *s, float *rho) {
 // Kick + drift per tile in the order of the last mgp_tiles_sort (a single
 // box with particle-array LPT displacements; the positions unchanged since
 // the sort), the particle arrays rewritten in that order into the second
-// buffers, which then become the arrays.  nblocks_out: the grid, whose
-// per-block partial sums k_finalize_kd reduces.
-int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a, int *nblocks_out) {
+// buffers, which then become the arrays.
+int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a) {
   if (!c->tile_ready || c->nbox != 1) return mgp_set_error(MGP_ESTATE, "tile kick without a current tile sort");
   const size_t bytes = sizeof(float) * 3 * (size_t)c->np;
   if (!c->s_alt) {
@@ -959,7 +949,7 @@ int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a, int *nblocks_out) {
                                                                c->s, c->v, (const float4 *)c->lpt, c->q_alt,  \
                                                                c->tile_off, c->tile_order, nt1, ntz,          \
                                                                c->dstate, c->s_alt, c->v_alt, c->partials,    \
-                                                               *a);                                           \
+                                                               c->kd_done, *a);                                           \
   } while (0)
   const bool narrow = 3 * c->np < 0xffffffffLL;
   if (T == kElong && ls >= 0 && narrow)
@@ -987,6 +977,5 @@ int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a, int *nblocks_out) {
   c->q_alt = t;
   c->permuted = 1;
   c->tile_ready = 0;  // the arrays are in the sort's order now, the positions drifted
-  *nblocks_out = nb;
   return MGP_OK;
 }
