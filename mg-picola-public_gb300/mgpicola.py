@@ -6,6 +6,7 @@ There is no CPU fallback: loading fails loudly when the shared library is
 missing, and mgp_create fails when no CUDA device is present.
 """
 import ctypes as C
+import mmap
 import os
 
 import numpy as np
@@ -194,6 +195,18 @@ def lib():
                                        C.c_double, C.c_int, C.POINTER(C.c_int), dp, dp, dp, dp, vp]
         _lib = L
     return _lib
+
+
+def _result(shape):
+    """FP32 array for a result that the library writes whole.  From 4 MB on numpy
+    offers its arrays for huge pages; with 64 KB base pages those are 512 MB, and a
+    copy that faults one in zeroes it all (21 ms for a 25 MB array).  Such results
+    take pages of their own (1 ms); smaller ones are better off with memory that was
+    in use before."""
+    n = 4 * int(np.prod(shape))
+    if n < 1 << 22:
+        return np.empty(shape, np.float32)
+    return np.frombuffer(mmap.mmap(-1, n, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS), np.float32).reshape(shape)
 
 
 def _check(rc):
@@ -438,10 +451,7 @@ class Context:
         return tuple(a[:m] for a in arrs)
 
     def get_particles(self):
-        pos = np.zeros((self.np, 3), np.float32)
-        vel = np.zeros((self.np, 3), np.float32)
-        d1 = np.zeros((self.np, 3), np.float32)
-        d2 = np.zeros((self.np, 3), np.float32)
+        pos, vel, d1, d2 = (_result((self.np, 3)) for _ in range(4))
         _check(lib().mgp_get_particles(self.h, pos.ctypes.data, vel.ctypes.data, d1.ctypes.data, d2.ctypes.data,
                                        self.np))
         return pos, vel, d1, d2
@@ -461,7 +471,7 @@ class Context:
         """Copy of grid `which` (its first `planes` x planes when given)."""
         nx = self.N if planes is None else int(planes)
         n = nx * self.N * 2 * (self.N // 2 + 1)
-        out = np.zeros(n, np.float32)
+        out = _result(n)
         _check(lib().mgp_copy_grid(self.h, which, out, n))
         return out.reshape(nx, self.N, 2 * (self.N // 2 + 1))
 
@@ -491,10 +501,11 @@ class Context:
         return lib().mgp_kernel_ms_step(self.h, name.encode(), step)
 
     def set_particle_order(self, tiles):
-        """Cell-tile particle order (mgp_set_particle_order): 2 the default
-        for single boxes (tile deposit, kick per tile with the arrays
-        rewritten in tile order every step), 1 the tile deposit with the
-        arrays in lattice order, 0 the deposit and kick in lattice order."""
+        """Cell-tile particle order (mgp_set_particle_order): 2 the tile
+        deposit and the kick per tile with the arrays rewritten in tile order
+        every step (a single box's start from Nmesh = 512 on), 1 the tile
+        deposit with the arrays in lattice order, 0 the deposit and kick in
+        lattice order (the start of smaller meshes)."""
         _check(lib().mgp_set_particle_order(self.h, int(tiles)))
 
     def set_fft_mode(self, mode):
@@ -555,8 +566,7 @@ class Batch:
 
     def particles(self, box):
         n = self.p.Nsample ** 3
-        pos = np.zeros((n, 3), np.float32)
-        vel = np.zeros((n, 3), np.float32)
+        pos, vel = _result((n, 3)), _result((n, 3))
         _check(lib().mgp_batch_get_particles(self.h, box, pos.ctypes.data, vel.ctypes.data, n))
         return pos, vel
 
