@@ -251,23 +251,25 @@ static int setup_pofk(mgp_ctx *c) {
   c->pk_n = (double *)calloc(nbins, sizeof(double));
   c->pk_k = (double *)calloc(nbins, sizeof(double));
   c->pk_host = (double *)calloc(nbins, sizeof(double));
-  // geometric mode counts and |k| sums with the reference's weights
-  for (int d0 = 0; d0 <= h; d0++) {
-    double m0 = (d0 == 0 || d0 == h) ? 1.0 : 2.0;
-    for (int d1 = 0; d1 <= h; d1++) {
-      double m1 = (d1 == 0 || d1 == h) ? 1.0 : 2.0;
-      for (int d2 = 0; d2 <= h; d2++) {
-        int rk = d0 * d0 + d1 * d1 + d2 * d2;
-        int b = rkb[rk];
-        if (b < 0) continue;
-        double w = m0 * m1 * ((d2 == 0 || d2 == h) ? 1.0 : 2.0);
-        c->pk_n[b] += w;
-        c->pk_k[b] += w * sqrt((double)rk);
-      }
+  // geometric mode counts and |k| sums with the reference's weights: the number of
+  // (d0, d1) per d0^2 + d1^2, and from it of modes per |k|^2 (h = 512: 56 M integer
+  // additions for 134 M modes)
+  {
+    std::vector<int> pairs(2 * h * h + 1, 0), modes(rkmax + 1, 0);
+    const auto weight = [h](int d) { return d == 0 || d == h ? 1 : 2; };
+    for (int d0 = 0; d0 <= h; d0++)
+      for (int d1 = 0; d1 <= h; d1++) pairs[d0 * d0 + d1 * d1] += weight(d0) * weight(d1);
+    for (int m = 0; m <= 2 * h * h; m++) {
+      if (!pairs[m]) continue;
+      for (int d2 = 0; d2 <= h; d2++) modes[m + d2 * d2] += pairs[m] * weight(d2);
+    }
+    for (int rk = 0; rk <= rkmax; rk++) {
+      const int b = rkb[rk];
+      if (b < 0) continue;
+      c->pk_n[b] += (double)modes[rk];
+      c->pk_k[b] += (double)modes[rk] * sqrt((double)rk);
     }
   }
-  MGP_CUDA(cudaMalloc(&c->rk_bin, sizeof(int) * (rkmax + 1)));
-  MGP_CUDA(cudaMemcpy(c->rk_bin, rkb.data(), sizeof(int) * (rkmax + 1), cudaMemcpyHostToDevice));
   // first |k|^2 of each bin: the bin index is monotone in |k|^2 over one
   // contiguous range [rlo, rhi) and -1 outside it
   {
@@ -397,7 +399,7 @@ extern "C" int mgp_destroy(mgp_ctx *c) {
   }
   free(c->box_p);
   void *bufs[] = {c->ic_scratch, c->ic_amp, c->ic_box, c->s, c->v, c->D1, c->D2, c->dstate, c->partials, c->kd_done, c->stage, c->rho, c->dk, c->frc, c->mg1,
-                  c->fft_work, c->rk_bin, c->pk_thr, c->win1d, c->pk_block, c->pk_sum, c->rsd_block, c->rsd_sum,
+                  c->fft_work, c->pk_thr, c->win1d, c->pk_block, c->pk_sum, c->rsd_block, c->rsd_sum,
                   c->pk_sum_tot, c->nu_tab_d, c->nu_row_d, c->nu_x_d, c->nu_den_d, c->scr_tab};
   for (size_t i = 0; i < sizeof(bufs) / sizeof(bufs[0]); i++)
     if (bufs[i]) cudaFree(bufs[i]);

@@ -105,7 +105,6 @@ struct mgp_ctx {
   /* P(k) */
   int pk_nbins, pk_bintype, pk_sub;
   double pk_kmin, pk_kmax;  /* integer-k units, adjusted */
-  int *rk_bin;              /* device: bin index per integer |k|^2 (or -1) */
   int *pk_thr;              /* device: first |k|^2 of each bin, [nbins] = end */
   float *win1d;             /* device: 1/sinc^4 per |d| in [0, N/2] */
   double *pk_block;         /* device: per-block FP64 bin partials */
