@@ -567,10 +567,16 @@ __device__ __forceinline__ int tile_row(int c, int xx, int yy) {
 // (scale-independent growth) stay in lattice order, packed 32 bytes per
 // particle in `lpt` and read through the lattice point.  kd_means takes the means.
 // PI: particle-array offset type, 32-bit when 3 np < 2^32 (fewer integer
-// instructions per access); NT: threads per block (512: two blocks per SM
-// within 64 registers a thread).
-template <int T, bool P2, typename PI, int NT>
-__global__ void __launch_bounds__(NT, NT >= 512 ? 2 : 0) k_ikd_tiles(
+// instructions per access).
+// Bound by the latency of dependent reads (offsets, then order and lattice point,
+// then the particle) beside the tile's copy: a thread's first PF particles are read
+// while the tile arrives, the next tile's order and lattice points while this one
+// is computed.  8 x 8 x 64 tiles hold 512 particles at Ns = N/2, so two blocks of 256
+// threads with PF = 3 and 123 registers have all of them in flight; 512 threads
+// within 64 registers spill and were 25% slower, three blocks an SM as well.  A kick
+// at N = 512, Ns = 256: 892 -> 716 us (4.8 TB/s), at 1024, 512: 6.92 -> 5.69 ms.
+template <int T, bool P2, typename PI, int NB, int PF>
+__global__ void __launch_bounds__(kThreads, NB) k_ikd_tiles(
     const float *__restrict__ frc, long long gf, int N, long long P, int Ns, int ls, long long np,
     const float *__restrict__ s, const float *__restrict__ v, const float4 *__restrict__ lpt,
     const unsigned *__restrict__ qs, const unsigned *__restrict__ off, const unsigned *__restrict__ order, int ntx,
@@ -578,53 +584,104 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 2 : 0) k_ikd_tiles(
     unsigned *__restrict__ done, mgp_kd_args a) {
   using FT = force_tile<T>;
   constexpr int X = FT::X, R = FT::R, COMP = FT::COMP, K = FT::PIECES, KX = FT::TX, KZ = FT::TZ;
-  constexpr int ROWS = NT / K;  // rows copied per pass of the block
+  constexpr int NT = kThreads, ROWS = NT / K;  // threads; rows copied per pass of the block
   extern __shared__ __align__(16) float fs[];  // FT::FLOATS
-  __shared__ long long rowoff[X * X];  // grid offset of row (x0 + xx, y0 + yy), periodic
-  const int sub = threadIdx.x / K, k = threadIdx.x - sub * K;  // this thread's row in a pass, its piece
+  __shared__ long long rowoff[3 * X * X];  // grid offset of a tile's row from the tile's own (no wrap)
+  const int tid = threadIdx.x, sub = tid / K, k = tid - sub * K;  // this thread's row in a pass, its piece
   const float ox = (float)(st->cx[0] * a.scale), oy = (float)(st->cx[1] * a.scale), oz = (float)(st->cx[2] * a.scale);
   const float inv_ns = 1.0f / (float)Ns;
   const int ntiles = ntx * ntx * ntz;
+  for (int r = tid; r < 3 * X * X; r += NT) {
+    const int c = r / (X * X), rr = r - c * X * X, xx = rr / X, yy = rr - xx * X;
+    rowoff[r] = c * gf + ((long long)xx * N + yy) * P - 2 * (yy & 1);
+  }
   float accD[3] = {0.f, 0.f, 0.f}, accV[3] = {0.f, 0.f, 0.f};
-  for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
+  const PI npi = (PI)np;
+  unsigned j0 = 0, j1 = 0, ord[PF], lat[PF];  // the current tile's particles, and the first PF of this thread's
+  auto fetch = [&](int L) {
+    j0 = j1 = 0;
+    if (L >= ntiles) return;
     const int tile = tile_at(L, ntx, ntz);
-    const unsigned j0 = off[tile], j1 = off[tile + 1];
-    if (j0 == j1) continue;
-    const int tz = tile % ntz, ty = (tile / ntz) % ntx, tx = tile / (ntz * ntx);
-    const int x0 = tx * KX, y0 = ty * KX, z0 = tz * KZ;
-    __syncthreads();  // the previous tile's reads of fs and rowoff are done
-    for (int r = threadIdx.x; r < X * X; r += NT) {
-      const int xx = r / X, yy = r - xx * X;
-      const int gx = x0 + xx >= N ? x0 + xx - N : x0 + xx, gy = y0 + yy >= N ? y0 + yy - N : y0 + yy;
-      rowoff[r] = ((long long)gx * N + gy) * P + z0 - 2 * (yy & 1);
-    }
-    __syncthreads();
-    if (sub < ROWS) {
-      for (int r = sub; r < 3 * X * X; r += ROWS) {
-        const int c = r >= 2 * X * X ? 2 : (r >= X * X ? 1 : 0), rr = r - c * X * X;
-        cp_async16(fs + c * COMP + rr * R + 4 * k, frc + c * gf + rowoff[rr] + 4 * k);
+    j0 = off[tile];
+    j1 = off[tile + 1];
+  };
+  auto fetch_index = [&]() {
+#pragma unroll
+    for (int c = 0; c < PF; c++) {
+      const unsigned j = j0 + tid + c * NT;
+      if (j < j1) {
+        ord[c] = order[j];
+        lat[c] = qs[j];
       }
     }
+  };
+  fetch(blockIdx.x);
+  fetch_index();
+  for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
+    if (j0 == j1) {
+      fetch(L + gridDim.x);
+      fetch_index();
+      continue;
+    }
+    const unsigned jb = j0, je = j1;
+    const int tile = tile_at(L, ntx, ntz);
+    const int tz = tile % ntz, ty = (tile / ntz) % ntx, tx = tile / (ntz * ntx);
+    const int x0 = tx * KX, y0 = ty * KX, z0 = tz * KZ;
+    const float *base = frc + ((long long)x0 * N + y0) * P + z0;
+    // the halo rows past the last plane or row are the first ones
+    const long long wx = x0 + KX == N ? (long long)N * N * P : 0, wy = y0 + KX == N ? (long long)N * P : 0;
+    const bool inside = wx == 0 && wy == 0;
+    __syncthreads();  // the previous tile's reads of fs are done (and rowoff is there)
+    if (sub < ROWS) {
+      float *d = fs + sub * R + 4 * k;
+      for (int r = sub; r < 3 * X * X; r += ROWS, d += ROWS * R) {
+        const float *g = base + rowoff[r] + 4 * k;
+        if (!inside) {
+          const int rr = r % (X * X);
+          if (rr / X == KX) g -= wx;
+          if (rr % X == KX) g -= wy;
+        }
+        cp_async16(d, g);
+      }
+    }
+    // this thread's first particles, read while the tile arrives
+    float sp[PF][3], vp[PF][3];
+    float4 l0[PF], l1[PF];
+    unsigned lc[PF];
+#pragma unroll
+    for (int c = 0; c < PF; c++) {
+      lc[c] = lat[c];
+      if (jb + tid + c * NT < je) {
+        const PI p = (PI)ord[c];
+#pragma unroll
+        for (int ax = 0; ax < 3; ax++) {
+          sp[c][ax] = s[(PI)ax * npi + p];
+          vp[c][ax] = v[(PI)ax * npi + p];
+        }
+        l0[c] = lpt[2 * (size_t)lc[c]];
+        l1[c] = lpt[2 * (size_t)lc[c] + 1];
+      }
+    }
+    fetch(L + gridDim.x);
     cp_async_wait_all();
     __syncthreads();
     if (z0 + KZ == N) {
       // last tile in z: the halo column z0 + KZ is z = 0 of the same row
-      for (int r = threadIdx.x; r < 3 * X * X; r += NT) {
-        const int c = r / (X * X), rr = r - c * X * X, yy = rr % X;
-        fs[c * COMP + rr * R + 2 * (yy & 1) + KZ] = frc[c * gf + rowoff[rr] + 2 * (yy & 1) - z0];
+      for (int r = tid; r < 3 * X * X; r += NT) {
+        const int rr = r % (X * X), yy = rr % X;
+        const float *g = base + rowoff[r] + 2 * (yy & 1) - z0;
+        if (rr / X == KX) g -= wx;
+        if (yy == KX) g -= wy;
+        fs[r * R + 2 * (yy & 1) + KZ] = *g;
       }
       __syncthreads();
     }
-    const PI npi = (PI)np;
-    for (unsigned j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-      const PI p = (PI)order[j];
-      const unsigned lat = qs[j];
-      const float sp[3] = {s[p], s[npi + p], s[2 * npi + p]};
-      const float4 l0 = lpt[2 * (size_t)lat], l1 = lpt[2 * (size_t)lat + 1];
-      const float D1p[3] = {l0.x, l0.y, l0.z}, D2p[3] = {l0.w, l1.x, l1.y};
+    fetch_index();
+    auto particle = [&](unsigned j, unsigned lattice, const float (&x)[3], const float (&u)[3], float4 q0, float4 q1) {
+      const float D1p[3] = {q0.x, q0.y, q0.z}, D2p[3] = {q0.w, q1.x, q1.y};
       int ix, iy, iz;
       float DX, DY, DZ;
-      cell_of<P2>(sp[0], sp[1], sp[2], lat, Ns, ls, inv_ns, N, a.scale, ox, oy, oz, ix, iy, iz, DX, DY, DZ);
+      cell_of<P2>(x[0], x[1], x[2], lattice, Ns, ls, inv_ns, N, a.scale, ox, oy, oz, ix, iy, iz, DX, DY, DZ);
       const float TX = 1.0f - DX, TY = 1.0f - DY, TZ = 1.0f - DZ;
       const float w000 = TX * TY * TZ, w001 = TX * TY * DZ, w010 = TX * DY * TZ, w011 = TX * DY * DZ;
       const float w100 = DX * TY * TZ, w101 = DX * TY * DZ, w110 = DX * DY * TZ, w111 = DX * DY * DZ;
@@ -644,24 +701,37 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 2 : 0) k_ikd_tiles(
         const long long xa = (long long)ix * N * P, xb = (ix + 1 == N ? 0 : (long long)(ix + 1) * N * P);
         const long long ya = (long long)iy * P, yb = (iy + 1 == N ? 0 : (long long)(iy + 1) * P);
         const long long za = iz, zb = iz + 1 == N ? 0 : iz + 1;
-#pragma unroll
+#pragma unroll 1
         for (int c = 0; c < 3; c++) {
           const float *F = frc + c * gf;
-          disp[c] = F[xa + ya + za] * w000 + F[xa + ya + zb] * w001 + F[xa + yb + za] * w010 +
-                    F[xa + yb + zb] * w011 + F[xb + ya + za] * w100 + F[xb + ya + zb] * w101 +
-                    F[xb + yb + za] * w110 + F[xb + yb + zb] * w111;
+          const float f = F[xa + ya + za] * w000 + F[xa + ya + zb] * w001 + F[xa + yb + za] * w010 +
+                          F[xa + yb + zb] * w011 + F[xb + ya + za] * w100 + F[xb + ya + zb] * w101 +
+                          F[xb + yb + za] * w110 + F[xb + yb + zb] * w111;
+          if (c == 0) disp[0] = f;
+          if (c == 1) disp[1] = f;
+          if (c == 2) disp[2] = f;
         }
       }
 #pragma unroll
       for (int ax = 0; ax < 3; ax++) {
-        const PI o = (PI)ax * npi, oj = o + (PI)j;
+        const PI oj = (PI)ax * npi + (PI)j;
         const float d1 = D1p[ax], d2 = D2p[ax];
-        const float vn = v[o + p] + a.kick_disp * disp[ax] + a.kick_d1 * d1 + a.kick_d2 * d2;
+        const float vn = u[ax] + a.kick_disp * disp[ax] + a.kick_d1 * d1 + a.kick_d2 * d2;
         v2[oj] = vn;
-        s2[oj] = a.do_drift ? sp[ax] + vn * a.dyyy + a.dD1 * d1 + a.dD2 * d2 : sp[ax];
+        s2[oj] = a.do_drift ? x[ax] + vn * a.dyyy + a.dD1 * d1 + a.dD2 * d2 : x[ax];
         accD[ax] += disp[ax];
         accV[ax] += vn;
       }
+    };
+#pragma unroll
+    for (int c = 0; c < PF; c++)
+      if (jb + tid + c * NT < je) particle(jb + tid + c * NT, lc[c], sp[c], vp[c], l0[c], l1[c]);
+#pragma unroll 1
+    for (unsigned j = jb + tid + PF * NT; j < je; j += NT) {
+      const PI p = (PI)order[j];
+      const unsigned lattice = qs[j];
+      const float x[3] = {s[p], s[npi + p], s[2 * npi + p]}, u[3] = {v[p], v[npi + p], v[2 * npi + p]};
+      particle(j, lattice, x, u, lpt[2 * (size_t)lattice], lpt[2 * (size_t)lattice + 1]);
     }
   }
   static_assert(6 * NT <= FT::FLOATS, "the sums reuse the force tile");
@@ -671,15 +741,17 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 2 : 0) k_ikd_tiles(
 
 }  // namespace
 
-// Whether a context left to choose buckets its particles.  Below 512^3 the mesh
-// and much of the three force grids stay in L2, the lattice-order deposit and
-// kick find their cells there, and the sort and the tiles cost more than they
-// save.  Microseconds a step (tiles; lattice order), Ns = N/2, cells of 0.5 and
-// of 2 Mpc/h: N = 64 96; 56 and 90; 55, 128 156; 97 and 142; 93, 256 578; 432 and
-// 528; 416, 384 3024; 2631 and 2923; 2553.  At 512 the two are even (3691; 3648 and
-// 3580; 3247) and at 1024 the tiles lead where the particles have moved far (29975;
-// 39071 and 29147; 29442).
-bool mgp_tiles_pay(int N) { return N >= 512; }
+// Whether a context left to choose buckets its particles.  On smaller meshes the
+// mesh and much of the force grids stay in L2, the lattice-order deposit and kick
+// find their cells there, and the sort and the tiles cost more than they save; the
+// cubic tiles cost more than the long ones, which need Nmesh a multiple of 64.
+// Microseconds a step (tiles; lattice order), Ns = N/2, cells of 0.5 and of 2 Mpc/h:
+//   N = 64   96; 56        90; 55          528 (16^3)   7624; 7094     7360; 6769
+//   128      156; 97       142; 93         784 (16^3)   32053; 31265   31577; 28864
+//   256      578; 432      528; 416        1008 (16^3)  99641; 102582  97987; 95058
+//   384      3024; 2631    2923; 2553      520 (8^3)    11493; 8686    11320; 8336
+//   512      3566; 3648    3392; 3247      1024         29148; 39071   27809; 29442
+bool mgp_tiles_pay(int N) { return N % kElong == 0 ? N >= 512 : N % 16 == 0 && N >= 960; }
 
 // Tile shape of the single-box tile path, or 0 when it does not apply (the
 // mesh must split into whole tiles and the indices fit 32 bits): 8 x 8 x 64
@@ -934,22 +1006,19 @@ int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a) {
   const int ls = lattice_log2(Ns);
   const long long ntiles = (long long)nt1 * nt1 * ntz;
   // forces per block: 16^3 tiles 68 KB (three blocks of 256 threads per
-  // SM), 8 x 8 x 64 tiles 65 KB (two blocks of 512), 8^3 tiles 12 KB (eight
-  // of 256)
+  // SM), 8 x 8 x 64 tiles 65 KB (two blocks), 8^3 tiles 12 KB (eight)
   const size_t smem = sizeof(float) * (T == kElong ? force_tile<kElong>::FLOATS
                                                    : (T == 16 ? force_tile<16>::FLOATS : force_tile<8>::FLOATS));
   int nb = T == kElong ? mgp_blocks_for(ntiles * 256, 2) : mgp_blocks_for(ntiles * 256, T == 8 ? 8 : 3);
   if (nb > c->max_blocks) nb = c->max_blocks;
 #define MGP_IKD_TILES(TT, PP, PI)                                                                             \
   do {                                                                                                        \
-    constexpr int NTT = TT == kElong ? 512 : 256;                                                             \
-    MGP_CUDA(cudaFuncSetAttribute(k_ikd_tiles<TT, PP, PI, NTT>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
-                                  (int)smem));                                                                \
-    k_ikd_tiles<TT, PP, PI, NTT><<<nb, NTT, smem, c->stream>>>(c->frc, c->g.nreal, N, c->g.P, Ns, ls, c->np,  \
-                                                               c->s, c->v, (const float4 *)c->lpt, c->q_alt,  \
-                                                               c->tile_off, c->tile_order, nt1, ntz,          \
-                                                               c->dstate, c->s_alt, c->v_alt, c->partials,    \
-                                                               c->kd_done, *a);                                           \
+    const auto kernel = TT == kElong ? k_ikd_tiles<TT, PP, PI, 2, 3> : k_ikd_tiles<TT, PP, PI, 3, 1>;         \
+    MGP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));           \
+    kernel<<<nb, kThreads, smem, c->stream>>>(c->frc, c->g.nreal, N, c->g.P, Ns, ls, c->np, c->s, c->v,       \
+                                              (const float4 *)c->lpt, c->q_alt, c->tile_off, c->tile_order,   \
+                                              nt1, ntz, c->dstate, c->s_alt, c->v_alt, c->partials,           \
+                                              c->kd_done, *a);                                                \
   } while (0)
   const bool narrow = 3 * c->np < 0xffffffffLL;
   if (T == kElong && ls >= 0 && narrow)

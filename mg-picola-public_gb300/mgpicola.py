@@ -503,9 +503,10 @@ class Context:
     def set_particle_order(self, tiles):
         """Cell-tile particle order (mgp_set_particle_order): 2 the tile
         deposit and the kick per tile with the arrays rewritten in tile order
-        every step (a single box's start from Nmesh = 512 on), 1 the tile
-        deposit with the arrays in lattice order, 0 the deposit and kick in
-        lattice order (the start of smaller meshes)."""
+        every step (what a single box starts with from Nmesh = 512 on, where
+        Nmesh is a multiple of 64), 1 the tile deposit with the arrays in
+        lattice order, 0 the deposit and kick in lattice order (what it
+        starts with else)."""
         _check(lib().mgp_set_particle_order(self.h, int(tiles)))
 
     def set_fft_mode(self, mode):

@@ -4,8 +4,8 @@ Default order: the density, the velocities and the positions of one step against
 both explicit orders, up to the order of float sums: a cell adds up to 16 weights
 (16 2^-24 of the largest cell, bound 2e-6); forces of the two densities agree to
 about 1e-6 rms as the transforms' own error is 5e-7 (bound 1e-5, also of the
-lattice spacing for positions).  Sizes on either side of the line (Nmesh 512), the
-smallest mesh with tiles and one without.
+lattice spacing for positions).  Sizes on either side of the line (Nmesh 512 in
+multiples of 64), the smallest mesh with tiles and one without.
 
 Means: Drift subtracts the mean velocity (src/main.c:747-787).  Particles with a
 large common velocity keep their mean position: positions are FP32 numbers below
@@ -26,7 +26,7 @@ def params(N, Ns):
     return M.default_params(Nmesh=N, Nsample=Ns, Box=2.0 * N, Seed=5001, Init_Redshift=19.0, pofk_nbins=8)
 
 
-@pytest.mark.parametrize("N,Ns", [(16, 8), (20, 10), (64, 32), (496, 32), (512, 32)])
+@pytest.mark.parametrize("N,Ns", [(16, 8), (20, 10), (64, 32), (496, 32), (512, 32), (520, 26)])
 def test_default_order_matches_explicit_orders(N, Ns):
     box = 2.0 * N
     rng = np.random.default_rng(N)
