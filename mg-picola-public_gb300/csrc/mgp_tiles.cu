@@ -44,6 +44,7 @@
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kSortItems = 2;                      // runs of 32 particles a warp has in flight
 constexpr int kScanItems = 16;                     // per thread in a scan block
 constexpr int kScanChunk = kThreads * kScanItems;  // elements per scan block
 
@@ -102,9 +103,9 @@ __device__ __forceinline__ void cp_async16(float *dst, const float *src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Tile of every particle and the per-tile counts.  The loop runs in whole
-// warps (warp-aligned starts, stride a multiple of 32) so that the lanes of
-// a warp can merge their count increments per tile.
+// Tile of every particle and the per-tile counts.  A warp takes kSortItems runs of
+// 32 particles at a time, all read before the first is counted;
+// the lanes of a run merge their count increments per tile.
 template <bool P2>
 __global__ void __launch_bounds__(kThreads) k_tile_key(const float *__restrict__ s, const mgp_dstate *__restrict__ st,
                                                        long long np, int Ns, int ls, int N, float scale, int sx,
@@ -120,21 +121,35 @@ __global__ void __launch_bounds__(kThreads) k_tile_key(const float *__restrict__
   const float ox = (float)(st->cx[0] * scale), oy = (float)(st->cx[1] * scale), oz = (float)(st->cx[2] * scale);
   const float inv_ns = 1.0f / (float)Ns;
   const int lane = threadIdx.x & 31;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < np; base += stride) {
-    const long long p = base + lane;
-    const bool on = p < np;
-    const unsigned am = __ballot_sync(0xffffffffu, on);
-    if (!on) continue;
-    int ix, iy, iz;
-    float DX, DY, DZ;
-    particle_cell<P2>(s, np, p, q ? q[p] : (unsigned)p, Ns, ls, inv_ns, N, scale, ox, oy, oz, ix, iy, iz, DX, DY,
-                      DZ);
-    const unsigned t = box * ntiles + ((unsigned)(ix >> sx) * (unsigned)ntx + (unsigned)(iy >> sx)) * (unsigned)ntz +
-                       (unsigned)(iz >> sz);
-    tile_of[p] = t;
-    const unsigned same = __match_any_sync(am, t);
-    if (lane == __ffs(same) - 1) atomicAdd(count + t, (unsigned)__popc(same));
+  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long base = 32LL * kSortItems * ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); base < np;
+       base += 32LL * kSortItems * nwarps) {
+    float x[kSortItems][3];
+    unsigned lat[kSortItems];
+#pragma unroll
+    for (int u = 0; u < kSortItems; u++) {
+      const long long p = base + 32 * u + lane;
+      if (p >= np) continue;
+      lat[u] = q ? q[p] : (unsigned)p;
+      x[u][0] = s[p];
+      x[u][1] = s[np + p];
+      x[u][2] = s[2 * np + p];
+    }
+#pragma unroll
+    for (int u = 0; u < kSortItems; u++) {
+      const long long p = base + 32 * u + lane;
+      const bool on = p < np;
+      const unsigned am = __ballot_sync(0xffffffffu, on);
+      if (!on) continue;
+      int ix, iy, iz;
+      float DX, DY, DZ;
+      cell_of<P2>(x[u][0], x[u][1], x[u][2], lat[u], Ns, ls, inv_ns, N, scale, ox, oy, oz, ix, iy, iz, DX, DY, DZ);
+      const unsigned t = box * ntiles + ((unsigned)(ix >> sx) * (unsigned)ntx + (unsigned)(iy >> sx)) * (unsigned)ntz +
+                         (unsigned)(iz >> sz);
+      tile_of[p] = t;
+      const unsigned same = __match_any_sync(am, t);
+      if (lane == __ffs(same) - 1) atomicAdd(count + t, (unsigned)__popc(same));
+    }
   }
 }
 
@@ -219,27 +234,46 @@ __global__ void k_scan_add(unsigned *__restrict__ off, unsigned *__restrict__ cu
 // warps claim their slots); with `lat` (a single box), also the lattice
 // point of every slot, lat[slot] = q[p] (p when q is NULL), so that the
 // deposit and the kick read it in slot order instead of through the index.
+// A warp takes kSortItems runs of 32 particles at a time: their reads and their
+// atomics, whose answers it waits for, are in flight together.  Key and scatter of 2^27 particles 1.27 ms with one
+// run at a time, 1.06 with two, 1.15 with four (48 registers).
 __global__ void __launch_bounds__(kThreads) k_tile_scatter(const unsigned *__restrict__ tile_of, long long np,
                                                            unsigned *__restrict__ cursor,
                                                            unsigned *__restrict__ order,
                                                            const unsigned *__restrict__ q,
                                                            unsigned *__restrict__ lat) {
   const int lane = threadIdx.x & 31;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long base = (long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < np; base += stride) {
-    const long long p = base + lane;
-    const bool on = p < np;
-    const unsigned am = __ballot_sync(0xffffffffu, on);
-    if (!on) continue;
-    const unsigned t = tile_of[p];
-    const unsigned same = __match_any_sync(am, t);
-    const int leader = __ffs(same) - 1;
-    unsigned first = 0;
-    if (lane == leader) first = atomicAdd(cursor + t, (unsigned)__popc(same));
-    first = __shfl_sync(same, first, leader);
-    const unsigned slot = first + __popc(same & ((1u << lane) - 1u));
-    order[slot] = (unsigned)p;
-    if (lat) lat[slot] = q ? q[p] : (unsigned)p;
+  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long base = 32LL * kSortItems * ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); base < np;
+       base += 32LL * kSortItems * nwarps) {
+    unsigned t[kSortItems], l[kSortItems], rank[kSortItems], first[kSortItems];
+    int leader[kSortItems];
+#pragma unroll
+    for (int u = 0; u < kSortItems; u++) {
+      const long long p = base + 32 * u + lane;
+      if (p >= np) continue;
+      t[u] = tile_of[p];
+      l[u] = q ? q[p] : (unsigned)p;
+    }
+#pragma unroll
+    for (int u = 0; u < kSortItems; u++) {
+      const bool on = base + 32 * u + lane < np;
+      const unsigned am = __ballot_sync(0xffffffffu, on);
+      if (!on) continue;
+      const unsigned same = __match_any_sync(am, t[u]);
+      leader[u] = __ffs(same) - 1;
+      rank[u] = __popc(same & ((1u << lane) - 1u));
+      if (lane == leader[u]) first[u] = atomicAdd(cursor + t[u], (unsigned)__popc(same));
+    }
+#pragma unroll
+    for (int u = 0; u < kSortItems; u++) {
+      const long long p = base + 32 * u + lane;
+      const unsigned am = __ballot_sync(0xffffffffu, p < np);
+      if (p >= np) continue;
+      const unsigned slot = __shfl_sync(am, first[u], leader[u]) + rank[u];
+      order[slot] = (unsigned)p;
+      if (lat) lat[slot] = l[u];
+    }
   }
 }
 
@@ -374,40 +408,80 @@ __device__ __forceinline__ void halo_pair(int h, int &xx, int &yy, int &zz) {
 // to the neighbours' interiors.  A particle whose base cell falls outside its
 // tile after all (not expected: the key pass rounds identically) is listed in
 // `spill` for k_cic_halo, after every interior has been stored.
+// Shared-memory float adds are compare-and-swap loops, and a tile's dependent reads
+// stood between them: the next tile's first two particles a thread are read while
+// this one is added and stored (48 registers, five blocks an SM; four blocks with
+// three particles were 4% slower, six spill), and rows are stored a group of lanes
+// each instead of by an index worked out per pair.  With k_cic_halo, N = 512, Ns =
+// 256: 590 -> 490 us; 1024, 512: 4.54 -> 3.90 ms.
 template <int T, bool P2>
-__global__ void __launch_bounds__(kThreads) k_cic_tiles_own(const float *__restrict__ s,
-                                                            const mgp_dstate *__restrict__ st, long long np, int Ns,
-                                                            int ls, int N, float scale, float wpar,
-                                                            float *__restrict__ rho, long long P,
-                                                            const unsigned *__restrict__ off,
-                                                            const unsigned *__restrict__ order,
-                                                            const unsigned *__restrict__ qs, int ntx, int ntz,
-                                                            float2 *__restrict__ halo, unsigned *__restrict__ spill,
-                                                            unsigned *__restrict__ nspill) {
+__global__ void __launch_bounds__(kThreads, 5) k_cic_tiles_own(const float *__restrict__ s,
+                                                               const mgp_dstate *__restrict__ st, long long np, int Ns,
+                                                               int ls, int N, float scale, float wpar,
+                                                               float *__restrict__ rho, long long P,
+                                                               const unsigned *__restrict__ off,
+                                                               const unsigned *__restrict__ order,
+                                                               const unsigned *__restrict__ qs, int ntx, int ntz,
+                                                               float2 *__restrict__ halo, unsigned *__restrict__ spill,
+                                                               unsigned *__restrict__ nspill) {
   using H = tile_halo<T>;
-  constexpr int KX = H::KX, KZ = H::KZ, BX = H::BX, BZ = H::BZ, BOX = BX * BX * BZ;
-  __shared__ __align__(16) float box[BOX];
+  constexpr int KX = H::KX, KZ = H::KZ, BX = H::BX, BZ = H::BZ, BOX = BX * BX * BZ, PF = 2;
+  constexpr int LR = KZ / 2 < 32 ? KZ / 2 : 32, WR = kThreads / LR;  // lanes of a row's pairs, rows at a time
+  __shared__ __align__(16) float box[(BOX + 3) / 4 * 4];
+  const int tid = threadIdx.x, zp = tid % LR;
   const float inv_ns = 1.0f / (float)Ns;
   const int ntiles = ntx * ntx * ntz;
   const float ox = (float)(st->cx[0] * scale), oy = (float)(st->cx[1] * scale), oz = (float)(st->cx[2] * scale);
+  unsigned j0 = 0, j1 = 0, ord[PF], lat[PF];  // the next tile's particles, and the first PF of this thread's
+  float x[PF][3];
+  auto fetch = [&](int L) {
+    j0 = j1 = 0;
+    if (L >= ntiles) return;
+    const int tile = tile_at(L, ntx, ntz);
+    j0 = off[tile];
+    j1 = off[tile + 1];
+  };
+  auto fetch_index = [&]() {
+#pragma unroll
+    for (int c = 0; c < PF; c++) {
+      const unsigned j = j0 + tid + c * kThreads;
+      if (j >= j1) continue;
+      ord[c] = order[j];
+      lat[c] = qs[j];
+    }
+  };
+  auto fetch_particles = [&]() {
+#pragma unroll
+    for (int c = 0; c < PF; c++) {
+      if (j0 + tid + c * kThreads >= j1) continue;
+      const long long p = (long long)ord[c];
+      x[c][0] = s[p];
+      x[c][1] = s[np + p];
+      x[c][2] = s[2 * np + p];
+    }
+  };
+  fetch(blockIdx.x);
+  fetch_index();
+  fetch_particles();
   for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
     const int tile = tile_at(L, ntx, ntz);
-    const unsigned j0 = off[tile], j1 = off[tile + 1];
     const int tz = tile % ntz, ty = (tile / ntz) % ntx, tx = tile / (ntz * ntx);
     const int x0 = tx * KX, y0 = ty * KX, z0 = tz * KZ;
-    for (int e = threadIdx.x; e < BOX; e += blockDim.x) box[e] = 0.0f;
+    const unsigned jb = j0, je = j1;
+    for (int e = tid; e < (BOX + 3) / 4; e += kThreads)
+      reinterpret_cast<float4 *>(box)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    fetch(L + gridDim.x);
     __syncthreads();
-    for (unsigned j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-      const long long p = (long long)order[j];
+    auto deposit = [&](unsigned j, unsigned lattice, float px, float py, float pz) {
       int ix, iy, iz;
       float DX, DY, DZ;
-      particle_cell<P2>(s, np, p, qs[j], Ns, ls, inv_ns, N, scale, ox, oy, oz, ix, iy, iz, DX, DY, DZ);
+      cell_of<P2>(px, py, pz, lattice, Ns, ls, inv_ns, N, scale, ox, oy, oz, ix, iy, iz, DX, DY, DZ);
       const float TX = 1.0f - DX, TY = (1.0f - DY) * wpar, TZ = 1.0f - DZ;
       DY *= wpar;
       const int lx = ix - x0, ly = iy - y0, lz = iz - z0;
       if ((unsigned)lx >= (unsigned)KX || (unsigned)ly >= (unsigned)KX || (unsigned)lz >= (unsigned)KZ) {
         spill[atomicAdd(nspill, 1u)] = j;  // at most np entries: every slot once
-        continue;
+        return;
       }
       const int b = (lx * BX + ly) * BZ + lz;
       atomicAdd(box + b, TX * TY * TZ);
@@ -418,24 +492,34 @@ __global__ void __launch_bounds__(kThreads) k_cic_tiles_own(const float *__restr
       atomicAdd(box + b + BX * BZ + 1, DX * TY * DZ);
       atomicAdd(box + b + BX * BZ + BZ, DX * DY * TZ);
       atomicAdd(box + b + BX * BZ + BZ + 1, DX * DY * DZ);
+    };
+#pragma unroll
+    for (int c = 0; c < PF; c++)
+      if (jb + tid + c * kThreads < je) deposit(jb + tid + c * kThreads, lat[c], x[c][0], x[c][1], x[c][2]);
+    fetch_index();
+#pragma unroll 1
+    for (unsigned j = jb + tid + PF * kThreads; j < je; j += kThreads) {
+      const long long p = (long long)order[j];
+      deposit(j, qs[j], s[p], s[np + p], s[2 * np + p]);
     }
+    fetch_particles();
     __syncthreads();
     // interior: rows of the mesh have even length and z0 is even, so every
     // pair is 8-byte aligned
-    for (int e = threadIdx.x; e < KX * KX * (KZ / 2); e += blockDim.x) {
-      const int zp = e % (KZ / 2), r = e / (KZ / 2), yy = r % KX, xx = r / KX;
-      const float2 v = *reinterpret_cast<const float2 *>(box + (xx * BX + yy) * BZ + 2 * zp);
-      *reinterpret_cast<float2 *>(rho + ((long long)(x0 + xx) * N + (y0 + yy)) * P + z0 + 2 * zp) =
-          make_float2(v.x - 1.0f, v.y - 1.0f);
-    }
-    if (z0 + KZ == N) {
-      for (int r = threadIdx.x; r < KX * KX; r += blockDim.x) {
-        const int yy = r % KX, xx = r / KX;
-        *reinterpret_cast<float2 *>(rho + ((long long)(x0 + xx) * N + (y0 + yy)) * P + N) = make_float2(-1.0f, -1.0f);
+    float2 *hp = halo + (long long)tile * H::PAIRS;
+    for (int r = tid / LR; r < KX * KX; r += WR) {
+      const int yy = r % KX, xx = r / KX;
+      const float2 *bp = reinterpret_cast<const float2 *>(box + (xx * BX + yy) * BZ);
+      float2 *g = reinterpret_cast<float2 *>(rho + ((long long)(x0 + xx) * N + (y0 + yy)) * P + z0);
+      const float2 v = bp[zp];
+      g[zp] = make_float2(v.x - 1.0f, v.y - 1.0f);
+      if (zp == 0) {
+        hp[H::FX + H::FY + r] = bp[KZ / 2];
+        if (z0 + KZ == N) g[KZ / 2] = make_float2(-1.0f, -1.0f);
       }
     }
-    float2 *hp = halo + (long long)tile * H::PAIRS;
-    for (int h = threadIdx.x; h < H::PAIRS; h += blockDim.x) {
+    // the faces x = KX and y = KX
+    for (int h = tid; h < H::FX + H::FY; h += kThreads) {
       int xx, yy, zz;
       halo_pair<T>(h, xx, yy, zz);
       hp[h] = *reinterpret_cast<const float2 *>(box + (xx * BX + yy) * BZ + zz);
@@ -444,8 +528,8 @@ __global__ void __launch_bounds__(kThreads) k_cic_tiles_own(const float *__restr
   }
 }
 
-// The halos of k_cic_tiles_own added to the mesh (float2 reductions, zero
-// pairs skipped; a pair never straddles the periodic wrap: z0 + KZ is even
+// The halos of k_cic_tiles_own added to the mesh, a block per tile (float2
+// reductions, zero pairs skipped; a pair never straddles the periodic wrap: z0 + KZ is even
 // and at most N), then the listed particles straight to the mesh.
 template <int T, bool P2>
 __global__ void __launch_bounds__(kThreads) k_cic_halo(const float2 *__restrict__ halo, int ntx, int ntz,
@@ -458,20 +542,28 @@ __global__ void __launch_bounds__(kThreads) k_cic_halo(const float2 *__restrict_
                                                        const unsigned *__restrict__ spill,
                                                        const unsigned *__restrict__ nspill) {
   using H = tile_halo<T>;
-  const long long n = (long long)ntx * ntx * ntz * H::PAIRS;
+  constexpr int U = (H::PAIRS + kThreads - 1) / kThreads < 4 ? (H::PAIRS + kThreads - 1) / kThreads : 4;
+  const int ntiles = ntx * ntx * ntz;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const float2 v = halo[i];
-    if (v.x == 0.0f && v.y == 0.0f) continue;
-    const int tile = (int)(i / H::PAIRS), h = (int)(i - (long long)tile * H::PAIRS);
-    int xx, yy, zz;
-    halo_pair<T>(h, xx, yy, zz);
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int tz = tile % ntz, ty = (tile / ntz) % ntx, tx = tile / (ntz * ntx);
-    int gx = tx * H::KX + xx, gy = ty * H::KX + yy, gz = tz * H::KZ + zz;
-    if (gx >= N) gx -= N;
-    if (gy >= N) gy -= N;
-    if (gz >= N) gz -= N;
-    atomicAdd(reinterpret_cast<float2 *>(rho + ((long long)gx * N + gy) * P + gz), v);
+    const float2 *hp = halo + (long long)tile * H::PAIRS;
+    for (int h0 = threadIdx.x; h0 < H::PAIRS; h0 += U * kThreads) {
+      float2 v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) v[u] = h0 + u * kThreads < H::PAIRS ? hp[h0 + u * kThreads] : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (v[u].x == 0.0f && v[u].y == 0.0f) continue;
+        int xx, yy, zz;
+        halo_pair<T>(h0 + u * kThreads, xx, yy, zz);
+        int gx = tx * H::KX + xx, gy = ty * H::KX + yy, gz = tz * H::KZ + zz;
+        if (gx >= N) gx -= N;
+        if (gy >= N) gy -= N;
+        if (gz >= N) gz -= N;
+        atomicAdd(reinterpret_cast<float2 *>(rho + ((long long)gx * N + gy) * P + gz), v[u]);
+      }
+    }
   }
   const unsigned ns = *nspill;
   if (ns == 0) return;
@@ -951,8 +1043,8 @@ int mgp_cic_tiles_own(mgp_ctx *c, float wpar, const float *s, float *rho) {
   const int ls = lattice_log2(Ns);
   const float scale = (float)(N / c->p.Box);
   float2 *halo = (float2 *)c->tile_halo;
-  const int nb = mgp_blocks_for(ntiles * kThreads, 8);
-  const int nh = mgp_blocks_for(ntiles * pairs, 8);
+  const int nb = mgp_blocks_for(ntiles * kThreads, 5);
+  const int nh = mgp_blocks_for(ntiles * kThreads, 8);
 #define MGP_CIC_OWN(TT, PP)                                                                                          \
   do {                                                                                                               \
     k_cic_tiles_own<TT, PP><<<nb, kThreads, 0, c->stream>>>(s, c->dstate, c->np, Ns, ls, N, scale, wpar, rho,       \

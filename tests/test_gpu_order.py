@@ -54,6 +54,30 @@ def test_default_order_matches_explicit_orders(N, Ns):
         assert np.sqrt(np.mean(dx ** 2)) < 1e-5 * box / Ns
 
 
+@pytest.mark.parametrize("N,Ns,size", [(64, 32, (10, 10, 36)), (40, 24, (9, 9, 20)), (512, 64, (20, 20, 72))])
+def test_crowded_tiles_match_lattice_order(N, Ns, size):
+    """All particles in one corner: tiles with several thousand beside empty ones,
+    more than a block reads ahead.  A cell adds about 75 weights, at most 128
+    (bound 128 2^-24 of the largest cell)."""
+    box = 2.0 * N
+    rng = np.random.default_rng(Ns)
+    scale = 2.0 * (Ns ** 3 / 9.0 / np.prod(size)) ** (1 / 3)  # nine particles a cell
+    pos = (rng.random((Ns ** 3, 3)) * np.array(size) * scale + 5.0).astype(np.float32)
+    assert pos.max() < box
+    vel, d1, d2 = (rng.normal(0, 1.0, pos.shape).astype(np.float32) for _ in range(3))
+    out = []
+    for order in (0, 2):
+        with M.Context(params(N, Ns)) as ctx:
+            ctx.set_particle_order(order)
+            ctx.set_particles(pos, vel, d1, d2)
+            ctx.get_displacements(0.5)
+            rho = ctx.grid(0)[:, :, :N].astype(np.float64)
+            ctx.kick_drift(0.45, 0.55, 0.5, 0.6, drift=False)
+            out.append((rho, ctx.get_particles()[1].astype(np.float64)))
+    assert np.abs(out[0][0] - out[1][0]).max() < 128 * 2.0 ** -24 * np.abs(out[0][0]).max()
+    assert np.sqrt(np.mean((out[0][1] - out[1][1]) ** 2)) < 1e-5 * np.sqrt(np.mean(out[0][1] ** 2))
+
+
 @pytest.mark.parametrize("order", [0, 2])
 @pytest.mark.parametrize("N,Ns", [(16, 2), (32, 17), (64, 64)])
 def test_drift_subtracts_mean_velocity(N, Ns, order):
