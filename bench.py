@@ -327,13 +327,13 @@ def algorithmic_bytes(N, Np, kernel):
 
 
 # DRAM bytes per launch measured by ncu (dram__bytes.sum.per_second x gpu__time_duration.sum)
-# on the nDGP step at 256^3 particles / 512^3 mesh, one launch each at step 46 of the 50-step
-# run (profiles/deposit_and_kick_late_ndgp_256_512.md; tile deposit and tile kick over
-# 8 x 8 x 64-cell tiles, the kick reading each slot's lattice point from the sort; the
-# deposit's figure is its two passes, tile sums with owner writes and the halo pass).  Every term of these kernels scales with the particle count or the
+# on the nDGP step at 256^3 particles / 512^3 mesh, one launch each in the last step of a
+# 10-step run (profiles/kernels_ndgp_256_512.md; tile deposit and tile kick over
+# 8 x 8 x 64-cell tiles; the deposit's figure is its two passes, tile sums with owner
+# writes and the halo pass).  Every term of these kernels scales with the particle count or the
 # cell count, which grow together between the configurations (Nmesh = 2 Nsample), so the
 # figure is scaled by the cell count.
-TRAFFIC_256_512 = {"interp_kick_drift": 4.154e9, "cic": 1.420e9}
+TRAFFIC_256_512 = {"interp_kick_drift": 4.114e9, "cic": 1.471e9}
 
 
 def measured_traffic(cfg, N, Np, kernel):
@@ -496,8 +496,10 @@ def run_gpu(args):
 
     peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))) if os.path.exists(
         os.path.join(ROOT, "MEASURED_PEAKS.json")) else {"hbm_gbs": 6800.0}
-    # stages that are one own kernel (the "mg" stage wraps two cuFFT calls)
-    own = {k: v for k, v in stage_ms.items() if k in ("cic", "pofk", "forces", "interp_kick_drift") and v > 0}
+    # stages that are one pass of this library's: the "mg" stage wraps the screening's transforms, and on
+    # the meshes of the library's own transforms the "forces" stage is two of their passes
+    alone = ("cic", "pofk", "interp_kick_drift") + (() if N in (64, 128, 256, 512, 1024) else ("forces",))
+    own = {k: v for k, v in stage_ms.items() if k in alone and v > 0}
     dom = max(own, key=own.get)
     abytes = algorithmic_bytes(N, Np, dom)
     achieved = abytes / (own[dom] * 1e-3) / 1e9
@@ -505,7 +507,7 @@ def run_gpu(args):
     traffic = measured_traffic(cfg, N, Np, dom)
     roof = {"bound": "hbm", "kernel": dom, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "traffic": traffic,
-            "traffic_source": ("ncu DRAM bytes of one launch at step 46 of the 50-step nDGP run at 256^3 particles / "
+            "traffic_source": ("ncu DRAM bytes of one launch in the last step of a 10-step nDGP run at 256^3 particles / "
                                "512^3 mesh (rate x duration), scaled by particles and cells") if traffic else
                               "no ncu capture of this kernel for this workload",
             "algorithmic_bytes_per_launch": abytes, "mean_launch_ms": round(own[dom], 4),
