@@ -186,10 +186,12 @@ int mgp_launch_cic_range(const float *s, const mgp_dstate *st, long long np, lon
 // on the host in double exactly as pofk_bin_index, compute_pofk.c:30-46).
 // Mode counts and k sums are geometric and also precomputed on the host.
 //
-// Accumulation: a warp reads 32 consecutive modes (coalesced); lanes with the
+// Accumulation: a warp reads 64 consecutive modes, two a lane; lanes with the
 // same bin are contiguous (|k| grows along kz), so a segmented warp scan sums
-// each run in FP32 and the last lane of a run adds it to an FP64 shared-memory
-// bin; blocks write FP64 partials that k_pofk_reduce sums in fixed order.
+// each run in FP32 and the last lane of a run adds it to a compensated
+// shared-memory bin; blocks write FP64 partials that k_pofk_reduce sums in fixed
+// order.  Bound by instructions: with one mode a lane and kz = N/2 as a mode of the
+// scan, 65 modes took three scans of 32 (stage at 512: 170 -> 122 us, at 1024: 0.90 -> 0.74 ms).
 // Bin lookup: with `thr` (first |k|^2 of every bin, thr[nbins] = end of the
 // binned range; bins are monotone in |k|^2) a float estimate of the bin is
 // corrected against the exact integer thresholds held in shared memory, which
@@ -246,6 +248,27 @@ __global__ void __launch_bounds__(MGP_THREADS, 4) k_pofk(mgp_pofk_kargs a) {
   const float inv_span = (float)nbins / (a.kmax - a.kmin);
   const float inv_logspan = a.bintype ? (float)nbins / logf(a.kmax / a.kmin) : 0.0f;
   const int lo = a.thr ? sthr[0] : 0, hi = a.thr ? sthr[nbins] : 0;
+  auto bin_of = [&](int rk) {
+    if (!a.thr) return a.rk_bin[rk];
+    if (rk < lo || rk >= hi) return -1;
+    const float km = sqrtf((float)rk);
+    const float x = a.bintype ? logf(km / a.kmin) * inv_logspan : (km - a.kmin) * inv_span;
+    int b = (int)floorf(x + 0.5f);
+    b = b < 0 ? 0 : (b >= nbins ? nbins - 1 : b);
+    while (b > 0 && sthr[b] > rk) b--;
+    while (b + 1 < nbins && sthr[b + 1] <= rk) b++;
+    return b;
+  };
+  auto add = [&](int b, float v) {
+    const float old = a.priv ? shi[b] : atomicAdd(&shi[b], v);
+    const float sum = old + v, bp = sum - old, err = (old - (sum - bp)) + (v - bp);
+    if (a.priv) {
+      shi[b] = sum;
+      slo[b] += err;
+    } else {
+      atomicAdd(&slo[b], err);
+    }
+  };
   // One warp per (|d0|, |d1|) pair: the up to four stored rows (i, j) with
   // i in {d0, N-d0}, j in {d1, N-d1} share |k|^2 along kz, hence the bins,
   // window and filter; their powers are summed before the warp scan.
@@ -256,85 +279,96 @@ __global__ void __launch_bounds__(MGP_THREADS, 4) k_pofk(mgp_pofk_kargs a) {
     const float w01 = swin[d0] * swin[d1];
     const bool mi = !(d0 == 0 || d0 == h), mj = !(d1 == 0 || d1 == h);
     const bool use[4] = {true, mj, mi, mi && mj};
-    // row (i, j): its kz = 0 value, and the distance to its kz = N/2 value
-    const float2 *row[4];
-    long long last[4];
+    const float2 *row[4];  // row (i, j): its kz = 0 value
 #pragma unroll
     for (int t = 0; t < 4; t++) {
       const int i = t < 2 ? d0 : N - d0, j = t & 1 ? N - d1 : d1;
       const long long plane = (long long)i * N * NH;
       row[t] = dkb + (a.planar ? plane + (long long)j * h : plane + (long long)j * NH);
-      last[t] = a.planar ? (long long)(N - j) * h + j : h;
     }
-    // the rows' next 32 modes are loaded while the current ones are binned
-    float2 zn[4];
-#pragma unroll
-    for (int t = 0; t < 4; t++)
-      if (use[t] && lane < NH) zn[t] = row[t][lane == h ? last[t] : lane];
-    for (int k0 = 0; k0 < NH; k0 += 32) {
-      const int kz = k0 + lane;
-      float2 z[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) z[t] = zn[t];
-      if (kz + 32 < NH) {
-#pragma unroll
-        for (int t = 0; t < 4; t++)
-          if (use[t]) zn[t] = row[t][kz + 32 == h ? last[t] : kz + 32];
-      }
-      int bin = -1;
-      float pk = 0.0f;
-      if (kz < NH) {
-        const int rk = rk01 + kz * kz;
-        if (a.thr) {
-          if (rk >= lo && rk < hi) {
-            float km = sqrtf((float)rk);
-            float x = a.bintype ? logf(km / a.kmin) * inv_logspan : (km - a.kmin) * inv_span;
-            int b = (int)floorf(x + 0.5f);
-            b = b < 0 ? 0 : (b >= nbins ? nbins - 1 : b);
-            while (b > 0 && sthr[b] > rk) b--;
-            while (b + 1 < nbins && sthr[b + 1] <= rk) b++;
-            bin = b;
-          }
-        } else {
-          bin = a.rk_bin[rk];
+    // kz = N/2 of the four rows, a lane each, added to its bin after the loop
+    float plast = 0.0f;
+    {
+      const int i = lane & 2 ? N - d0 : d0, j = lane & 1 ? N - d1 : d1;
+      if (lane < 4 && (mi || !(lane & 2)) && (mj || !(lane & 1))) {
+        const long long plane = (long long)i * N * NH;
+        const long long o = a.planar ? plane + (long long)N * h + j : plane + (long long)j * NH + h;
+        const float2 z = dkb[o];
+        plast = z.x * z.x + z.y * z.y;
+        if (a.fuse_kind) {
+          const float f = mg_kfilter(rk01 + h * h, a.fuse_kind, a.filter, a.fuse_a, a.fuse_b);
+          fob[o] = make_float2(f * z.x, f * z.y);
         }
-        const float f = a.fuse_kind ? mg_kfilter(rk, a.fuse_kind, a.filter, a.fuse_a, a.fuse_b) : 0.0f;
-        float p2 = 0.0f;
+      }
+    }
+    for (int k0 = 0; k0 < h; k0 += 64) {
+      const int kz = k0 + 2 * lane;
+      // two modes a lane
+      int bin[2] = {-1, -1};
+      float pk[2] = {0.0f, 0.0f};
+      if (kz < h) {
+        const bool two = kz + 1 < h;
+        float4 z[4];  // both modes' values of a row; planar rows are 16-byte aligned (h even)
 #pragma unroll
         for (int t = 0; t < 4; t++)
           if (use[t]) {
-            p2 += z[t].x * z[t].x + z[t].y * z[t].y;
-            if (a.fuse_kind) fob[(row[t] - dkb) + kz] = make_float2(f * z[t].x, f * z[t].y);
+            if (a.planar) {
+              z[t] = *reinterpret_cast<const float4 *>(row[t] + kz);
+            } else {
+              const float2 z0 = row[t][kz], z1 = two ? row[t][kz + 1] : make_float2(0.0f, 0.0f);
+              z[t] = make_float4(z0.x, z0.y, z1.x, z1.y);
+            }
           }
-        if (bin >= 0) {
-          float w = (kz == 0 || 2 * kz == N) ? 1.0f : 2.0f;
-          pk = p2 * (w01 * swin[kz] * w);
+        float p2[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int t = 0; t < 4; t++)
+          if (use[t]) {
+            p2[0] += z[t].x * z[t].x + z[t].y * z[t].y;
+            p2[1] += z[t].z * z[t].z + z[t].w * z[t].w;
+          }
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+          if (m && !two) {
+            bin[1] = bin[0];
+            continue;
+          }
+          const int rk = rk01 + (kz + m) * (kz + m);
+          bin[m] = bin_of(rk);
+          if (bin[m] >= 0) pk[m] = p2[m] * (w01 * swin[kz + m] * (kz + m ? 2.0f : 1.0f));
+          if (a.fuse_kind) {
+            const float f = mg_kfilter(rk, a.fuse_kind, a.filter, a.fuse_a, a.fuse_b);
+#pragma unroll
+            for (int t = 0; t < 4; t++)
+              if (use[t])
+                fob[(row[t] - dkb) + kz + m] = m ? make_float2(f * z[t].z, f * z[t].w) : make_float2(f * z[t].x, f * z[t].y);
+          }
         }
       }
-      // segmented inclusive scan over runs of equal bin (|k| grows with kz)
-      int prev = __shfl_up_sync(0xffffffffu, bin, 1);
-      bool head = lane == 0 || prev != bin;
-      unsigned heads = __ballot_sync(0xffffffffu, head);
-      unsigned below = heads & ((2u << lane) - 1u);
-      int seg0 = 31 - __clz(below);
-      float acc = pk;
+      // segmented inclusive scan over the lanes' trailing runs of equal bin (|k|
+      // grows with kz); a lane with two bins ends the run before it as well
+      const bool one = bin[0] == bin[1];
+      const int prev = __shfl_up_sync(0xffffffffu, bin[1], 1);
+      const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || !one || prev != bin[0]);
+      const int seg0 = 31 - __clz(heads & ((2u << lane) - 1u));
+      float acc = one ? pk[0] + pk[1] : pk[1];
       for (int o = 1; o < 32; o <<= 1) {
-        float t = __shfl_up_sync(0xffffffffu, acc, o);
+        const float t = __shfl_up_sync(0xffffffffu, acc, o);
         if (lane - o >= seg0) acc += t;
       }
-      int nbin = __shfl_down_sync(0xffffffffu, bin, 1);
-      bool tail = lane == 31 || nbin != bin;
-      if (tail && bin >= 0) {
-        float old = a.priv ? shi[bin] : atomicAdd(&shi[bin], acc);
-        float sum = old + acc, bp = sum - old, err = (old - (sum - bp)) + (acc - bp);
-        if (a.priv) {
-          shi[bin] = sum;
-          slo[bin] += err;
-        } else {
-          atomicAdd(&slo[bin], err);
-        }
-      }
+      const float before = __shfl_up_sync(0xffffffffu, acc, 1);
+      const int next = __shfl_down_sync(0xffffffffu, bin[0], 1);
+      // every run ends once, so these lanes' bins are distinct
+      if (!one && bin[0] >= 0) add(bin[0], lane > 0 && prev == bin[0] ? pk[0] + before : pk[0]);
+      if ((lane == 31 || next != bin[1]) && bin[1] >= 0) add(bin[1], acc);
+      __syncwarp();  // a bin may go on in the next 64 modes
     }
+    plast += __shfl_xor_sync(0xffffffffu, plast, 1);
+    plast += __shfl_xor_sync(0xffffffffu, plast, 2);
+    if (lane == 0) {
+      const int b = bin_of(rk01 + h * h);
+      if (b >= 0) add(b, plast * (w01 * swin[h]));
+    }
+    __syncwarp();
   }
   __syncthreads();
   for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
