@@ -85,31 +85,58 @@ __host__ __device__ __forceinline__ int lattice_log2(int Ns) {
   return l;
 }
 
+// A thread's FP32 sum; kd_sum also keeps what its additions rounded away (Knuth's
+// TwoSum).
+struct kd_plain {
+  static constexpr bool two = false;
+  float s = 0.f;
+  __device__ __forceinline__ void add(float x) { s += x; }
+  __device__ __forceinline__ float rest() const { return 0.f; }
+};
+struct kd_sum {
+  static constexpr bool two = true;
+  float s = 0.f, r = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = s + x, b = t - s;
+    r += (s - (t - b)) + (x - b);
+    s = t;
+  }
+  __device__ __forceinline__ float rest() const { return r; }
+};
+
 // Means over all particles of the interpolated forces and the new velocities
 // at the end of a kick, and the FP64 offsets they move (Kick and Drift subtract
 // them, src/main.c:688-787).  Every block adds its threads' FP32 sums in FP64
 // and leaves six numbers in `partials`; the block that arrives last at `done`
 // adds the blocks' in index order and updates the state (done returns to 0 for
-// the next launch).  red: 6 NT floats of shared memory that are free.
+// the next launch).  acc: the forces' three sums, then the velocities'; red: 6 NT
+// floats of shared memory that are free.
 // FP64 runs at 1/64 of the FP32 rate here, so the adds are what counts: six
 // warps sum NT / 32 values a lane and then one tree each, instead of six trees
 // in every warp and a serial sum over warps (2^18 particles: 38 us the kick and
 // 11 us a kernel for the blocks' sums; one kernel of 21 us now).
-template <int NT>
-__device__ __forceinline__ void kd_means(const float (&accD)[3], const float (&accV)[3], float *red,
-                                         double *partials, int block, int nblocks, unsigned *done, mgp_dstate *st,
-                                         const mgp_kd_args &a) {
+template <int NT, class SUM>
+__device__ __forceinline__ void kd_means(const SUM (&acc)[6], float *red, double *partials, int block, int nblocks,
+                                         unsigned *done, mgp_dstate *st, const mgp_kd_args &a) {
   __shared__ double tot[6];
   __shared__ int last;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  float y = 0.0f;  // what the additions rounded away: FP32 is more than enough for its sum
+  if (SUM::two) {
 #pragma unroll
-  for (int q = 0; q < 3; q++) {
-    red[q * NT + tid] = accD[q];
-    red[(3 + q) * NT + tid] = accV[q];
+    for (int q = 0; q < 6; q++) red[q * NT + tid] = acc[q].rest();
+    __syncthreads();
+    if (w < 6) {
+#pragma unroll 4
+      for (int i = 0; i < NT / 32; i++) y += red[w * NT + 32 * i + lane];
+    }
+    __syncthreads();
   }
+#pragma unroll
+  for (int q = 0; q < 6; q++) red[q * NT + tid] = acc[q].s;
   __syncthreads();
   if (w < 6) {
-    double x = 0.0;
+    double x = (double)y;
 #pragma unroll 4
     for (int i = 0; i < NT / 32; i++) x += (double)red[w * NT + 32 * i + lane];
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);

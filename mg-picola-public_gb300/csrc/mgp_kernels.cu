@@ -597,7 +597,9 @@ __global__ void __launch_bounds__(MGP_THREADS, 4) k_interp_kick_drift(
   const float ox = (float)(st->cx[0] * a.scale), oy = (float)(st->cx[1] * a.scale), oz = (float)(st->cx[2] * a.scale);
   const float *F0 = frc, *F1 = frc + gf, *F2 = frc + 2 * gf;
   const IDX Pi = (IDX)P, NPi = (IDX)N * (IDX)P;
-  float accD[3] = {0.f, 0.f, 0.f}, accV[3] = {0.f, 0.f, 0.f};
+  // sums for the means, with the roundings of each addition in a second number: a
+  // thread takes as many particles as four blocks an SM leave it (108 of 2^24)
+  kd_sum acc[6];
   long long stride = (long long)gridDim.x * blockDim.x;
   const float inv_ns = 1.0f / (float)Ns;
   for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += stride) {
@@ -649,11 +651,11 @@ __global__ void __launch_bounds__(MGP_THREADS, 4) k_interp_kick_drift(
       float vn = v[o] + a.kick_disp * disp[ax] + a.kick_d1 * d1 + a.kick_d2 * d2;
       v[o] = vn;
       if (a.do_drift) s[o] = sp[ax] + vn * a.dyyy + a.dD1 * d1 + a.dD2 * d2;
-      accD[ax] += disp[ax];
-      accV[ax] += vn;
+      acc[ax].add(disp[ax]);
+      acc[3 + ax].add(vn);
     }
   }
-  kd_means<MGP_THREADS>(accD, accV, red, partials, blockIdx.x, gridDim.x, done, st, a);
+  kd_means<MGP_THREADS>(acc, red, partials, blockIdx.x, gridDim.x, done, st, a);
 }
 
 int mgp_ikd_blocks(long long np) { return blocks_for(np, 8); }

@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kThreads, NB) k_ikd_tiles(
     const int c = r / (X * X), rr = r - c * X * X, xx = rr / X, yy = rr - xx * X;
     rowoff[r] = c * gf + ((long long)xx * N + yy) * P - 2 * (yy & 1);
   }
-  float accD[3] = {0.f, 0.f, 0.f}, accV[3] = {0.f, 0.f, 0.f};
+  kd_plain acc[6];
   const PI npi = (PI)np;
   unsigned j0 = 0, j1 = 0, ord[PF], lat[PF];  // the current tile's particles, and the first PF of this thread's
   auto fetch = [&](int L) {
@@ -811,8 +811,8 @@ __global__ void __launch_bounds__(kThreads, NB) k_ikd_tiles(
         const float vn = u[ax] + a.kick_disp * disp[ax] + a.kick_d1 * d1 + a.kick_d2 * d2;
         v2[oj] = vn;
         s2[oj] = a.do_drift ? x[ax] + vn * a.dyyy + a.dD1 * d1 + a.dD2 * d2 : x[ax];
-        accD[ax] += disp[ax];
-        accV[ax] += vn;
+        acc[ax].add(disp[ax]);
+        acc[3 + ax].add(vn);
       }
     };
 #pragma unroll
@@ -828,7 +828,7 @@ __global__ void __launch_bounds__(kThreads, NB) k_ikd_tiles(
   }
   static_assert(6 * NT <= FT::FLOATS, "the sums reuse the force tile");
   __syncthreads();  // the last tile's reads of fs are done
-  kd_means<NT>(accD, accV, fs, partials, blockIdx.x, gridDim.x, done, st, a);
+  kd_means<NT>(acc, fs, partials, blockIdx.x, gridDim.x, done, st, a);
 }
 
 }  // namespace
@@ -1101,7 +1101,9 @@ int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a) {
   // SM), 8 x 8 x 64 tiles 65 KB (two blocks), 8^3 tiles 12 KB (eight)
   const size_t smem = sizeof(float) * (T == kElong ? force_tile<kElong>::FLOATS
                                                    : (T == 16 ? force_tile<16>::FLOATS : force_tile<8>::FLOATS));
-  int nb = T == kElong ? mgp_blocks_for(ntiles * 256, 2) : mgp_blocks_for(ntiles * 256, T == 8 ? 8 : 3);
+  // (8 x 8 x 64: a grid of twice the resident blocks, which halves the particles in a
+  // thread's FP32 sums for the means)
+  int nb = T == kElong ? mgp_blocks_for(ntiles * 256, 4) : mgp_blocks_for(ntiles * 256, T == 8 ? 8 : 3);
   if (nb > c->max_blocks) nb = c->max_blocks;
 #define MGP_IKD_TILES(TT, PP, PI)                                                                             \
   do {                                                                                                        \
