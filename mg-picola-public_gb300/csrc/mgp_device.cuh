@@ -182,4 +182,20 @@ __device__ __forceinline__ float mg_kfilter(int rk, int kind, int filter, float 
   return f * norm;
 }
 
+// Screening factors (src/mg.h:174-176, 241-250 with the functions of
+// src/user_defined_functions.h:725-773): min(1, |phi_crit / Phi|) where Phi < 0;
+// 2 (sqrt(1 + f) - 1) / f with f = pref (1 + delta_R), 1 below f = 1e-5.
+__device__ __forceinline__ float screen_pot(float ph, float phicrit) {
+  float f = 1.0f;
+  if (ph < 0.0f) {
+    f = fabsf(phicrit / ph);
+    if (f > 1.0f) f = 1.0f;
+  }
+  return f;
+}
+__device__ __forceinline__ float screen_den(float dsm, float pref) {
+  float fac = pref * (1.0f + dsm);
+  return fac < 1e-5f ? 1.0f : 2.0f * (sqrtf(1.0f + fac) - 1.0f) / fac;
+}
+
 #endif

@@ -759,14 +759,6 @@ int mgp_launch_smooth(const float *dk, float *out, int N, int filter, float kR1,
 // Potential screening (src/mg.h:174-176, screening_factor_potential at
 // src/user_defined_functions.h:725-750): rho *= min(1, |phicrit / Phi_N|)
 // where Phi_N < 0, else 1.  Padding entries are included as in the reference.
-__device__ __forceinline__ float screen_pot(float ph, float phicrit) {
-  float f = 1.0f;
-  if (ph < 0.0f) {
-    f = fabsf(phicrit / ph);
-    if (f > 1.0f) f = 1.0f;
-  }
-  return f;
-}
 __global__ void k_screen_potential(float *__restrict__ rho, const float *__restrict__ phi, long long n, float phicrit,
                                    const mgp_box_scalars *__restrict__ bs) {
   // box blockIdx.y: grids n floats apart
@@ -798,10 +790,6 @@ int mgp_launch_screen_potential(float *rho, const float *phi, long long n, float
 // Density screening (src/mg.h:241-250, screening_factor_density at
 // src/user_defined_functions.h:757-773): rho *= coupling * 2(sqrt(1+f)-1)/f,
 // f = pref (1 + delta_R), factor 1 when f < 1e-5.
-__device__ __forceinline__ float screen_den(float dsm, float pref) {
-  float fac = pref * (1.0f + dsm);
-  return fac < 1e-5f ? 1.0f : 2.0f * (sqrtf(1.0f + fac) - 1.0f) / fac;
-}
 // base 1: rho *= 1 + coupling * S, i.e. the density plus its fifth-force
 // source in one field (the force pass then reads one spectrum).
 __global__ void k_screen_density(float *__restrict__ rho, const float *__restrict__ dsm, long long n, float coupling,
