@@ -1334,7 +1334,7 @@ extern "C" int mgp_pofk_rsd(mgp_ctx *c, double A, int cap, int *nbins, double *k
   if (nbins) *nbins = nb;
   if (cap < nb) return mgp_set_error(MGP_EINVAL, "RSD capacity %d < %d bins", cap, nb);
   if (!c->rsd_block) {
-    MGP_CUDA(cudaMalloc(&c->rsd_block, sizeof(double) * 3 * (size_t)nb * (c->pk_blocks + 1)));
+    MGP_CUDA(cudaMalloc(&c->rsd_block, sizeof(double) * 3 * (size_t)nb * c->pk_blocks));
     MGP_CUDA(cudaMalloc(&c->rsd_sum, sizeof(double) * 3 * (size_t)nb));
   }
   const mgp_params *p = &c->p;

@@ -426,7 +426,7 @@ int mgp_launch_rsd_shift(const float *s, const float *v, const float *D1, const 
                          int lpt_pitch, const mgp_dstate *st, long long np, int Ns, int axis, float shift, float g1,
                          float g2, const unsigned *qlat, float *out, cudaStream_t stream);
 /* sums of P, P mu^2, P mu^4 per bin, mu along grid axis `los` (1 y, 2 z);
- * block_part: 3 nbins (nblocks + 1) values */
+ * block_part: 3 nbins nblocks values */
 int mgp_launch_pofk_mu(const float *dk, int N, const int *thr, const float *win, int nbins, int bintype, double kmin,
                        double kmax, int los, int planar, double *block_part, int nblocks, double *sums,
                        cudaStream_t st);

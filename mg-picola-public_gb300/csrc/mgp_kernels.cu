@@ -1733,23 +1733,28 @@ int mgp_launch_rsd_shift(const float *s, const float *v, const float *D1, const 
 // P mu^4 per bin with mu = k_los/|k|, mu = 0 for the k = 0 mode.  As k_pofk: a warp
 // takes the four rows that share (|kx|, |ky|), 32 modes at a time, sums the runs
 // of equal bin with a segmented scan (three values), and adds each run's total to
-// its own bins in FP32 with the rounding error kept apart; blocks write FP64
-// partials.  One FP64 shared-memory addition per mode and moment -- a
-// compare-and-swap loop, with all modes of a row falling into few bins -- took 2.9
-// of the 5.5 ms of a line of sight at 512^3.  The modes with all |k_i| < 32, whose
-// bins hold few modes and carry the multipoles' weight (35 P4 - 30 P2 + 3 P0
-// amplifies their rounding), are FP64 throughout, added to the partial row after
-// the blocks' (zeroed by the launcher).
+// its own bins; blocks write their partials.  FP64 from the modes' powers on: 35 P4 -
+// 30 P2 + 3 P0 amplifies the rounding of the moments.  FP64 instructions, a 64th of the
+// FP32 rate here, are what bounds it: the four powers are added and mu^2 is divided as an FP32
+// number and its remainder (Knuth's TwoSum; the remainder of the division is exact), and a scan
+// stops at the length of its longest run (bins as wide as a mode hold a few).  One shared-memory addition
+// per mode and moment -- a compare-and-swap loop, with all modes of a row falling
+// into few bins -- took 2.9 of the 5.5 ms of a line of sight at 512^3.
 #define MGP_MU_THREADS 128
+// a + b as an FP32 sum and what it rounded away
+__device__ __forceinline__ float2 two_sum(float a, float b) {
+  const float s = a + b, c = s - a;
+  return make_float2(s, (a - (s - c)) + (b - c));
+}
 __global__ void __launch_bounds__(MGP_MU_THREADS) k_pofk_mu(mgp_pofk_kargs a, int los) {
-  extern __shared__ float shf[];
+  extern __shared__ double shd[];
   const int N = a.N, nbins = a.nbins, NH = N / 2 + 1, h = N / 2, nwb = blockDim.x >> 5;
-  float *acc0 = shf;  // [warp][moment][hi, lo][nbins]
+  double *acc0 = shd;  // [warp][moment][nbins]
   const int *sthr = a.thr;  // priv: with room for them, the tables in shared memory too
   const float *swin = a.win;
-  for (int b = threadIdx.x; b < 6 * nwb * nbins; b += blockDim.x) acc0[b] = 0.0f;
+  for (int b = threadIdx.x; b < 3 * nwb * nbins; b += blockDim.x) acc0[b] = 0.0;
   if (a.priv) {
-    int *t = (int *)(acc0 + 6 * (size_t)nwb * nbins);
+    int *t = (int *)(acc0 + 3 * (size_t)nwb * nbins);
     float *w = (float *)(t + nbins + 1);
     for (int b = threadIdx.x; b <= nbins; b += blockDim.x) t[b] = a.thr[b];
     for (int d = threadIdx.x; d <= h; d += blockDim.x) w[d] = a.win[d];
@@ -1758,7 +1763,7 @@ __global__ void __launch_bounds__(MGP_MU_THREADS) k_pofk_mu(mgp_pofk_kargs a, in
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  float *acc = acc0 + 6 * (size_t)(threadIdx.x >> 5) * nbins;
+  double *acc = acc0 + 3 * (size_t)(threadIdx.x >> 5) * nbins;
   const long long wid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
   const float inv_span = (float)nbins / (a.kmax - a.kmin);
@@ -1783,21 +1788,21 @@ __global__ void __launch_bounds__(MGP_MU_THREADS) k_pofk_mu(mgp_pofk_kargs a, in
     for (int k0 = 0; k0 < NH; k0 += 32) {
       const int kz = k0 + lane;
       int bin = -1;
-      float m0 = 0.0f, m2 = 0.0f, m4 = 0.0f;
+      double m0 = 0.0, m2 = 0.0, m4 = 0.0;
       if (kz < NH) {
         const int rk = rk01 + kz * kz;
         if (rk >= lo && rk < hi) {
-          float p2 = 0.0f;
-          double e2 = 0.0;
-          const bool exact = k0 == 0 && d0 < 32 && d1 < 32;
+          float p[4];
 #pragma unroll
-          for (int t = 0; t < 4; t++)
+          for (int t = 0; t < 4; t++) {
+            p[t] = 0.0f;
             if (use[t]) {
               const float2 z = row[t][kz == h ? last[t] : kz];
-              const float p1 = z.x * z.x + z.y * z.y;
-              p2 += p1;
-              if (exact) e2 += (double)p1;
+              p[t] = z.x * z.x + z.y * z.y;
             }
+          }
+          const float2 pa = two_sum(p[0], p[1]), pb = two_sum(p[2], p[3]), ps = two_sum(pa.x, pb.x);
+          const double p2 = (double)ps.x + (double)(ps.y + (pa.y + pb.y));
           const float km = sqrtf((float)rk);
           const float x = a.bintype ? logf(km / a.kmin) * inv_logspan : (km - a.kmin) * inv_span;
           int b = (int)floorf(x + 0.5f);
@@ -1806,17 +1811,9 @@ __global__ void __launch_bounds__(MGP_MU_THREADS) k_pofk_mu(mgp_pofk_kargs a, in
           while (b + 1 < nbins && sthr[b + 1] <= rk) b++;
           bin = b;
           const int kl = los == 2 ? kz : d1;
-          if (exact) {
-            const double w = (double)(w01 * swin[kz]) * ((kz == 0 || 2 * kz == N) ? 1.0 : 2.0);
-            const double mu = rk == 0 ? 0.0 : (double)(kl * kl) / (double)rk, pk = e2 * w;
-            double *o = a.block_part + (long long)gridDim.x * 3 * nbins + b;
-            atomicAdd(o, pk);
-            atomicAdd(o + nbins, pk * mu);
-            atomicAdd(o + 2 * nbins, pk * mu * mu);
-            p2 = 0.0f;
-          }
-          const float mu2 = rk == 0 ? 0.0f : (float)(kl * kl) / (float)rk;
-          m0 = p2 * (w01 * swin[kz] * ((kz == 0 || 2 * kz == N) ? 1.0f : 2.0f));
+          const float frk = rk == 0 ? 1.0f : (float)rk, fkl = (float)(kl * kl), mh = fkl / frk;  // below 2^24: exact
+          const double mu2 = (double)mh + (double)(fmaf(-mh, frk, fkl) / frk);
+          m0 = p2 * (double)(w01 * swin[kz] * ((kz == 0 || 2 * kz == N) ? 1.0f : 2.0f));
           m2 = m0 * mu2;
           m4 = m2 * mu2;
         }
@@ -1824,9 +1821,9 @@ __global__ void __launch_bounds__(MGP_MU_THREADS) k_pofk_mu(mgp_pofk_kargs a, in
       const int prev = __shfl_up_sync(0xffffffffu, bin, 1);
       const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != bin);
       const int seg0 = 31 - __clz(heads & ((2u << lane) - 1u));
-      for (int o = 1; o < 32; o <<= 1) {
-        const float t0 = __shfl_up_sync(0xffffffffu, m0, o), t2 = __shfl_up_sync(0xffffffffu, m2, o),
-                    t4 = __shfl_up_sync(0xffffffffu, m4, o);
+      for (int o = 1; __any_sync(0xffffffffu, bin >= 0 && lane - o >= seg0); o <<= 1) {
+        const double t0 = __shfl_up_sync(0xffffffffu, m0, o), t2 = __shfl_up_sync(0xffffffffu, m2, o),
+                     t4 = __shfl_up_sync(0xffffffffu, m4, o);
         if (lane - o >= seg0) {
           m0 += t0;
           m2 += t2;
@@ -1835,26 +1832,17 @@ __global__ void __launch_bounds__(MGP_MU_THREADS) k_pofk_mu(mgp_pofk_kargs a, in
       }
       const int nbin = __shfl_down_sync(0xffffffffu, bin, 1);
       if ((lane == 31 || nbin != bin) && bin >= 0) {
-        const float m[3] = {m0, m2, m4};
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          float *p = acc + 2 * c * nbins + bin;
-          const float old = p[0], sum = old + m[c], bp = sum - old;
-          p[0] = sum;
-          p[nbins] += (old - (sum - bp)) + (m[c] - bp);
-        }
+        acc[bin] += m0;
+        acc[nbins + bin] += m2;
+        acc[2 * nbins + bin] += m4;
       }
       __syncwarp();  // a bin may go on in the next 32 modes
     }
   }
   __syncthreads();
   for (int b = threadIdx.x; b < 3 * nbins; b += blockDim.x) {
-    const int c = b / nbins, k = b - c * nbins;
     double t = 0.0;
-    for (int w = 0; w < nwb; w++) {
-      const float *p = acc0 + 6 * (size_t)w * nbins + 2 * c * nbins + k;
-      t += (double)p[0] + (double)p[nbins];
-    }
+    for (int w = 0; w < nwb; w++) t += acc0[3 * (size_t)w * nbins + b];
     a.block_part[(long long)blockIdx.x * 3 * nbins + b] = t;
   }
 }
@@ -1886,11 +1874,10 @@ int mgp_launch_pofk_mu(const float *dk, int N, const int *thr, const float *win,
       return mgp_set_error(MGP_EINVAL, "RSD P(k) needs %zu bytes of shared memory", shmem);
     }
   }
-  MGP_CUDA(cudaMemsetAsync(block_part + (size_t)nblocks * 3 * nbins, 0, sizeof(double) * 3 * nbins, st));
   k_pofk_mu<<<nblocks, threads, shmem, st>>>(ka, los);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
-  k_pofk_reduce<<<reduce_blocks(3 * nbins), 128, 0, st>>>(block_part, nblocks + 1, 3 * nbins, sums, 0, 0);
+  k_pofk_reduce<<<reduce_blocks(3 * nbins), 128, 0, st>>>(block_part, nblocks, 3 * nbins, sums, 0, 0);
   MGP_CHECK_LAUNCH();
   g_kernel_launches++;
   return MGP_OK;
