@@ -316,7 +316,8 @@ __global__ void __launch_bounds__(kThreadsConv, 2) k_conv_fwd(const bf16 *__rest
 // one is computed.  Warp (dk, ks) owns the nine taps of its k shift and 16 of the
 // 64 voxels: it holds the dY^T fragments of the 8 rows (ldmatrix.trans) and runs
 // every X fragment against all of them whose tap it is, 32 ldmatrix for 144 MMAs;
-// the dk = 1 warps also multiply dY^T by a ones fragment for the bias.  (A warp
+// the dk = 1 warps also multiply dY^T by a ones fragment for the bias, whose sums over
+// tiles keep what they round away (one warp's sum holds a 608th of the voxels).  (A warp
 // per staged-row offset, three taps, took 4 for 6: 384 us a layer at 192^3; now
 // 315, the tensor pipe 55% busy with the 12 warps that the sums leave room for.)
 // Sums stay in registers across tiles; at the end the four voxel quarters are
@@ -337,13 +338,15 @@ __global__ void __launch_bounds__(kThreadsWg, 1) k_conv_wgrad(const bf16 *__rest
   bf16 *buf = reinterpret_cast<bf16 *>(wg_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int dk = warp % 3, ks = warp / 3;
-  float acc[9][NT][4], bacc[4] = {0.f, 0.f, 0.f, 0.f};
+  float acc[9][NT][4];
+  __shared__ float2 bias[4][NN_CH];  // kd_sum of the dk = 1 warps, a lane's own; registers are short
 #pragma unroll
   for (int t = 0; t < 9; t++)
 #pragma unroll
     for (int n = 0; n < NT; n++)
 #pragma unroll
       for (int q = 0; q < 4; q++) acc[t][n][q] = 0.f;
+  if (tid < 4 * NN_CH) bias[tid / NN_CH][tid % NN_CH] = make_float2(0.f, 0.f);  // read past the first tile's barrier
   const uint32_t ones = 0x3F803F80u;  // two bf16 1.0
   // ldmatrix.trans lane roles: A = dY^T (16 out x 16 voxels), B = X (16 voxels x 16 in)
   const int a_vox = (lane & 7) + 8 * (lane >> 4), a_half = (lane >> 3) & 1;
@@ -377,11 +380,21 @@ __global__ void __launch_bounds__(kThreadsWg, 1) k_conv_wgrad(const bf16 *__rest
     const bf16 *xs = buf + slot * (kWgX + kWgY), *ys = xs + kWgX;
     if (16 * ks < N - t % nseg * CT_SEG) {  // the warp's voxels hold data
       uint32_t a[WG_OUT][4];
+      float bt[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int o = 0; o < WG_OUT; o++) {
         const int q = 16 * ks + a_vox;
         ldsm_x4_t(smem_u32(ys + (o * CT_SEG + q) * NN_CH + 8 * swz_half(q, a_half)), a[o][0], a[o][1], a[o][2], a[o][3]);
-        if (dk == 1) mma16816(bacc, a[o][0], a[o][1], a[o][2], a[o][3], ones, ones);
+        if (dk == 1) mma16816(bt, a[o][0], a[o][1], a[o][2], a[o][3], ones, ones);
+      }
+      if (dk == 1 && (lane & 3) == 0) {  // every column of the ones product holds the row sum
+#pragma unroll
+        for (int o = 0; o < 2; o++) {
+          float2 &b = bias[ks][(lane >> 2) + 8 * o];
+          kd_sum x{b.x, b.y};
+          x.add(bt[2 * o]);
+          b = make_float2(x.s, x.r);
+        }
       }
 #pragma unroll
       for (int r = 0; r < WG_ROWS; r++) {
@@ -418,10 +431,8 @@ __global__ void __launch_bounds__(kThreadsWg, 1) k_conv_wgrad(const bf16 *__rest
         w[(o0 + 8) * NN_CH] += acc[t][n][2];
         w[(o0 + 8) * NN_CH + 1] += acc[t][n][3];
       }
-    if (dk == 1 && (lane & 3) == 0) {  // every column of the ones product holds the row sum
-      sum[NN_WSIZE + o0] += bacc[0];
-      sum[NN_WSIZE + o0 + 8] += bacc[2];
-    }
+    if (dk == 1 && (lane & 3) == 0)
+      for (int o = o0; o < NN_CH; o += 8) sum[NN_WSIZE + o] += bias[ks][o].x + bias[ks][o].y;
   }
   __syncthreads();
   float *pb = partial + (size_t)blockIdx.x * kWgPartial;
