@@ -110,14 +110,16 @@ struct kd_sum {
 // and leaves six numbers in `partials`; the block that arrives last at `done`
 // adds the blocks' in index order and updates the state (done returns to 0 for
 // the next launch).  acc: the forces' three sums, then the velocities'; red: 6 NT
-// floats of shared memory that are free.
+// floats of shared memory that are free; keep (or NULL): as many sums that the
+// threads have put aside, in the same order.
 // FP64 runs at 1/64 of the FP32 rate here, so the adds are what counts: six
 // warps sum NT / 32 values a lane and then one tree each, instead of six trees
 // in every warp and a serial sum over warps (2^18 particles: 38 us the kick and
 // 11 us a kernel for the blocks' sums; one kernel of 21 us now).
 template <int NT, class SUM>
 __device__ __forceinline__ void kd_means(const SUM (&acc)[6], float *red, double *partials, int block, int nblocks,
-                                         unsigned *done, mgp_dstate *st, const mgp_kd_args &a) {
+                                         unsigned *done, mgp_dstate *st, const mgp_kd_args &a,
+                                         const float *keep = nullptr) {
   __shared__ double tot[6];
   __shared__ int last;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -139,6 +141,9 @@ __device__ __forceinline__ void kd_means(const SUM (&acc)[6], float *red, double
     double x = (double)y;
 #pragma unroll 4
     for (int i = 0; i < NT / 32; i++) x += (double)red[w * NT + 32 * i + lane];
+    if (keep)
+#pragma unroll 4
+      for (int i = 0; i < NT / 32; i++) x += (double)keep[w * NT + 32 * i + lane];
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
     if (lane == 0) {
       partials[(long long)block * 6 + w] = x;

@@ -667,17 +667,21 @@ __device__ __forceinline__ int tile_row(int c, int xx, int yy) {
 // threads with PF = 3 and 123 registers have all of them in flight; 512 threads
 // within 64 registers spill and were 25% slower, three blocks an SM as well.  A kick
 // at N = 512, Ns = 256: 892 -> 716 us (4.8 TB/s), at 1024, 512: 6.92 -> 5.69 ms.
-template <int T, bool P2, typename PI, int NB, int PF>
-__global__ void __launch_bounds__(kThreads, NB) k_ikd_tiles(
+// With half the threads of k_ikd_tiles_loop a thread has twice the particles in its sums for
+// the means, so it puts the sums aside once, in the middle of its tiles.
+template <bool P2, typename PI>
+__global__ void __launch_bounds__(kThreads, 2) k_ikd_tiles(
     const float *__restrict__ frc, long long gf, int N, long long P, int Ns, int ls, long long np,
     const float *__restrict__ s, const float *__restrict__ v, const float4 *__restrict__ lpt,
     const unsigned *__restrict__ qs, const unsigned *__restrict__ off, const unsigned *__restrict__ order, int ntx,
     int ntz, mgp_dstate *st, float *__restrict__ s2, float *__restrict__ v2, double *__restrict__ partials,
     unsigned *__restrict__ done, mgp_kd_args a) {
+  constexpr int T = kElong, PF = 3;
   using FT = force_tile<T>;
   constexpr int X = FT::X, R = FT::R, COMP = FT::COMP, K = FT::PIECES, KX = FT::TX, KZ = FT::TZ;
   constexpr int NT = kThreads, ROWS = NT / K;  // threads; rows copied per pass of the block
   extern __shared__ __align__(16) float fs[];  // FT::FLOATS
+  __shared__ float keep[6 * NT];
   __shared__ long long rowoff[3 * X * X];  // grid offset of a tile's row from the tile's own (no wrap)
   const int tid = threadIdx.x, sub = tid / K, k = tid - sub * K;  // this thread's row in a pass, its piece
   const float ox = (float)(st->cx[0] * a.scale), oy = (float)(st->cx[1] * a.scale), oz = (float)(st->cx[2] * a.scale);
@@ -688,6 +692,9 @@ __global__ void __launch_bounds__(kThreads, NB) k_ikd_tiles(
     rowoff[r] = c * gf + ((long long)xx * N + yy) * P - 2 * (yy & 1);
   }
   kd_plain acc[6];
+  int mid = (int)blockIdx.x + (ntiles / (int)gridDim.x + 1) / 2 * (int)gridDim.x;
+#pragma unroll
+  for (int q = 0; q < 6; q++) keep[q * NT + tid] = 0.f;
   const PI npi = (PI)np;
   unsigned j0 = 0, j1 = 0, ord[PF], lat[PF];  // the current tile's particles, and the first PF of this thread's
   auto fetch = [&](int L) {
@@ -710,6 +717,14 @@ __global__ void __launch_bounds__(kThreads, NB) k_ikd_tiles(
   fetch(blockIdx.x);
   fetch_index();
   for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
+    if (L >= mid) {
+      mid = ntiles;
+#pragma unroll
+      for (int q = 0; q < 6; q++) {
+        keep[q * NT + tid] = acc[q].s;
+        acc[q].s = 0.f;
+      }
+    }
     if (j0 == j1) {
       fetch(L + gridDim.x);
       fetch_index();
@@ -828,7 +843,119 @@ __global__ void __launch_bounds__(kThreads, NB) k_ikd_tiles(
   }
   static_assert(6 * NT <= FT::FLOATS, "the sums reuse the force tile");
   __syncthreads();  // the last tile's reads of fs are done
+  kd_means<NT>(acc, fs, partials, blockIdx.x, gridDim.x, done, st, a, keep);
+}
+
+// The same without reading ahead: for 8 x 8 x 64 tiles with more particles than the threads of
+// k_ikd_tiles have in flight, where the loop over them takes the time (512 threads within
+// 64 registers, two blocks an SM), and for cubic tiles, whose kernel is short of registers
+// for it (256 threads; N = 1008, Ns = 336: 6.9 ms a kick with one particle ahead, 6.0 without).
+template <int T, bool P2, typename PI, int NT>
+__global__ void __launch_bounds__(NT, NT >= 512 ? 2 : 0) k_ikd_tiles_loop(
+    const float *__restrict__ frc, long long gf, int N, long long P, int Ns, int ls, long long np,
+    const float *__restrict__ s, const float *__restrict__ v, const float4 *__restrict__ lpt,
+    const unsigned *__restrict__ qs, const unsigned *__restrict__ off, const unsigned *__restrict__ order, int ntx,
+    int ntz, mgp_dstate *st, float *__restrict__ s2, float *__restrict__ v2, double *__restrict__ partials,
+    unsigned *__restrict__ done, mgp_kd_args a) {
+  using FT = force_tile<T>;
+  constexpr int X = FT::X, R = FT::R, COMP = FT::COMP, K = FT::PIECES, KX = FT::TX, KZ = FT::TZ;
+  constexpr int ROWS = NT / K;  // rows copied per pass of the block
+  extern __shared__ __align__(16) float fs[];  // FT::FLOATS
+  __shared__ long long rowoff[X * X];  // grid offset of row (x0 + xx, y0 + yy), periodic
+  const int sub = threadIdx.x / K, k = threadIdx.x - sub * K;  // this thread's row in a pass, its piece
+  const float ox = (float)(st->cx[0] * a.scale), oy = (float)(st->cx[1] * a.scale), oz = (float)(st->cx[2] * a.scale);
+  const float inv_ns = 1.0f / (float)Ns;
+  const int ntiles = ntx * ntx * ntz;
+  kd_plain acc[6];
+  for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
+    const int tile = tile_at(L, ntx, ntz);
+    const unsigned j0 = off[tile], j1 = off[tile + 1];
+    if (j0 == j1) continue;
+    const int tz = tile % ntz, ty = (tile / ntz) % ntx, tx = tile / (ntz * ntx);
+    const int x0 = tx * KX, y0 = ty * KX, z0 = tz * KZ;
+    __syncthreads();  // the previous tile's reads of fs and rowoff are done
+    for (int r = threadIdx.x; r < X * X; r += NT) {
+      const int xx = r / X, yy = r - xx * X;
+      const int gx = x0 + xx >= N ? x0 + xx - N : x0 + xx, gy = y0 + yy >= N ? y0 + yy - N : y0 + yy;
+      rowoff[r] = ((long long)gx * N + gy) * P + z0 - 2 * (yy & 1);
+    }
+    __syncthreads();
+    if (sub < ROWS) {
+      for (int r = sub; r < 3 * X * X; r += ROWS) {
+        const int c = r >= 2 * X * X ? 2 : (r >= X * X ? 1 : 0), rr = r - c * X * X;
+        cp_async16(fs + c * COMP + rr * R + 4 * k, frc + c * gf + rowoff[rr] + 4 * k);
+      }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    if (z0 + KZ == N) {
+      // last tile in z: the halo column z0 + KZ is z = 0 of the same row
+      for (int r = threadIdx.x; r < 3 * X * X; r += NT) {
+        const int c = r / (X * X), rr = r - c * X * X, yy = rr % X;
+        fs[c * COMP + rr * R + 2 * (yy & 1) + KZ] = frc[c * gf + rowoff[rr] + 2 * (yy & 1) - z0];
+      }
+      __syncthreads();
+    }
+    const PI npi = (PI)np;
+    for (unsigned j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
+      const PI p = (PI)order[j];
+      const unsigned lat = qs[j];
+      const float sp[3] = {s[p], s[npi + p], s[2 * npi + p]};
+      const float4 l0 = lpt[2 * (size_t)lat], l1 = lpt[2 * (size_t)lat + 1];
+      const float D1p[3] = {l0.x, l0.y, l0.z}, D2p[3] = {l0.w, l1.x, l1.y};
+      int ix, iy, iz;
+      float DX, DY, DZ;
+      cell_of<P2>(sp[0], sp[1], sp[2], lat, Ns, ls, inv_ns, N, a.scale, ox, oy, oz, ix, iy, iz, DX, DY, DZ);
+      const float TX = 1.0f - DX, TY = 1.0f - DY, TZ = 1.0f - DZ;
+      const float w000 = TX * TY * TZ, w001 = TX * TY * DZ, w010 = TX * DY * TZ, w011 = TX * DY * DZ;
+      const float w100 = DX * TY * TZ, w101 = DX * TY * DZ, w110 = DX * DY * TZ, w111 = DX * DY * DZ;
+      const int lx = ix - x0, ly = iy - y0, lz = iz - z0;
+      float disp[3];
+      if ((unsigned)lx < (unsigned)KX && (unsigned)ly < (unsigned)KX && (unsigned)lz < (unsigned)KZ) {
+        // row (lx, ly + 1) is in the other parity's box
+        const float *f = fs + tile_row<T>(0, lx, ly) + lz;
+        const int dy = R + ((ly & 1) ? -2 : 2), dx = X * R;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const float *F = f + c * COMP;
+          disp[c] = F[0] * w000 + F[1] * w001 + F[dy] * w010 + F[dy + 1] * w011 + F[dx] * w100 + F[dx + 1] * w101 +
+                    F[dx + dy] * w110 + F[dx + dy + 1] * w111;
+        }
+      } else {
+        const long long xa = (long long)ix * N * P, xb = (ix + 1 == N ? 0 : (long long)(ix + 1) * N * P);
+        const long long ya = (long long)iy * P, yb = (iy + 1 == N ? 0 : (long long)(iy + 1) * P);
+        const long long za = iz, zb = iz + 1 == N ? 0 : iz + 1;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const float *F = frc + c * gf;
+          disp[c] = F[xa + ya + za] * w000 + F[xa + ya + zb] * w001 + F[xa + yb + za] * w010 +
+                    F[xa + yb + zb] * w011 + F[xb + ya + za] * w100 + F[xb + ya + zb] * w101 +
+                    F[xb + yb + za] * w110 + F[xb + yb + zb] * w111;
+        }
+      }
+#pragma unroll
+      for (int ax = 0; ax < 3; ax++) {
+        const PI o = (PI)ax * npi, oj = o + (PI)j;
+        const float d1 = D1p[ax], d2 = D2p[ax];
+        const float vn = v[o + p] + a.kick_disp * disp[ax] + a.kick_d1 * d1 + a.kick_d2 * d2;
+        v2[oj] = vn;
+        s2[oj] = a.do_drift ? sp[ax] + vn * a.dyyy + a.dD1 * d1 + a.dD2 * d2 : sp[ax];
+        acc[ax].add(disp[ax]);
+        acc[3 + ax].add(vn);
+      }
+    }
+  }
+  static_assert(6 * NT <= FT::FLOATS, "the sums reuse the force tile");
+  __syncthreads();  // the last tile's reads of fs are done
   kd_means<NT>(acc, fs, partials, blockIdx.x, gridDim.x, done, st, a);
+}
+
+template <int T, bool P2, typename PI>
+auto ikd_kernel(bool dense) {
+  if constexpr (T == kElong)
+    return dense ? k_ikd_tiles_loop<T, P2, PI, 512> : k_ikd_tiles<P2, PI>;
+  else
+    return k_ikd_tiles_loop<T, P2, PI, kThreads>;
 }
 
 }  // namespace
@@ -1098,18 +1225,24 @@ int mgp_ikd_tiles(mgp_ctx *c, const mgp_kd_args *a) {
   const int ls = lattice_log2(Ns);
   const long long ntiles = (long long)nt1 * nt1 * ntz;
   // forces per block: 16^3 tiles 68 KB (three blocks of 256 threads per
-  // SM), 8 x 8 x 64 tiles 65 KB (two blocks), 8^3 tiles 12 KB (eight)
+  // SM), 8 x 8 x 64 tiles 65 KB (two blocks of 256 or 512), 8^3 tiles 12 KB (eight)
   const size_t smem = sizeof(float) * (T == kElong ? force_tile<kElong>::FLOATS
                                                    : (T == 16 ? force_tile<16>::FLOATS : force_tile<8>::FLOATS));
-  // (8 x 8 x 64: a grid of twice the resident blocks, which halves the particles in a
-  // thread's FP32 sums for the means)
-  int nb = T == kElong ? mgp_blocks_for(ntiles * 256, 4) : mgp_blocks_for(ntiles * 256, T == 8 ? 8 : 3);
+  int nb = T == kElong ? mgp_blocks_for(ntiles * 256, 2) : mgp_blocks_for(ntiles * 256, T == 8 ? 8 : 3);
   if (nb > c->max_blocks) nb = c->max_blocks;
+  // more particles a tile than 256 threads hold ahead.  Microseconds a kick (k_ikd_tiles;
+  // k_ikd_tiles_loop), cells of 0.5 and 2 Mpc/h:
+  //   N = 512, Ns = 256    512 a tile   879; 932      729; 885
+  //   704, 400             751          3099; 2968    2593; 2636
+  //   512, 300             824          1340; 1266    1140; 1136
+  //   1024, 640            1000         12464; 11620  11189; 10629
+  //   640, 640             4096         10515; 8291   9155; 7160
+  const bool dense = c->np > 768 * ntiles;
 #define MGP_IKD_TILES(TT, PP, PI)                                                                             \
   do {                                                                                                        \
-    const auto kernel = TT == kElong ? k_ikd_tiles<TT, PP, PI, 2, 3> : k_ikd_tiles<TT, PP, PI, 3, 1>;         \
+    const auto kernel = ikd_kernel<TT, PP, PI>(dense);                                                        \
     MGP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));           \
-    kernel<<<nb, kThreads, smem, c->stream>>>(c->frc, c->g.nreal, N, c->g.P, Ns, ls, c->np, c->s, c->v,       \
+    kernel<<<nb, T == kElong && dense ? 512 : kThreads, smem, c->stream>>>(c->frc, c->g.nreal, N, c->g.P, Ns, ls, c->np, c->s, c->v,       \
                                               (const float4 *)c->lpt, c->q_alt, c->tile_off, c->tile_order,   \
                                               nt1, ntz, c->dstate, c->s_alt, c->v_alt, c->partials,           \
                                               c->kd_done, *a);                                                \

@@ -10,11 +10,10 @@ in the offset of all particles, so what is left of the displacement is the
 mean's error times dt, and the rounding of two FP32 numbers of that size and of
 their FP32 factor: 3 2^-24 c dt, plus the rounding of positions, 2^-24 box.
 
-2^24 particles on 152 SMs: with four blocks of 256 threads an SM a thread has 108
-particles in either order (in tile order, tiles of 8 x 8 x 64 cells with 512
-particles on this uniform lattice).  b = 18 in lattice order, where the sums keep what
-they round away: without that, exact up to 64; b = 17 in tile order: exact up to 128,
-past what a thread has.
+2^24 particles on 152 SMs: in lattice order, with four blocks of 256 threads an SM, a
+thread has 108 particles, and its sums keep what they round away (b = 18: without that,
+exact up to 64); in tile order, with two blocks and tiles of 512 particles on this
+uniform lattice, it has 216 and puts its sums aside half-way (b = 17: exact up to 128).
 """
 import numpy as np
 import pytest
