@@ -502,8 +502,10 @@ int mgp_mark(mgp_ctx *ctx, int slot);
  * reference).  Every step the particles are bucketed by the tile of the mesh
  * (8 x 8 x 64, 16^3 or 8^3 cells) holding their CIC base cell and deposited per tile
  * in shared memory (tiles = 1 or 2).  A single box starts out with 2 where
- * that is the faster order (Nmesh a multiple of 64 from 512 on, or of 16 from
- * 960 on), else with 0; a call here sets the order whatever the size.  tiles = 2: the kick also runs per tile -- the three force grids over the
+ * the mesh splits into tiles and is large (Nmesh a multiple of 64 from 512 on,
+ * of 16 from 640 on, of 8 with 2^28 particles and more), else with 0; a call
+ * here sets the order whatever the size.  tiles = 2: the kick also runs per
+ * tile -- the three force grids over the
  * tile staged in shared memory -- and writes the particles back in the
  * tile order, so the arrays follow the particles (with scale-independent
  * growth; the scale-dependent LPT fields keep the array-order kick); entry

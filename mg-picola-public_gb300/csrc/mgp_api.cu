@@ -997,7 +997,7 @@ static int fields_from_density(mgp_ctx *c, double A);
 
 // Tile shape of a single box's deposit, 0: in lattice order.
 static int tile_side(const mgp_ctx *c) {
-  if (!c->tile_mode || (c->tile_mode == 2 && !mgp_tiles_pay(c->g.N))) return 0;
+  if (!c->tile_mode || (c->tile_mode == 2 && !mgp_tiles_pay(c->g.N, c->np))) return 0;
   return mgp_tile_side(c->g.N, c->np);
 }
 

@@ -370,7 +370,7 @@ int mgp_launch_ikd(const float *frc, long long grid_floats, int N, long long P, 
 int mgp_ikd_blocks(long long np);
 /* cell-tile order (mgp_tiles.cu) */
 int mgp_tile_side(int N, long long np);
-bool mgp_tiles_pay(int N);
+bool mgp_tiles_pay(int N, long long np);
 int mgp_tiles_check(const mgp_ctx *c, int T);
 int mgp_tiles_alloc(mgp_ctx *c, int T);
 void mgp_tiles_free(mgp_ctx *c);

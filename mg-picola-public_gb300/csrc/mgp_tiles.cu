@@ -960,17 +960,30 @@ auto ikd_kernel(bool dense) {
 
 }  // namespace
 
-// Whether a context left to choose buckets its particles.  On smaller meshes the
-// mesh and much of the force grids stay in L2, the lattice-order deposit and kick
-// find their cells there, and the sort and the tiles cost more than they save; the
-// cubic tiles cost more than the long ones, which need Nmesh a multiple of 64.
-// Microseconds a step (tiles; lattice order), Ns = N/2, cells of 0.5 and of 2 Mpc/h:
-//   N = 64   96; 56        90; 55          528 (16^3)   7624; 7094     7360; 6769
-//   128      156; 97       142; 93         784 (16^3)   32053; 31265   31577; 28864
-//   256      578; 432      528; 416        1008 (16^3)  99641; 102582  97987; 95058
-//   384      3024; 2631    2923; 2553      520 (8^3)    11493; 8686    11320; 8336
-//   512      3566; 3648    3392; 3247      1024         29148; 39071   27809; 29442
-bool mgp_tiles_pay(int N) { return N % kElong == 0 ? N >= 512 : N % 16 == 0 && N >= 960; }
+// Whether a context left to choose buckets its particles.  Lattice order wins where the
+// mesh and much of the force grids stay in L2 and the particles are near their lattice
+// cells: on small meshes, and with large cells (a displacement is fewer of them).  Tiles win
+// on large meshes with many particles or small cells.  The cells grow and the particles
+// spread through a run, so the line goes by the sizes alone, and lies where neither order is
+// far behind: a step in tile order is 10% behind at most where this chooses it, one in
+// lattice order 1% at most.  Milliseconds a step (lattice order; tiles), cells of 0.5 and
+// of 2 Mpc/h:
+//   8 x 8 x 64 tiles (Nmesh a multiple of 64)
+//   N = 256, Ns = 128    0.416; 0.578  0.416; 0.528      512, 170    4.03; 4.27  3.93; 4.22
+//   384, 192             2.63; 3.02    2.55; 2.92        512, 512    14.9; 12.2  11.0; 10.2
+//   768, 256             33.8; 32.9    32.6; 32.8        1024, 512   39.1; 29.1  29.4; 27.8
+//   16^3
+//   528, 264             7.09; 7.62    6.77; 7.36        656, 328    45.0; 44.6  43.2; 43.6
+//   592, 592             47.0; 47.7    41.6; 43.2        656, 656    69.1; 65.9  58.7; 60.5
+//   720, 240             25.2; 25.6    24.4; 25.0        912, 608    123; 108    103; 105
+//   8^3
+//   600, 600             36.0; 36.5    29.8; 33.6        808, 808    157; 140    127; 134
+//   1000, 500            77.7; 79.9    66.5; 78.3        968, 646    106; 94.1   80.3; 88.3
+bool mgp_tiles_pay(int N, long long np) {
+  if (N % kElong == 0) return N >= 512;
+  if (N % 16 == 0) return N >= 640;
+  return np >= 1LL << 28;
+}
 
 // Tile shape of the single-box tile path, or 0 when it does not apply (the
 // mesh must split into whole tiles and the indices fit 32 bits): 8 x 8 x 64

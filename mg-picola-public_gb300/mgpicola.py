@@ -503,10 +503,10 @@ class Context:
     def set_particle_order(self, tiles):
         """Cell-tile particle order (mgp_set_particle_order): 2 the tile
         deposit and the kick per tile with the arrays rewritten in tile order
-        every step (what a single box starts with from Nmesh = 512 on, where
-        Nmesh is a multiple of 64), 1 the tile deposit with the arrays in
-        lattice order, 0 the deposit and kick in lattice order (what it
-        starts with else)."""
+        every step (what a single box starts with where Nmesh is a multiple
+        of 64 from 512 on, of 16 from 640 on, or of 8 with 2^28 particles
+        and more), 1 the tile deposit with the arrays in lattice order, 0 the
+        deposit and kick in lattice order (what it starts with else)."""
         _check(lib().mgp_set_particle_order(self.h, int(tiles)))
 
     def set_fft_mode(self, mode):
