@@ -641,6 +641,21 @@ static int ic_prepare(mgp_ctx *c, int namp, int draw) {
                            mgp_cosmo_growth_lcdm0(c0), c->stream);
 }
 
+// Scratch grids of the IC, kept by the context for its next IC (runs of many ICs --
+// the boxes of a batch, repeated runs -- allocate them once).
+int mgp_ic_scratch(mgp_ctx *c, int grids) {
+  if (c->ic_grids >= grids) return MGP_OK;
+  if (c->ic_scratch) {
+    MGP_CUDA(cudaStreamSynchronize(c->stream));
+    cudaFree(c->ic_scratch);
+    c->ic_scratch = NULL;
+    c->ic_grids = 0;
+  }
+  MGP_CUDA(cudaMalloc(&c->ic_scratch, sizeof(float) * (size_t)grids * c->g.nreal));
+  c->ic_grids = grids;
+  return MGP_OK;
+}
+
 // Mode cut of the draw (the cube cut of 2LPT.c:383-386 with the reference's
 // double expression: the largest |d| it keeps) and the number of amplitudes.
 static int ic_cut(const mgp_ctx *c, int *namp) {
@@ -742,10 +757,8 @@ static int ic_box(mgp_ctx *c, int bx, const double *pos01, size_t npos) {
   const double vD2 = pb->UseCOLA ? 0.0 : mgp_cosmo_growth(cb, 4, ai);
   const int nblk = mgp_ikd_blocks(c->np);
   // six scratch grids for the displacement gradients and the six
-  // displacement fields (2LPT.c:1214-1219, 1300-1306), kept by the context
-  // for its next IC (runs of many ICs -- the boxes of a batch, repeated
-  // runs -- allocate them once)
-  if (!c->ic_scratch) MGP_CUDA(cudaMalloc(&c->ic_scratch, sizeof(float) * 6 * (size_t)gf));
+  // displacement fields (2LPT.c:1214-1219, 1300-1306)
+  RET_IF(mgp_ic_scratch(c, 6));
   float *g6 = c->ic_scratch;
   if (pos01)
     RET_IF(ic_density(c, pos01, npos, false));
@@ -1094,6 +1107,7 @@ static int user_screen_pass(mgp_ctx *c, const mgp_fft_plan *f) {
 
 static int fields_own(mgp_ctx *c, double A) {
   mgp_fft_plan f = field_plan(c, A, NULL);
+  c->have_forces = 0;  // the passes before the forces use their grids
   tstart(c, T_R2C);
   RET_IF(mgp_fft_density(c, &f));
   tstop(c, T_R2C);
@@ -1133,7 +1147,9 @@ static int fields_from_density(mgp_ctx *c, double A) {
   c->rho_planar = 0;
   // a closure whose high-pass keeps more than the mean out adds its residual
   // to force spectra in cuFFT's layout
-  if (own_fft(c) && !(c->closure && !mgp_closure_real(c->closure))) return fields_own(c, A);
+  // (without room for the scratch grid the 3D plans, which need none, still run)
+  if (own_fft(c) && !(c->closure && !mgp_closure_real(c->closure)) && mgp_fft_scratch(c) == MGP_OK)
+    return fields_own(c, A);
   const int N = c->g.N;
   c->dk_planar = 0;
   tstart(c, T_R2C);

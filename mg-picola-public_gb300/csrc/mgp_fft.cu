@@ -137,14 +137,24 @@ struct passes {
     a.bs_in = a.bs_out = gs / 2;
     return z(MGP_Z_R2C, a);
   }
-  int z_c2r(const float *in, float *out, long long gs, int n) const {
+  int z_c2r(const float *in, float *out, long long gs, int n) const { return z_c2r(in, gs, out, gs, n); }
+  int z_c2r(const float *in, long long gs_in, float *out, long long gs_out, int n) const {
     mgp_fft_z a;
     memset(&a, 0, sizeof(a));
     a.in = (const float2 *)in;
     a.real = (float2 *)out;
     a.rows = rows(n);
-    a.bs_in = a.bs_real = gs / 2;
+    a.bs_in = gs_in / 2;
+    a.bs_real = gs_out / 2;
     return z(MGP_Z_C2R, a);
+  }
+  // z rows of three spectra to the grids g, g + gs, g + 2 gs: those in the second and
+  // third go down by one, the one in `last` to the third, one after the other (a row of
+  // a grid and of its spectrum do not lie in the same place).  n boxes.
+  int z_c2r_down(float *g, long long gs, long long bs, const float *last, long long bs_last, int n) const {
+    RET_IF(z_c2r(g + gs, bs, g, bs, n));
+    RET_IF(z_c2r(g + 2 * gs, bs, g + gs, bs, n));
+    return z_c2r(last, bs_last, g + 2 * gs, bs, n);
   }
   int y(int dir, float *g, long long gs, int n) const {
     mgp_fft_y a;
@@ -152,13 +162,13 @@ struct passes {
     a.ntask = 1;
     a.task[0].in = (const float2 *)g;
     a.task[0].out[0] = (float2 *)g;
+    a.task[0].bs_in = a.task[0].bs_out[0] = gs / 2;
     a.task[0].nout = 1;
-    return y(dir, 0, a, gs, n);
+    return y(dir, 0, a, n);
   }
-  int y(int dir, int gen, mgp_fft_y a, long long gs, int n, int kc = 1 << 30) const {
+  int y(int dir, int gen, mgp_fft_y a, int n, int kc = 1 << 30) const {
     a.tw = tw;
     a.nbox = n;
-    a.bs = gs / 2;
     a.kc = kc;
     return launched(o->y(dir, gen, a, sms, c->stream));
   }
@@ -201,6 +211,22 @@ int mgp_fft_c2r(mgp_ctx *c, int N, float *in, float *out, int n, long long gs) {
   return p.z_c2r(in, out, gs, n);
 }
 
+// The same of the three planar spectra at g + gs, g + 2 gs and last into the grids g,
+// g + gs and g + 2 gs.
+int mgp_fft_c2r_down(mgp_ctx *c, int N, float *g, float *last, long long gs) {
+  const passes p(c, N);
+  if (!p.ok()) return mgp_set_error(MGP_EINVAL, "no transform of size %d", N);
+  for (int q = 0; q < 2; q++) {
+    float *s = q ? last : g + gs;
+    const int n = q ? 1 : 2;
+    mgp_fft_x a = x_args(s, gs);
+    a.o[0] = (float2 *)s;
+    RET_IF(p.x(0, MGP_X_INV, a, n));
+    RET_IF(p.y(1, s, gs, n));
+  }
+  return p.z_c2r_down(g, gs, 0, last, 0, 1);
+}
+
 // A planar spectrum's x planes x0 .. x1 - 1 in the [N][N][N/2+1] layout.
 __global__ void k_planar_rows(const float2 *__restrict__ in, float2 *__restrict__ out, int N, long long rows) {
   const int lane = threadIdx.x & 31, h = N / 2;
@@ -221,31 +247,56 @@ int mgp_fft_planar_rows(int N, const float *in, float *out, int x0, int x1, cuda
   return MGP_OK;
 }
 
-// Scratch spectra of the field passes and the IC: three per box.
+// Scratch spectra of the field passes and the IC.  A batch takes its density grid, which
+// nothing reads after the fifth force's source spectrum; a single box keeps that grid
+// for its caller and has one of its own, or three where they are small (64 MB, meshes up to 128),
+// which saves two launches a step.
 int mgp_fft_scratch(mgp_ctx *c) {
-  if (!c->fft_scr) MGP_CUDA(cudaMalloc(&c->fft_scr, sizeof(float) * 3 * (size_t)c->g.nreal * c->nbox));
+  if (c->nbox > 1 || c->fft_scr) return MGP_OK;
+  const size_t bytes = sizeof(float) * (size_t)c->g.nreal;
+  const int grids = 3 * bytes <= (64u << 20) ? 3 : 1;
+  if (cudaMalloc(&c->fft_scr, grids * bytes) != cudaSuccess) {
+    cudaGetLastError();
+    c->fft_scr = NULL;
+    return mgp_set_error(MGP_ECUDA, "no memory for the transforms' scratch grid");
+  }
+  c->fft_scr_grids = grids;
   return MGP_OK;
 }
 
 // The field passes of the PM step (src/auxPM.c:358-555, src/mg.h:21-309) from
 // the density in rho: delta(k) in dk, the fifth force's source spectrum in
 // rho (both planar), and the three force grids, for all boxes of the context.
-// The P(k) and neutrino passes between them are the caller's.  Spectra live in
-// three scratch grids F0, F1, F2 a box (box stride 3 grids):
-//   density  rho -> dk; with a filter its inverse x lines -> F0; else, one
-//            spectrum being all the forces need, their x lines -> F0, F2
-//   screen   F0 -> mg1 (real), rho -> F1
-//   force_x  F1 (or dk) -> F0 (k_x G), F2 (G), the source spectrum -> rho
-//   force_y  F0 -> F0, F2 -> F1, F2
-//   force_z  F0, F1, F2 -> the force grids
-static float *scr(const mgp_ctx *c, int q) { return c->fft_scr + (size_t)q * c->g.nreal; }
+// The P(k) and neutrino passes between them are the caller's.  Spectra live in the
+// second and third force grid of a box, F1 and F2, and in its scratch grid F3 (three grids
+// of scratch a box before, which made the largest batch smaller by a quarter), or in three
+// scratch grids:
+//   density  rho -> dk; with a filter its inverse x lines -> F1; else, one
+//            spectrum being all the forces need, their x lines -> F1, F2
+//   screen   F1 -> mg1 (real), rho -> F2
+//   force_x  F2 (or dk) -> F1 (k_x G), F2 (G), the source spectrum -> rho
+//   force_y  F1 -> F1, F2 -> F2, F3
+//   force_z  F1, F2, F3 -> the force grids
+static float *frc(const mgp_ctx *c, int q) { return c->frc + (size_t)q * c->g.nreal; }
+static bool apart(const mgp_ctx *c) { return c->nbox == 1 && c->fft_scr_grids == 3; }
+static float *F(const mgp_ctx *c, int q) {
+  if (apart(c)) return c->fft_scr + (size_t)(q - 1) * c->g.nreal;
+  return q < 3 ? frc(c, q) : (c->nbox == 1 ? c->fft_scr : c->rho);
+}
+// z rows of F1, F2, F3 to the force grids
+static int z_forces(const passes &p) {
+  mgp_ctx *c = p.c;
+  const long long gs = c->g.nreal;
+  if (apart(c)) return p.z_c2r(F(c, 1), c->frc, gs, 3);
+  return p.z_c2r_down(c->frc, gs, 3 * gs, F(c, 3), gs, c->nbox);
+}
 
 static mgp_fft_x force_args(mgp_ctx *c, const mgp_fft_plan *f, float *in, long long bs_in, float *spec) {
   mgp_fft_x a = x_args(in, c->g.nreal);
   a.bs_in = bs_in;
   a.spec = (float2 *)spec;
-  a.o[0] = (float2 *)scr(c, 0);
-  a.o[1] = (float2 *)scr(c, 2);
+  a.o[0] = (float2 *)F(c, 1);
+  a.o[1] = (float2 *)F(c, 2);
   a.bs_o = 3 * c->g.nreal / 2;
   a.mg_kind = f->mg_kind;
   a.cfac = f->cfac;
@@ -261,7 +312,7 @@ static mgp_fft_x force_args(mgp_ctx *c, const mgp_fft_plan *f, float *in, long l
 
 static mgp_fft_x filter_args(mgp_ctx *c, const mgp_fft_plan *f) {
   mgp_fft_x a = x_args(c->dk, c->g.nreal);
-  a.o[0] = (float2 *)scr(c, 0);
+  a.o[0] = (float2 *)F(c, 1);
   a.bs_o = 3 * c->g.nreal / 2;
   a.filter_kind = f->filter_kind;
   a.filter = f->filter;
@@ -291,8 +342,8 @@ int mgp_fft_screen(mgp_ctx *c, const mgp_fft_plan *f, int (*user)(mgp_ctx *, con
   const long long gs = c->g.nreal;
   mgp_fft_z a;
   memset(&a, 0, sizeof(a));
-  a.in = (const float2 *)scr(c, 0);
-  a.out = (float2 *)scr(c, 1);
+  a.in = (const float2 *)F(c, 1);
+  a.out = (float2 *)F(c, 2);
   a.bs_in = a.bs_out = 3 * gs / 2;
   a.real = (float2 *)c->mg1;
   a.rho = (const float2 *)c->rho;
@@ -300,7 +351,7 @@ int mgp_fft_screen(mgp_ctx *c, const mgp_fft_plan *f, int (*user)(mgp_ctx *, con
   a.rows = p.rows(n);
   if (f->filter_kind) {
     if (f->split) RET_IF(p.x(0, MGP_X_INV, filter_args(c, f), n));
-    RET_IF(p.y(1, scr(c, 0), 3 * gs, n));
+    RET_IF(p.y(1, F(c, 1), 3 * gs, n));
     if (user) {
       RET_IF(p.z(MGP_Z_C2R, a));
       RET_IF(user(c, f));
@@ -319,45 +370,41 @@ int mgp_fft_screen(mgp_ctx *c, const mgp_fft_plan *f, int (*user)(mgp_ctx *, con
     a.bs_in = gs / 2;
     RET_IF(p.z(MGP_Z_R2C, a));
   }
-  return p.y(-1, scr(c, 1), 3 * gs, n);
+  return p.y(-1, F(c, 2), 3 * gs, n);
 }
 
 int mgp_fft_force_x(mgp_ctx *c, const mgp_fft_plan *f) {
   const passes p(c, c->g.N);
   const long long gs = c->g.nreal;
   if (!f->from_rho) return p.x(0, MGP_X_FORCE, force_args(c, f, c->dk, gs / 2, NULL), c->nbox);
-  RET_IF(p.x(1, MGP_X_FORCE, force_args(c, f, scr(c, 1), 3 * gs / 2, c->rho), c->nbox));
+  RET_IF(p.x(1, MGP_X_FORCE, force_args(c, f, F(c, 2), 3 * gs / 2, c->rho), c->nbox));
   c->rho_planar = 1;
   return MGP_OK;
 }
 
-// y pass of the force fields f[0] (kx G) and f[2] (G) after their x lines
-static mgp_fft_y force_y_args(float2 *const *f) {
+// y pass of the force fields kx G in F1 and G in F2 after their x lines: F_x in F1, F_y =
+// ky G in F2, F_z = kz G in F3
+static mgp_fft_y force_y_args(const mgp_ctx *c) {
+  const long long bs = 3 * c->g.nreal / 2;
   mgp_fft_y a;
   memset(&a, 0, sizeof(a));
   a.ntask = 2;
-  a.task[0].in = f[0];
-  a.task[0].out[0] = f[0];
+  a.task[0].in = a.task[0].out[0] = (float2 *)F(c, 1);
+  a.task[0].bs_in = a.task[0].bs_out[0] = bs;
   a.task[0].nout = 1;
-  a.task[1].in = f[2];  // inverse x transform of G: F_y = ky G, F_z = kz G
-  a.task[1].out[0] = f[1];
+  a.task[1].in = a.task[1].out[0] = (float2 *)F(c, 2);
+  a.task[1].bs_in = a.task[1].bs_out[0] = bs;
   a.task[1].ypow[0] = 1;
-  a.task[1].out[1] = f[2];
+  a.task[1].out[1] = (float2 *)F(c, 3);
+  a.task[1].bs_out[1] = c->g.nreal / 2;
   a.task[1].zpow[1] = 1;
   a.task[1].nout = 2;
   return a;
 }
 
-int mgp_fft_force_y(mgp_ctx *c) {
-  const passes p(c, c->g.N);
-  float2 *f[3] = {(float2 *)scr(c, 0), (float2 *)scr(c, 1), (float2 *)scr(c, 2)};
-  return p.y(1, 1, force_y_args(f), 3 * c->g.nreal, c->nbox);
-}
+int mgp_fft_force_y(mgp_ctx *c) { return passes(c, c->g.N).y(1, 1, force_y_args(c), c->nbox); }
 
-int mgp_fft_force_z(mgp_ctx *c) {
-  const passes p(c, c->g.N);
-  return p.z_c2r(scr(c, 0), c->frc, c->g.nreal, 3 * c->nbox);
-}
+int mgp_fft_force_z(mgp_ctx *c) { return z_forces(passes(c, c->g.N)); }
 
 // The 2LPT source's spectrum in rho from delta(k) in dk (src/2LPT.c:1224-1290),
 // both planar, for all boxes: three inverse x transforms of -delta / k^2 times 1,
@@ -365,54 +412,68 @@ int mgp_fft_force_z(mgp_ctx *c) {
 // inverts the six rows, forms the source and transforms it forward.  delta is
 // zero beyond |k| <= kc: columns and tiles beyond it are skipped (at Nmesh = 2
 // Nsample a quarter of the x columns and half of the y columns are left).
-// Gradients 00, 01, 02 in the force grids, 11, 12, 22 in the scratch spectra.
+// A box's six gradients take the force grids: of two boxes in a batch, which goes by as
+// many boxes as have room there; a single box has its scratch and, with one grid of it,
+// two more.
 int mgp_fft_ic_source(mgp_ctx *c, int kc) {
   const passes p(c, c->g.N);
-  const int n = c->nbox;
   const long long gs = c->g.nreal;
+  const int per = c->nbox == 1 ? 1 : c->nbox / 2;
   RET_IF(mgp_fft_scratch(c));
+  const int own = c->nbox > 1 ? 3 : c->fft_scr_grids;
+  if (own == 1) RET_IF(mgp_ic_scratch(c, 2));
   float2 *g[6];
-  for (int q = 0; q < 6; q++) g[q] = (float2 *)((q < 3 ? c->frc : c->fft_scr) + (q % 3) * gs);
-  mgp_fft_x x = x_args(c->dk, gs);
-  x.o[0] = g[5];
-  x.o[1] = g[2];
-  x.o[2] = g[0];
-  x.bs_o = 3 * gs / 2;
-  x.kc = kc;
-  RET_IF(p.x(0, MGP_X_IC, x, n));
-  mgp_fft_y y;
-  memset(&y, 0, sizeof(y));
-  y.ntask = 3;
-  y.neg = 1;
-  y.task[0].in = y.task[0].out[0] = g[0];
-  y.task[0].nout = 1;
-  y.task[1].in = g[2];
-  y.task[1].out[0] = g[1];
-  y.task[1].ypow[0] = 1;
-  y.task[1].out[1] = g[2];
-  y.task[1].zpow[1] = 1;
-  y.task[1].nout = 2;
-  y.task[2].in = g[5];
-  y.task[2].out[0] = g[3];
-  y.task[2].ypow[0] = 2;
-  y.task[2].out[1] = g[4];
-  y.task[2].ypow[1] = y.task[2].zpow[1] = 1;
-  y.task[2].out[2] = g[5];
-  y.task[2].zpow[2] = 2;
-  y.task[2].nout = 3;
-  RET_IF(p.y(1, 1, y, 3 * gs, n, kc));
-  mgp_fft_z z;
-  memset(&z, 0, sizeof(z));
-  for (int q = 0; q < 6; q++) z.grad[q] = g[q];
-  z.out = (float2 *)c->rho;
-  z.rows = p.rows(n);
-  z.bs_in = 3 * gs / 2;
-  z.bs_out = gs / 2;
-  z.kc = kc;
-  RET_IF(p.z(MGP_Z_SOURCE, z));
-  RET_IF(p.y(-1, c->rho, gs, n));
+  for (int q = 0; q < 6; q++) {
+    float *more = c->nbox > 1 ? frc(c, 3) : c->fft_scr;
+    g[q] = (float2 *)(q < 3 ? frc(c, q) : q < 3 + own ? more + (q - 3) * gs : c->ic_scratch + (q - 4) * gs);
+  }
+  for (int b = 0; b < c->nbox; b += per) {
+    const int n = c->nbox - b < per ? c->nbox - b : per;
+    mgp_fft_x x = x_args(c->dk + b * gs, gs);
+    x.o[0] = g[5];
+    x.o[1] = g[2];
+    x.o[2] = g[0];
+    x.bs_o = 6 * gs / 2;
+    x.kc = kc;
+    RET_IF(p.x(0, MGP_X_IC, x, n));
+    mgp_fft_y y;
+    memset(&y, 0, sizeof(y));
+    y.ntask = 3;
+    y.neg = 1;
+    y.task[0].in = y.task[0].out[0] = g[0];
+    y.task[0].nout = 1;
+    y.task[1].in = g[2];
+    y.task[1].out[0] = g[1];
+    y.task[1].ypow[0] = 1;
+    y.task[1].out[1] = g[2];
+    y.task[1].zpow[1] = 1;
+    y.task[1].nout = 2;
+    y.task[2].in = g[5];
+    y.task[2].out[0] = g[3];
+    y.task[2].ypow[0] = 2;
+    y.task[2].out[1] = g[4];
+    y.task[2].ypow[1] = y.task[2].zpow[1] = 1;
+    y.task[2].out[2] = g[5];
+    y.task[2].zpow[2] = 2;
+    y.task[2].nout = 3;
+    for (int t = 0; t < 3; t++) {
+      y.task[t].bs_in = 6 * gs / 2;
+      for (int q = 0; q < 3; q++) y.task[t].bs_out[q] = 6 * gs / 2;
+    }
+    RET_IF(p.y(1, 1, y, n, kc));
+    mgp_fft_z z;
+    memset(&z, 0, sizeof(z));
+    for (int q = 0; q < 6; q++) z.grad[q] = g[q];
+    z.out = (float2 *)(c->rho + b * gs);
+    z.rows = p.rows(n);
+    z.bs_in = 6 * gs / 2;
+    z.bs_out = gs / 2;
+    z.kc = kc;
+    RET_IF(p.z(MGP_Z_SOURCE, z));
+  }
+  RET_IF(p.y(-1, c->rho, gs, c->nbox));
   c->rho_planar = 1;
-  return p.x(1, MGP_X_NONE, x_args(c->rho, gs), n);
+  return p.x(1, MGP_X_NONE, x_args(c->rho, gs), c->nbox);
 }
 
 // The particles' D1, D2, s and v from delta(k) in dk and the 2LPT source in rho.
@@ -428,27 +489,28 @@ int mgp_fft_ic_fields(mgp_ctx *c) {
   RET_IF(mgp_launch_ic_take(c->frc, 3 * gs, gs, N, N / Ns, Ns, c->np, c->ic_box, n, 0, 1.0f, c->D1, c->D2, c->s, c->v,
                             c->stream));
   if (N != Ns) {
-    // three lattice grids a box, from the scratch spectra to the force grids
+    // three lattice grids a box, all boxes' spectra and then all grids in the force
+    // grids (at most 3/4 of a mesh grid a box)
     const long long ls = (long long)Ns * Ns * (Ns + 2);
-    RET_IF(mgp_launch_ic_fold(c->rho, gs, N, Ns, c->p.Box, c->fft_scr, ls, n, c->stream));
-    RET_IF(mgp_fft_c2r(c, Ns, c->fft_scr, c->frc, 3 * n, ls));
-    return mgp_launch_ic_take(c->frc, 3 * ls, ls, Ns, 1, Ns, c->np, c->ic_box, n, 1, mult, c->D1, c->D2, c->s, c->v,
+    float *out = c->frc + 3 * n * ls;
+    RET_IF(mgp_launch_ic_fold(c->rho, gs, N, Ns, c->p.Box, c->frc, ls, n, c->stream));
+    RET_IF(mgp_fft_c2r(c, Ns, c->frc, out, 3 * n, ls));
+    return mgp_launch_ic_take(out, 3 * ls, ls, Ns, 1, Ns, c->np, c->ic_box, n, 1, mult, c->D1, c->D2, c->s, c->v,
                               c->stream);
   }
-  // the force pass's x and y passes with g = -Box/2pi / k^2 on the source
+  // the force pass's x, y and z passes with g = -Box/2pi / k^2 on the source
   const passes p(c, N);
-  float2 *f[3] = {(float2 *)c->frc, (float2 *)(c->frc + gs), (float2 *)(c->frc + 2 * gs)};
   mgp_fft_x x = x_args(c->rho, gs);
-  x.o[0] = f[0];
-  x.o[1] = f[2];
+  x.o[0] = (float2 *)F(c, 1);
+  x.o[1] = (float2 *)F(c, 2);
   x.bs_o = 3 * gs / 2;
   x.cfac = (float)(-c->p.Box / (2.0 * M_PI));
   x.neg = 1;
   RET_IF(p.x(0, MGP_X_FORCE, x, n));
-  mgp_fft_y y = force_y_args(f);
+  mgp_fft_y y = force_y_args(c);
   y.neg = 1;
-  RET_IF(p.y(1, 1, y, 3 * gs, n));
-  RET_IF(p.z_c2r(c->frc, c->fft_scr, gs, 3 * n));
-  return mgp_launch_ic_take(c->fft_scr, 3 * gs, gs, N, 1, Ns, c->np, c->ic_box, n, 1, mult, c->D1, c->D2, c->s, c->v,
+  RET_IF(p.y(1, 1, y, n));
+  RET_IF(z_forces(p));
+  return mgp_launch_ic_take(c->frc, 3 * gs, gs, N, 1, Ns, c->np, c->ic_box, n, 1, mult, c->D1, c->D2, c->s, c->v,
                             c->stream);
 }

@@ -27,16 +27,17 @@ typedef struct {
   int neg; /* X_FORCE: wave number -N/2 at the Nyquist index (the IC's convention), else +N/2 */
 } mgp_fft_x;
 
+/* strides between boxes in complex values */
 typedef struct {
   const float2 *in;
   float2 *out[3];
+  long long bs_in, bs_out[3];
   int nout, ypow[3], zpow[3];
 } mgp_fft_ytask;
 
 typedef struct {
   mgp_fft_ytask task[3];
   int ntask, nbox;
-  long long bs;
   const float2 *tw;
   int kc, neg;
 } mgp_fft_y;

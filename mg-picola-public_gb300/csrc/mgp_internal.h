@@ -87,7 +87,8 @@ struct mgp_ctx {
 
   /* grids */
   float *rho, *dk, *frc, *mg1;
-  float *ic_scratch;        /* six grids for the 2LPT IC (lazy, kept for the next IC) */
+  float *ic_scratch;        /* grids for the 2LPT IC (lazy, kept for the next IC) */
+  int ic_grids;             /* how many */
   double *ic_amp;           /* device: per box the amplitude per integer |k|^2 up to the IC's mode cut, then a growth column (lazy) */
   mgp_ic_box *ic_box;       /* device: per box (lazy) */
   void *fft_work;
@@ -99,7 +100,8 @@ struct mgp_ctx {
    * Gaussian smoothing factor per stored index */
   int fft_mode;
   float *fft_tw, *fft_tw_s, *fft_gauss;
-  float *fft_scr;           /* scratch spectra, three a box (lazy) */
+  float *fft_scr;           /* scratch spectra of a single box (lazy) */
+  int fft_scr_grids;        /* how many: 1, or 3 on small meshes */
   int dk_planar, rho_planar; /* dk / rho hold a spectrum in the planar layout of mgp_fft.cuh */
 
   /* P(k) */
@@ -320,8 +322,10 @@ int mgp_fft_supported(const mgp_ctx *c);
 int mgp_fft_setup(mgp_ctx *c);
 void mgp_fft_free(mgp_ctx *c);
 int mgp_fft_scratch(mgp_ctx *c);
+int mgp_ic_scratch(mgp_ctx *c, int grids);
 int mgp_fft_r2c(mgp_ctx *c, const float *in, float *out, int n, long long gs);
 int mgp_fft_c2r(mgp_ctx *c, int N, float *in, float *out, int n, long long gs);
+int mgp_fft_c2r_down(mgp_ctx *c, int N, float *g, float *last, long long gs);
 int mgp_fft_ic_source(mgp_ctx *c, int kc);
 int mgp_fft_ic_fields(mgp_ctx *c);
 int mgp_fft_planar_rows(int N, const float *in, float *out, int x0, int x1, cudaStream_t st);

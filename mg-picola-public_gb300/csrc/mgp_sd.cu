@@ -96,12 +96,12 @@ __global__ void k_sd_table(const double *__restrict__ cols, SdRecipe r, long lon
 // One thread per output mode k' of the Ns half-complex grid; sums the r^3
 // aliases of the full spectrum F_a(k) = i d_a T(|k|^2) . (delta, -S2) for one
 // or two fields (table components xy -> field 0, zw -> field 1;
-// nfields -1: field 1 alone, to out0).  planar, oplanar: the layouts of the stored and the folded spectra (mgp_fft.cuh).
+// nfields -1: field 1 alone, to out0).  last0: the first output's third component.  planar, oplanar: the layouts of the stored and the folded spectra (mgp_fft.cuh).
 __global__ void __launch_bounds__(kThreads) k_sd_fold(const float2 *__restrict__ d1, const float2 *__restrict__ d2,
                                                        const float4 *__restrict__ tab, int N, int Ns, int r,
                                                        int nfields, float2 *__restrict__ out0,
-                                                       float2 *__restrict__ out1, long long ostride, int planar,
-                                                       int oplanar) {
+                                                       float2 *__restrict__ last0, float2 *__restrict__ out1,
+                                                       long long ostride, int planar, int oplanar) {
   const int NH = N / 2 + 1, NHs = Ns / 2 + 1;
   // one warp per folded (kx, ky) row, lanes along kz: no division per mode
   const int lane = threadIdx.x & 31;
@@ -159,8 +159,9 @@ __global__ void __launch_bounds__(kThreads) k_sd_fold(const float2 *__restrict__
     }
     const long long op = (long long)kxp * Ns * NHs;
     const long long w = !oplanar ? o : 2 * kzp == Ns ? op + (long long)Ns * kzp + kyp : op + (long long)kyp * (Ns / 2) + kzp;
-#pragma unroll
-    for (int a = 0; a < 3; a++) out0[a * ostride + w] = G[0][a];
+    out0[w] = G[0][0];
+    out0[ostride + w] = G[0][1];
+    last0[w] = G[0][2];
     if (nfields > 1) {
 #pragma unroll
       for (int a = 0; a < 3; a++) out1[a * ostride + w] = G[1][a];
@@ -443,26 +444,35 @@ static int fields_pass(mgp_ctx *c, double A, double AFF, int n, const int *types
     }
     return MGP_OK;
   }
-  // the Ns^3 inverse transforms: this library's (from planar spectra in
-  // scratch, six at most 3/4 of three mesh grids for Nmesh >= 2 Nsample, or
-  // two calls of three) where the lattice size has them, else cuFFT's in place
-  const bool own = c->fft_mode && mgp_fft_has(Ns) && mgp_fft_supported(c);
-  if (own) RET_IF(mgp_fft_scratch(c));
+  // the Ns^3 inverse transforms: this library's (where the lattice size has them) from
+  // planar spectra, else cuFFT's in place.  Nmesh >= 2 Nsample: the spectra of both fields
+  // fit the scratch grid (3/4 of it); Nmesh = Nsample: a field at a time, in its own
+  // second and third component and the scratch grid.
+  const bool own = c->fft_mode && mgp_fft_has(Ns) && mgp_fft_supported(c) && mgp_fft_scratch(c) == MGP_OK;
   const int per = own && c->g.N == Ns ? 1 : n;  // fields per fold
   for (int f0 = 0; f0 < n; f0 += per) {
     float *o[2] = {c->sd_slot[slot_of(types[f0])], per > 1 ? c->sd_slot[slot_of(types[f0 + 1])] : NULL};
-    if (own) {
+    float *last = o[0] + 2 * c->sd_grid;  // third component of the first field
+    if (own && c->g.N == Ns) {
+      o[0] += c->sd_grid;
+      last = c->fft_scr;
+    } else if (own) {
       o[0] = c->fft_scr;
       o[1] = c->fft_scr + 3 * c->sd_grid;
+      last = o[0] + 2 * c->sd_grid;
     }
     const float4 *tab = (const float4 *)c->sd_tab;
     k_sd_fold<<<mgp_blocks_for((long long)Ns * Ns * 32, 8), kThreads, 0, c->stream>>>(
         (const float2 *)c->sd_dk[0], (const float2 *)c->sd_dk[1], tab, c->g.N, Ns, c->sd_fold, f0 ? -per : per,
-        (float2 *)o[0], (float2 *)o[1], c->sd_grid / 2, c->sd_planar, own);
+        (float2 *)o[0], (float2 *)last, (float2 *)o[1], c->sd_grid / 2, c->sd_planar, own);
     MGP_CHECK_LAUNCH();
     g_kernel_launches++;
     for (int f = 0; f < per; f++) {
       float *base = c->sd_slot[slot_of(types[f0 + f])];
+      if (own && c->g.N == Ns) {
+        RET_IF(mgp_fft_c2r_down(c, Ns, base, c->fft_scr, c->sd_grid));
+        continue;
+      }
       if (own) {
         RET_IF(mgp_fft_c2r(c, Ns, o[f], base, 3, c->sd_grid));
         continue;
