@@ -403,6 +403,10 @@ extern "C" int mgp_destroy(mgp_ctx *c) {
                   c->pk_sum_tot, c->nu_tab_d, c->nu_row_d, c->nu_x_d, c->nu_den_d, c->scr_tab};
   for (size_t i = 0; i < sizeof(bufs) / sizeof(bufs[0]); i++)
     if (bufs[i]) cudaFree(bufs[i]);
+  for (int q = 0; q < 2; q++) {
+    if (c->up_host[q]) cudaFreeHost(c->up_host[q]);
+    if (c->up_ev[q]) cudaEventDestroy(c->up_ev[q]);
+  }
   if (c->nu_row_h) cudaFreeHost(c->nu_row_h);
   for (int q = 0; q < 2; q++)
     if (c->nu_ev[q]) cudaEventDestroy(c->nu_ev[q]);
@@ -567,20 +571,60 @@ extern "C" int mgp_batch_create(const mgp_params *p, int nbox, const mgp_box_par
 }
 
 // ---------------------------------------------------------------- IC
+// A host table to the device on the context's stream without waiting for it: through
+// page-locked slots, since a copy from pageable memory may read it after the call returns (it is
+// staged first only where the device cannot read such memory itself).
+int mgp_upload(mgp_ctx *c, void *dst, const void *src, size_t bytes) {
+  const int q = c->up_slot ^= 1;
+  if (!c->up_ev[q])
+    MGP_CUDA(cudaEventCreateWithFlags(&c->up_ev[q], cudaEventDisableTiming));
+  else
+    MGP_CUDA(cudaEventSynchronize(c->up_ev[q]));  // the copy two uploads ago is done
+  if (c->up_bytes[q] < bytes) {
+    if (c->up_host[q]) cudaFreeHost(c->up_host[q]);
+    c->up_host[q] = NULL;
+    c->up_bytes[q] = 0;
+    MGP_CUDA(cudaMallocHost(&c->up_host[q], bytes));
+    c->up_bytes[q] = bytes;
+  }
+  memcpy(c->up_host[q], src, bytes);
+  MGP_CUDA(cudaMemcpyAsync(dst, c->up_host[q], bytes, cudaMemcpyHostToDevice, c->stream));
+  MGP_CUDA(cudaEventRecord(c->up_ev[q], c->stream));
+  return MGP_OK;
+}
+
+// Host tables of an IC, which its copies read until the stream has come that far.
+struct ic_host {
+  cudaStream_t st;
+  std::vector<mgp_ic_box> box;
+  std::vector<std::vector<double>> tab;
+
+  explicit ic_host(cudaStream_t s) : st(s) {}
+  ~ic_host() { cudaStreamSynchronize(st); }
+  // `t` to the device, kept here
+  int copy(double *dst, std::vector<double> &t) {
+    tab.push_back(std::vector<double>());
+    tab.back().swap(t);
+    MGP_CUDA(cudaMemcpyAsync(dst, tab.back().data(), sizeof(double) * tab.back().size(), cudaMemcpyHostToDevice, st));
+    return MGP_OK;
+  }
+};
+
 // What the IC kernels need of every box (device, c->ic_box), and with `draw` the
 // amplitudes per integer |k|^2 < namp of the Gaussian draw (k in h/Mpc = 2 pi/Box
 // sqrt(RK)) into c->ic_amp, namp a box, with the P(k) rescaling for MG runs whose
 // input spectrum is LCDM (2LPT.c:323-327, 395-407): mg_pofk_ratio(k, 1), per k when
 // the growth is scale dependent.  The analytic spectrum is evaluated on the
 // device; tabulated spectra and CAMB files on the host.
-static int ic_prepare(mgp_ctx *c, int namp, int draw) {
+static int ic_prepare(mgp_ctx *c, ic_host &host, int namp, int draw) {
   const int n = c->nbox;
   const double box = c->p.Box, kf = 2.0 * M_PI / box, ai = 1.0 / (1.0 + c->p.Init_Redshift);
   const mgp_cosmo *c0 = &c->cosmo;
   const int ny = c0->sd ? c0->sd_tab[0].ny : 0;
   if (!c->ic_box) MGP_CUDA(cudaMalloc(&c->ic_box, sizeof(mgp_ic_box) * n));
   if (!c->ic_amp) MGP_CUDA(cudaMalloc(&c->ic_amp, sizeof(double) * ((size_t)namp * n + 2 * ny)));
-  std::vector<mgp_ic_box> hb(n);
+  std::vector<mgp_ic_box> &hb = host.box;
+  hb.resize(n);
   mgp_eh_spectrum eh;
   const int analytic = mgp_cosmo_power_eh(c0, &eh);
   bool per_k = false;
@@ -623,11 +667,9 @@ static int ic_prepare(mgp_ctx *c, int namp, int draw) {
     if (rescale) mgp_cosmo_pofk_ratio_many(cb, 1.0, namp - 1, kk.data() + 1, ratio.data() + 1);
     for (int rk = 1; rk < namp; rk++)
       amp[rk] = pow(box, -1.5) * sqrt(mgp_cosmo_power(cb, kk[rk]) * ratio[rk] * o.fac);
-    // pageable sources: the copies have been staged when the calls return
-    MGP_CUDA(cudaMemcpyAsync(c->ic_amp + (size_t)b * namp, amp.data(), sizeof(double) * namp, cudaMemcpyHostToDevice,
-                             c->stream));
+    RET_IF(host.copy(c->ic_amp + (size_t)b * namp, amp));
   }
-  MGP_CUDA(cudaMemcpyAsync(c->ic_box, hb.data(), sizeof(mgp_ic_box) * n, cudaMemcpyHostToDevice, c->stream));
+  MGP_CUDA(cudaMemcpyAsync(c->ic_box, host.box.data(), sizeof(mgp_ic_box) * n, cudaMemcpyHostToDevice, c->stream));
   if (!draw || !analytic) return MGP_OK;
   if (!per_k)
     return mgp_launch_ic_amp(c->ic_amp, namp, kf, pow(box, -1.5), &eh, c->ic_box, n, NULL, 0, 0.0, 1.0, 1.0, c->stream);
@@ -636,7 +678,7 @@ static int ic_prepare(mgp_ctx *c, int namp, int draw) {
   RET_IF(mgp_cosmo_sd_column(c0, 0, 1.0, col.data(), col.data() + ny));
   const double *y = c0->sd_tab[0].y, dy = (y[ny - 1] - y[0]) / (double)(ny - 1);
   double *dcol = c->ic_amp + namp;
-  MGP_CUDA(cudaMemcpyAsync(dcol, col.data(), sizeof(double) * 2 * ny, cudaMemcpyHostToDevice, c->stream));
+  RET_IF(host.copy(dcol, col));
   return mgp_launch_ic_amp(c->ic_amp, namp, kf, pow(box, -1.5), &eh, c->ic_box, 1, dcol, ny, y[0], dy,
                            mgp_cosmo_growth_lcdm0(c0), c->stream);
 }
@@ -668,7 +710,7 @@ static int ic_cut(const mgp_ctx *c, int *namp) {
 // delta(k) of box 0 in dk from particles in [0,1) of the box, as the linear field at
 // a = 1: their CIC density at a_i (readICfromfile.c:640-676), deconvolved and
 // rescaled (701-777).
-static int ic_density(mgp_ctx *c, const double *pos01, size_t npos, bool own) {
+static int ic_density(mgp_ctx *c, ic_host &host, const double *pos01, size_t npos, bool own) {
   const mgp_params *pb = &c->box_p[0];
   const mgp_cosmo *cb = &c->cosmo;
   const int N = c->g.N, Ns = c->Ns, h = N / 2, rkmax = 3 * h * h;
@@ -693,8 +735,8 @@ static int ic_density(mgp_ctx *c, const double *pos01, size_t npos, bool own) {
   MGP_CUDA(cudaMalloc(&b_gc.p, sizeof(double) * gcw.size()));
   MGP_CUDA(cudaMalloc(&b_resc.p, sizeof(double) * resc.size()));
   MGP_CUDA(cudaMemcpyAsync(b_pos.p, pos01, sizeof(double) * 3 * npos, cudaMemcpyHostToDevice, c->stream));
-  MGP_CUDA(cudaMemcpyAsync(b_gc.p, gcw.data(), sizeof(double) * gcw.size(), cudaMemcpyHostToDevice, c->stream));
-  MGP_CUDA(cudaMemcpyAsync(b_resc.p, resc.data(), sizeof(double) * resc.size(), cudaMemcpyHostToDevice, c->stream));
+  RET_IF(host.copy(b_gc.p, gcw));
+  RET_IF(host.copy(b_resc.p, resc));
   int rc = mgp_launch_fill(c->rho, c->g.nreal, -1.0f, c->stream);
   if (rc == MGP_OK)
     rc = mgp_launch_cic_unit(b_pos.p, (long long)npos, N, c->g.P, (float)pow((double)N / Ns, 3), c->rho, c->stream);
@@ -719,13 +761,13 @@ static int ic_sd(mgp_ctx *c, const float *src, int planar) {
 }
 
 // The IC of every box with the transforms of mgp_fft.cu.
-static int ic_own(mgp_ctx *c, const double *pos01, size_t npos) {
+static int ic_own(mgp_ctx *c, ic_host &host, const double *pos01, size_t npos) {
   const int N = c->g.N, Ns = c->Ns;
   int namp, kc = ic_cut(c, &namp);
   c->dk_planar = 1;
-  RET_IF(ic_prepare(c, namp, pos01 == NULL));
+  RET_IF(ic_prepare(c, host, namp, pos01 == NULL));
   if (pos01) {
-    RET_IF(ic_density(c, pos01, npos, true));
+    RET_IF(ic_density(c, host, pos01, npos, true));
     kc = N > Ns ? Ns / 2 : N / 2;
   } else {
     RET_IF(mgp_launch_ic_delta(c->ic_box, c->nbox, c->ic_amp, namp, N, Ns, kc, c->p.Box, c->dk, c->g.nreal, 1, c->stream));
@@ -740,7 +782,7 @@ static int ic_own(mgp_ctx *c, const double *pos01, size_t npos) {
 // 2LPT initial conditions of box bx with cuFFT's 3D plans (displacement_fields,
 // src/2LPT.c:185-495, 1209-1519): delta(k), the 2LPT fields, the lattice
 // read-out and the particle state.
-static int ic_box(mgp_ctx *c, int bx, const double *pos01, size_t npos) {
+static int ic_box(mgp_ctx *c, ic_host &host, int bx, const double *pos01, size_t npos) {
   const mgp_params *pb = &c->box_p[bx];
   const mgp_cosmo *cb = cosmo_of(c, bx);
   float *dkb = c->dk + (size_t)bx * c->g.nreal;
@@ -761,7 +803,7 @@ static int ic_box(mgp_ctx *c, int bx, const double *pos01, size_t npos) {
   RET_IF(mgp_ic_scratch(c, 6));
   float *g6 = c->ic_scratch;
   if (pos01)
-    RET_IF(ic_density(c, pos01, npos, false));
+    RET_IF(ic_density(c, host, pos01, npos, false));
   else
     RET_IF(mgp_launch_ic_delta(c->ic_box + bx, 1, c->ic_amp + (size_t)bx * namp, namp, N, Ns, kc, box, dkb, gf, 0,
                                c->stream));
@@ -785,6 +827,7 @@ static int ic_box(mgp_ctx *c, int bx, const double *pos01, size_t npos) {
 // src/readICfromfile.c:533-777).  With the transforms of mgp_fft.cu where the
 // lattice points are mesh points and the lattice size has them too.
 static int ic_boxes(mgp_ctx *c, const double *pos01, size_t npos) {
+  ic_host host(c->stream);
   const int N = c->g.N, Ns = c->Ns;
   // the IC writes every particle array in lattice order
   c->permuted = 0;
@@ -792,12 +835,12 @@ static int ic_boxes(mgp_ctx *c, const double *pos01, size_t npos) {
   c->dk_planar = c->rho_planar = 0;
   c->have_density = c->have_forces = 0;
   if (own_fft(c) && (N == Ns || (N % Ns == 0 && mgp_fft_has(Ns)))) {
-    RET_IF(ic_own(c, pos01, npos));
+    RET_IF(ic_own(c, host, pos01, npos));
   } else {
     int namp;
     ic_cut(c, &namp);
-    RET_IF(ic_prepare(c, namp, pos01 == NULL));
-    for (int b = 0; b < c->nbox; b++) RET_IF(ic_box(c, b, pos01, npos));
+    RET_IF(ic_prepare(c, host, namp, pos01 == NULL));
+    for (int b = 0; b < c->nbox; b++) RET_IF(ic_box(c, host, b, pos01, npos));
   }
   c->lpt_ver++;  // new D1/D2
   MGP_CUDA(cudaMemsetAsync(c->dstate, 0, sizeof(mgp_dstate) * c->nbox, c->stream));
@@ -849,8 +892,7 @@ static int require_particles(mgp_ctx *c) {
 // A user's screening_factor_potential (density = 0, argument the Newtonian
 // potential of mg1) or screening_factor_density (density = 1, argument the
 // smoothed density of mg1) applied to rho through a table of the function at
-// this a: MGP_SCREEN_TABLE values at t = asinh(u/u_s) uniform in [t0, t1],
-// copied from pageable memory (the copy has been staged when it returns).
+// this a: MGP_SCREEN_TABLE values at t = asinh(u/u_s) uniform in [t0, t1].
 static int user_screening(mgp_ctx *c, double A, int density, double mult, long long nr) {
   const mgp_model_hooks *h = &c->cosmo.hooks;
   const int nt = MGP_SCREEN_TABLE;
@@ -862,7 +904,7 @@ static int user_screening(mgp_ctx *c, double A, int density, double mult, long l
     const double u = us * sinh(t0 + dt * j);
     tab[j] = (float)(density ? h->screening_factor_density(A, u, h->user) : h->screening_factor_potential(A, u, h->user));
   }
-  MGP_CUDA(cudaMemcpyAsync(c->scr_tab, tab.data(), sizeof(float) * nt, cudaMemcpyHostToDevice, c->stream));
+  RET_IF(mgp_upload(c, c->scr_tab, tab.data(), sizeof(float) * nt));
   return mgp_launch_screen_table(c->rho, c->mg1, nr, (float)mult, c->scr_tab, nt, us, t0, dt, c->stream);
 }
 

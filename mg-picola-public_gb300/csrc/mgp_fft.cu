@@ -55,6 +55,13 @@ static int launched(int rc) {
   return MGP_OK;
 }
 
+// A table to the device, there when the call returns (at context creation).
+static int upload(mgp_ctx *c, float *dst, const void *src, size_t bytes) {
+  MGP_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream));
+  MGP_CUDA(cudaStreamSynchronize(c->stream));
+  return MGP_OK;
+}
+
 // Twiddle tables of size N on the device: W_N^m (m < N), then the row passes'
 // tables (mgp_fft.cuh, fft_row).
 static int make_table(mgp_ctx *c, int N, float **out) {
@@ -73,9 +80,7 @@ static int make_table(mgp_ctx *c, int N, float **out) {
     ns *= o->radix[p];
   }
   MGP_CUDA(cudaMalloc(out, sizeof(float2) * h.size()));
-  // pageable source: the copy has been staged when the call returns
-  MGP_CUDA(cudaMemcpyAsync(*out, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice, c->stream));
-  return MGP_OK;
+  return upload(c, *out, h.data(), sizeof(float2) * h.size());
 }
 
 // Tables of the mesh and, where the lattice transforms apply, of the lattice
@@ -94,7 +99,7 @@ int mgp_fft_setup(mgp_ctx *c) {
       h[i] = (float)exp(-0.5 * x * x);
     }
     MGP_CUDA(cudaMalloc(&c->fft_gauss, sizeof(float) * N));
-    MGP_CUDA(cudaMemcpyAsync(c->fft_gauss, h.data(), sizeof(float) * N, cudaMemcpyHostToDevice, c->stream));
+    RET_IF(upload(c, c->fft_gauss, h.data(), sizeof(float) * N));
   }
   return MGP_OK;
 }

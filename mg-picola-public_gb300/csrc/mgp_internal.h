@@ -123,6 +123,10 @@ struct mgp_ctx {
   float *nu_tab_d;
   int nu_nx;
   cudaEvent_t nu_ev[2];
+  void *up_host[2];        /* page-locked slots of mgp_upload, the events of their last copies */
+  size_t up_bytes[2];
+  cudaEvent_t up_ev[2];
+  int up_slot;
   int nu_slot;
   double nu_cdmfac;
   int pk_blocks;
@@ -323,6 +327,7 @@ int mgp_fft_setup(mgp_ctx *c);
 void mgp_fft_free(mgp_ctx *c);
 int mgp_fft_scratch(mgp_ctx *c);
 int mgp_ic_scratch(mgp_ctx *c, int grids);
+int mgp_upload(mgp_ctx *c, void *dst, const void *src, size_t bytes);
 int mgp_fft_r2c(mgp_ctx *c, const float *in, float *out, int n, long long gs);
 int mgp_fft_c2r(mgp_ctx *c, int N, float *in, float *out, int n, long long gs);
 int mgp_fft_c2r_down(mgp_ctx *c, int N, float *g, float *last, long long gs);

@@ -408,8 +408,7 @@ static int fields_pass(mgp_ctx *c, double A, double AFF, int n, const int *types
       }
     }
   }
-  MGP_CUDA(cudaMemcpyAsync(c->sd_cols, cols.data(), sizeof(double) * 2 * ny * ncol, cudaMemcpyHostToDevice,
-                           c->stream));
+  RET_IF(mgp_upload(c, c->sd_cols, cols.data(), sizeof(double) * 2 * ny * ncol));
   k_sd_table<<<mgp_blocks_for(c->sd_nmax + 1, 8), kThreads, 0, c->stream>>>(c->sd_cols, r, c->sd_nmax,
                                                                             (float4 *)c->sd_tab);
   MGP_CHECK_LAUNCH();
