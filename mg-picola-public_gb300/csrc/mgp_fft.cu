@@ -252,17 +252,19 @@ int mgp_fft_planar_rows(int N, const float *in, float *out, int x0, int x1, cuda
   return MGP_OK;
 }
 
-// Scratch spectra of the field passes and the IC.  A batch takes its density grid, which
-// nothing reads after the fifth force's source spectrum; a single box keeps that grid
-// for its caller and has one of its own, or three where they are small (64 MB, meshes up to 128),
-// which saves two launches a step.
+// Scratch spectra of the field passes and the IC: three a box where they are small (64 MB in
+// all), which saves two launches a step; else a batch takes its density grid, which nothing
+// reads after the fifth force's source spectrum, and a single box, which keeps that grid
+// for its caller, has one of its own.
 int mgp_fft_scratch(mgp_ctx *c) {
-  if (c->nbox > 1 || c->fft_scr) return MGP_OK;
-  const size_t bytes = sizeof(float) * (size_t)c->g.nreal;
+  if (c->fft_scr) return MGP_OK;
+  const size_t bytes = sizeof(float) * (size_t)c->g.nreal * c->nbox;
   const int grids = 3 * bytes <= (64u << 20) ? 3 : 1;
+  if (grids == 1 && c->nbox > 1) return MGP_OK;
   if (cudaMalloc(&c->fft_scr, grids * bytes) != cudaSuccess) {
     cudaGetLastError();
     c->fft_scr = NULL;
+    if (c->nbox > 1) return MGP_OK;
     return mgp_set_error(MGP_ECUDA, "no memory for the transforms' scratch grid");
   }
   c->fft_scr_grids = grids;
@@ -283,7 +285,7 @@ int mgp_fft_scratch(mgp_ctx *c) {
 //   force_y  F1 -> F1, F2 -> F2, F3
 //   force_z  F1, F2, F3 -> the force grids
 static float *frc(const mgp_ctx *c, int q) { return c->frc + (size_t)q * c->g.nreal; }
-static bool apart(const mgp_ctx *c) { return c->nbox == 1 && c->fft_scr_grids == 3; }
+static bool apart(const mgp_ctx *c) { return c->fft_scr_grids == 3; }
 static float *F(const mgp_ctx *c, int q) {
   if (apart(c)) return c->fft_scr + (size_t)(q - 1) * c->g.nreal;
   return q < 3 ? frc(c, q) : (c->nbox == 1 ? c->fft_scr : c->rho);
@@ -292,7 +294,7 @@ static float *F(const mgp_ctx *c, int q) {
 static int z_forces(const passes &p) {
   mgp_ctx *c = p.c;
   const long long gs = c->g.nreal;
-  if (apart(c)) return p.z_c2r(F(c, 1), c->frc, gs, 3);
+  if (apart(c)) return p.z_c2r(F(c, 1), c->frc, gs, 3 * c->nbox);
   return p.z_c2r_down(c->frc, gs, 3 * gs, F(c, 3), gs, c->nbox);
 }
 
@@ -401,7 +403,7 @@ static mgp_fft_y force_y_args(const mgp_ctx *c) {
   a.task[1].bs_in = a.task[1].bs_out[0] = bs;
   a.task[1].ypow[0] = 1;
   a.task[1].out[1] = (float2 *)F(c, 3);
-  a.task[1].bs_out[1] = c->g.nreal / 2;
+  a.task[1].bs_out[1] = apart(c) ? bs : c->g.nreal / 2;
   a.task[1].zpow[1] = 1;
   a.task[1].nout = 2;
   return a;

@@ -100,8 +100,8 @@ struct mgp_ctx {
    * Gaussian smoothing factor per stored index */
   int fft_mode;
   float *fft_tw, *fft_tw_s, *fft_gauss;
-  float *fft_scr;           /* scratch spectra of a single box (lazy) */
-  int fft_scr_grids;        /* how many: 1, or 3 on small meshes */
+  float *fft_scr;           /* scratch spectra (lazy) */
+  int fft_scr_grids;        /* how many a box: 3 where they are small, else 1 of a single box */
   int dk_planar, rho_planar; /* dk / rho hold a spectrum in the planar layout of mgp_fft.cuh */
 
   /* P(k) */
