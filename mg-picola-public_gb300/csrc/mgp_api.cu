@@ -1422,7 +1422,12 @@ extern "C" int mgp_pofk_rsd(mgp_ctx *c, double A, int cap, int *nbins, double *k
   // the grid axes as they are
   const int side = tile_side(c);
   const bool own = own_fft(c);
-  RET_IF(ensure_stage(c));
+  // the shifted displacements: in the third force grid where they fit (Nmesh >= 1.45 Nsample)
+  float *shifted = c->frc + 2 * c->g.nreal;
+  if (3 * c->np > c->g.nreal) {
+    RET_IF(ensure_stage(c, 1));
+    shifted = c->stage;
+  }
   if (side)
     c->tile_ready = 0;  // the sort's arrays describe the shifted positions
   else
@@ -1432,14 +1437,14 @@ extern "C" int mgp_pofk_rsd(mgp_ctx *c, double A, int cap, int *nbins, double *k
   const double norm = pow(p->Box, 3) / pow((double)N, 6), shot = c->pk_sub ? pow(p->Box / (double)c->Ns, 3) : 0.0;
   for (int ax = 0; ax < 2; ax++) {
     RET_IF(mgp_launch_rsd_shift(c->s, c->v, L1, L2, lstride, lpitch, c->dstate, c->np, c->Ns, ax + 1,
-                                (float)(vnorm * p->Box / N), g1, g2, c->permuted ? c->q : NULL, c->stage, c->stream));
+                                (float)(vnorm * p->Box / N), g1, g2, c->permuted ? c->q : NULL, shifted, c->stream));
     if (side) {
-      RET_IF(mgp_tiles_sort(c, side, c->stage));
-      RET_IF(mgp_cic_tiles_own(c, (float)wpar, c->stage, dens));
+      RET_IF(mgp_tiles_sort(c, side, shifted));
+      RET_IF(mgp_cic_tiles_own(c, (float)wpar, shifted, dens));
       c->tile_ready = 0;
     } else {
       RET_IF(mgp_launch_fill(dens, c->g.nreal, -1.0f, c->stream));
-      RET_IF(mgp_launch_cic(c->stage, c->dstate, c->np, c->Ns, N, p->Box, (float)wpar, dens, c->g.P, c->stream));
+      RET_IF(mgp_launch_cic(shifted, c->dstate, c->np, c->Ns, N, p->Box, (float)wpar, dens, c->g.P, c->stream));
     }
     if (own)
       RET_IF(mgp_fft_r2c(c, dens, dkr, 1, c->g.nreal));

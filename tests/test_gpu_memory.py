@@ -46,3 +46,15 @@ def test_single_box_scratch():
         assert (_used() - before) / GRID < base + 1
         ctx.displacement_fields()
         assert (_used() - before) / GRID < base + 3
+
+
+@pytest.mark.parametrize("n,ns,more", [(256, 128, 0.0), (256, 256, 3.0)])
+def test_rsd_multipoles_reuse_the_force_grids(n, ns, more):
+    """The redshift-space displacements (three floats a particle) lie in a force grid where they
+    fit, else in one staging array; bound 0.2 grids for the bins' sums."""
+    p = M.default_params(Nmesh=n, Nsample=ns, Box=256.0, Seed=1, Init_Redshift=9.0, WhichSpectrum=2, pofk_nbins=64)
+    with M.Context(p) as ctx:
+        ctx.displacement_fields()
+        before = _used()
+        ctx.pofk_rsd(0.1)
+        assert (_used() - before) / GRID < more + 0.2
