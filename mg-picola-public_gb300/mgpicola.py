@@ -206,7 +206,11 @@ def _result(shape):
     n = 4 * int(np.prod(shape))
     if n < 1 << 22:
         return np.empty(shape, np.float32)
-    return np.frombuffer(mmap.mmap(-1, n, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS), np.float32).reshape(shape)
+    try:
+        pages = mmap.mmap(-1, n, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+    except (OSError, OverflowError) as e:
+        raise MemoryError("no memory for a result of %d bytes" % n) from e
+    return np.frombuffer(pages, np.float32).reshape(shape)
 
 
 def _check(rc):
