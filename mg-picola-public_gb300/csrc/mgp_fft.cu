@@ -252,14 +252,14 @@ int mgp_fft_planar_rows(int N, const float *in, float *out, int x0, int x1, cuda
   return MGP_OK;
 }
 
-// Scratch spectra of the field passes and the IC: three a box where they are small (64 MB in
-// all), which saves two launches a step; else a batch takes its density grid, which nothing
+// Scratch spectra of the field passes and the IC: three a box where they are small (256 MB in
+// all), so that one launch does the force rows (256^3: 76 us, 88 in three); else a batch takes its density grid, which nothing
 // reads after the fifth force's source spectrum, and a single box, which keeps that grid
 // for its caller, has one of its own.
 int mgp_fft_scratch(mgp_ctx *c) {
   if (c->fft_scr) return MGP_OK;
   const size_t bytes = sizeof(float) * (size_t)c->g.nreal * c->nbox;
-  const int grids = 3 * bytes <= (64u << 20) ? 3 : 1;
+  const int grids = 3 * bytes <= (256u << 20) ? 3 : 1;
   if (grids == 1 && c->nbox > 1) return MGP_OK;
   if (cudaMalloc(&c->fft_scr, grids * bytes) != cudaSuccess) {
     cudaGetLastError();
