@@ -333,7 +333,7 @@ def algorithmic_bytes(N, Np, kernel):
 # writes and the halo pass).  Every term of these kernels scales with the particle count or the
 # cell count, which grow together between the configurations (Nmesh = 2 Nsample), so the
 # figure is scaled by the cell count.
-TRAFFIC_256_512 = {"interp_kick_drift": 4.114e9, "cic": 1.471e9}
+TRAFFIC_256_512 = {"interp_kick_drift": 4.215e9, "cic": 1.479e9}
 
 
 def measured_traffic(cfg, N, Np, kernel):

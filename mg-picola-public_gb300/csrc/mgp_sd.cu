@@ -96,7 +96,8 @@ __global__ void k_sd_table(const double *__restrict__ cols, SdRecipe r, long lon
 // One thread per output mode k' of the Ns half-complex grid; sums the r^3
 // aliases of the full spectrum F_a(k) = i d_a T(|k|^2) . (delta, -S2) for one
 // or two fields (table components xy -> field 0, zw -> field 1;
-// nfields -1: field 1 alone, to out0).  last0: the first output's third component.  planar, oplanar: the layouts of the stored and the folded spectra (mgp_fft.cuh).
+// nfields -1: field 1 alone, to out0).  last0: the first output's third component.
+// planar, oplanar: the layouts of the stored and the folded spectra (mgp_fft.cuh).
 __global__ void __launch_bounds__(kThreads) k_sd_fold(const float2 *__restrict__ d1, const float2 *__restrict__ d2,
                                                        const float4 *__restrict__ tab, int N, int Ns, int r,
                                                        int nfields, float2 *__restrict__ out0,

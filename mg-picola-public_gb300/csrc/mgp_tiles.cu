@@ -25,7 +25,9 @@
 //                   writes every particle's s and v to its slot in the tile
 //                   order (the sort's lattice map then describes the arrays),
 //                   so that the arrays follow the particles and the next
-//                   step's reads stay nearly sequential.
+//                   step's reads stay nearly sequential;
+//   k_ikd_tiles_loop  the same without reading particles ahead, for full or
+//                   cubic tiles.
 // Any order gives the same density and forces (up to the order of
 // floating-point sums); the tile order restores the locality that the
 // Lagrangian order loses as the particles cluster.
