@@ -85,23 +85,14 @@ __host__ __device__ __forceinline__ int lattice_log2(int Ns) {
   return l;
 }
 
-// A thread's FP32 sum; kd_sum also keeps what its additions rounded away (Knuth's
-// TwoSum).
-struct kd_plain {
-  static constexpr bool two = false;
-  float s = 0.f;
-  __device__ __forceinline__ void add(float x) { s += x; }
-  __device__ __forceinline__ float rest() const { return 0.f; }
-};
+// An FP32 sum that keeps what its additions rounded away (Knuth's TwoSum).
 struct kd_sum {
-  static constexpr bool two = true;
   float s = 0.f, r = 0.f;
   __device__ __forceinline__ void add(float x) {
     const float t = s + x, b = t - s;
     r += (s - (t - b)) + (x - b);
     s = t;
   }
-  __device__ __forceinline__ float rest() const { return r; }
 };
 
 // Means over all particles of the interpolated forces and the new velocities
@@ -110,35 +101,43 @@ struct kd_sum {
 // and leaves six numbers in `partials`; the block that arrives last at `done`
 // adds the blocks' in index order and updates the state (done returns to 0 for
 // the next launch).  acc: the forces' three sums, then the velocities'; red: 6 NT
-// floats of shared memory that are free; keep (or NULL): as many sums that the
-// threads have put aside, in the same order.
+// floats of shared memory that are free, or hold (kept) sums that the threads have put aside
+// half-way, in the same order, so that a sum holds as few particles as with twice the
+// threads; keep (or NULL): such sums elsewhere.
 // FP64 runs at 1/64 of the FP32 rate here, so the adds are what counts: six
 // warps sum NT / 32 values a lane and then one tree each, instead of six trees
 // in every warp and a serial sum over warps (2^18 particles: 38 us the kick and
 // 11 us a kernel for the blocks' sums; one kernel of 21 us now).
-template <int NT, class SUM>
-__device__ __forceinline__ void kd_means(const SUM (&acc)[6], float *red, double *partials, int block, int nblocks,
+template <int NT>
+__device__ __forceinline__ void kd_means(float (&acc)[6], float *red, double *partials, int block, int nblocks,
                                          unsigned *done, mgp_dstate *st, const mgp_kd_args &a,
-                                         const float *keep = nullptr) {
+                                         bool kept, const float *keep = nullptr) {
   __shared__ double tot[6];
   __shared__ int last;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  float y = 0.0f;  // what the additions rounded away: FP32 is more than enough for its sum
-  if (SUM::two) {
+  double x = 0.0;
+  if (kept) {
+    // both halves as one FP32 sum and what it rounded away, whose sum takes no FP64
+    float y = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 6; q++) red[q * NT + tid] = acc[q].rest();
+    for (int q = 0; q < 6; q++) {
+      kd_sum h{red[q * NT + tid], 0.0f};
+      h.add(acc[q]);
+      acc[q] = h.s;
+      red[q * NT + tid] = h.r;
+    }
     __syncthreads();
     if (w < 6) {
 #pragma unroll 4
       for (int i = 0; i < NT / 32; i++) y += red[w * NT + 32 * i + lane];
+      x = (double)y;
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int q = 0; q < 6; q++) red[q * NT + tid] = acc[q].s;
+  for (int q = 0; q < 6; q++) red[q * NT + tid] = acc[q];
   __syncthreads();
   if (w < 6) {
-    double x = (double)y;
 #pragma unroll 4
     for (int i = 0; i < NT / 32; i++) x += (double)red[w * NT + 32 * i + lane];
     if (keep)
@@ -156,7 +155,7 @@ __device__ __forceinline__ void kd_means(const SUM (&acc)[6], float *red, double
   if (!last) return;
   if (w < 6) {
     __threadfence();
-    double x = 0.0;
+    x = 0.0;
     for (int b = lane; b < nblocks; b += 32) x += __ldcg(partials + (long long)b * 6 + w);
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
     if (lane == 0) tot[w] = x;

@@ -597,12 +597,23 @@ __global__ void __launch_bounds__(MGP_THREADS, 4) k_interp_kick_drift(
   const float ox = (float)(st->cx[0] * a.scale), oy = (float)(st->cx[1] * a.scale), oz = (float)(st->cx[2] * a.scale);
   const float *F0 = frc, *F1 = frc + gf, *F2 = frc + 2 * gf;
   const IDX Pi = (IDX)P, NPi = (IDX)N * (IDX)P;
-  // sums for the means, with the roundings of each addition in a second number: a
-  // thread takes as many particles as four blocks an SM leave it (108 of 2^24)
-  kd_sum acc[6];
+  // sums for the means, put aside half-way: a thread takes as many particles as four
+  // blocks an SM leave it (108 of 2^24).  (In `red`: shared memory of its own took L1 from the
+  // gathers, 100 -> 112 us at 128^3/256^3.)
+  float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   long long stride = (long long)gridDim.x * blockDim.x;
+  const long long mid = (np / stride + 1) / 2 * stride;
   const float inv_ns = 1.0f / (float)Ns;
+#pragma unroll
+  for (int q = 0; q < 6; q++) red[q * MGP_THREADS + threadIdx.x] = 0.f;
   for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < np; p += stride) {
+    if (p >= mid && p < mid + stride) {
+#pragma unroll
+      for (int q = 0; q < 6; q++) {
+        red[q * MGP_THREADS + threadIdx.x] = acc[q];
+        acc[q] = 0.f;
+      }
+    }
     // lattice point of the particle in slot p: qlat[p] when the arrays are
     // held in cell-tile order, else p itself
     const long long lat = qlat ? (long long)qlat[p] : p;
@@ -651,11 +662,11 @@ __global__ void __launch_bounds__(MGP_THREADS, 4) k_interp_kick_drift(
       float vn = v[o] + a.kick_disp * disp[ax] + a.kick_d1 * d1 + a.kick_d2 * d2;
       v[o] = vn;
       if (a.do_drift) s[o] = sp[ax] + vn * a.dyyy + a.dD1 * d1 + a.dD2 * d2;
-      acc[ax].add(disp[ax]);
-      acc[3 + ax].add(vn);
+      acc[ax] += disp[ax];
+      acc[3 + ax] += vn;
     }
   }
-  kd_means<MGP_THREADS>(acc, red, partials, blockIdx.x, gridDim.x, done, st, a);
+  kd_means<MGP_THREADS>(acc, red, partials, blockIdx.x, gridDim.x, done, st, a, true);
 }
 
 int mgp_ikd_blocks(long long np) { return blocks_for(np, 8); }

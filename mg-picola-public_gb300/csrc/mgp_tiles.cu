@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_ikd_tiles(
     const int c = r / (X * X), rr = r - c * X * X, xx = rr / X, yy = rr - xx * X;
     rowoff[r] = c * gf + ((long long)xx * N + yy) * P - 2 * (yy & 1);
   }
-  kd_plain acc[6];
+  float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   int mid = (int)blockIdx.x + (ntiles / (int)gridDim.x + 1) / 2 * (int)gridDim.x;
 #pragma unroll
   for (int q = 0; q < 6; q++) keep[q * NT + tid] = 0.f;
@@ -723,8 +723,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_ikd_tiles(
       mid = ntiles;
 #pragma unroll
       for (int q = 0; q < 6; q++) {
-        keep[q * NT + tid] = acc[q].s;
-        acc[q].s = 0.f;
+        keep[q * NT + tid] = acc[q];
+        acc[q] = 0.f;
       }
     }
     if (j0 == j1) {
@@ -828,8 +828,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_ikd_tiles(
         const float vn = u[ax] + a.kick_disp * disp[ax] + a.kick_d1 * d1 + a.kick_d2 * d2;
         v2[oj] = vn;
         s2[oj] = a.do_drift ? x[ax] + vn * a.dyyy + a.dD1 * d1 + a.dD2 * d2 : x[ax];
-        acc[ax].add(disp[ax]);
-        acc[3 + ax].add(vn);
+        acc[ax] += disp[ax];
+        acc[3 + ax] += vn;
       }
     };
 #pragma unroll
@@ -845,7 +845,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_ikd_tiles(
   }
   static_assert(6 * NT <= FT::FLOATS, "the sums reuse the force tile");
   __syncthreads();  // the last tile's reads of fs are done
-  kd_means<NT>(acc, fs, partials, blockIdx.x, gridDim.x, done, st, a, keep);
+  kd_means<NT>(acc, fs, partials, blockIdx.x, gridDim.x, done, st, a, false, keep);
 }
 
 // The same without reading ahead: for 8 x 8 x 64 tiles with more particles than the threads of
@@ -868,7 +868,7 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 2 : 0) k_ikd_tiles_loop(
   const float ox = (float)(st->cx[0] * a.scale), oy = (float)(st->cx[1] * a.scale), oz = (float)(st->cx[2] * a.scale);
   const float inv_ns = 1.0f / (float)Ns;
   const int ntiles = ntx * ntx * ntz;
-  kd_plain acc[6];
+  float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int L = blockIdx.x; L < ntiles; L += gridDim.x) {
     const int tile = tile_at(L, ntx, ntz);
     const unsigned j0 = off[tile], j1 = off[tile + 1];
@@ -942,14 +942,14 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 2 : 0) k_ikd_tiles_loop(
         const float vn = v[o + p] + a.kick_disp * disp[ax] + a.kick_d1 * d1 + a.kick_d2 * d2;
         v2[oj] = vn;
         s2[oj] = a.do_drift ? sp[ax] + vn * a.dyyy + a.dD1 * d1 + a.dD2 * d2 : sp[ax];
-        acc[ax].add(disp[ax]);
-        acc[3 + ax].add(vn);
+        acc[ax] += disp[ax];
+        acc[3 + ax] += vn;
       }
     }
   }
   static_assert(6 * NT <= FT::FLOATS, "the sums reuse the force tile");
   __syncthreads();  // the last tile's reads of fs are done
-  kd_means<NT>(acc, fs, partials, blockIdx.x, gridDim.x, done, st, a);
+  kd_means<NT>(acc, fs, partials, blockIdx.x, gridDim.x, done, st, a, false);
 }
 
 template <int T, bool P2, typename PI>

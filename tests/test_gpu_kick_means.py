@@ -11,9 +11,9 @@ mean's error times dt, and the rounding of two FP32 numbers of that size and of
 their FP32 factor: 3 2^-24 c dt, plus the rounding of positions, 2^-24 box.
 
 2^24 particles on 152 SMs: in lattice order, with four blocks of 256 threads an SM, a
-thread has 108 particles, and its sums keep what they round away (b = 18: without that,
-exact up to 64); in tile order, with two blocks and tiles of 512 particles on this
-uniform lattice, it has 216 and puts its sums aside half-way (b = 17: exact up to 128).
+thread has 108 particles and puts its sums aside half-way (b = 18: exact up to 64); in tile
+order, with two blocks and tiles of 512 particles on this uniform lattice, it has 216
+and does the same (b = 17: exact up to 128).
 """
 import numpy as np
 import pytest
